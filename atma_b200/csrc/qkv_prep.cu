@@ -220,19 +220,21 @@ qkv_prep_kernel(const PrepArgs a) {
 
   // ---- stage the tile: every 16-byte piece by one asynchronous copy (whole rows per pass of the CTA) ---
   {
-    const int per_row = nu * pieces;                              // 16-byte pieces per tile row (<= 256)
-    const int rows_per_pass = kPrepThreads / per_row;
-    const int r_off = tid / per_row, j = tid - r_off * per_row;
-    const int ul = j / pieces, pc = j - ul * pieces;
+    const int per_row = nu * pieces;                              // 16-byte pieces per tile row (256 with eight fp32 heads of 128)
+    const int rows_per_pass = max(1, kPrepThreads / per_row);     // rows wider than the CTA take several strides of a pass
+    const int r_off = per_row <= kPrepThreads ? tid / per_row : 0;
     if (r_off < rows_per_pass) {
-      const T* src; int64_t row_st; int which, head;
-      unit_src(u0 + ul, src, row_st, which, head);
-      src += pc * kVec;
-      T* dst = tile + ul * dk + pc * kVec;
-      for (int r = r_off; r < kRows; r += rows_per_pass) {
-        const int t = t0 - (K - 1) + r;
-        const bool ok = t >= 0 && t < a.total;
-        prep_cp_async16(dst + r * row_elems, src + (ok ? (int64_t)t * row_st : 0), ok);
+      for (int j = tid - r_off * per_row; j < per_row; j += kPrepThreads) {
+        const int ul = j / pieces, pc = j - ul * pieces;
+        const T* src; int64_t row_st; int which, head;
+        unit_src(u0 + ul, src, row_st, which, head);
+        src += pc * kVec;
+        T* dst = tile + ul * dk + pc * kVec;
+        for (int r = r_off; r < kRows; r += rows_per_pass) {
+          const int t = t0 - (K - 1) + r;
+          const bool ok = t >= 0 && t < a.total;
+          prep_cp_async16(dst + r * row_elems, src + (ok ? (int64_t)t * row_st : 0), ok);
+        }
       }
     }
   }

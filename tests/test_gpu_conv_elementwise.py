@@ -158,6 +158,12 @@ def test_qkv_prep_prefill_matches_the_op_by_op_oracle(dtype, tol, dk, lens, cont
     _check_prep_against_oracle(dtype, tol, dk, lens, continued)
 
 
+@pytest.mark.parametrize("H,Hkv,dk", [(8, 2, 128), (5, 4, 128), (16, 2, 64), (8, 8, 72)])
+def test_qkv_prep_prefill_fp32_rows_wider_than_a_block(H, Hkv, dk):
+    """Eight fp32 heads of 128 are 256 sixteen-byte pieces, twice the threads of a block."""
+    _check_prep_against_oracle(torch.float32, 1e-4, dk, [2, 37, 1, 64, 29], True, H=H, Hkv=Hkv)
+
+
 @pytest.mark.parametrize("H,Hkv", [(3, 1), (5, 2), (1, 1)])
 def test_qkv_prep_prefill_with_an_odd_number_of_head_rows(H, Hkv):
     """The direct form pairs head rows two to a warp; with H + 2 Hkv odd the last pair is half empty and
