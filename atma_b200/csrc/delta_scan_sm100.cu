@@ -18,12 +18,14 @@
 //   the chunks.  v is on the 128 TMEM lanes of every accumulator; the A operands S^T, R^T, U^T sit in TMEM as two 16-bit
 //   terms, the B operands are the K and Q rows exactly as TMA delivers them and M1, M2 as two terms.  Issue order per
 //   chunk: P = S^T K^T | first half of S^T Q^T | U^T = R^T M1^T | second half of S^T Q^T | dS^T = U^T K | R^T M2^T, so that
-//   the products the next step does not wait for run under the thread phases.
+//   the products the next step does not wait for run under the thread phases.  Few long sequences are cut into segments that
+//   are walked side by side (plan_kernel, delta_compose_kernel).
 //     warp 0 TMA producer (two stages), warp 1 MMA issuer, warps 2-17 state warps (TMEM lanes 32 (warp % 4) .. + 31, column
 //     quarter (warp - 2) / 4); what a thread phase reads from shared memory is fetched while the product before it runs.
 //     TMEM: S hi/lo [0,128) | P, U [128,192) | dS [192,320) | R hi/lo [320,384) | U hi/lo, then R M2 [384,448) | S Q [448,512)
 // Every mbarrier wait is bounded; on expiry a CTA frees its TMEM, returns and leaves a status word for the host.
 #include "delta_rule.cuh"
+#include "mma_sync.cuh"
 #include "sm100.cuh"
 
 namespace atma {
@@ -39,6 +41,23 @@ constexpr int kRecBytes = 4 * kC * kC * 2;          // M1 hi, M2 hi, M1 lo, M2 l
 constexpr int kScal = 256;                          // floats per record: a k_inv [64] | a q_inv [64] | (a_C/a) k_inv [64] | a_C
 constexpr int kThreads = 320;
 
+// One walk of the recurrence over chunks [first, last) of a sequence, for every head and block of 128 value channels.
+// Planes are [head and block][128 k][128 v] fp32 in the scratch; -1 = none.
+enum { kWalk = 0, kOffset = 1, kTransfer = 2 };     // from the true state, with outputs | from zero | from the identity with v = 0
+struct Item {
+  int seq, first, last, kind;
+  int from;                                          // plane of the state before (kWalk; -1 = the state table or zero)
+  int to;                                            // plane of the state after (-1 = the state table where `last` ends the sequence)
+  int middle, at;                                    // plane of the state before chunk `at` (kOffset, kTransfer)
+};
+// A cut (a segment's first chunk that is not its sequence's) e owns planes 6 e ..: the true state before it and in its
+// middle, its offset and transfer to its end, its offset and transfer to its middle.
+enum { kPlaneState = 0, kPlaneMiddle = 1, kPlaneOffset = 2, kPlaneTransfer = 3, kPlaneOffsetMid = 4, kPlaneTransferMid = 5, kPlanes = 6 };
+struct Plan {
+  int n_first, n_second, n_chains, pad;              // items of the two launches, sequences that are cut
+};
+struct Chain { int first_cut, n_cuts; };
+
 struct Params {
   const float *q_inv, *k_inv, *log_decay, *beta;
   const int32_t *cu_rows, *start_pos, *cu_chunks;
@@ -46,6 +65,9 @@ struct Params {
   uint8_t* recs; float* scal;
   float* state; int64_t state_ss;
   void* o;
+  const Plan* plan; const Item* items; const Chain* chains; float* planes;
+  int second;                                        // which launch of the recurrence: 0, or 1 = from the composed states
+  int max_items;
   int n_seqs, NC, H, G, vdim;
 };
 
@@ -64,10 +86,23 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint3
 }
 __device__ __forceinline__ void worker_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
-// ---- chunk offsets of the sequences ------------------------------------------------------------------------------------
-__global__ void chunk_offsets_kernel(const int32_t* __restrict__ cu_rows, const int32_t* __restrict__ start_pos, int n_seqs,
-                                     int32_t* __restrict__ cu_chunks) {
-  if (threadIdx.x == 0) {
+// ---- chunk offsets of the sequences, and how the recurrence walks them ---------------------------------------------------
+// A walk is a serial chain of about 3.2 us a chunk on one SM per head and value block, so few long sequences leave most of the
+// machine idle.  They are then cut into segments that are walked side by side: S' = T S + B over a segment, T from the identity
+// with v = 0, B from zero (first launch, without outputs; a sequence's first segment is walked for real), the true states at the
+// cuts in fp32 (delta_compose_kernel), and the later segments again from them, with outputs, each as two halves (second launch:
+// their middles' T and B are kept on the way).  `room` walks fit the machine at a time.  The segment length is the shortest whose
+// 2 s - 1 walks per sequence of s segments fit; it is taken if one and a half segments and the composition (about ten chunks'
+// time, with the launches) are shorter than the longest sequence.  Measured, 8 heads of 128: one sequence of 32768 rows 1634 us
+// uncut, cut into nine 339 us (197 + 34 for the states + 105, plan 3); sequences of 3001 and 1876 rows 154 -> 87 us.
+constexpr int kComposeChunks = 10;
+
+__device__ __forceinline__ int n_chunks_of(const int32_t* cu_chunks, int s) { return cu_chunks[s + 1] - cu_chunks[s]; }
+
+__global__ void plan_kernel(const int32_t* __restrict__ cu_rows, const int32_t* __restrict__ start_pos, int n_seqs, int room,
+                            int32_t* cu_chunks, Plan* plan, Item* items, int max_items, Chain* chains) {
+  const int lane = threadIdx.x;
+  if (lane == 0) {
     int at = 0;
     cu_chunks[0] = 0;
     for (int s = 0; s < n_seqs; ++s) {
@@ -75,6 +110,60 @@ __global__ void chunk_offsets_kernel(const int32_t* __restrict__ cu_rows, const 
       cu_chunks[s + 1] = at;
     }
   }
+  __syncwarp();
+  int length = 1 << 30;                              // chunks of a segment
+  if (n_seqs + 2 <= room) {
+    int longest = 0;
+    for (int s = 0; s < n_seqs; ++s) longest = max(longest, n_chunks_of(cu_chunks, s));
+    for (int base = 4; base < longest; base += 32) {
+      int walks = 0;
+      for (int s = 0; s < n_seqs; ++s) {
+        const int n = n_chunks_of(cu_chunks, s);
+        if (n > 0) walks += 2 * ((n + base + lane - 1) / (base + lane)) - 1;
+      }
+      const unsigned fits = __ballot_sync(0xffffffffu, walks <= room);
+      if (fits) {
+        const int l = base + __ffs(fits) - 1;
+        if (l + (l + 1) / 2 + kComposeChunks < longest) length = l;
+        break;
+      }
+    }
+  }
+  if (length == 1 << 30) {                           // every sequence in one walk
+    for (int s = lane; s < n_seqs; s += 32) items[s] = Item{s, 0, n_chunks_of(cu_chunks, s), kWalk, -1, -1, -1, 0};
+    if (lane == 0) *plan = Plan{n_seqs, 0, 0, 0};
+    return;
+  }
+  int first = 0, cuts = 0, n_chains = 0;
+  Item* after = items + max_items;
+  for (int s = 0; s < n_seqs; ++s) {
+    const int n = n_chunks_of(cu_chunks, s);
+    if (n == 0) continue;
+    const int parts = (n + length - 1) / length, longer = n % parts, base = n / parts;      // the first `longer` segments are a chunk longer
+    if (lane == 0 && parts > 1) chains[n_chains] = Chain{cuts, parts - 1};
+    for (int j = lane; j < parts; j += 32) {
+      const int a = j * base + min(j, longer), b = a + base + (j < longer ? 1 : 0), mid = (a + b + 1) / 2;
+      if (j == 0) {
+        items[first] = Item{s, a, b, kWalk, -1, parts > 1 ? cuts * kPlanes + kPlaneState : -1, -1, 0};
+        continue;
+      }
+      const int cut = cuts + j - 1, e = cut * kPlanes;
+      Item* two = items + first + 2 * j - 1;
+      if (j + 1 < parts) {                             // the last segment's end is reached by its own walk
+        two[0] = Item{s, a, b, kOffset, -1, e + kPlaneOffset, e + kPlaneOffsetMid, mid};
+        two[1] = Item{s, a, b, kTransfer, -1, e + kPlaneTransfer, e + kPlaneTransferMid, mid};
+      } else {                                         // only its middle is asked for
+        two[0] = Item{s, a, mid, kOffset, -1, e + kPlaneOffsetMid, -1, 0};
+        two[1] = Item{s, a, mid, kTransfer, -1, e + kPlaneTransferMid, -1, 0};
+      }
+      after[2 * cut] = Item{s, a, mid, kWalk, e + kPlaneState, -1, -1, 0};
+      after[2 * cut + 1] = Item{s, mid, b, kWalk, e + kPlaneMiddle, -1, -1, 0};             // may be empty
+    }
+    first += 2 * parts - 1;
+    cuts += parts - 1;
+    n_chains += parts > 1 ? 1 : 0;
+  }
+  if (lane == 0) *plan = Plan{first, 2 * cuts, n_chains, 0};
 }
 
 // ======================================= factors =========================================================================
@@ -412,6 +501,9 @@ struct RecurBarriers {
   uint64_t s_ready, pq_full, r_ready, uo_full, us_ready, s_done;
 };
 
+// kCuts: the walks may be offsets and transfers (the first launch where sequences can be cut); without them the state warps' loop
+// needs fewer registers than the 96 that eighteen warps leave a thread.
+template <bool kCuts>
 __global__ void __launch_bounds__(kRecurThreads, 1)
 delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_m, const Params p) {
@@ -423,18 +515,23 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int vblocks = p.vdim / kD;
-  const int hv = blockIdx.x, h = hv / vblocks, b = blockIdx.y, g = h / (p.H / p.G);
-  const int c0 = p.cu_chunks[b], n_chunks = p.cu_chunks[b + 1] - c0;
-  const int64_t slot = p.slots[b];
-  if (n_chunks <= 0 || slot < 0) return;              // the whole CTA, before anything is allocated
-  const int row_begin = p.cu_rows[b], row_end = p.cu_rows[b + 1];
-  const int64_t rec0 = (int64_t)h * p.NC + c0;
+  const int hv = blockIdx.x, h = hv / vblocks, g = h / (p.H / p.G);
+  if ((int)blockIdx.y >= (p.second ? p.plan->n_second : p.plan->n_first)) return;      // the whole CTA, before anything is allocated
+  const Item entry = p.items[(p.second ? p.max_items : 0) + blockIdx.y];
+  const int b = entry.seq, n_chunks = entry.last - entry.first;
+  if (n_chunks <= 0 || p.slots[b] < 0 || (kCuts && entry.kind == kTransfer && hv % vblocks != 0)) return;
+  const int row_begin = p.cu_rows[b] + entry.first * kC, row_end = p.cu_rows[b + 1];
+  const int64_t rec0 = (int64_t)h * p.NC + p.cu_chunks[b] + entry.first;
+  __shared__ Item s_item;
+  const volatile Item& item = s_item;                 // read where it is needed: the loop's registers are all taken
 
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) { mbar_init(&bar.in_full[i], 1); mbar_init(&bar.m_full[i], 1); mbar_init(&bar.empty[i], 1 + kStateWarps); }
     mbar_init(&bar.s_ready, kStateWarps); mbar_init(&bar.r_ready, kStateWarps); mbar_init(&bar.us_ready, kStateWarps);
     mbar_init(&bar.pq_full, 1); mbar_init(&bar.uo_full, 1); mbar_init(&bar.s_done, 1);
     s_abort = 0;
+    s_item = entry;
+    s_item.at = entry.middle >= 0 ? entry.at - entry.first : -1;
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc(&s_tmem_base, 512);
@@ -471,7 +568,8 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   } else if (warp == 1) {
     // ---- MMA issuer --------------------------------------------------------------------------------------------
     if (lane == 0) {
-      constexpr uint32_t idesc_k = make_idesc(128, 128, 1, 0, 0);      // B rows as they lie: [K; Q] or [M1; M2]
+      // B rows as they lie: [K; Q] or [M1; M2]; without outputs only the first half
+      const uint32_t idesc_k = !kCuts || item.kind == kWalk ? make_idesc(128, 128, 1, 0, 0) : make_idesc(128, 64, 1, 0, 0);
       constexpr uint32_t idesc_ds = make_idesc(128, 128, 1, 0, 1);     // B = K [s][k], MN-major
       const uint64_t hi_k = (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(16 >> 4) << 16);
       const uint64_t hi_mn = (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(16384 >> 4) << 16);
@@ -522,16 +620,31 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const int v = 32 * quad + lane;                    // TMEM lane = value channel of this CTA's block
     const uint32_t lane_base = tbase + (uint32_t(32 * quad) << 16);
     const int vcol = (hv % vblocks) * kD + v;
-    float* plane = p.state + slot * p.state_ss + ((int64_t)h * kD + 32 * qt) * p.vdim + vcol;   // element (k = 32 qt + j, v)
-    const bool fresh = p.start_pos[b] == 0;
+    auto table = [&] { return p.state + p.slots[b] * p.state_ss + ((int64_t)h * kD + 32 * qt) * p.vdim + vcol; };   // element (k = 32 qt + j, v)
+    auto plane_of = [&](int i) {
+      int unit = hv;
+      asm volatile("" : "+r"(unit));                    // no part of the address is kept through the loop
+      return p.planes + ((int64_t)i * gridDim.x + unit) * (kD * kD) + 32 * qt * kD + v;
+    };
     float S[32];
-    {
-      const float* src = plane;
-      int64_t step = p.vdim;
+    if (kCuts && item.kind != kWalk) {
+      const bool identity = item.kind == kTransfer;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) S[j] = identity && 32 * qt + j == v ? 1.f : 0.f;
+    } else {
+      const int from = item.from;
+      const bool fresh = from < 0 && p.start_pos[b] == 0;
+      const float* src = from < 0 ? table() : plane_of(from);
+      int64_t step = from < 0 ? p.vdim : kD;
       asm volatile("" : "+l"(step));                    // not a loop invariant: its multiples would be kept in registers
 #pragma unroll
       for (int j = 0; j < 32; ++j) { S[j] = fresh ? 0.f : *src; src += step; }
     }
+    auto put = [&](float* dst, int64_t step) {
+      asm volatile("" : "+l"(step));
+#pragma unroll
+      for (int j = 0; j < 32; ++j) { *dst = S[j]; dst += step; }
+    };
     float gC = 0.f;                                    // decay over the chunk before
     bool ok = true;
     for (int i = 0; i <= n_chunks; ++i) {
@@ -546,6 +659,7 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         for (int j = 0; j < 32; ++j) S[j] = fmaf(gC, S[j], __uint_as_float(d[j]));
       }
       if (i == n_chunks) break;
+      if (kCuts && i == item.at) put(plane_of(item.middle), kD);
       // ---- S^T as two 16-bit terms (the dS columns have been read: the next products may overwrite them) ----
       {
         uint32_t hi[16], lo[16];
@@ -574,6 +688,10 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
         for (int j = 0; j < 16; ++j) {
           const int t = 16 * qt + j;
           vv[j] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(vb + t * 128 + ((ch ^ (t & 7)) << 4)));
+        }
+        if (kCuts && item.kind == kTransfer) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) vv[j] = 0.f;
         }
 #pragma unroll
         for (int j = 0; j < 16; j += 4) {
@@ -627,7 +745,7 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       {
         gC = reinterpret_cast<const float*>(st + kOffRS)[192];
         const int t0 = row_begin + i * kC + 16 * qt;
-        const int n_ok = min(16, row_end - t0);
+        const int n_ok = !kCuts || item.kind == kWalk ? min(16, row_end - t0) : 0;      // without outputs whatever the columns hold stays here
         uint16_t* oc = static_cast<uint16_t*>(p.o) + ((int64_t)t0 * p.H + h) * p.vdim + vcol;
         int64_t orow = (int64_t)p.H * p.vdim;
         asm volatile("" : "+l"(orow));
@@ -648,16 +766,91 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       }
     }
     if (ok) {
-      int64_t step = p.vdim;
-      asm volatile("" : "+l"(step));
-#pragma unroll
-      for (int j = 0; j < 32; ++j) { *plane = S[j]; plane += step; }
+      if (kCuts && item.to >= 0) put(plane_of(item.to), kD);
+      else if (item.last == n_chunks_of(p.cu_chunks, b)) put(table(), p.vdim);
     }
   }
   tc_fence_before();
   __syncthreads();
   if (tid == 0 && s_abort) atomicExch(&g_delta_status, 1);
   if (warp == 1) tmem_dealloc(tbase, 512);
+}
+
+// ---- the true states at the cuts ------------------------------------------------------------------------------------------
+// S_next = T S + B along a sequence's cuts, and the state in the middle of every segment beside it, in fp32.  A CTA owns eight
+// value channels of a head (columns are independent): 128 threads hold two rows of T x four channels each, the other 128 the
+// middle's.  The matrices do not depend on the states, so their quarters (32 columns; row stride 36: sixteen-byte reads of
+// neighbouring rows hit different banks) stream through six stages of shared memory ahead of the chain.
+constexpr int kComposeCols = 8, kComposeLd = 36, kComposePart = kD * kComposeLd, kComposeStages = 6;
+constexpr int kComposeSmem = 2 * kComposeStages * kComposePart * 4;
+
+__global__ void __launch_bounds__(256, 1) delta_compose_kernel(const Params p) {
+  extern __shared__ __align__(16) float parts[];
+  __shared__ __align__(16) float S[2][kD][kComposeCols];
+  if ((int)blockIdx.y >= p.plan->n_chains) return;
+  const Chain chain = p.chains[blockIdx.y];
+  const int vblocks = p.vdim / kD, HV = p.H * vblocks;
+  const int hv = blockIdx.x / (kD / kComposeCols), v0 = blockIdx.x % (kD / kComposeCols) * kComposeCols;
+  const int tid = threadIdx.x & 127, side = threadIdx.x >> 7, k = tid >> 1, half = tid & 1;      // side 1: the middle's matrix
+  auto plane = [&](int i, int unit) { return p.planes + ((int64_t)(chain.first_cut * kPlanes + i) * HV + unit) * (kD * kD); };
+  float* mine = parts + side * kComposeStages * kComposePart;
+  const int64_t at = (int64_t)k * kD + v0 + 4 * half;                                            // rows k and k + 64
+  const int units = 4 * chain.n_cuts;
+  auto active = [&](int c) { return side == 1 || c + 1 < chain.n_cuts; };                        // the last segment's end is not composed
+  auto request = [&](int u) {
+    if (u < units && active(u >> 2)) {
+      const float* T = plane((u >> 2) * kPlanes + (side ? kPlaneTransferMid : kPlaneTransfer), hv - hv % vblocks) + (u & 3) * 32;
+      float* dst = mine + u % kComposeStages * kComposePart;
+#pragma unroll
+      for (int i = tid; i < kD * 8; i += 128)
+        mma::cp_async16(mma::smem_u32(dst + (i >> 3) * kComposeLd + (i & 7) * 4), T + (i >> 3) * kD + (i & 7) * 4);
+    }
+    mma::cp_async_commit();
+  };
+
+  for (int u = 0; u < kComposeStages - 1; ++u) request(u);
+#pragma unroll
+  for (int r = 0; r < 2; ++r)                          // both sides write the same
+    *reinterpret_cast<float4*>(&S[0][k + 64 * r][4 * half]) = *reinterpret_cast<const float4*>(plane(kPlaneState, hv) + at + 64 * r * kD);
+  float2 acc[2][2];
+  float4 off[2];
+  for (int u = 0; u < units; ++u) {
+    const int c = u >> 2, base = c * kPlanes;
+    mma::cp_async_wait<kComposeStages - 2>();
+    __syncthreads();                                   // the part has landed for everyone, and the stage asked for below is free
+    request(u + kComposeStages - 1);
+    if (!active(c)) continue;
+    if ((u & 3) == 0) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        acc[r][0] = acc[r][1] = make_float2(0.f, 0.f);
+        off[r] = *reinterpret_cast<const float4*>(plane(base + (side ? kPlaneOffsetMid : kPlaneOffset), hv) + at + 64 * r * kD);
+      }
+    }
+    const float* row = mine + u % kComposeStages * kComposePart + k * kComposeLd;
+    const float* s = &S[c & 1][32 * (u & 3)][4 * half];
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+      const float4 t0 = *reinterpret_cast<const float4*>(row + j), t1 = *reinterpret_cast<const float4*>(row + 64 * kComposeLd + j);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float w0 = e == 0 ? t0.x : e == 1 ? t0.y : e == 2 ? t0.z : t0.w, w1 = e == 0 ? t1.x : e == 1 ? t1.y : e == 2 ? t1.z : t1.w;
+        const float4 x = *reinterpret_cast<const float4*>(s + (j + e) * kComposeCols);
+        const float2 lo = make_float2(x.x, x.y), hi = make_float2(x.z, x.w);
+        acc[0][0] = __ffma2_rn(make_float2(w0, w0), lo, acc[0][0]); acc[0][1] = __ffma2_rn(make_float2(w0, w0), hi, acc[0][1]);
+        acc[1][0] = __ffma2_rn(make_float2(w1, w1), lo, acc[1][0]); acc[1][1] = __ffma2_rn(make_float2(w1, w1), hi, acc[1][1]);
+      }
+    }
+    if ((u & 3) == 3) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float4 x = make_float4(acc[r][0].x + off[r].x, acc[r][0].y + off[r].y, acc[r][1].x + off[r].z, acc[r][1].y + off[r].w);
+        *reinterpret_cast<float4*>(plane(side ? base + kPlaneMiddle : base + kPlanes + kPlaneState, hv) + at + 64 * r * kD) = x;
+        if (side == 0) *reinterpret_cast<float4*>(&S[(c & 1) ^ 1][k + 64 * r][4 * half]) = x;
+      }
+    }
+  }
+  mma::cp_async_wait<0>();
 }
 
 // (channel, head, row) view of a (rows, heads, 128) tensor; boxes of 64 channels x 64 rows of one head
@@ -671,6 +864,29 @@ int heads_map(CUtensorMap* out, const void* base, int heads, int64_t rows) {
 int64_t max_chunks(const atma_delta_args& a) { return a.total_rows / kC + a.n_seqs; }
 int64_t align_up(int64_t n) { return (n + 1023) & ~int64_t(1023); }
 
+// Where the scratch's parts lie, from launch-time sizes only.
+struct Layout {
+  int room, max_items;                                // walks that fit the machine at a time; items of either launch
+  bool cuts;                                          // whether a sequence may be cut at all
+  int64_t cu, plan, items, chains, scal, recs, planes, bytes;
+};
+Layout layout_of(const atma_delta_args& a) {
+  Layout l{};
+  const int64_t n = max_chunks(a) * a.H;
+  const int walks = a.H * (a.vdim / kD);
+  l.room = sm_count_of_current_device() / walks;
+  l.cuts = a.n_seqs + 2 <= l.room && (a.total_rows + kC - 1) / kC > 6 + kComposeChunks;
+  l.max_items = l.cuts ? l.room : a.n_seqs;
+  l.plan = align_up(4 * ((int64_t)a.n_seqs + 1));
+  l.items = l.plan + align_up(sizeof(Plan));
+  l.chains = l.items + align_up(2 * (int64_t)l.max_items * sizeof(Item));
+  l.scal = l.chains + align_up((int64_t)a.n_seqs * sizeof(Chain));
+  l.recs = l.scal + n * kScal * 4;
+  l.planes = l.recs + n * kRecBytes;
+  l.bytes = l.planes + (l.cuts ? (int64_t)(l.room / 2) * kPlanes * walks * kD * kD * 4 : 0);
+  return l;
+}
+
 }  // namespace
 
 bool delta_scan_sm100_supported(const atma_delta_args& a) {
@@ -678,10 +894,7 @@ bool delta_scan_sm100_supported(const atma_delta_args& a) {
          max_chunks(a) * a.H * 256 < (int64_t(1) << 31);
 }
 
-int64_t delta_scan_sm100_scratch_bytes(const atma_delta_args& a) {
-  const int64_t n = max_chunks(a) * a.H;
-  return align_up(4 * ((int64_t)a.n_seqs + 1)) + n * kScal * 4 + n * kRecBytes + 1024;
-}
+int64_t delta_scan_sm100_scratch_bytes(const atma_delta_args& a) { return layout_of(a).bytes + 1024; }
 
 int delta_scan_sm100(const atma_delta_args& a, const void* q, const void* k, const void* v, const float* q_inv, const float* k_inv,
                      const float* log_decay, const float* beta, void* o, void* scratch, cudaStream_t st) {
@@ -691,9 +904,15 @@ int delta_scan_sm100(const atma_delta_args& a, const void* q, const void* k, con
   const int64_t NC = max_chunks(a);
   Params p{};
   uint8_t* base = reinterpret_cast<uint8_t*>(align_up((int64_t)reinterpret_cast<uintptr_t>(scratch)));
+  const Layout l = layout_of(a);
   int32_t* cu_chunks = reinterpret_cast<int32_t*>(base);
-  p.scal = reinterpret_cast<float*>(base + align_up(4 * ((int64_t)a.n_seqs + 1)));
-  p.recs = reinterpret_cast<uint8_t*>(p.scal + NC * a.H * kScal);
+  Plan* plan = reinterpret_cast<Plan*>(base + l.plan);
+  Item* items = reinterpret_cast<Item*>(base + l.items);
+  Chain* chains = reinterpret_cast<Chain*>(base + l.chains);
+  p.plan = plan; p.items = items; p.chains = chains; p.max_items = l.max_items;
+  p.planes = reinterpret_cast<float*>(base + l.planes);
+  p.scal = reinterpret_cast<float*>(base + l.scal);
+  p.recs = base + l.recs;
   p.q_inv = q_inv; p.k_inv = k_inv; p.log_decay = log_decay; p.beta = beta;
   p.cu_rows = a.cu_rows; p.start_pos = a.start_pos; p.cu_chunks = cu_chunks; p.slots = a.slots;
   p.state = a.state_table; p.state_ss = a.state_ss; p.o = o;
@@ -710,13 +929,22 @@ int delta_scan_sm100(const atma_delta_args& a, const void* q, const void* k, con
     rc = make_tmap_16bit_4d(&mm, p.recs, 1, dims, strides, box);
   }
   if (rc != ATMA_OK) return rc;
-  chunk_offsets_kernel<<<1, 32, 0, st>>>(a.cu_rows, a.start_pos, a.n_seqs, cu_chunks);
+  plan_kernel<<<1, 32, 0, st>>>(a.cu_rows, a.start_pos, a.n_seqs, l.cuts ? l.room : 0, cu_chunks, plan, items, l.max_items, chains);
   const int64_t tiles = (NC + 1) / 2 * a.H;
   const int sms = sm_count_of_current_device();
   ATMA_CUDA_OK(cudaFuncSetAttribute(delta_factors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
   delta_factors_kernel<<<(unsigned)(tiles < 2 * sms ? tiles : 2 * sms), kThreads, kFactorSmem, st>>>(mq, mk, p);
-  ATMA_CUDA_OK(cudaFuncSetAttribute(delta_recur_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecurSmem));
-  delta_recur_kernel<<<dim3(a.H * (a.vdim / kD), a.n_seqs), kRecurThreads, kRecurSmem, st>>>(mq, mk, mv, mm, p);
+  ATMA_CUDA_OK(cudaFuncSetAttribute(delta_recur_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecurSmem));
+  const int walks = a.H * (a.vdim / kD);
+  const dim3 grid(walks, l.max_items);
+  if (l.cuts) {                                       // whether one is cut is decided on the device: the last two may find nothing to do
+    ATMA_CUDA_OK(cudaFuncSetAttribute(delta_recur_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecurSmem));
+    ATMA_CUDA_OK(cudaFuncSetAttribute(delta_compose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kComposeSmem));
+    delta_recur_kernel<true><<<grid, kRecurThreads, kRecurSmem, st>>>(mq, mk, mv, mm, p);
+    delta_compose_kernel<<<dim3(walks * (kD / kComposeCols), a.n_seqs), 256, kComposeSmem, st>>>(p);
+    p.second = 1;
+  }
+  delta_recur_kernel<false><<<grid, kRecurThreads, kRecurSmem, st>>>(mq, mk, mv, mm, p);
   return launch_status("delta_scan (tcgen05)");
 }
 

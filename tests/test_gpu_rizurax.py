@@ -216,10 +216,11 @@ def test_which_kernel_serves_which_shape():
 DELTA_SHAPES = [(4, 2, 128, 128, 4), (2, 2, 128, 256, 3), (3, 1, 33, 65, 2), (1, 1, 5, 7, 1), (6, 3, 20, 12, 5), (2, 1, 256, 40, 4), (4, 4, 64, 32, 7)]
 
 
-def _delta_case(shape, dtype, T, seed, decay_shift=0.0):
+def _delta_case(shape, dtype, T, seed, decay_shift=0.0, weights_seed=None):
     H, G, K, V, taps = shape
     ch = 2 * G * K + H * V
     z = rand((T, ch + H * V + 2 * H), seed, dtype, 1.5)
+    seed = seed if weights_seed is None else weights_seed
     conv = [rand((n, taps), seed + i, dtype, 0.6) for i, n in enumerate((G * K, G * K, H * V), 1)]
     A_log, dt = rand((H,), seed + 5) * 0.7 - 1, rand((H,), seed + 6) - 2 + decay_shift
     norm = (1 + rand((V,), seed + 7, scale=0.3)).to(dtype)
@@ -314,6 +315,35 @@ def test_delta_with_slow_and_fast_decay(shift):
     out = torch.empty(400, 256, dtype=BF16, device="cuda")
     ops().delta_prefill(z, w, conv, state, group([400], [0], [0], [[0]]), out, eps)
     assert torch.isfinite(out).all() and max_rel(out, want) < 2e-2 and max_rel(state[0], S) < 5e-4
+
+
+@pytest.mark.parametrize("shift", [-6.0, 0.0, 8.0])
+@pytest.mark.parametrize("shape,lens,first", [((4, 2, 128, 128, 4), [2113], [0]), ((2, 2, 128, 256, 3), [1025], [1]),       # 1025: 17 chunks, the shortest cut
+                                              ((2, 1, 128, 128, 4), [1300, 70, 1999], [64, 0, 65]), ((8, 8, 128, 128, 4), [1024, 1600], [0, 3])])
+def test_delta_long_sequences_cut_into_segments(shape, lens, first, shift):
+    """Few long sequences are walked in segments side by side: the same outputs and the same fp32 accuracy of the state as the
+    uncut walk has (the bounds of the tests above), with decays that forget a segment and decays that carry it through."""
+    cases = [_delta_case(shape, BF16, f + n, 40 + i, decay_shift=shift) for i, (n, f) in enumerate(zip(lens, first))]
+    w, n_seqs = cases[0][1], len(lens)
+    wants = [c[2:4] for c in cases]
+    for i in range(1, n_seqs):                                                      # one layer's weights for all of them
+        cases[i] = _delta_case(shape, BF16, first[i] + lens[i], 40 + i, decay_shift=shift, weights_seed=40)
+        wants[i] = cases[i][2:4]
+    conv, state = _delta_tables(w, n_seqs + 1, BF16)
+    slots = [n_seqs - i for i in range(n_seqs)]
+    call = lambda z, *g: ops().delta_prefill(z, w, conv, state, group(*g), torch.empty(z.shape[0], w.heads * w.vdim, dtype=BF16, device="cuda"), 1e-5)
+    for i in range(n_seqs):
+        if first[i]:
+            call(cases[i][0][:first[i]], [first[i]], [0], [slots[i]], [[0]])
+    z = torch.cat([c[0][f:] for c, f in zip(cases, first)])
+    out = call(z, lens, first, slots, [[0]] * n_seqs)
+    at = 0
+    for i in range(n_seqs):
+        o, S = wants[i]
+        assert max_rel(out[at:at + lens[i]], o[first[i]:]) < 2e-2, i
+        assert max_rel(state[slots[i]], S) < (5e-4 if shift else 2e-4), i
+        at += lens[i]
+    assert (state[0] == 33).all() and ops().device_status() == 0
 
 
 # ---- the whole model through the engine ----------------------------------------------------------------------------------------
