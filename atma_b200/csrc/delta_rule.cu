@@ -8,6 +8,7 @@
 // not read.
 #include "common.cuh"
 #include "../../include/atma_decoder.h"
+#include "delta_blocks.cuh"
 #include "delta_rule.cuh"
 
 namespace atma {
@@ -346,7 +347,7 @@ delta_conv_state_kernel(const atma_delta_args a, int ctot) {
     table[(int64_t)((start + i) % a.taps) * ctot + c] = static_cast<const T*>(a.z)[(int64_t)(r0 + i) * a.z_rs + c];
 }
 
-// ---- scan: a warp owns four value columns of one head's state, its lanes the key rows -------------------------------
+// ---- scan without scratch memory, row by row: a warp owns four value columns of one head's state, its lanes the key rows ---
 constexpr int kScanWarps = 8, kScanCols = 4;
 
 template <typename T, int RPL>
@@ -689,7 +690,9 @@ extern "C" int atma_delta_prepare(const atma_delta_args* a, void* q, void* k, vo
 
 extern "C" int atma_delta_scan_path(const atma_delta_args* a) { return a != nullptr && delta_scan_sm100_supported(*a) ? 1 : 0; }
 extern "C" int64_t atma_delta_scan_scratch_bytes(const atma_delta_args* a) {
-  return a != nullptr && delta_scan_sm100_supported(*a) ? delta_scan_sm100_scratch_bytes(*a) : 0;
+  if (a == nullptr) return 0;
+  return delta_scan_sm100_supported(*a) ? delta_scan_sm100_scratch_bytes(*a)
+                                        : delta_blocks_scratch_bytes(a->total_rows, a->n_seqs, a->H, a->dim);
 }
 
 extern "C" int atma_delta_scan(const atma_delta_args* a, const void* q, const void* k, const void* v, const float* q_inv,
@@ -699,6 +702,17 @@ extern "C" int atma_delta_scan(const atma_delta_args* a, const void* q, const vo
   if (a->total_rows <= 0 || a->n_seqs <= 0) return ATMA_OK;
   cudaStream_t st = (cudaStream_t)stream;
   if (delta_scan_sm100_supported(*a)) return delta_scan_sm100(*a, q, k, v, q_inv, k_inv, log_decay, beta, o, scratch, st);
+  if (scratch != nullptr && delta_blocks_supported(a->total_rows, a->n_seqs, a->H, a->dim)) {
+    DeltaBlocks d{};
+    d.q = q; d.k = k; d.v = v; d.o = o;
+    d.q_inv = q_inv; d.k_inv = k_inv; d.q_scale = 1.f;
+    d.log_decay = log_decay; d.beta = beta;
+    d.cu_rows = a->cu_rows; d.start_pos = a->start_pos; d.slots = a->slots;
+    d.state_in = a->state_table; d.state_out = a->state_table; d.state_ss = a->state_ss;
+    d.n_seqs = a->n_seqs; d.total_rows = a->total_rows;
+    d.H = a->H; d.Hq = a->G; d.G = a->G; d.Hv = a->H; d.dk = a->dim; d.dv = a->vdim; d.dtype = a->dtype;
+    return delta_blocks_scan(d, scratch, st);
+  }
   if (a->dtype == ATMA_F32) return scan_t<float>(*a, q, k, v, q_inv, k_inv, log_decay, beta, o, st);
   return scan_t<__nv_bfloat16>(*a, q, k, v, q_inv, k_inv, log_decay, beta, o, st);
 }

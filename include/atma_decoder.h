@@ -131,7 +131,8 @@ typedef struct {
 int atma_delta_prepare(const atma_delta_args* args, void* q, void* k, void* v, float* q_inv, float* k_inv, float* log_decay,
                        float* beta, void* stream);
 /* The recurrence over those rows, state in and out through the slot table; o [rows][H][vdim] (dtype).  scratch:
- * atma_delta_scan_scratch_bytes() bytes (chunk factors of the tensor-core path; 0 for other shapes). */
+ * atma_delta_scan_scratch_bytes() bytes (factors of chunks or blocks of rows).  NULL where the tensor-core kernels do not
+ * serve the shape (atma_delta_scan_path() = 0): row by row, slower. */
 int atma_delta_scan(const atma_delta_args* args, const void* q, const void* k, const void* v, const float* q_inv, const float* k_inv,
                     const float* log_decay, const float* beta, void* o, void* scratch, void* stream);
 int atma_delta_scan_path(const atma_delta_args* args);

@@ -254,3 +254,33 @@ def test_scan_cut_into_segments_equals_the_single_pass(B, T, segments):
     o_ref, S_ref = oracle.chunk_gated_delta_rule_oracle(q, k, v, glog, beta, initial_state=S0)
     assert max_rel(o2, o_ref) < 2e-2 and max_rel(S2, S_ref) < 2e-2
     assert atma_b200.device_status() == 0            # no bounded wait of the tcgen05 scan kernels ran out
+
+
+@pytest.mark.parametrize("B,T,H,Hkv,dk,dv", [(1, 1, 1, 1, 1, 1), (2, 7, 2, 1, 64, 33), (1, 8, 3, 3, 65, 4), (3, 9, 4, 2, 128, 127),
+                                             (8, 31, 8, 2, 128, 128), (5, 70, 8, 4, 20, 128)])
+def test_fp32_blocks_of_rows(B, T, H, Hkv, dk, dv):
+    """Edges of the eight-row blocks, of the padded head sizes and of both widths of the walk; a decay of zero, and an
+    infinite value, which must not reach rows in front of it."""
+    q, k, v, glog, beta, S0 = _scan_inputs(B, T, H, dk, dv, torch.float32, seed=T + dk, gamma_bias=1.0)
+    k, v = k[:, :, :Hkv].contiguous(), v[:, :, :Hkv].contiguous()
+    glog[:, T // 2] = float("-inf")
+    wide = [x.repeat_interleave(H // Hkv, 2) for x in (k, v)]
+
+    def exact(S):
+        """Row by row in 64 bits (a decay of zero has no logarithm to subtract)."""
+        S, out = S.double(), []
+        qn, kn = (x.double() / x.double().norm(dim=-1, keepdim=True) for x in (q, wide[0]))
+        for t in range(T):
+            S = S * glog[:, t, :, None, None].double().exp()
+            u = beta[:, t, :, None].double() * (wide[1][:, t].double() - torch.einsum("bhk,bhkv->bhv", kn[:, t], S))
+            S = S + kn[:, t, :, :, None] * u[:, :, None]
+            out.append(torch.einsum("bhk,bhkv->bhv", qn[:, t], S))
+        return torch.stack(out, 1), S
+
+    o, S = _scan(q, k, v, glog, beta, S0)
+    o_ref, S_ref = exact(S0)
+    # sums of at most 128 products and 70 updates of unit vectors in fp32: a few hundred rounding steps of 6e-8
+    assert max_rel(o, o_ref.float()) < 2e-5 and max_rel(S, S_ref.float()) < 2e-5
+    v[:, T - 1] = float("inf")
+    again, _ = _scan(q, k, v, glog, beta, S0)
+    assert torch.equal(again[:, :T - 1], o[:, :T - 1])
