@@ -116,6 +116,8 @@ _SIGNATURES = {
                                      c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                      c_float, c_int, c_void_p]),
     "atma_add_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]),
+    "atma_linear_f32": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "atma_linear_f32_scratch_bytes": (c_int64, [c_int, c_int, c_int]),
     "atma_decode_linear": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int,
                                    c_void_p]),
     "atma_gated_delta_scan_segmented": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
@@ -187,7 +189,7 @@ _DECODER_SIGNATURES = {
     "atma_delta_scan_scratch_bytes": (c_int64, [POINTER(DeltaArgs)]),
     "atma_delta_step": (c_int, [POINTER(DeltaArgs), c_void_p, c_void_p, c_int64, c_float, c_void_p]),
 }
-_SHARED_SYMBOLS = ("atma_last_error", "atma_decode_linear")
+_SHARED_SYMBOLS = ("atma_last_error", "atma_decode_linear", "atma_linear_f32", "atma_linear_f32_scratch_bytes")
 
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
 DECODER_SYMBOLS = tuple(_DECODER_SIGNATURES)

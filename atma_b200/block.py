@@ -4,8 +4,8 @@ Host-side mirror of the reference's ``Block.forward`` with a Polar attention cor
 gated-delta memory branch (model/reference.py:127-195,230-233; model/blocks.py:463-490;
 model/layers.py:19-31): pre-norm RMSNorm, q/k/v projections, per-head RMSNorm of q and k,
 the three Canon depthwise convs (residual form), Polar attention, the additive memory channel,
-then the squared-ReLU gated MLP.  Projections and norms are library calls (cuBLAS through
-``F.linear``, ``F.rms_norm``); every mixing step goes through the C ABI:
+then the squared-ReLU gated MLP.  Norms are library calls (``F.rms_norm``) and so are projections, but for fp32 rows in
+numbers (``linear_f32``); every mixing step goes through the C ABI:
 
     Canon convs        -> causal_conv1d_fn (packed prefill conv kernel)
     Polar core         -> polar_attention_fwd (un-expanded KV heads, (B,T,H,dk) storage viewed as (B,H,T,dk))
@@ -21,14 +21,14 @@ import torch.nn.functional as F
 
 from .causal_conv1d import causal_conv1d_fn
 from .gated_delta import chunk_gated_delta_rule
-from .inference_ops import squared_relu_gate
+from .inference_ops import linear, squared_relu_gate
 from .polar import polar_attention_fwd
 
 
 def _linear(x, sd, name):
     w = sd[name + ".weight"].to(x.dtype)
     b = sd.get(name + ".bias")
-    return F.linear(x, w, None if b is None else b.to(x.dtype))
+    return linear(x, w, None if b is None else b.to(x.dtype))
 
 
 def _canon(x_btc, weight):

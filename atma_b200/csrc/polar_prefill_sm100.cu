@@ -23,6 +23,7 @@
 // the result is unchanged), which keeps the read-modify-write of O out of most iterations.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a
 // status word for the host.
+#include "linear_f32.cuh"
 #include "polar_prefill.cuh"
 #include "sm100.cuh"
 #include "gated_delta_scan.cuh"
@@ -606,10 +607,11 @@ int sm100_status_fetch_and_clear(int* out) {
 // the device; clears the flag).
 extern "C" int atma_device_status(int* status) {
   ATMA_REQUIRE(status != nullptr, "device_status: null out pointer");
-  int a = 0, b = 0, c = 0;
+  int a = 0, b = 0, c = 0, d = 0;
   int rc = atma::sm100_status_fetch_and_clear(&a);
   if (rc == ATMA_OK) rc = atma::scan_sm100_status_fetch_and_clear(&b);
   if (rc == ATMA_OK) rc = atma::scan_local_status_fetch_and_clear(&c);
-  *status = a | b | c;
+  if (rc == ATMA_OK) rc = atma::linear_f32_status_fetch_and_clear(&d);
+  *status = a | b | c | d;
   return rc;
 }

@@ -274,13 +274,19 @@ def delta_step(z, weights, conv_table, state_table, group, out, eps):
     return out
 
 
+def _product(x, weight):
+    from .inference_ops import linear_f32, linear_f32_supported
+    return linear_f32(x, weight, lib=_lib.load_decoder()) if linear_f32_supported(x, weight) else torch.mm(x, weight.t())
+
+
 def linear(x, weight, out=None):
-    """x @ weight.T in the activation dtype: the weight-streaming kernel for up to 16 16-bit rows, cuBLAS otherwise."""
+    """x @ weight.T in the activation dtype: the weight-streaming kernel for up to 16 16-bit rows, ``linear_f32`` for
+    fp32 rows in numbers, cuBLAS otherwise."""
     from .inference_ops import decode_linear, decode_linear_supported
     if decode_linear_supported(x, weight):
         return decode_linear(x, weight, out=out, lib=_lib.load_decoder())
     if out is None:
-        return torch.mm(x, weight.t())
+        return _product(x, weight)
     return torch.mm(x, weight.t(), out=out)
 
 
@@ -289,7 +295,7 @@ def squared_relu_linear(x, weight, bias=None):
     from .inference_ops import decode_linear, decode_linear_supported
     if decode_linear_supported(x, weight):
         return decode_linear(x, weight, bias=bias, gated="plain_squared_relu", lib=_lib.load_decoder())
-    z = torch.mm(x, weight.t())
+    z = _product(x, weight)
     return bias_squared_relu(z, bias, z)
 
 
@@ -298,7 +304,7 @@ def gelu_gated_linear(x, weight, out):
     from .inference_ops import decode_linear, decode_linear_supported
     if decode_linear_supported(x, weight, gated=True):
         return decode_linear(x, weight, gated="gelu_tanh", out=out, lib=_lib.load_decoder())
-    gu = torch.mm(x, weight.t())
+    gu = _product(x, weight)
     half = weight.shape[0] // 2
     return gelu_gate(gu[:, :half], gu[:, half:], out)
 

@@ -2,6 +2,7 @@
 (kernel/inference_ops_triton.py:124-223)."""
 
 import torch
+import torch.nn.functional as F
 
 from . import _lib
 
@@ -321,6 +322,63 @@ def decode_linear_supported(x, weight, gated=False):
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype and x.ndim == 2 and
             0 < x.shape[0] <= DECODE_LINEAR_MAX_ROWS and x.shape[1] % 32 == 0 and weight.shape[0] % (32 if gated else 16) == 0 and
             weight.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+
+
+LINEAR_F32_MIN_ROWS, LINEAR_F32_MIN_SIZE = 128, 64        # fewer rows, or a narrower product: the library is faster
+
+
+def linear_f32_supported(x, weight):
+    """Whether ``linear_f32`` serves this product: plain fp32 CUDA tensors, enough rows, and nothing around the call that a
+    library product would obey (autograd, transforms, tracing, autocast, a caller's choice of TF32)."""
+    if not (type(x) in _PLAIN and type(weight) in _PLAIN and x.is_cuda and weight.is_cuda and x.dtype == weight.dtype == torch.float32):
+        return False
+    if x.ndim < 2 or weight.ndim != 2 or not weight.is_contiguous() or min(x.shape[-1], weight.shape[0]) < LINEAR_F32_MIN_SIZE:
+        return False
+    if x.numel() < LINEAR_F32_MIN_ROWS * x.shape[-1]:
+        return False
+    if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
+        return False
+    if torch.is_autocast_enabled() or torch.compiler.is_compiling() or torch.jit.is_tracing():
+        return False
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    try:
+        return not torch.backends.cuda.matmul.allow_tf32
+    except RuntimeError:                       # chosen through another of torch's switches
+        return False
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def linear_f32(x, weight, bias=None, out=None, lib=None):
+    """x @ weight.T + bias in fp32 on the tensor cores: x (..., K) fp32, weight (N, K) contiguous.  ``out`` (rows, N):
+    where the result goes (contiguous rows, any row stride); ``lib``: as for ``decode_linear``."""
+    _lib.require_cuda(x, "linear_f32")
+    lib = _lib.load() if lib is None else lib
+    K, N = x.shape[-1], weight.shape[0]
+    if weight.shape[1] != K or x.dtype != torch.float32 or weight.dtype != torch.float32 or not weight.is_contiguous():
+        raise ValueError("weight must be a contiguous fp32 (N, K) tensor and x fp32")
+    rows = x.reshape(-1, K)
+    if rows.stride(1) != 1:
+        rows = rows.contiguous()
+    if bias is not None:
+        bias = bias.float().contiguous()
+    M = rows.shape[0]
+    y = torch.empty((M, N), device=x.device, dtype=torch.float32) if out is None else out
+    if y.shape != (M, N) or y.dtype != torch.float32 or y.stride(1) != 1:
+        raise ValueError("out must have the result's shape and dtype and contiguous rows")
+    scratch = torch.empty(int(lib.atma_linear_f32_scratch_bytes(M, N, K)), device=x.device, dtype=torch.uint8)
+    _lib.check(lib.atma_linear_f32(_lib.ptr(rows), rows.stride(0), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), y.stride(0),
+                                   M, N, K, _lib.ptr(scratch), _lib.stream_ptr()), lib)
+    return y.view(*x.shape[:-1], N) if out is None else y
+
+
+def linear(x, weight, bias=None):
+    """x @ weight.T + bias: fp32 rows in numbers through ``linear_f32``, the library's product otherwise."""
+    if linear_f32_supported(x, weight) and (bias is None or bias.dtype == torch.float32):
+        return linear_f32(x, weight, bias)
+    return F.linear(x, weight, bias)
 
 
 _GATES = {False: 0, None: 0, True: 1, "squared_relu": 1, "gelu_tanh": 2, "plain_squared_relu": 3}

@@ -4,7 +4,7 @@ Host-side mirror of the packed ("grouped") prefill branch of the reference's
 ``AtmaGlobalAttention.forward`` (inference/models/atma.py:389-399,429-441,466-510) together with
 the per-token maps its model runner builds (inference/engine/model_runner.py:395-404):
 
-    q|gate, k, v projections      cuBLAS (F.linear)
+    q|gate, k, v projections      cuBLAS, linear_f32 for fp32
     RMSNorm + Canon convs + cache  qkv_prep_prefill            one launch, conv-state rows and K/V pages written
     Polar attention                polar_attention_packed_fwd  un-expanded KV heads, one launch for all sequences
     memory branch                  packed_gated_delta_prefill  one call for all sequences, state rows in place,
@@ -20,7 +20,7 @@ import torch
 import torch.nn.functional as F
 
 from .gated_delta import packed_gated_delta_prefill
-from .inference_ops import qkv_prep_prefill, rms_sigmoid_gate, sigmoid_gate_mul
+from .inference_ops import linear, qkv_prep_prefill, rms_sigmoid_gate, sigmoid_gate_mul
 from .mixing import _side_stream
 from .polar import polar_attention_fwd, polar_attention_packed_fwd
 
@@ -52,7 +52,7 @@ class PackedMaps:
 
 def _linear(x, sd, name):
     b = sd.get(name + ".bias")
-    return F.linear(x, sd[name + ".weight"].to(x.dtype), None if b is None else b.to(x.dtype))
+    return linear(x, sd[name + ".weight"].to(x.dtype), None if b is None else b.to(x.dtype))
 
 
 @torch.no_grad()

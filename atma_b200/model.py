@@ -7,7 +7,7 @@ fourth one (i % 4 == 2) a global Polar + gated-delta layer, the others LFM2 gate
 each followed by the squared-ReLU gated MLP; final RMSNorm, LM head, logit soft-cap.  It takes
 the reference's ``state_dict`` as is (inference/utils/loader.py:5-39).
 
-Projections are cuBLAS (``F.linear``); everything between them is this library:
+Projections are cuBLAS (``linear_f32`` for fp32 prompts); everything between them is this library:
 
     prefill (packed fresh prompts)          decode (one token per sequence, CUDA-graph safe)
     add_rms_norm                            add_rms_norm
@@ -35,7 +35,7 @@ import hashlib
 from .gated_delta import gated_delta_decode_step, gated_delta_decode_step_fused, packed_gated_delta_prefill
 from .inference_ops import qkv_prep_prefill, sigmoid_gate_mul
 from .polar import polar_attention_fwd
-from .inference_ops import (add_rms_norm, decode_linear, decode_linear_supported, lfm2_conv_decode_step, lfm2_conv_packed,
+from .inference_ops import (add_rms_norm, decode_linear, decode_linear_supported, lfm2_conv_decode_step, lfm2_conv_packed, linear,
                             qkv_prep_decode, rms_sigmoid_gate, softcap_logits, squared_relu_gate)
 from .layer import PackedMaps, global_attention_prefill_packed
 from .polar import DECODE_BESIDE_MAX_ROWS, polar_attention_decode
@@ -138,14 +138,14 @@ class AtmaModel:
         """Decode batches of up to 16 rows stream the weights through this library's kernel; larger ones are cuBLAS."""
         if self.small_batch_linear and decode_linear_supported(x, w):
             return decode_linear(x, w, b)
-        return F.linear(x, w, b)
+        return linear(x, w, b)
 
     def _mlp(self, h, i):
         w, b = self.sd[f"blocks.{i}.mlp.fc.weight"], self.sd.get(f"blocks.{i}.mlp.fc.bias")
         if self.small_batch_linear and decode_linear_supported(h, w, gated=True):
             act = decode_linear(h, w, b, gated=True)            # fc GEMM and the squared-ReLU gate in one launch
         else:
-            fc = F.linear(h, w, b)
+            fc = linear(h, w, b)
             half = fc.shape[-1] // 2
             act = squared_relu_gate(fc[:, :half], fc[:, half:])
         return self._lin(act, f"blocks.{i}.mlp.proj")

@@ -230,6 +230,12 @@ int atma_qkv_prep_decode(const void* q_gate, int64_t qg_row, int64_t qg_head, co
 int atma_add_rms_norm(const void* x, const void* y, const void* weight, void* x_out, void* h_out, int rows, int D,
                       float eps, int dtype, void* stream);
 
+/* fp32 linear layer on the tensor cores at fp32 accuracy: out[m][n] = sum_k x[m][k] * w[n][k] + bias[n] (bias may be
+ * NULL); x rows and out rows with strides in elements, w [N][K] dense.  scratch: atma_linear_f32_scratch_bytes() bytes. */
+int atma_linear_f32(const float* x, int64_t x_row_stride, const float* w, const float* bias, float* out, int64_t out_row_stride,
+                    int M, int N, int K, void* scratch, void* stream);
+int64_t atma_linear_f32_scratch_bytes(int M, int N, int K);
+
 /* Weight-streaming linear layer for decode batches of up to 16 rows (16-bit types): out[b][n] =
  * sum_k x[b][k] * weight[n][k] + bias[n] (bias may be NULL), weight [N][K] dense in torch's Linear
  * layout, fp32 accumulation, one rounding to `dtype`.  gated = 1: the N outputs are the two halves

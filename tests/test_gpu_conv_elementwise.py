@@ -366,3 +366,27 @@ def test_decode_linear_rejects_what_it_does_not_serve():
         atma_b200.decode_linear(x[:4, :48].contiguous(), w[:, :48].contiguous())   # K not a multiple of 32
     assert atma_b200.decode_linear(x[:0], w).shape == (0, 32)
     assert atma_b200.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (128, 64, 64), (129, 65, 63), (127, 4100, 257), (300, 1027, 130), (2000, 128, 2049)])
+@pytest.mark.parametrize("spread", [0.0, 4.0])
+def test_linear_f32(M, K, N, spread):
+    """Edges of tiles and planes, strided and unaligned rows, values of very different size in one row.  A product's terms
+    are right to 2^-22 and 2^-51 of their row's largest value, and fp32 sums add a few units of 2^-24."""
+    from atma_b200.inference_ops import linear_f32
+    g = torch.Generator().manual_seed(M + K)
+    wide = lambda *s: torch.randn(*s, generator=g) * torch.exp(torch.randn(*s, generator=g) * spread)      # noqa: E731
+    x, w, b = wide(M, K + 3).cuda()[:, 1:K + 1], wide(N, K).cuda(), torch.randn(N, generator=g).cuda()
+    out = torch.full((M, N + 5), 7.0, device="cuda")
+    y = linear_f32(x, w, b, out=out[:, 2:N + 2])
+    xd, wd = x.double(), w.double()
+    bound = xd.abs() @ wd.abs().t() * 2 ** -20 + b.abs() * 2 ** -23
+    bound = bound + 2 ** -50 * (xd.abs().amax(1, True) * wd.abs().sum(1) + xd.abs().sum(1, True) * wd.abs().amax(1))
+    assert ((y - (xd @ wd.t() + b)).abs() <= bound).all()
+    assert (out[:, :2] == 7).all() and (out[:, N + 2:] == 7).all()
+    assert torch.equal(linear_f32(x.contiguous(), w, b), y)
+    x, w = x.clone(), w.clone()
+    x[M // 2, 0], w[N // 2, K // 2] = float("inf"), float("nan")
+    odd, want = linear_f32(x, w), (x.double() @ w.double().t())
+    assert torch.equal(odd.isnan(), want.isnan()) and torch.equal(odd.isinf(), want.isinf())
+    assert atma_b200.device_status() == 0
