@@ -17,6 +17,7 @@
 // against row by row, 2048 rows 1117 -> 216 us against chunks of 64 in fp32; errors against 64 bits unchanged (4.8e-6 of a
 // whole model, 8.5e-7 of a block).
 #include "delta_blocks.cuh"
+#include "f32x2.cuh"
 
 namespace atma {
 
@@ -36,27 +37,6 @@ __device__ __forceinline__ Rows rows_of(const DeltaBlocks& a, int s) {
   if (a.cu_rows == nullptr) return {(int64_t)s * a.len, a.len};
   const int r0 = a.cu_rows[s];
   return {r0, a.cu_rows[s + 1] - r0};
-}
-
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t pair(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float2 halves(uint64_t p) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p));
-  return f;
 }
 
 template <typename T, int DK>
@@ -207,8 +187,8 @@ delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, in
       x[0][e] = ok && c0 ? p[0] : 0.f;
       x[1][e] = ok && c1 ? p[1] : 0.f;
     }
-    S[0][m] = pair(x[0][0], x[0][1]);
-    S[1][m] = pair(x[1][0], x[1][1]);
+    S[0][m] = pack2(x[0][0], x[0][1]);
+    S[1][m] = pack2(x[1][0], x[1][1]);
   }
 
   const float* rec = recs + ((int64_t)h * n_records + first_record(seq.r0, s)) * kRec;
@@ -255,7 +235,7 @@ delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, in
         t0 = fma2(x.y, S[0][2 * m + 1], t0);
         t1 = fma2(x.y, S[1][2 * m + 1], t1);
       }
-      const float2 f0 = halves(t0), f1 = halves(t1);
+      const float2 f0 = unpack2(t0), f1 = unpack2(t1);
       d[0][i] = f0.x + f0.y;
       d[1][i] = f1.x + f1.y;
     }
@@ -279,12 +259,12 @@ delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, in
       r0[j] = __shfl_sync(0xffffffffu, rhs0, j, 16);
       r1[j] = __shfl_sync(0xffffffffu, rhs1, j, 16);
     }
-    const uint64_t fade = pair(e_all, e_all);
+    const uint64_t fade = pack2(e_all, e_all);
 #pragma unroll
     for (int m = 0; m < 2 * R4; ++m) { S[0][m] = mul2(S[0][m], fade); S[1][m] = mul2(S[1][m], fade); }
 #pragma unroll
     for (int j = 0; j < kN; ++j) {
-      const uint64_t p0 = pair(r0[j], r0[j]), p1 = pair(r1[j], r1[j]);
+      const uint64_t p0 = pack2(r0[j], r0[j]), p1 = pack2(r1[j], r1[j]);
 #pragma unroll
       for (int m = 0; m < R4; ++m) {
         const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(now + (2 * kN + j) * DK + 64 * m + 4 * l);
@@ -314,7 +294,7 @@ delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, in
   if (a.state_out == nullptr) return;
 #pragma unroll
   for (int m = 0; m < 2 * R4; ++m) {
-    const float2 f0 = halves(S[0][m]), f1 = halves(S[1][m]);
+    const float2 f0 = unpack2(S[0][m]), f1 = unpack2(S[1][m]);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int row = 64 * (m >> 1) + 4 * l + 2 * (m & 1) + e;

@@ -1,5 +1,5 @@
 // atma_polar_prefill: argument validation and the choice between the tensor-core tile kernel
-// (16-bit inputs, head_dim 128) and the fp32 CUDA-core kernel (everything else).
+// (16-bit inputs, head_dim 128) and the two fp32 CUDA-core kernels (everything else).
 #include "polar_prefill.cuh"
 
 using namespace atma;
@@ -41,5 +41,6 @@ extern "C" int atma_polar_prefill(const atma_polar_prefill_args* args, void* str
   if (rc != ATMA_OK) return rc;
   if (a.B == 0 || a.Tq == 0) return ATMA_OK;
   if (polar_prefill_sm100_supported(a)) return polar_prefill_sm100(a, (cudaStream_t)stream);
+  if (polar_rows_f32_supported(a)) return polar_rows_f32(a, (cudaStream_t)stream);
   return polar_prefill_simt(a, (cudaStream_t)stream);
 }

@@ -1,0 +1,205 @@
+// Polar Attention prefill of fp32 tensors with a head size of 64 or 128, fp32 arithmetic, 64 rows x 64 keys per step: the
+// same results as polar_prefill_simt_kernel, which keeps the other types and sizes.
+//
+// There a lane owns one key and a warp four rows, with a shuffle for every weight; here a thread owns 4 x 4 scores and
+// 4 rows x DK / 16 channels (rows_f32.cuh).  K and V take turns in one buffer, V under the statistics, and two CTAs share an
+// SM; later rows have more keys, so those of all heads come first.  Measured, 2048 rows, 8 heads of 128: 1049 -> 423 us (527
+// with the heads one after another and the scores one channel at a time).
+#include "polar_prefill.cuh"
+#include "rows_f32.cuh"
+
+namespace atma {
+
+namespace {
+
+using namespace rows_f32;
+constexpr float kNegBig = -1e38f;
+
+template <int DK>
+__global__ void __launch_bounds__(kThreads, 2)
+polar_rows_f32_kernel(const atma_polar_prefill_args a) {
+  constexpr int VM = DK / 64, ld = DK + kPad;
+  extern __shared__ __align__(16) float sm[];
+  float* sQ = sm;                              // [64][ld]
+  float* sKV = sQ + kM * ld;                   // K [64][ld], then V [64][DK]
+  float* sP = sKV + kN * ld;                   // [64][kLdP]
+  __shared__ float s_lo[kThreads / 32], s_hi[kThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
+  const int h = blockIdx.x % a.H, b = blockIdx.y, kvh = h / (a.H / a.Hkv);
+
+  // ---- which query rows of which sequence ----
+  const bool packed = a.n_tiles > 0;
+  const int block = ((int)(gridDim.x - blockIdx.x) - 1) / a.H;
+  int q0 = block * kM, seq0 = 0, q_limit = a.Tq, k_limit = a.Tk;
+  if (packed) {
+    const int t = block / (128 / kM);
+    seq0 = a.tile_seq_start[t];
+    q0 = a.tile_q_start[t] + block % (128 / kM) * kM;
+    q_limit = k_limit = a.tile_seq_len[t];
+  }
+  if (q0 >= q_limit) return;
+  const float* Q = static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh + (int64_t)seq0 * a.q_st;
+  const float* K = static_cast<const float*>(a.k) + b * a.k_sb + kvh * a.k_sh + (int64_t)seq0 * a.k_st;
+  const float* V = static_cast<const float*>(a.v) + b * a.v_sb + kvh * a.v_sh + (int64_t)seq0 * a.v_st;
+  for (int i = tid; i < kM * (DK / 4); i += kThreads) {
+    const int r = i / (DK / 4), c = 4 * (i - r * (DK / 4));
+    const bool there = q0 + r < q_limit;
+    copy16(sQ + r * ld + c, there ? Q + (int64_t)(q0 + r) * a.q_st + c : Q, there);
+  }
+
+  float n[4], temp[4], m[4], L[4], Q2[4];
+  uint64_t acc[4][2 * VM];
+  float lo = 3.0e38f, hi = -1.0f;              // key counts of this warp's rows
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = q0 + 4 * ty + i;
+    const bool ok = r < q_limit;
+    n[i] = !ok ? 0.f : (packed ? (float)(r + 1) : (a.n_keys ? a.n_keys[r] : a.n_base + (float)(r + 1)));
+    const float nc = fmaxf(a.window > 0 ? fminf(n[i], (float)a.window) : n[i], 1.0f);
+    temp[i] = 1.0f + a.spg[h] * logf(nc);
+    if (ok) { lo = fminf(lo, n[i]); hi = fmaxf(hi, n[i]); }
+    m[i] = kNegBig; L[i] = 0.f; Q2[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 2 * VM; ++c) acc[i][c] = 0;
+    if (a.stats_in_m != nullptr && ok) {
+      const int64_t row = ((int64_t)b * a.H + h) * a.Tq + r;
+      m[i] = a.stats_in_m[row]; L[i] = a.stats_in_l[row]; Q2[i] = a.stats_in_q2[row];
+#pragma unroll
+      for (int c = 0; c < VM; ++c) {
+        const float* p = a.stats_in_s + row * DK + 64 * c + 4 * tx;
+        acc[i][2 * c] = pack2(p[0], p[1]);
+        acc[i][2 * c + 1] = pack2(p[2], p[3]);
+      }
+    }
+  }
+  const float inv_sqrt_dk = rsqrtf((float)DK);
+  lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, 16));
+  hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, 16));
+  if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
+  __syncthreads();
+  float all_lo = lo, all_hi = hi;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) { all_lo = fminf(all_lo, s_lo[w]); all_hi = fmaxf(all_hi, s_hi[w]); }
+
+  // ---- key tiles that some row sees ----
+  const float koff = (float)a.key_offset;
+  const int j_end = max((int)fminf((float)k_limit, ceilf(all_hi - koff)), 0);
+  int j_begin = 0;
+  if (a.window > 0) {
+    const float first = all_lo - (float)a.window - koff;
+    if (first > 0.f) j_begin = (int)fminf(first, (float)k_limit) / kN * kN;
+  }
+  for (int k0 = j_begin; k0 < j_end; k0 += kN) {
+    auto fetch = [&](const float* src, int64_t stride, int dst_ld) {
+      for (int i = tid; i < kN * (DK / 4); i += kThreads) {
+        const int j = i / (DK / 4), c = 4 * (i - j * (DK / 4));
+        const bool there = k0 + j < k_limit;
+        copy16(sKV + j * dst_ld + c, there ? src + (int64_t)(k0 + j) * stride + c : src, there);
+      }
+    };
+    __syncthreads();                           // the last tile's V is read
+    fetch(K, a.k_st, ld);
+    copies_done();
+    float sc[4][4];
+    dots<true>(sQ, sKV, ld, DK / 4, ty, tx, sc);
+    __syncthreads();
+    fetch(V, a.v_st, DK);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float f = temp[i] * inv_sqrt_dk;
+      float top = kNegBig;
+      bool valid[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = k0 + tx + 16 * j;
+        const float pos = (float)key + koff;
+        valid[j] = key < k_limit && pos < n[i] && (a.window <= 0 || pos >= n[i] - (float)a.window);
+        sc[i][j] = valid[j] ? sc[i][j] * f : kNegBig;
+        top = fmaxf(top, sc[i][j]);
+      }
+      const float mn = fmaxf(m[i], row_max(top));
+      const float al = expf(m[i] - mn);
+      float sum = 0.f, sq = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float p = valid[j] ? expf(sc[i][j] - mn) : 0.f;
+        sP[(4 * ty + i) * kLdP + tx + 16 * j] = p;
+        sum += p;
+        sq = fmaf(p, p, sq);
+      }
+      L[i] = L[i] * al + row_sum(sum);
+      Q2[i] = Q2[i] * al * al + row_sum(sq);
+      m[i] = mn;
+      times<VM>(acc[i], al);
+    }
+    // keys that some row of this warp sees: nothing beyond them enters its sums
+    const int j1 = min(min(kN, k_limit - k0), (int)fminf(fmaxf(ceilf(hi - koff) - (float)k0, 0.f), (float)kN));
+    const int j0 = a.window > 0 ? (int)fminf(fmaxf(lo - (float)a.window - koff - (float)k0, 0.f), (float)kN) & ~3 : 0;
+    copies_done();
+    weigh<VM>(sP, sKV, ty, tx, j0, j1, acc);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+
+  // ---- result ----
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = q0 + 4 * ty + i;
+    const bool ok = r < q_limit;
+    const int64_t row = ((int64_t)b * a.H + h) * a.Tq + r;
+    if (!a.finalize) {
+      if (ok) {
+        if (tx == 0) { a.stats_out_m[row] = m[i]; a.stats_out_l[row] = L[i]; a.stats_out_q2[row] = Q2[i]; }
+#pragma unroll
+        for (int c = 0; c < 4 * VM; ++c) a.stats_out_s[row * DK + 64 * (c >> 2) + 4 * tx + (c & 3)] = at<VM>(acc[i], c);
+      }
+      continue;
+    }
+    const float nc = fmaxf(a.window > 0 ? fminf(n[i], (float)a.window) : n[i], 1.0f);
+    const float a_n = temp[i] * (a.null_base[h] + a.sps[h] * sqrtf(logf(nc + 1.0f)));
+    const float mn = fmaxf(m[i], a_n);
+    const float al = expf(m[i] - mn);
+    const float Lf = L[i] * al, Q2f = Q2[i] * al * al;
+    const float p_n = expf(a_n - mn);
+    const float Z = Lf + p_n;
+    float sv[4 * VM], sq = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4 * VM; ++c) {
+      sv[c] = at<VM>(acc[i], c) * al + p_n * a.v_null[h * DK + 64 * (c >> 2) + 4 * tx + (c & 3)];
+      sq = fmaf(sv[c], sv[c], sq);
+    }
+    const float inv = 1.0f / fmaxf(sqrtf(row_sum(sq)), a.eps);
+    if (ok) {
+      float* cp = static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)(seq0 + r) * a.c_st;
+#pragma unroll
+      for (int c = 0; c < 4 * VM; ++c) cp[64 * (c >> 2) + 4 * tx + (c & 3)] = sv[c] * inv;
+      if (tx == 0) {
+        const float n_eff = Lf * Lf / fmaxf(Q2f, 1e-30f);
+        const float m_eff = n_eff * (Lf / fmaxf(Z, a.eps));
+        static_cast<float*>(a.mag)[b * a.mag_sb + h * a.mag_sh + (int64_t)(seq0 + r) * a.mag_st] = tanhf(a.beta[h] * log1pf(m_eff));
+      }
+    }
+  }
+}
+
+template <int DK>
+int launch(const atma_polar_prefill_args& a, cudaStream_t st) {
+  const int smem = 4 * (kM * (DK + kPad) + kN * (DK + kPad) + kM * kLdP);
+  ATMA_CUDA_OK(cudaFuncSetAttribute(polar_rows_f32_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  const int blocks = a.n_tiles > 0 ? a.n_tiles * (128 / kM) : (a.Tq + kM - 1) / kM;
+  polar_rows_f32_kernel<DK><<<dim3(blocks * a.H, a.B), kThreads, smem, st>>>(a);
+  return launch_status("polar_prefill (fp32, 64 x 64)");
+}
+
+}  // namespace
+
+// Rows in quadruples of channels, and more rows than one CTA of the other kernel holds.
+bool polar_rows_f32_supported(const atma_polar_prefill_args& a) {
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  auto rows = [](int64_t sb, int64_t sh, int64_t st) { return sb % 4 == 0 && sh % 4 == 0 && st % 4 == 0; };
+  return a.dtype == ATMA_F32 && (a.dk == 64 || a.dk == 128) && (a.n_tiles > 0 || a.Tq > 32) && al(a.q) && al(a.k) && al(a.v) &&
+         rows(a.q_sb, a.q_sh, a.q_st) && rows(a.k_sb, a.k_sh, a.k_st) && rows(a.v_sb, a.v_sh, a.v_st);
+}
+
+int polar_rows_f32(const atma_polar_prefill_args& a, cudaStream_t st) { return a.dk == 64 ? launch<64>(a, st) : launch<128>(a, st); }
+
+}  // namespace atma

@@ -1,6 +1,6 @@
-// Causal softmax attention over a paged cache, fp32 arithmetic throughout: the path for fp32 models and for head sizes
-// the tensor-core kernels do not serve, prompts and single tokens alike, with one or two maps per head, windows, a sink,
-// the differential combination and the output gate.  Also the entry points that choose between the kernels.
+// Causal softmax attention over a paged cache, fp32 arithmetic throughout: the path for fp32 models' single tokens and short
+// steps and for head sizes the tiled kernels do not serve, with one or two maps per head, windows, a sink, the differential
+// combination and the output gate.  Also the entry points that choose between the kernels.
 //
 // A CTA of eight warps holds 16 query rows of one head, two per warp.  Keys come in tiles of 32: a lane owns a key for
 // the scores, and vdim / 32 value channels for the weighted sum, so the softmax statistics of a row are warp reductions.
@@ -205,6 +205,7 @@ extern "C" int atma_softmax_prefill(const atma_softmax_args* a, void* stream) {
   if (a->n_seqs <= 0 || a->max_rows <= 0) return ATMA_OK;
   const atma_softmax_args b = bounded(*a);
   if (softmax_prefill_sm100_supported(b)) return softmax_prefill_sm100(b, (cudaStream_t)stream);
+  if (softmax_rows_f32_supported(b)) return softmax_rows_f32(b, (cudaStream_t)stream);
   return rows_path(b, b.max_rows, (cudaStream_t)stream);
 }
 

@@ -1,0 +1,185 @@
+// Causal softmax attention of fp32 prompts over a paged cache, fp32 arithmetic, 64 rows x 64 keys per step: one or two maps,
+// windows, a sink, the differential combination and the output gate as in softmax_rows_kernel, which keeps the other types
+// and sizes and short steps.
+//
+// There a lane owns one key and a warp two rows: two loads from shared memory for two FMAs.  Here a thread owns 4 x 4 scores
+// and 4 rows x 4 VM channels (rows_f32.cuh), so that FMAs and shared memory are both busy; K and V take turns in one buffer,
+// V under the statistics, and two CTAs share an SM, one loading while the other computes.  Later rows have more keys, so
+// those of all heads come first.  Measured, 1500 rows, 8 heads, two maps of 64, 128 value channels: 1089 -> 549 us (679 with
+// the heads one after another).
+#include "rows_f32.cuh"
+#include "softmax_attention.cuh"
+
+namespace atma {
+
+namespace {
+
+using namespace rows_f32;
+
+template <int M, int VM>
+__global__ void __launch_bounds__(kThreads, 2)
+softmax_rows_f32_kernel(const atma_softmax_args a) {
+  extern __shared__ __align__(16) float sm[];
+  const int kd = M * a.dim, ld = kd + kPad;
+  float* sQ = sm;                              // [64][ld]
+  float* sKV = sQ + kM * ld;                   // K [64][ld], then V [64][64 VM]
+  float* sP = sKV + kN * max(ld, 64 * VM);     // [M][64][kLdP]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
+  const int s = blockIdx.y, h = blockIdx.x % a.H;
+  const int r_begin = a.cu_rows[s], n_rows = a.cu_rows[s + 1] - r_begin;
+  const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM;
+  if (q0 >= n_rows) return;
+  const int start = a.start_pos[s];
+  const int g = h / (a.H / a.G);
+  float* out = static_cast<float*>(a.out);
+  if (start < 0) {                             // padded sequence
+    for (int i = tid; i < min(kM, n_rows - q0) * a.vdim; i += kThreads)
+      out[(int64_t)(r_begin + q0 + i / a.vdim) * a.out_rs + (int64_t)h * a.vdim + i % a.vdim] = 0.f;
+    return;
+  }
+  const float* Q = static_cast<const float*>(a.q);
+  const float* K = static_cast<const float*>(a.k_cache);
+  const float* V = static_cast<const float*>(a.v_cache);
+  for (int i = tid; i < kM * (kd / 4); i += kThreads) {
+    const int r = i / (kd / 4), c = 4 * (i - r * (kd / 4));
+    float4 x = {0.f, 0.f, 0.f, 0.f};
+    if (q0 + r < n_rows) x = *reinterpret_cast<const float4*>(Q + ((int64_t)(r_begin + q0 + r) * a.H + h) * kd + c);
+    *reinterpret_cast<float4*>(sQ + r * ld + c) = make_float4(x.x * a.scale, x.y * a.scale, x.z * a.scale, x.w * a.scale);
+  }
+  const int last_pos = start + min(q0 + kM, n_rows) - 1;      // the last row's own position
+  const int n_keys = min(last_pos + 1, a.max_blocks * a.block_size);
+  const KeyTiles tiles(start + q0, last_pos, a.max_blocks * a.block_size, a.window, a.keep_first, kN);
+  const int32_t* bt = a.block_tables + s * a.bt_stride;
+  const int first_pos = start + q0 + 8 * warp;                // of this warp's eight rows
+
+  float m[4][M], l[4][M];
+  uint64_t acc[M][4][2 * VM];
+#pragma unroll
+  for (int t = 0; t < M; ++t)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      m[i][t] = a.sink;                        // the sink is a key that was seen before the others
+      l[i][t] = a.sink > -INFINITY ? 1.f : 0.f;
+#pragma unroll
+      for (int c = 0; c < 2 * VM; ++c) acc[t][i][c] = 0;
+    }
+
+  for (int kt = 0; kt < tiles.n; ++kt) {
+    const int k0 = tiles[kt] * kN;
+    auto fetch = [&](const float* cache, int width, int row_len, int dst_ld) {      // the tile's rows of one cache, zeros behind them
+      const int per_row = row_len / 4;
+      for (int i = tid; i < kN * per_row; i += kThreads) {
+        const int j = i / per_row, c = 4 * (i - j * per_row), pos = k0 + j;
+        const float* src = cache;
+        const bool there = pos < n_keys && c < width;
+        if (there) {
+          const int blk = pos / a.block_size;
+          const int phys = min(max(bt[blk], 0), a.num_blocks - 1);
+          src = cache + (((int64_t)phys * a.block_size + (pos - blk * a.block_size)) * a.G + g) * width + c;
+        }
+        copy16(sKV + j * dst_ld + c, src, there);
+      }
+    };
+    __syncthreads();                           // the last tile's V is read
+    fetch(K, kd, kd, ld);
+    copies_done();
+    // columns that some row of the warp may see: nothing beyond them enters its sums
+    const int j1 = min(min(kN, n_keys - k0), first_pos + 8 - k0);
+    const int j0 = k0 >= a.keep_first ? max(0, first_pos - a.window + 1 - k0) & ~3 : 0;
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      float sc[4][4];
+      dots<M == 1>(sQ + t * a.dim, sKV + t * a.dim, ld, a.dim / 4, ty, tx, sc);
+      if (t == M - 1) {
+        __syncthreads();                       // K is read
+        fetch(V, a.vdim, 64 * VM, 64 * VM);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int pos = start + q0 + 4 * ty + i;
+        float top = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = k0 + tx + 16 * j;
+          sc[i][j] = key < n_keys && key_visible(pos, key, a.window, a.keep_first) ? sc[i][j] : -INFINITY;
+          top = fmaxf(top, sc[i][j]);
+        }
+        const float mn = fmaxf(m[i][t], row_max(top));
+        const float al = mn == -INFINITY ? 1.f : expf(m[i][t] - mn);
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float p = mn == -INFINITY ? 0.f : expf(sc[i][j] - mn);
+          sP[(t * kM + 4 * ty + i) * kLdP + tx + 16 * j] = p;
+          sum += p;
+        }
+        l[i][t] = l[i][t] * al + row_sum(sum);
+        m[i][t] = mn;
+        times<VM>(acc[t][i], al);
+      }
+    }
+    copies_done();
+#pragma unroll
+    for (int t = 0; t < M; ++t) weigh<VM>(sP + t * kM * kLdP, sKV, ty, tx, j0, j1, acc[t]);
+  }
+
+  const bool vec = a.out_rs % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = q0 + 4 * ty + i;
+    float o[4 * VM], ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4 * VM; ++c) {
+      o[c] = l[i][0] > 0.f ? at<VM>(acc[0][i], c) / l[i][0] : 0.f;
+      if constexpr (M == 2) o[c] -= l[i][M - 1] > 0.f ? a.lambda * (at<VM>(acc[M - 1][i], c) / l[i][M - 1]) : 0.f;
+      ss = fmaf(o[c], o[c], ss);               // channels behind vdim are zero
+    }
+    float f = 1.f;
+    if constexpr (M == 2) f = a.out_scale / sqrtf(row_sum(ss) / (float)a.vdim + a.eps);
+    if (row < n_rows) {
+      float* op = out + (int64_t)(r_begin + row) * a.out_rs + (int64_t)h * a.vdim;
+      const float* gp = a.gate == nullptr ? nullptr : static_cast<const float*>(a.gate) + (int64_t)(r_begin + row) * a.gate_rs + (int64_t)h * a.vdim;
+#pragma unroll
+      for (int c = 0; c < VM; ++c) {
+        const int at0 = 64 * c + 4 * tx;
+        if (at0 >= a.vdim) continue;
+        float y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] = o[4 * c + e] * f * (gp != nullptr ? sigmoid_gate(gp[at0 + e]) : 1.f);
+        if (vec) *reinterpret_cast<float4*>(op + at0) = make_float4(y[0], y[1], y[2], y[3]);
+        else
+#pragma unroll
+          for (int e = 0; e < 4; ++e) op[at0 + e] = y[e];
+      }
+    }
+  }
+}
+
+int smem_bytes(const atma_softmax_args& a) {
+  const int ld = a.maps * a.dim + kPad, vm = a.vdim <= 64 ? 64 : 128;
+  return 4 * (kM * ld + kN * (ld > vm ? ld : vm) + a.maps * kM * kLdP);
+}
+
+template <int M, int VM>
+int launch(const atma_softmax_args& a, cudaStream_t st) {
+  const int smem = smem_bytes(a);
+  ATMA_CUDA_OK(cudaFuncSetAttribute(softmax_rows_f32_kernel<M, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  softmax_rows_f32_kernel<M, VM><<<dim3((a.max_rows + kM - 1) / kM * a.H, a.n_seqs), kThreads, smem, st>>>(a);
+  return launch_status("softmax attention (fp32, 64 x 64)");
+}
+
+}  // namespace
+
+// Rows in quadruples of channels, sizes that leave room for two CTAs, and more rows than two CTAs of the other kernel hold.
+bool softmax_rows_f32_supported(const atma_softmax_args& a) {
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  return a.dtype == ATMA_F32 && a.max_rows > 32 && a.dim % 4 == 0 && a.vdim % 4 == 0 && a.maps * a.dim <= 128 && a.vdim <= 128 && al(a.q) &&
+         al(a.k_cache) && al(a.v_cache);
+}
+
+int softmax_rows_f32(const atma_softmax_args& a, cudaStream_t st) {
+  if (a.maps == 1) return a.vdim <= 64 ? launch<1, 1>(a, st) : launch<1, 2>(a, st);
+  return a.vdim <= 64 ? launch<2, 1>(a, st) : launch<2, 2>(a, st);
+}
+
+}  // namespace atma

@@ -222,3 +222,20 @@ def test_tensor_core_path_is_taken_and_no_wait_ran_out():
     status = c_int(-1)
     _lib.check(lib.atma_device_status(byref(status)))
     assert status.value == 0
+
+
+@pytest.mark.parametrize("Tq,Tk", [(33, 33), (64, 64), (65, 130), (190, 200)])
+@pytest.mark.parametrize("H,Hkv,dk", [(2, 1, 64), (4, 2, 128)])
+@pytest.mark.parametrize("window", [None, 37])
+def test_fp32_tiles_of_rows_against_short_calls(Tq, Tk, H, Hkv, dk, window):
+    """The 64-row kernel against the 32-row kernel on the same rows in portions, whose key counts are not in order; both sum
+    at most 200 fp32 terms in their own order."""
+    q, k, v = rand((2, H, Tq, dk), 1).cuda(), rand((2, Hkv, Tk, dk), 2).cuda(), rand((2, Hkv, Tk, dk), 3).cuda()
+    n = (torch.arange(Tq) * 37 % Tk + 1).float().cuda()
+    p = dict(v_null=rand((H, dk), 4).cuda(), null_base=rand((H,), 5).cuda(), null_slope_raw=rand((H,), 6).cuda(), len_gain_raw=rand((H,), 7).cuda(),
+             mag_beta_raw=rand((H,), 8).cuda())
+    c, mag = atma_b200.polar_attention_fwd(q, k, v, n, window=window, is_causal=False, **p)
+    for a in range(0, Tq, 32):
+        s = slice(a, a + 32)
+        wc, wm = atma_b200.polar_attention_fwd(q[:, :, s].contiguous(), k, v, n[s].contiguous(), window=window, is_causal=False, **p)
+        assert max_rel(c[:, :, s], wc) < 1e-5 and max_rel(mag[:, :, s], wm) < 1e-5

@@ -421,3 +421,29 @@ def test_saved_folder_command_line_and_replay(tmp_path, capsys, monkeypatch):
     assert capsys.readouterr().out.split() == ["done", "0", "done", "1", "done", "2"]
     got = np.concatenate([np.fromfile(tmp_path / "o" / f, "<f4") for f in ("0.f32", "2.f32")]).reshape(3, -1)
     close(torch.tensor(got), Z.forward(cfg, w, p)[0][[14, 2, 19]], F32)
+
+
+@pytest.mark.parametrize("H,G,maps,dim,vdim", [(2, 1, 1, 4, 4), (3, 1, 1, 128, 128), (2, 2, 1, 60, 68), (4, 2, 2, 64, 128), (2, 1, 2, 8, 64)])
+@pytest.mark.parametrize("window,keep", [(EVERY, 0), (40, 3), (65, 70)])
+@pytest.mark.parametrize("rows,start", [(33, 0), (64, 1), (65, 63), (200, 130)])
+def test_fp32_tiles_of_rows_against_short_steps(H, G, maps, dim, vdim, window, keep, rows, start):
+    """The 64-row kernel on a prompt against the 16-row kernel on the same rows in portions of 32: edges of tiles, windows
+    and kept keys.  Both sum at most 330 fp32 terms in their own order.  An infinite value stays behind the rows in front."""
+    n = rows + start
+    q, kc, vc = rand((rows, H, maps, dim), 1), rand((8, 64, G, maps * dim), 2), rand((8, 64, G, vdim), 3)
+    q, kc, vc = q.cuda(), kc.cuda(), vc.cuda()
+    table = [[5, 2, 7, 0, 1, 3]]
+    kw = dict(scale=dim ** -0.5, lam=0.3, out_scale=0.7, eps=1e-6, window=None if window == EVERY else window, keep_first=keep, sink=0.5,
+              gate=rand((rows, H * vdim), 4).cuda())
+
+    def whole():
+        out = torch.zeros(rows, H * vdim, device="cuda")
+        return ops().softmax_prefill(q, kc, vc, group([rows], [start], [0], table), out, **kw)
+
+    out, want = whole(), torch.zeros(rows, H * vdim, device="cuda")
+    for a in range(0, rows, 32):
+        b = min(a + 32, rows)
+        ops().softmax_prefill(q[a:b], kc, vc, group([b - a], [start + a], [0], table), want[a:b], **{**kw, "gate": kw["gate"][a:b]})
+    assert max_rel(out, want) < 1e-5
+    vc[table[0][(n - 1) // 64], (n - 1) % 64] = float("inf")
+    assert torch.equal(whole()[:max(rows - 12, 0)], out[:max(rows - 12, 0)])
