@@ -196,15 +196,19 @@ def _sm_count(device=None):
     return _sm_counts[idx]
 
 
-def decode_num_splits(B, Hkv, max_context, sm_count=None, ctas_per_sm=2, min_keys=1024):
+def decode_num_splits(B, Hkv, max_context, sm_count=None, ctas_per_sm=2, min_keys=1024, few_keys=None):
     """Key ranges per (sequence, KV head).  The split kernel keeps ``ctas_per_sm`` CTAs resident
     per SM, so the grid B*Hkv*n runs in ceil(B*Hkv*n / (sm_count*ctas_per_sm)) waves; pick the n
     (at least ``min_keys`` keys per range, at most 64 ranges) whose last wave is fullest, preferring
-    more ranges on a tie-ish.  Depends only on launch-time shapes (CUDA-graph safe)."""
+    more ranges on a tie-ish.  With ``few_keys``, while everything fits one wave, up to 16 ranges of at least that many keys
+    each (3 sequences of 1000 keys: 14.1 us in one range, 4.2 in 16; SMs would be idle otherwise).  Depends only on launch-time shapes (CUDA-graph safe)."""
     if sm_count is None:
         sm_count = _sm_count() if torch.cuda.is_available() else 148
     slots = sm_count * ctas_per_sm
-    n_max = int(max(1, min(64, max_context // min_keys)))
+    n_max = max_context // min_keys
+    if few_keys is not None:
+        n_max = max(n_max, min(max_context // few_keys, slots // (B * Hkv), 16))
+    n_max = int(max(1, min(64, n_max)))
     best_n, best_eff = 1, -1.0
     for n in range(1, n_max + 1):
         ctas = B * Hkv * n
@@ -276,7 +280,7 @@ def polar_attention_decode(q, k_cache, v_cache, block_tables, context_lens, *,
     if context_lens.dtype != torch.int32 or not context_lens.is_contiguous():
         context_lens = context_lens.to(torch.int32).contiguous()
     params = _params(v_null, null_base, null_slope_raw, len_gain_raw, mag_beta_raw, q.device)
-    n_splits = num_splits or decode_num_splits(B, Hkv, max_blocks * block_size)
+    n_splits = num_splits or decode_num_splits(B, Hkv, max_blocks * block_size, few_keys=64)
     scratch = _decode_scratch(q.device, lib.atma_polar_decode_scratch_floats(B, H, dk, n_splits))
     a = _lib.PolarDecodeArgs()
     if out is None:
