@@ -13,6 +13,7 @@
 // Rounding follows eager execution: every op of the reference rounds its result to the
 // activation dtype, and so do the corresponding points here.
 #include "common.cuh"
+#include "early.cuh"
 
 namespace atma {
 
@@ -70,6 +71,7 @@ __device__ __forceinline__ void store_run(T* p, const T (&v)[N]) {
 template <typename T, int CPL, int K>
 __global__ void __launch_bounds__(128)
 qkv_prep_decode_kernel(const PrepDecodeArgs a, const int wide) {
+  early_start();
   const int lane = threadIdx.x & 31;
   const int unit = blockIdx.x * 4 + (threadIdx.x >> 5);
   const int units = a.H + 2 * a.Hkv;
@@ -187,8 +189,8 @@ add_rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* _
 // the latency of a decode step's 2 x layers launches of this kernel, not its bandwidth, is what counts.
 template <typename T>
 __global__ void __launch_bounds__(512)
-add_rms_norm_row_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* __restrict__ w, T* __restrict__ x_out,
-                        T* __restrict__ h_out, int D, float eps) {
+add_rms_norm_row_kernel(const T* x, const T* y, const T* w, T* x_out, T* h_out, int D, float eps) {
+  early_start();
   __shared__ float s_part[16];
   const int row = blockIdx.x, tid = threadIdx.x;
   const int c = tid * 8;
@@ -264,9 +266,9 @@ extern "C" int atma_qkv_prep_decode(const void* q_gate, int64_t qg_row, int64_t 
                     al(k_out, 16) && al(v_out, 16) && al(k_cache, 16) && al(v_cache, 16)) ? 1 : 0;
 #define ATMA_PD(CPLV)                                                                        \
   switch (K) {                                                                               \
-    case 2: qkv_prep_decode_kernel<T, CPLV, 2><<<grid, block, 0, st>>>(a, wide); break;      \
-    case 3: qkv_prep_decode_kernel<T, CPLV, 3><<<grid, block, 0, st>>>(a, wide); break;      \
-    default: qkv_prep_decode_kernel<T, CPLV, 4><<<grid, block, 0, st>>>(a, wide); break;     \
+    case 2: launch_early(B, qkv_prep_decode_kernel<T, CPLV, 2>, grid, block, 0, st, a, wide); break;      \
+    case 3: launch_early(B, qkv_prep_decode_kernel<T, CPLV, 3>, grid, block, 0, st, a, wide); break;      \
+    default: launch_early(B, qkv_prep_decode_kernel<T, CPLV, 4>, grid, block, 0, st, a, wide); break;     \
   }
   ATMA_DISPATCH_DTYPE(dtype, T, {
     switch (dk) {
@@ -291,11 +293,11 @@ extern "C" int atma_add_rms_norm(const void* x, const void* y, const void* weigh
   if (dtype != ATMA_F32 && D % 8 == 0 && al16(x) && al16(y) && al16(weight) && al16(x_out) && al16(h_out)) {
     const int threads = ((D / 8 + 31) / 32) * 32;                // <= 512 for D <= 4096
     if (dtype == ATMA_BF16)
-      add_rms_norm_row_kernel<__nv_bfloat16><<<rows, threads, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)y,
-          (const __nv_bfloat16*)weight, (__nv_bfloat16*)x_out, (__nv_bfloat16*)h_out, D, eps);
+      launch_early(rows, add_rms_norm_row_kernel<__nv_bfloat16>, rows, threads, 0, st, (const __nv_bfloat16*)x, (const __nv_bfloat16*)y,
+                   (const __nv_bfloat16*)weight, (__nv_bfloat16*)x_out, (__nv_bfloat16*)h_out, D, eps);
     else
-      add_rms_norm_row_kernel<__half><<<rows, threads, 0, st>>>((const __half*)x, (const __half*)y, (const __half*)weight,
-                                                                (__half*)x_out, (__half*)h_out, D, eps);
+      launch_early(rows, add_rms_norm_row_kernel<__half>, rows, threads, 0, st, (const __half*)x, (const __half*)y, (const __half*)weight,
+                   (__half*)x_out, (__half*)h_out, D, eps);
     return launch_status("add_rms_norm");
   }
   const dim3 grid((rows + 3) / 4), block(128);

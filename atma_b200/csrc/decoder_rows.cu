@@ -1,6 +1,7 @@
 // Row operations of the decoder models: token + bigram and token + learned-position embeddings, the fp32 residual
 // stream with RMS norms of the stream or of what a sublayer adds to it, the feed-forward activations and the per-head
 // norm with a silu gate.  Everything is one pass over rows, 16 bytes per thread and access where the shapes allow it.
+#include "early.cuh"
 #include "common.cuh"
 #include "../../include/atma_decoder.h"
 
@@ -42,8 +43,8 @@ constexpr int kNormThreads = 256;
 // One CTA per row; the row stays in registers between the sum of squares and the outputs.
 template <typename T, int NV>
 __global__ void __launch_bounds__(kNormThreads)
-residual_norms_kernel(const float* __restrict__ x, const T* __restrict__ y, float* __restrict__ x_out, const T* __restrict__ w1,
-                      T* __restrict__ h1, const T* __restrict__ w2, T* __restrict__ h2, int D, float eps, float offset) {
+residual_norms_kernel(const float* x, const T* y, float* x_out, const T* w1, T* h1, const T* w2, T* h2, int D, float eps, float offset) {
+  early_start();
   __shared__ float s_part[kNormThreads / 32];
   const int64_t base = (int64_t)blockIdx.x * D;
   const int tid = threadIdx.x;
@@ -163,6 +164,7 @@ struct EmbedNormArgs {
 template <typename T, int VEC, int NV>
 __global__ void __launch_bounds__(kNormThreads)
 embed_position_norm_kernel(const EmbedNormArgs a) {
+  early_start();
   __shared__ float s_part[kNormThreads / 32];
   const int64_t row = blockIdx.x;
   const T* e = static_cast<const T*>(a.embed) + (int64_t)min(max(a.ids[row], 0), a.vocab - 1) * a.D;
@@ -213,6 +215,7 @@ struct PostNormArgs {
 template <typename T, int VEC, int NV>
 __global__ void __launch_bounds__(kNormThreads)
 residual_post_norm_kernel(const PostNormArgs a) {
+  early_start();
   __shared__ float s_part[2][kNormThreads / 32];
   const int64_t base = (int64_t)blockIdx.x * a.D;
   const T *y = static_cast<const T*>(a.y) + base, *bias = static_cast<const T*>(a.bias), *w = static_cast<const T*>(a.w);
@@ -380,11 +383,11 @@ using namespace atma;
   do {                                                                                                     \
     int threads = 0;                                                                                       \
     const int nv = row_groups<VEC>(a.D, &threads);                                                         \
-    if (nv == 1) KERNEL<T, VEC, 1><<<rows, threads, 0, st>>>(a);                                           \
-    else if (nv == 2) KERNEL<T, VEC, 2><<<rows, threads, 0, st>>>(a);                                      \
-    else if (nv == 4) KERNEL<T, VEC, 4><<<rows, threads, 0, st>>>(a);                                      \
-    else if (nv == 8) KERNEL<T, VEC, 8><<<rows, threads, 0, st>>>(a);                                      \
-    else KERNEL<T, VEC, 16><<<rows, threads, 0, st>>>(a);                                                  \
+    if (nv == 1) launch_early(rows, KERNEL<T, VEC, 1>, rows, threads, 0, st, a);                                           \
+    else if (nv == 2) launch_early(rows, KERNEL<T, VEC, 2>, rows, threads, 0, st, a);                                      \
+    else if (nv == 4) launch_early(rows, KERNEL<T, VEC, 4>, rows, threads, 0, st, a);                                      \
+    else if (nv == 8) launch_early(rows, KERNEL<T, VEC, 8>, rows, threads, 0, st, a);                                      \
+    else launch_early(rows, KERNEL<T, VEC, 16>, rows, threads, 0, st, a);                                                  \
   } while (0)
 
 extern "C" int atma_decoder_abi_version(void) { return 2; }
@@ -472,10 +475,10 @@ extern "C" int atma_residual_norms(const float* x, const void* y, float* x_out, 
     const int nv = (D / 4 + kNormThreads - 1) / kNormThreads;
     const int threads = min(kNormThreads, ((D / 4 + 31) / 32) * 32);
     if (!vec) residual_norms_any_kernel<T><<<rows, kNormThreads, 0, st>>>(x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
-    else if (nv <= 1) residual_norms_kernel<T, 1><<<rows, threads, 0, st>>>(x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
-    else if (nv <= 2) residual_norms_kernel<T, 2><<<rows, threads, 0, st>>>(x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
-    else if (nv <= 4) residual_norms_kernel<T, 4><<<rows, threads, 0, st>>>(x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
-    else residual_norms_kernel<T, 8><<<rows, threads, 0, st>>>(x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
+    else if (nv <= 1) launch_early(rows, residual_norms_kernel<T, 1>, rows, threads, 0, st, x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
+    else if (nv <= 2) launch_early(rows, residual_norms_kernel<T, 2>, rows, threads, 0, st, x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
+    else if (nv <= 4) launch_early(rows, residual_norms_kernel<T, 4>, rows, threads, 0, st, x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
+    else launch_early(rows, residual_norms_kernel<T, 8>, rows, threads, 0, st, x, yp, x_out, w1p, h1p, w2p, h2p, D, eps, offset);
   });
   return launch_status("residual_norms");
 }

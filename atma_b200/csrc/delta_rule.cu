@@ -8,6 +8,7 @@
 // not read.
 #include "common.cuh"
 #include "../../include/atma_decoder.h"
+#include "early.cuh"
 #include "delta_blocks.cuh"
 #include "delta_rule.cuh"
 
@@ -429,13 +430,15 @@ delta_scan_kernel(const atma_delta_args a, const T* __restrict__ q, const T* __r
 }
 
 // ---- step: one CTA per (sequence, head) -----------------------------------------------------------------------------
-// Warp w holds rows w, w + 8, ... of the state plane, lane l the VEC columns VEC * l of a block of 32 * VEC columns; the
-// first block's loads are in flight while the convolutions run.
-constexpr int kStepWarps = 8;
+// Warp w holds rows w, w + 16, ... of the state plane, lane l the VEC columns VEC * l of a block of 32 * VEC columns; the
+// first block's loads are in flight while the convolutions run.  Sixteen warps and the corrections summed once, by a thread per
+// column: 8 sequences x 8 heads 9.5 -> 7.7 us (8 warps, every thread summing for itself).
+constexpr int kStepWarps = 16;
 
 template <typename T, int VEC, int RPW, int TAPS>             // TAPS 0: any number
 __global__ void __launch_bounds__(kStepWarps * 32)
-delta_step_kernel(const atma_delta_args a, const T* __restrict__ norm_w, T* __restrict__ out, int64_t out_rs, float eps) {
+delta_step_kernel(const atma_delta_args a, const T* norm_w, T* out, int64_t out_rs, float eps) {
+  early_start();
   extern __shared__ float sm[];
   const int K = a.dim, V = a.vdim;
   float* s_q = sm;                              // [K]
@@ -443,6 +446,7 @@ delta_step_kernel(const atma_delta_args a, const T* __restrict__ norm_w, T* __re
   float* s_v = s_k + K;                         // [V]
   float* s_o = s_v + V;                         // [V]
   __shared__ __align__(16) float s_red[kStepWarps][32 * VEC];
+  __shared__ __align__(16) float s_u[32 * VEC];
   __shared__ float s_sum[3][kStepWarps];
   const int b = blockIdx.y, h = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -481,7 +485,7 @@ delta_step_kernel(const atma_delta_args a, const T* __restrict__ norm_w, T* __re
   const float za = to_f32(zr[goff + h]), zb = to_f32(zr[goff + a.H + h]), alog = a.A_log[h], dtb = a.dt_bias[h];
   float gate_c = 0.f, norm_c = 0.f;              // V <= 256: one output channel per thread
   if (tid < V) { gate_c = to_f32(zr[2 * nq + a.H * V + h * V + tid]); norm_c = to_f32(norm_w[tid]); }
-  constexpr int kRounds = 3, TA = TAPS > 0 ? TAPS : 1;           // 2 K + V <= 768 channels
+  constexpr int kRounds = 2, TA = TAPS > 0 ? TAPS : 1;           // 2 K + V <= 768 channels
   float qs = 0.f, ks = 0.f;
   float hist[kRounds][TA], wt[kRounds][TA];
   auto locate = [&](int i, int& part, int& c, int& pc, int& zc) {
@@ -553,16 +557,17 @@ delta_step_kernel(const atma_delta_args a, const T* __restrict__ norm_w, T* __re
     __syncthreads();                            // s_red is free again
     *reinterpret_cast<FV*>(&s_red[warp][lane * VEC]) = *reinterpret_cast<const FV*>(p);
     __syncthreads();
-    alignas(16) float rd[VEC] = {};
-    float u[VEC] = {};
+    if (tid < 32 * VEC) {
+      const int cc = cb * 32 * VEC + tid;
+      float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < kStepWarps; ++w) {
-      const FV t = *reinterpret_cast<const FV*>(&s_red[w][lane * VEC]);
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) u[e] += t.e[e];
+      for (int w = 0; w < kStepWarps; ++w) t += s_red[w][tid];
+      s_u[tid] = cc < V ? bt * (s_v[cc] - t) : 0.f;
     }
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) u[e] = c + e < V ? bt * (s_v[c + e] - u[e]) : 0.f;
+    __syncthreads();
+    alignas(16) float rd[VEC] = {};
+    alignas(16) float u[VEC];
+    *reinterpret_cast<FV*>(u) = *reinterpret_cast<const FV*>(&s_u[lane * VEC]);
 #pragma unroll
     for (int i = 0; i < RPW; ++i) {
       const int r = warp + kStepWarps * i;
@@ -664,10 +669,10 @@ int step_t(const atma_delta_args& a, const void* w, void* out, int64_t out_rs, f
   const dim3 grid(a.H, a.n_seqs);
   const int smem = (2 * a.dim + 2 * a.vdim) * 4;
   const bool vec = a.vdim % 4 == 0 && a.state_ss % 4 == 0 && (reinterpret_cast<uintptr_t>(a.state_table) & 15) == 0;
-#define ATMA_STEPT(V, R, K) delta_step_kernel<T, V, R, K><<<grid, kStepWarps * 32, smem, st>>>(a, (const T*)w, (T*)out, out_rs, eps)
+#define ATMA_STEPT(V, R, K) launch_early(a.n_seqs, delta_step_kernel<T, V, R, K>, grid, kStepWarps * 32, smem, st, a, (const T*)w, (T*)out, out_rs, eps)
 #define ATMA_STEP(V, R) do { if (a.taps == 4) ATMA_STEPT(V, R, 4); else ATMA_STEPT(V, R, 0); } while (0)
-  if (vec) { if (a.dim <= 64) ATMA_STEP(4, 8); else if (a.dim <= 128) ATMA_STEP(4, 16); else ATMA_STEP(4, 32); }
-  else { if (a.dim <= 64) ATMA_STEP(1, 8); else if (a.dim <= 128) ATMA_STEP(1, 16); else ATMA_STEP(1, 32); }
+  if (vec) { if (a.dim <= 64) ATMA_STEP(4, 4); else if (a.dim <= 128) ATMA_STEP(4, 8); else ATMA_STEP(4, 16); }
+  else { if (a.dim <= 64) ATMA_STEP(1, 4); else if (a.dim <= 128) ATMA_STEP(1, 8); else ATMA_STEP(1, 16); }
 #undef ATMA_STEPT
 #undef ATMA_STEP
   return launch_status("delta_step");

@@ -5,6 +5,7 @@
 // B*x' never reaches memory (only its last K-1 values, the conv state), and y is written once.
 // Rounding to the activation dtype happens where the separate ops round: after B*x', after the
 // conv, after the product with C.
+#include "early.cuh"
 #include "common.cuh"
 
 namespace atma {
@@ -44,9 +45,9 @@ __global__ void lfm2_conv_step_kernel(const T* __restrict__ proj, int64_t proj_s
 // stores.  Same rounding points as the channel-per-thread form.
 template <typename T, int K>
 __global__ void __launch_bounds__(128)
-lfm2_conv_step_wide_kernel(const T* __restrict__ proj, int64_t proj_sb, const T* __restrict__ w,
-                           const int64_t* __restrict__ slots, T* __restrict__ state, int64_t state_ss,
-                           T* __restrict__ out, int64_t out_sb, int D) {
+lfm2_conv_step_wide_kernel(const T* proj, int64_t proj_sb, const T* w, const int64_t* slots, T* state, int64_t state_ss, T* out,
+                           int64_t out_sb, int D) {
+  early_start();
   const int b = blockIdx.x;
   const int d0 = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   if (d0 >= D) return;
@@ -297,9 +298,9 @@ int launch_lfm2_step(const void* proj, int64_t proj_sb, const void* w, const int
     if (D % 8 == 0 && proj_sb % 8 == 0 && out_sb % 8 == 0 && state_ss % 8 == 0 && al(proj) && al(w) && al(state) && al(out)) {
       dim3 wgrid(B, (D / 8 + 127) / 128), wblock(128);
       switch (K) {
-        case 2: lfm2_conv_step_wide_kernel<T, 2><<<wgrid, wblock, 0, st>>>((const T*)proj, proj_sb, (const T*)w, slots, (T*)state, state_ss, (T*)out, out_sb, D); break;
-        case 3: lfm2_conv_step_wide_kernel<T, 3><<<wgrid, wblock, 0, st>>>((const T*)proj, proj_sb, (const T*)w, slots, (T*)state, state_ss, (T*)out, out_sb, D); break;
-        case 4: lfm2_conv_step_wide_kernel<T, 4><<<wgrid, wblock, 0, st>>>((const T*)proj, proj_sb, (const T*)w, slots, (T*)state, state_ss, (T*)out, out_sb, D); break;
+        case 2: launch_early(B, lfm2_conv_step_wide_kernel<T, 2>, wgrid, wblock, 0, st, (const T*)proj, proj_sb, (const T*)w, slots, (T*)state, state_ss, (T*)out, out_sb, D); break;
+        case 3: launch_early(B, lfm2_conv_step_wide_kernel<T, 3>, wgrid, wblock, 0, st, (const T*)proj, proj_sb, (const T*)w, slots, (T*)state, state_ss, (T*)out, out_sb, D); break;
+        case 4: launch_early(B, lfm2_conv_step_wide_kernel<T, 4>, wgrid, wblock, 0, st, (const T*)proj, proj_sb, (const T*)w, slots, (T*)state, state_ss, (T*)out, out_sb, D); break;
         default: return fail(ATMA_ERR_UNSUPPORTED, "lfm2_conv_decode_step: kernel size %d not in 2..4", K);
       }
       return launch_status("lfm2_conv_decode_step");

@@ -2,6 +2,7 @@
 //
 // One CTA per row.  A thread holds up to NV groups of VEC channels between the sums of squares (q and k at once) and the
 // results; a group belongs to one part of the row (the vector form needs part widths that are multiples of VEC).
+#include "early.cuh"
 #include "common.cuh"
 #include "../../include/atma_decoder.h"
 
@@ -24,6 +25,7 @@ struct NormStoreArgs {
 template <typename T, int VEC, int NV>
 __global__ void __launch_bounds__(kThreads)
 norm_store_kernel(const NormStoreArgs a) {
+  early_start();
   struct alignas(VEC * sizeof(T)) Pack { T e[VEC]; };
   __shared__ float s_q[kThreads / 32], s_k[kThreads / 32];
   const int64_t row = blockIdx.x;
@@ -89,11 +91,11 @@ int launch(const NormStoreArgs& a, int rows, cudaStream_t st) {
   const int nv = max((groups + kThreads - 1) / kThreads, rows >= 2048 && groups >= 128 ? 2 : 1);
   ATMA_REQUIRE(nv <= 32, "norm_store: rows of %d channels", groups * VEC);
   const auto threads = [&](int n) { return min(kThreads, ((groups + n - 1) / n + 31) / 32 * 32); };
-  if (nv <= 1) norm_store_kernel<T, VEC, 1><<<rows, threads(1), 0, st>>>(a);
-  else if (nv <= 2) norm_store_kernel<T, VEC, 2><<<rows, threads(2), 0, st>>>(a);
-  else if (nv <= 4) norm_store_kernel<T, VEC, 4><<<rows, threads(4), 0, st>>>(a);
-  else if (nv <= 8) norm_store_kernel<T, VEC, 8><<<rows, threads(8), 0, st>>>(a);
-  else norm_store_kernel<T, VEC, 32><<<rows, threads(32), 0, st>>>(a);
+  if (nv <= 1) launch_early(rows, norm_store_kernel<T, VEC, 1>, rows, threads(1), 0, st, a);
+  else if (nv <= 2) launch_early(rows, norm_store_kernel<T, VEC, 2>, rows, threads(2), 0, st, a);
+  else if (nv <= 4) launch_early(rows, norm_store_kernel<T, VEC, 4>, rows, threads(4), 0, st, a);
+  else if (nv <= 8) launch_early(rows, norm_store_kernel<T, VEC, 8>, rows, threads(8), 0, st, a);
+  else launch_early(rows, norm_store_kernel<T, VEC, 32>, rows, threads(32), 0, st, a);
   return launch_status("norm_store");
 }
 

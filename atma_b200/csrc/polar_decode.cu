@@ -15,6 +15,7 @@
 //     writes c and mag.
 // Launch shapes depend only on host-side arguments, loop bounds come from context_lens on the
 // device: the pair of launches is CUDA-graph capturable.
+#include "early.cuh"
 #include "common.cuh"
 
 namespace atma {
@@ -238,16 +239,17 @@ polar_decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache
 
 // Merge the key-range partials of one (sequence, head), fold the null sink, emit c and mag.
 template <typename T>
-__global__ void polar_decode_merge_kernel(const float* __restrict__ scratch,
-                                          const int32_t* __restrict__ context_lens,
-                                          const float* __restrict__ v_null,
-                                          const float* __restrict__ spg,
-                                          const float* __restrict__ null_base,
-                                          const float* __restrict__ sps,
-                                          const float* __restrict__ beta, T* __restrict__ c,
-                                          T* __restrict__ mag, int B, int H, int dk, int n_splits,
-                                          int window, int max_ctx, float eps, const T* __restrict__ gate,
+__global__ void polar_decode_merge_kernel(const float* scratch,
+                                          const int32_t* context_lens,
+                                          const float* v_null,
+                                          const float* spg,
+                                          const float* null_base,
+                                          const float* sps,
+                                          const float* beta, T* c,
+                                          T* mag, int B, int H, int dk, int n_splits,
+                                          int window, int max_ctx, float eps, const T* gate,
                                           int64_t gate_sb, int64_t gate_sh, int64_t c_sb, int64_t mag_sb) {
+  early_start();
   const int bh = blockIdx.x, b = bh / H, h = bh % H;
   const int tid = threadIdx.x;
   const float* stats = scratch + (int64_t)bh * n_splits * 4;
@@ -364,8 +366,7 @@ int launch_decode(const atma_polar_decode_args& a, cudaStream_t st) {
   if (polar_decode_mma_supported(a)) {
     int rc = polar_decode_split_mma(a, st);
     if (rc != ATMA_OK || a.skip_merge) return rc;
-    polar_decode_merge_kernel<T><<<a.B * a.H, 128, 0, st>>>(
-        a.scratch, a.context_lens, a.v_null, a.spg, a.null_base, a.sps, a.beta, (T*)a.c, (T*)a.mag,
+    launch_early(a.B, polar_decode_merge_kernel<T>, a.B * a.H, 128, 0, st, a.scratch, a.context_lens, a.v_null, a.spg, a.null_base, a.sps, a.beta, (T*)a.c, (T*)a.mag,
         a.B, a.H, a.dk, a.n_splits, a.window, a.max_blocks * a.block_size, a.eps, (const T*)a.gate, a.gate_sb, a.gate_sh,
         a.c_sb, a.mag_sb);
     return launch_status("polar_decode (merge)");
@@ -388,8 +389,7 @@ int launch_decode(const atma_polar_decode_args& a, cudaStream_t st) {
 #undef ATMA_LAUNCH
   int rc = launch_status("polar_decode (split)");
   if (rc != ATMA_OK || a.skip_merge) return rc;
-  polar_decode_merge_kernel<T><<<a.B * a.H, 128, 0, st>>>(
-      a.scratch, a.context_lens, a.v_null, a.spg, a.null_base, a.sps, a.beta, (T*)a.c, (T*)a.mag,
+  launch_early(a.B, polar_decode_merge_kernel<T>, a.B * a.H, 128, 0, st, a.scratch, a.context_lens, a.v_null, a.spg, a.null_base, a.sps, a.beta, (T*)a.c, (T*)a.mag,
       a.B, a.H, a.dk, a.n_splits, a.window, a.max_blocks * a.block_size, a.eps, (const T*)a.gate, a.gate_sb, a.gate_sh,
       a.c_sb, a.mag_sb);
   return launch_status("polar_decode (merge)");
@@ -435,8 +435,7 @@ extern "C" int atma_polar_decode_merge(const atma_polar_decode_args* args, void*
   ATMA_REQUIRE(a.dk >= 1 && a.dk <= 256, "polar_decode_merge: head_dim %d", a.dk);
   if (a.B <= 0) return ATMA_OK;
   ATMA_DISPATCH_DTYPE(a.dtype, T, {
-    polar_decode_merge_kernel<T><<<a.B * a.H, 128, 0, (cudaStream_t)stream>>>(
-        a.scratch, a.context_lens, a.v_null, a.spg, a.null_base, a.sps, a.beta, (T*)a.c, (T*)a.mag, a.B, a.H, a.dk, a.n_splits,
+    launch_early(a.B, polar_decode_merge_kernel<T>, a.B * a.H, 128, 0, (cudaStream_t)stream, a.scratch, a.context_lens, a.v_null, a.spg, a.null_base, a.sps, a.beta, (T*)a.c, (T*)a.mag, a.B, a.H, a.dk, a.n_splits,
         a.window, 0x7fffffff, a.eps, (const T*)a.gate, a.gate_sb, a.gate_sh, a.c_sb, a.mag_sb);
   });
   return launch_status("polar_decode (merge)");

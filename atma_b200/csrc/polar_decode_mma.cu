@@ -13,6 +13,7 @@
 // rescale disappear from the steady state; L, Q2 and O stay relative to that reference.
 // The four warps are merged once at the end and the partial statistics go to the scratch
 // layout the merge kernel reads.
+#include "early.cuh"
 #include "common.cuh"
 #include "mma_sync.cuh"
 
@@ -36,13 +37,14 @@ __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t a) {
 
 template <bool kBf16, int DK, int STAGES>
 __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2)
-polar_decode_split_mma_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k_cache,
-                              const uint16_t* __restrict__ v_cache, const int32_t* __restrict__ block_tables,
-                              int64_t bt_stride, const int32_t* __restrict__ context_lens, const int32_t* __restrict__ temp_lens,
-                              const float* __restrict__ spg, float* __restrict__ scratch, int B, int H, int Hkv,
+polar_decode_split_mma_kernel(const uint16_t* q, const uint16_t* k_cache,
+                              const uint16_t* v_cache, const int32_t* block_tables,
+                              int64_t bt_stride, const int32_t* context_lens, const int32_t* temp_lens,
+                              const float* spg, float* scratch, int B, int H, int Hkv,
                               int block_size, int max_blocks, int num_blocks, int n_splits, int window,
-                              const uint16_t* __restrict__ append_k, int64_t append_k_st, const uint16_t* __restrict__ append_v,
-                              int64_t append_v_st, const int32_t* __restrict__ append_slots) {
+                              const uint16_t* append_k, int64_t append_k_st, const uint16_t* append_v,
+                              int64_t append_v_st, const int32_t* append_slots) {
+  early_start();
   constexpr int KS = DK / 16;                 // k-steps of K Q^T
   constexpr int MT = DK / 16;                 // m-tiles of V^T P^T
   constexpr int CH = DK / 8;                  // 16-byte chunks per row
@@ -295,7 +297,7 @@ int polar_decode_split_mma(const atma_polar_decode_args& a, cudaStream_t st) {
   do {                                                                                                          \
     auto kern = polar_decode_split_mma_kernel<BF, DKK, kStages>;                                                \
     ATMA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));                \
-    kern<<<grid, 128, smem, st>>>((const uint16_t*)a.q, (const uint16_t*)a.k_cache, (const uint16_t*)a.v_cache, \
+    launch_early(a.B, kern, grid, 128, smem, st, (const uint16_t*)a.q, (const uint16_t*)a.k_cache, (const uint16_t*)a.v_cache, \
                                   a.block_tables, a.bt_stride, a.context_lens, a.temp_lens, a.spg, a.scratch, a.B, a.H,      \
                                   a.Hkv, a.block_size, a.max_blocks, a.num_blocks, a.n_splits, a.window,        \
                                   (const uint16_t*)ak, a.append_k_stride, (const uint16_t*)a.append_v, a.append_v_stride, \

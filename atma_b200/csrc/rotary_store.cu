@@ -1,5 +1,6 @@
 // Rotary positions on q and k and the K/V cache write, one pass over the projection rows.  The table holds
 // (cos, sin) per position and channel pair, so scaled frequencies and amplitudes are the caller's business.
+#include "early.cuh"
 #include "common.cuh"
 #include "../../include/atma_decoder.h"
 
@@ -19,6 +20,7 @@ struct RotArgs {
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256)
 rotary_store_kernel(const RotArgs a) {
+  early_start();
   struct alignas(VEC * sizeof(T)) Vec { T e[VEC]; };
   const int per_row = (a.nq + a.nk + a.nv) / VEC;
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
@@ -80,11 +82,11 @@ extern "C" int atma_rotary_store(const void* z, int64_t z_rs, const int32_t* pos
   const unsigned grid = (unsigned)((n + 255) / 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == ATMA_F32) {
-    if (vec) rotary_store_kernel<float, 4><<<grid, 256, 0, st>>>(a);
-    else rotary_store_kernel<float, 1><<<grid, 256, 0, st>>>(a);
+    if (vec) launch_early(a.rows, rotary_store_kernel<float, 4>, grid, 256, 0, st, a);
+    else launch_early(a.rows, rotary_store_kernel<float, 1>, grid, 256, 0, st, a);
   } else {
-    if (vec) rotary_store_kernel<__nv_bfloat16, 8><<<grid, 256, 0, st>>>(a);
-    else rotary_store_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>(a);
+    if (vec) launch_early(a.rows, rotary_store_kernel<__nv_bfloat16, 8>, grid, 256, 0, st, a);
+    else launch_early(a.rows, rotary_store_kernel<__nv_bfloat16, 1>, grid, 256, 0, st, a);
   }
   return launch_status("rotary_store");
 }

@@ -316,15 +316,18 @@ def add_rms_norm(x, y, weight, eps=1e-6):
 DECODE_LINEAR_MAX_ROWS = 16
 
 
-def decode_linear_supported(x, weight, gated=False):
+def decode_linear_supported(x, weight, gated=False, k_unit=32):
     """Whether ``decode_linear`` serves this product: CUDA, 16-bit, 1..16 rows, K a multiple of 32, N a multiple of 16
-    (32 for the gated form), 16-byte aligned rows."""
+    (32 for the gated form), 16-byte aligned rows.  ``k_unit`` 8: whether it does with ``any_k``."""
     return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype and x.ndim == 2 and
-            0 < x.shape[0] <= DECODE_LINEAR_MAX_ROWS and x.shape[1] % 32 == 0 and weight.shape[0] % (32 if gated else 16) == 0 and
+            0 < x.shape[0] <= DECODE_LINEAR_MAX_ROWS and x.shape[1] % k_unit == 0 and x.shape[1] >= 32 and weight.shape[0] % (32 if gated else 16) == 0 and
             weight.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
 
 
-LINEAR_F32_MIN_ROWS, LINEAR_F32_MIN_SIZE = 128, 64        # fewer rows, or a narrower product: the library is faster
+# Fewer rows, or a narrower product: the library is faster.  Less work than 512 x 1024 x 1024: either takes less time on the
+# GPU than the host needs for a layer's calls, and the library's is the shorter one there (a block of a few hundred rows:
+# 1127 us with every product on linear_f32, 1090 without).
+LINEAR_F32_MIN_ROWS, LINEAR_F32_MIN_SIZE, LINEAR_F32_MIN_WORK = 128, 64, 1 << 29
 
 
 def linear_f32_supported(x, weight):
@@ -334,7 +337,7 @@ def linear_f32_supported(x, weight):
         return False
     if x.ndim < 2 or weight.ndim != 2 or not weight.is_contiguous() or min(x.shape[-1], weight.shape[0]) < LINEAR_F32_MIN_SIZE:
         return False
-    if x.numel() < LINEAR_F32_MIN_ROWS * x.shape[-1]:
+    if x.numel() < LINEAR_F32_MIN_ROWS * x.shape[-1] or x.numel() * weight.shape[0] < LINEAR_F32_MIN_WORK:
         return False
     if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
         return False
@@ -359,19 +362,19 @@ def linear_f32(x, weight, bias=None, out=None, lib=None):
     K, N = x.shape[-1], weight.shape[0]
     if weight.shape[1] != K or x.dtype != torch.float32 or weight.dtype != torch.float32 or not weight.is_contiguous():
         raise ValueError("weight must be a contiguous fp32 (N, K) tensor and x fp32")
-    rows = x.reshape(-1, K)
+    rows = x if x.ndim == 2 else x.reshape(-1, K)
     if rows.stride(1) != 1:
         rows = rows.contiguous()
-    if bias is not None:
+    if bias is not None and (bias.dtype != torch.float32 or not bias.is_contiguous()):
         bias = bias.float().contiguous()
     M = rows.shape[0]
     y = torch.empty((M, N), device=x.device, dtype=torch.float32) if out is None else out
-    if y.shape != (M, N) or y.dtype != torch.float32 or y.stride(1) != 1:
+    if out is not None and (y.shape != (M, N) or y.dtype != torch.float32 or y.stride(1) != 1):
         raise ValueError("out must have the result's shape and dtype and contiguous rows")
-    scratch = torch.empty(int(lib.atma_linear_f32_scratch_bytes(M, N, K)), device=x.device, dtype=torch.uint8)
-    _lib.check(lib.atma_linear_f32(_lib.ptr(rows), rows.stride(0), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(y), y.stride(0),
-                                   M, N, K, _lib.ptr(scratch), _lib.stream_ptr()), lib)
-    return y.view(*x.shape[:-1], N) if out is None else y
+    scratch = torch.empty(lib.atma_linear_f32_scratch_bytes(M, N, K), device=x.device, dtype=torch.uint8)
+    _lib.check(lib.atma_linear_f32(rows.data_ptr(), rows.stride(0), weight.data_ptr(), None if bias is None else bias.data_ptr(), y.data_ptr(),
+                                   y.stride(0), M, N, K, scratch.data_ptr(), _lib.stream_ptr()), lib)
+    return y.view(*x.shape[:-1], N) if out is None and x.ndim != 2 else y
 
 
 def linear(x, weight, bias=None):
@@ -386,14 +389,15 @@ _HALVES = (1, 2)                      # forms whose weight holds two projections
 
 
 @torch.no_grad()
-def decode_linear(x, weight, bias=None, gated=False, out=None, lib=None):
+def decode_linear(x, weight, bias=None, gated=False, out=None, lib=None, any_k=False):
     """x @ weight.T + bias for a decode batch of up to 16 rows, the weights streamed once from HBM
     (``F.linear`` at these sizes).  ``gated``: the weight holds two projections (2F, K), first half and second half,
     and the result is (rows, F): True / "squared_relu" = second * relu(first)^2 - the fc GEMM and
     ``squared_relu_gate`` of inference/models/atma.py:87-97 in one launch -, "gelu_tanh" = gelu_tanh(first) * second.
     "plain_squared_relu" has no second half: (rows, N) = relu(x @ weight.T + bias)^2.
     x (rows, K), weight (N, K) contiguous, 16-bit.  ``out``: where the result goes (contiguous rows, any row stride);
-    ``lib``: the library to call (None = libatma_b200.so; libatma_decoder.so has the same entry)."""
+    ``lib``: the library to call (None = libatma_b200.so; libatma_decoder.so has the same entry).  ``any_k``: K may be any
+    multiple of 8 (libatma_b200.so only)."""
     _lib.require_cuda(x, "decode_linear")
     lib = _lib.load() if lib is None else lib
     B, K = x.shape
@@ -409,6 +413,7 @@ def decode_linear(x, weight, bias=None, gated=False, out=None, lib=None):
         out = torch.empty((B, N // 2 if gate in _HALVES else N), device=x.device, dtype=x.dtype)
     elif out.shape != (B, N // 2 if gate in _HALVES else N) or out.dtype != x.dtype or out.stride(1) != 1:
         raise ValueError("out must have the result's shape and dtype and contiguous rows")
-    _lib.check(lib.atma_decode_linear(_lib.ptr(x), x.stride(0), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(out), out.stride(0),
-                                      B, N, K, gate, _lib.dtype_code(x), _lib.stream_ptr()), lib)
+    entry = lib.atma_decode_linear_k8 if any_k else lib.atma_decode_linear
+    _lib.check(entry(_lib.ptr(x), x.stride(0), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(out), out.stride(0),
+                     B, N, K, gate, _lib.dtype_code(x), _lib.stream_ptr()), lib)
     return out

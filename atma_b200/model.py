@@ -136,8 +136,8 @@ class AtmaModel:
 
     def _linear(self, x, w, b):
         """Decode batches of up to 16 rows stream the weights through this library's kernel; larger ones are cuBLAS."""
-        if self.small_batch_linear and decode_linear_supported(x, w):
-            return decode_linear(x, w, b)
+        if self.small_batch_linear and decode_linear_supported(x, w, k_unit=8):
+            return decode_linear(x, w, b, any_k=x.shape[1] % 32 != 0)
         return linear(x, w, b)
 
     def _mlp(self, h, i):

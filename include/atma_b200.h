@@ -248,6 +248,9 @@ int64_t atma_linear_f32_scratch_bytes(int M, int N, int K);
  * K a multiple of 32, N of 16 (32 when gated); x rows 16-byte aligned. */
 int atma_decode_linear(const void* x, int64_t x_row_stride, const void* weight, const void* bias, void* out,
                        int64_t out_row_stride, int B, int N, int K, int gated, int dtype, void* stream);
+/* The same for K a multiple of 8 (32 at least): a layer's joint output projection, whose rows are not whole 32s. */
+int atma_decode_linear_k8(const void* x, int64_t x_row_stride, const void* weight, const void* bias, void* out,
+                          int64_t out_row_stride, int B, int N, int K, int gated, int dtype, void* stream);
 
 /* ------------------------------------------------------------------------------------
  * Gated-delta chunked scan.  Replaces the third-party flash-linear-attention call

@@ -390,3 +390,50 @@ def test_linear_f32(M, K, N, spread):
     odd, want = linear_f32(x, w), (x.double() @ w.double().t())
     assert torch.equal(odd.isnan(), want.isnan()) and torch.equal(odd.isinf(), want.isinf())
     assert atma_b200.device_status() == 0
+
+
+@pytest.mark.parametrize("B,N,K", [(1, 16, 40), (3, 1024, 2056), (16, 48, 1000), (5, 160, 72)])
+def test_decode_linear_with_a_short_last_range(B, N, K):
+    """K a multiple of 8 only: the last K range has fewer columns, or none."""
+    g = torch.Generator().manual_seed(K)
+    x, w, b = (torch.randn(*s, generator=g).to(torch.bfloat16).cuda() for s in ((B, K), (N, K), (N,)))
+    want = x.double() @ w.double().t() + b.double()
+    got = atma_b200.decode_linear(x, w, b, any_k=True)
+    assert max_rel(got, want.float()) < 6e-3                              # one rounding to bf16 of an fp32 sum
+    with pytest.raises(ValueError):
+        atma_b200.decode_linear(x, w, b)
+
+
+def test_kernels_that_start_early_follow_a_join_in_a_graph():
+    """A chain of small launches, forked and joined as a decode step's, replayed: every kernel sees what those in front wrote."""
+    from atma_b200.inference_ops import add_rms_norm
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn(4, 1024, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(8, 1024, 1024, generator=g) / 32).to(torch.bfloat16).cuda()
+    norm, side = torch.ones(1024, dtype=torch.bfloat16, device="cuda"), torch.cuda.Stream()
+
+    def chain():
+        h = x
+        for i in range(0, 8, 2):
+            a = atma_b200.decode_linear(h, w[i])
+            cur = torch.cuda.current_stream()
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                c = atma_b200.decode_linear(a, w[i + 1])
+            b = atma_b200.decode_linear(a, w[i])
+            cur.wait_stream(side)
+            _, h = add_rms_norm(b, c, norm, 1e-6)
+        return h
+
+    want = chain()
+    torch.cuda.synchronize()
+    side2 = torch.cuda.Stream()
+    side2.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain()
+    for s in range(30):
+        x.copy_(torch.randn(4, 1024, generator=torch.Generator().manual_seed(s)))
+        graph.replay()
+        assert torch.equal(got, chain())
+    assert want.shape == got.shape
