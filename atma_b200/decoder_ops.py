@@ -85,6 +85,8 @@ def residual_post_norm(x, y, weight, eps, bias=None, next_weight=None, offset=0.
 def bias_squared_relu(z, bias, out):
     """out = relu(z + bias)^2 (bias None = none; rows may be strided; out may be z)."""
     _rows(z, "z"), _rows(out, "out")
+    if bias is not None and (tuple(bias.shape) != (z.shape[1],) or bias.device != z.device):
+        raise ValueError(f"bias must have {z.shape[1]} values on z's device, not the shape {tuple(bias.shape)}")
     _check(_lib.load_decoder().atma_bias_squared_relu(_ptr(z), z.stride(0), _ptr(bias), _ptr(out), out.stride(0), z.shape[0], z.shape[1],
                                                       _lib.dtype_code(z), _lib.stream_ptr()))
     return out

@@ -316,42 +316,61 @@ def add_rms_norm(x, y, weight, eps=1e-6):
 DECODE_LINEAR_MAX_ROWS = 16
 
 
-def decode_linear_supported(x, weight, gated=False, k_unit=32):
+def _one_device(x, *others):
+    """Whether x and the others (None = not there) are on the device that a launch goes to."""
+    return all(t is None or t.device == x.device for t in others) and x.device.index == torch.cuda.current_device()
+
+
+def _bias_fits(bias, N):
+    return bias is None or tuple(bias.shape) == (N,)
+
+
+def decode_linear_supported(x, weight, gated=False, k_unit=32, bias=None):
     """Whether ``decode_linear`` serves this product: CUDA, 16-bit, 1..16 rows, K a multiple of 32, N a multiple of 16
-    (32 for the gated form), 16-byte aligned rows.  ``k_unit`` 8: whether it does with ``any_k``."""
-    return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype and x.ndim == 2 and
+    (32 for the gated form), 16-byte aligned rows, a bias of N values.  ``k_unit`` 8: whether it does with ``any_k``."""
+    return (x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and weight.dtype == x.dtype and x.ndim == 2 and weight.ndim == 2 and
             0 < x.shape[0] <= DECODE_LINEAR_MAX_ROWS and x.shape[1] % k_unit == 0 and x.shape[1] >= 32 and weight.shape[0] % (32 if gated else 16) == 0 and
-            weight.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0)
+            weight.shape[1] == x.shape[1] and weight.is_contiguous() and x.stride(1) == 1 and x.stride(0) % 8 == 0 and
+            x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and _bias_fits(bias, weight.shape[0]) and _one_device(x, weight, bias))
 
 
 # Fewer rows, or a narrower product: the library is faster.  Less work than 512 x 1024 x 1024: either takes less time on the
 # GPU than the host needs for a layer's calls, and the library's is the shorter one there (a block of a few hundred rows:
 # 1127 us with every product on linear_f32, 1090 without).
 LINEAR_F32_MIN_ROWS, LINEAR_F32_MIN_SIZE, LINEAR_F32_MIN_WORK = 128, 64, 1 << 29
+LINEAR_F32_MAX_ROWS, LINEAR_F32_MAX_N, LINEAR_F32_MAX_K = 1 << 29, 1 << 21, 1 << 24      # what the entry takes
 
 
-def linear_f32_supported(x, weight):
-    """Whether ``linear_f32`` serves this product: plain fp32 CUDA tensors, enough rows, and nothing around the call that a
-    library product would obey (autograd, transforms, tracing, autocast, a caller's choice of TF32)."""
-    if not (type(x) in _PLAIN and type(weight) in _PLAIN and x.is_cuda and weight.is_cuda and x.dtype == weight.dtype == torch.float32):
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def linear_f32_supported(x, weight, bias=None):
+    """Whether ``linear_f32`` serves this product: plain fp32 tensors on the current CUDA device, a bias of N values or none,
+    enough rows, and nothing around the call that a library product would obey (autograd, transforms, tracing, autocast,
+    modes that see every call, a caller's choice of TF32)."""
+    tensors = (x, weight) if bias is None else (x, weight, bias)
+    for t in tensors:
+        if type(t) not in _PLAIN or t.dtype != torch.float32 or not t.is_cuda or t.is_neg():
+            return False
+    if x.ndim < 2 or weight.ndim != 2 or not weight.is_contiguous() or not _bias_fits(bias, weight.shape[0]) or not _one_device(*tensors):
         return False
-    if x.ndim < 2 or weight.ndim != 2 or not weight.is_contiguous() or min(x.shape[-1], weight.shape[0]) < LINEAR_F32_MIN_SIZE:
+    K, N = x.shape[-1], weight.shape[0]
+    if weight.shape[1] != K or min(K, N) < LINEAR_F32_MIN_SIZE or K > LINEAR_F32_MAX_K or N > LINEAR_F32_MAX_N:
         return False
-    if x.numel() < LINEAR_F32_MIN_ROWS * x.shape[-1] or x.numel() * weight.shape[0] < LINEAR_F32_MIN_WORK:
+    if not LINEAR_F32_MIN_ROWS * K <= x.numel() <= LINEAR_F32_MAX_ROWS * K or x.numel() * N < LINEAR_F32_MIN_WORK:
         return False
-    if torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
         return False
     if torch.is_autocast_enabled() or torch.compiler.is_compiling() or torch.jit.is_tracing():
         return False
     if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
         return False
+    if torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack():
+        return False
     try:
         return not torch.backends.cuda.matmul.allow_tf32
     except RuntimeError:                       # chosen through another of torch's switches
         return False
-
-
-_PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
 def linear_f32(x, weight, bias=None, out=None, lib=None):
@@ -362,6 +381,10 @@ def linear_f32(x, weight, bias=None, out=None, lib=None):
     K, N = x.shape[-1], weight.shape[0]
     if weight.shape[1] != K or x.dtype != torch.float32 or weight.dtype != torch.float32 or not weight.is_contiguous():
         raise ValueError("weight must be a contiguous fp32 (N, K) tensor and x fp32")
+    if not _bias_fits(bias, N):
+        raise ValueError(f"bias must have {N} values, not the shape {tuple(bias.shape)}")
+    if not _one_device(x, weight, bias, out):
+        raise ValueError("x, weight, bias and out must be on the current device")
     rows = x if x.ndim == 2 else x.reshape(-1, K)
     if rows.stride(1) != 1:
         rows = rows.contiguous()
@@ -379,7 +402,7 @@ def linear_f32(x, weight, bias=None, out=None, lib=None):
 
 def linear(x, weight, bias=None):
     """x @ weight.T + bias: fp32 rows in numbers through ``linear_f32``, the library's product otherwise."""
-    if linear_f32_supported(x, weight) and (bias is None or bias.dtype == torch.float32):
+    if linear_f32_supported(x, weight, bias):
         return linear_f32(x, weight, bias)
     return F.linear(x, weight, bias)
 
@@ -404,6 +427,10 @@ def decode_linear(x, weight, bias=None, gated=False, out=None, lib=None, any_k=F
     N = weight.shape[0]
     if weight.shape[1] != K or weight.dtype != x.dtype or not weight.is_contiguous():
         raise ValueError("weight must be a contiguous (N, K) tensor in x's dtype")
+    if not _bias_fits(bias, N):
+        raise ValueError(f"bias must have {N} values, not the shape {tuple(bias.shape)}")
+    if not _one_device(x, weight, bias, out):
+        raise ValueError("x, weight, bias and out must be on the current device")
     if x.stride(1) != 1:
         x = x.contiguous()
     if bias is not None:

@@ -136,13 +136,13 @@ class AtmaModel:
 
     def _linear(self, x, w, b):
         """Decode batches of up to 16 rows stream the weights through this library's kernel; larger ones are cuBLAS."""
-        if self.small_batch_linear and decode_linear_supported(x, w, k_unit=8):
+        if self.small_batch_linear and decode_linear_supported(x, w, k_unit=8, bias=b):
             return decode_linear(x, w, b, any_k=x.shape[1] % 32 != 0)
         return linear(x, w, b)
 
     def _mlp(self, h, i):
         w, b = self.sd[f"blocks.{i}.mlp.fc.weight"], self.sd.get(f"blocks.{i}.mlp.fc.bias")
-        if self.small_batch_linear and decode_linear_supported(h, w, gated=True):
+        if self.small_batch_linear and decode_linear_supported(h, w, gated=True, bias=b):
             act = decode_linear(h, w, b, gated=True)            # fc GEMM and the squared-ReLU gate in one launch
         else:
             fc = linear(h, w, b)
