@@ -1,25 +1,27 @@
 // fp32 matrix product on the tensor cores: out[m][n] = sum_k x[m][k] w[n][k] + bias[n], at fp32 accuracy.
 //
 // fp32 arithmetic outside the tensor cores reaches 40-50 TFLOP/s here.  A row times a power of two that brings its largest
-// value into [2^14, 2^15) is the sum of an fp16 term and 2^-11 times another, to 2^-22 of a value (2^-51 of the row's
-// largest, where a value is that much smaller).  Three products of terms - lo hi, hi lo, hi hi, small ones first, the last
-// scaling down what is there by 2^11 on its way - leave out 2^-22 of a product, with random signs.  The tensor core rounds
+// value into [2^14, 2^15) is the sum of an fp16 term and 2^-11 times another, to 2^-22 of a value that is not 2^28 times
+// smaller than that.  Three products of terms - lo hi, hi lo, hi hi, small ones first, the last scaling down what is there by
+// 2^11 on its way - leave out 2^-22 of a product, with random signs.  The tensor core rounds
 // its fp32 sums towards zero, so a sum stays there for 64 columns only; the columns' sums are added in registers, rounded to
 // nearest.  Error against 64 bits, 2-norm, beside the library's fp32 product (1500 rows, random normal): K = 1024 1.1e-7
 // against 4.1e-7, K = 5120 1.5e-7 against 9.0e-7.
-//   split kernel: one CTA per row of x and of w, two fp16 planes each and the row's power of two.
+// What the smaller values of a row lose is summed when it is split.  A result that this could change by more than 2^-24 of
+// itself - large values that meet zeros and small ones that do not - is summed again in fp32 from the inputs, a warp for
+// four, and so are the results of a row with an infinity or a NaN, which has no fp16 terms.  Rows of random values, squared
+// activations among them, have next to none, and the test costs nothing that shows; where every result needs it, 1500 x 8192 x
+// 1024 takes 7.8 ms instead of 0.12, with one such row of x 0.31.
+//   split kernel: one CTA per row of x and of w, two fp16 planes each, the row's power of two and what it lost.
 //   product kernel: a CTA owns 128 rows x BN columns.  Warp 0 TMA (both planes of 64 columns of x and of w per stage),
 //   warp 1 MMA, warps 2-9 add the sums of one stage out of one half of the accumulator columns while the next stage's
 //   products go to the other half, scale them back and write whole 128-byte lines.
 // Bound by L2 -> shared memory traffic (96 KB per 64 columns and CTA at BN = 256, 62 B per clock and SM if the tensor cores
 // were to wait for nothing).  Narrower BN where wide tiles would leave SMs without one; see pick_bn.
-// Infinities and NaN have no fp16 terms: a tile that meets one in its rows is computed in fp32 arithmetic instead.
-// Measured with the split, out of HBM, beside the library's: 1500 x 8192 x 1024 120 us (497), 1500 x 1024 x 5120 93 us (353),
-// 4096 x 8192 x 1024 261 us (1195).  Below 128 rows, 64 columns or K = 64 the split costs more than it gives (32 x 512 x
+// Measured with the split, out of HBM, beside the library's: 1500 x 8192 x 1024 118 us (499), 1500 x 1024 x 5120 95 us (346),
+// 4096 x 8192 x 1024 251 us (1094).  Below 128 rows, 64 columns or K = 64 the split costs more than it gives (32 x 512 x
 // 2048: 36 us against 26) and callers stay with the library.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status word for the host.
-#include <climits>
-
 #include "common.cuh"
 #include "linear_f32.cuh"
 #include "sm100.cuh"
@@ -32,18 +34,26 @@ using namespace sm100;
 
 constexpr int kBM = 128, kBK = 64;
 constexpr int kThreads = 320;
-constexpr int kNotFinite = INT_MIN;
 constexpr int kLoBits = 11;                 // the second plane is 2^11 times what the first leaves
+constexpr float kWhole = 1.0f / (1 << 13);  // scaled values from here on are in the two terms to 2^-22 of themselves
+constexpr float kGone = 8.6736174e-19f;      // 2^-60: from there down nothing is left (and scaling may have made it zero already)
+constexpr float kLossUnits = 4.6116860e18f; // 2^62: a row's loss, at most 2^-36 of each of 2^24 values, is counted in these
 
 __device__ int g_linear_status = 0;
+
+// From where on a sum whose row or column has that loss is trusted: it meets values below 2^15, and 2^-24 of the sum is accepted.
+__device__ __forceinline__ float trusted_from(unsigned long long loss) { return (float)loss * (549755813888.0f / kLossUnits); }      // 2^39
 
 __device__ __forceinline__ float pow2i(int n) { return __int_as_float((n + 127) << 23); }      // -126 <= n <= 127
 
 // ---- rows into two fp16 planes ----------------------------------------------------------------------------------------
-template <bool VEC>
-__global__ void __launch_bounds__(256)
+// Out of HBM and latency: a row of 1024 is one load, two barriers and one store per thread, so rows in flight count (9692 rows 20 us
+// with 32 registers, 25 with 40; the bytes alone are 12).
+// KEPT: groups of four values a thread has in registers between the two passes (1024 columns each); the others are read again.
+template <bool VEC, int KEPT>
+__global__ void __launch_bounds__(256, KEPT == 1 ? 8 : 6)
 split_rows_kernel(const float* __restrict__ x, int64_t x_rs, int M, const float* __restrict__ w, int N, int K, int Kp,
-                  __half* __restrict__ xp, __half* __restrict__ wp, int* __restrict__ exps) {
+                  __half* __restrict__ xp, __half* __restrict__ wp, int* __restrict__ exps, unsigned long long* __restrict__ losses) {
   __shared__ uint32_t s_max[8];
   const int tid = threadIdx.x;
   const bool is_x = (int)blockIdx.x < M;
@@ -63,37 +73,62 @@ split_rows_kernel(const float* __restrict__ x, int64_t x_rs, int M, const float*
     }
     return v;
   };
-  constexpr int kKept = 4;                  // rows of up to 4096 stay in registers between the two passes
-  float4 kept[kKept];
+  float4 kept[KEPT];
   uint32_t most = 0;
   auto largest = [&](const float4& v) {
     most = max(max(most, __float_as_uint(v.x) & 0x7fffffffu), max(__float_as_uint(v.y) & 0x7fffffffu,
                max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu)));
   };
 #pragma unroll
-  for (int j = 0; j < kKept; ++j) { kept[j] = load(tid + 256 * j); largest(kept[j]); }
-  for (int i = tid + 256 * kKept; 4 * i < K; i += 256) largest(load(i));
+  for (int j = 0; j < KEPT; ++j) { kept[j] = load(tid + 256 * j); largest(kept[j]); }
+  for (int i = tid + 256 * KEPT; 4 * i < K; i += 256) largest(load(i));
   most = __reduce_max_sync(0xffffffffu, most);
   if ((tid & 31) == 0) s_max[tid >> 5] = most;
+  if (tid == 0) losses[blockIdx.x] = 0;
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 8; ++j) most = max(most, s_max[j]);
-  const bool finite = most < 0x7f800000u;
+  if (most >= 0x7f800000u) {                // an infinity or a NaN: its results are summed in fp32
+    for (int i = tid; 4 * i < Kp; i += 256) {
+      reinterpret_cast<uint2*>(hi)[i] = uint2{0, 0};
+      reinterpret_cast<uint2*>(lo)[i] = uint2{0, 0};
+    }
+    if (tid == 0) { exps[blockIdx.x] = 0; losses[blockIdx.x] = 1; }     // sums of zeros: none of them is trusted
+    return;
+  }
   const int s = min(14 + 127 - (int)(most >> 23), 126);
-  if (tid == 0) exps[blockIdx.x] = finite ? s : kNotFinite;
-  const float scale = finite ? pow2i(s) : 0.f;
+  if (tid == 0) exps[blockIdx.x] = s;
+  const float scale = pow2i(s);
+  const uint32_t small = 2 * __float_as_uint(kWhole / scale) - 1;     // twice the bits drop the sign, and a zero's less one are the largest
   auto store = [&](int i, const float4& v) {
-    const float e[4] = {v.x * scale, v.y * scale, v.z * scale, v.w * scale};
+    const float x[4] = {v.x, v.y, v.z, v.w};
     alignas(8) __half h[4], l[4];
+    uint32_t least = 0xffffffffu;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) { h[j] = __float2half_rn(e[j]); l[j] = __float2half_rn((e[j] - __half2float(h[j])) * (1 << kLoBits)); }
+    for (int j = 0; j < 4; ++j) {
+      const float e = x[j] * scale;
+      h[j] = __float2half_rn(e);
+      l[j] = __float2half_rn((e - __half2float(h[j])) * (1 << kLoBits));
+      least = min(least, 2 * __float_as_uint(x[j]) - 1);
+    }
+    if (least < small) {                    // whole numbers: their sum has no order
+      unsigned long long loss = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = x[j] * scale;
+        if (fabsf(e) < kWhole && x[j] != 0.f)                  // what both terms leave: exact, as the differences are
+          loss += (unsigned long long)ceilf(fmaxf(fabsf(e - __half2float(h[j]) - __half2float(l[j]) * (1.0f / (1 << kLoBits))),
+                                                  fabsf(e) < kGone ? kGone : 0.f) * kLossUnits);
+      }
+      if (loss != 0) atomicAdd(losses + blockIdx.x, loss);
+    }
     reinterpret_cast<uint2*>(hi)[i] = *reinterpret_cast<const uint2*>(h);
     reinterpret_cast<uint2*>(lo)[i] = *reinterpret_cast<const uint2*>(l);
   };
 #pragma unroll
-  for (int j = 0; j < kKept; ++j)
+  for (int j = 0; j < KEPT; ++j)
     if (4 * (tid + 256 * j) < Kp) store(tid + 256 * j, kept[j]);
-  for (int i = tid + 256 * kKept; 4 * i < Kp; i += 256) store(i, load(i));
+  for (int i = tid + 256 * KEPT; 4 * i < Kp; i += 256) store(i, load(i));
 }
 
 // D[tmem] = A * B + 2^-kLoBits D
@@ -117,41 +152,63 @@ struct Tile {
 
 struct Product {
   const float *x, *w, *bias;
-  const int* exps;
+  const int* exps;                          // [M + N]
+  const unsigned long long* losses;         // [M + N]
   float* out;
   int64_t x_rs, out_rs;
   int M, N, K, Kp;
 };
 
+// A warp's rows from m0 on and its lanes' columns n: the results that the terms alone don't settle, in fp32 arithmetic.
+__device__ __noinline__ void sum_again(const Product& p, int m0, int rows, int n, const float* sums, int ld, const float* row_least, float least,
+                                       float bias) {
+  const int lane = threadIdx.x & 31;
+  for (int r = 0; r < rows; ++r) {
+    uint32_t lanes = __ballot_sync(0xffffffffu, n < p.N && fabsf(sums[r * ld]) < row_least[r] + least);
+    const float* x = p.x + (m0 + r) * p.x_rs;
+    while (lanes != 0) {                    // four at a time: their loads do not wait for one another
+      int l[4];
+      float acc[4] = {};
+      const float* w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        l[j] = j > 0 && lanes == 0 ? l[0] : __ffs(lanes) - 1;
+        lanes &= lanes - 1;
+        w[j] = p.w + (int64_t)(n - lane + l[j]) * p.K;
+      }
+#pragma unroll 4
+      for (int k = lane; k < p.K; k += 32) {
+        const float a = x[k];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = fmaf(a, w[j][k], acc[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float sum = warp_sum(acc[j]);
+        if (lane == l[j]) p.out[(m0 + r) * p.out_rs + n] = sum + bias;
+      }
+    }
+  }
+}
+
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
-linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, const Product p) {
+linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
+                  const __grid_constant__ Product p) {
   using L = Tile<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[L::kStages], empty[L::kStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort_v;
   __shared__ int s_ex[kBM];
+  __shared__ float s_least[kBM];            // a result is trusted from here on
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
 
-  int bad = 0;
   for (int i = tid; i < kBM; i += kThreads) {
     s_ex[i] = m0 + i < p.M ? p.exps[m0 + i] : 0;
-    bad |= s_ex[i] == kNotFinite;
-  }
-  for (int i = tid; i < BN; i += kThreads) bad |= n0 + i < p.N && p.exps[p.M + n0 + i] == kNotFinite;
-  if (__syncthreads_or(bad)) {
-    for (int i = tid; i < kBM * BN; i += kThreads) {
-      const int m = m0 + i / BN, n = n0 + i % BN;
-      if (m >= p.M || n >= p.N) continue;
-      const float *xr = p.x + m * p.x_rs, *wr = p.w + (int64_t)n * p.K;
-      float acc = 0.f;
-      for (int k = 0; k < p.K; ++k) acc = fmaf(xr[k], wr[k], acc);
-      p.out[m * p.out_rs + n] = acc + (p.bias ? p.bias[n] : 0.f);
-    }
-    return;
+    s_least[i] = m0 + i < p.M ? trusted_from(p.losses[m0 + i]) : 0.f;
   }
 
   if (warp == 0) tmem_alloc(&s_tmem, L::kCols);
@@ -229,24 +286,31 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       mbar_arrive(&acc_empty[buf]);
     }
     if (ok) {                               // every product is done: the stages' memory is free
-      float* s = reinterpret_cast<float*>(smem) + (warp - 2) * 32 * 33;
+      constexpr int kLd = kMine + 1;
+      static_assert(8 * 32 * kLd * 4 <= L::kStages * L::kStageBytes, "the sums don't fit where the stages were");
+      float* s = reinterpret_cast<float*>(smem) + (warp - 2) * 32 * kLd;
 #pragma unroll
-      for (int c = 0; c < kMine; c += 32) {
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) s[lane * 33 + i] = acc[c + i];
-        __syncwarp();
-        const int n = n0 + side * kMine + c + lane;
+      for (int i = 0; i < kMine; ++i) s[lane * kLd + i] = acc[i];
+      __syncwarp();
+      const int mw = m0 + 32 * quarter, rows = min(32, p.M - mw);
+      const int* ex = s_ex + 32 * quarter;
+      const float row_least = warp_max(s_least[32 * quarter + lane]);
+      for (int c = lane; c < kMine; c += 32) {
+        const int n = n0 + side * kMine + c;
         const bool in = n < p.N;
         const int ew = in ? p.exps[p.M + n] : 0;
+        const float least = in ? trusted_from(p.losses[p.M + n]) : 0.f;
         const float bias = in && p.bias ? p.bias[n] : 0.f;
-        for (int r = 0; r < 32; ++r) {
-          const int m = 32 * quarter + r;
-          if (m0 + m >= p.M) break;
-          const int e = -(s_ex[m] + ew);
-          const float v = s[r * 33 + lane] * pow2i(e / 2) * pow2i(e - e / 2);
-          if (in) p.out[(m0 + m) * p.out_rs + n] = v + bias;
+        float low = INFINITY;
+#pragma unroll 8
+        for (int r = 0; r < rows; ++r) {
+          const float sum = s[r * kLd + c];
+          const int e = -(ex[r] + ew);
+          const float v = sum * pow2i(e / 2) * pow2i(e - e / 2);
+          low = fminf(low, fabsf(sum));
+          if (in) p.out[(int64_t)(mw + r) * p.out_rs + n] = v + bias;
         }
+        if (__any_sync(0xffffffffu, in && low < row_least + least)) sum_again(p, mw, rows, n, s + c, kLd, s_least + 32 * quarter, least, bias);
       }
     }
   }
@@ -307,7 +371,7 @@ using namespace atma;
 
 extern "C" int64_t atma_linear_f32_scratch_bytes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  return round256((int64_t)M * padded(K) * 4) + round256((int64_t)N * padded(K) * 4) + round256(((int64_t)M + N) * 4) + 256;
+  return round256((int64_t)M * padded(K) * 4) + round256((int64_t)N * padded(K) * 4) + round256(((int64_t)M + N) * 4) + round256(((int64_t)M + N) * 8) + 256;
 }
 
 extern "C" int atma_linear_f32(const float* x, int64_t x_rs, const float* w, const float* bias, float* out, int64_t out_rs, int M, int N,
@@ -322,12 +386,15 @@ extern "C" int atma_linear_f32(const float* x, int64_t x_rs, const float* w, con
   __half* xp = reinterpret_cast<__half*>(at);
   __half* wp = reinterpret_cast<__half*>(at + round256((int64_t)M * Kp * 4));
   int* exps = reinterpret_cast<int*>(at + round256((int64_t)M * Kp * 4) + round256((int64_t)N * Kp * 4));
+  auto* losses = reinterpret_cast<unsigned long long*>(reinterpret_cast<uint8_t*>(exps) + round256(((int64_t)M + N) * 4));
   const bool vec = K % 4 == 0 && x_rs % 4 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
-  if (vec) split_rows_kernel<true><<<M + N, 256, 0, st>>>(x, x_rs, M, w, N, K, Kp, xp, wp, exps);
-  else split_rows_kernel<false><<<M + N, 256, 0, st>>>(x, x_rs, M, w, N, K, Kp, xp, wp, exps);
+#define ATMA_SPLIT(VEC, KEPT) split_rows_kernel<VEC, KEPT><<<M + N, 256, 0, st>>>(x, x_rs, M, w, N, K, Kp, xp, wp, exps, losses)
+  if (vec) { if (Kp <= 1024) ATMA_SPLIT(true, 1); else ATMA_SPLIT(true, 4); }
+  else { if (Kp <= 1024) ATMA_SPLIT(false, 1); else ATMA_SPLIT(false, 4); }
+#undef ATMA_SPLIT
   int rc = launch_status("linear_f32 (split)");
   if (rc != ATMA_OK) return rc;
-  const Product p{x, w, bias, exps, out, x_rs, out_rs, M, N, K, Kp};
+  const Product p{x, w, bias, exps, losses, out, x_rs, out_rs, M, N, K, Kp};
   if (bn == 256) return launch<256>(p, xp, wp, st);
   if (bn == 128) return launch<128>(p, xp, wp, st);
   return launch<64>(p, xp, wp, st);

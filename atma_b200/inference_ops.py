@@ -375,7 +375,12 @@ def linear_f32_supported(x, weight, bias=None):
 
 def linear_f32(x, weight, bias=None, out=None, lib=None):
     """x @ weight.T + bias in fp32 on the tensor cores: x (..., K) fp32, weight (N, K) contiguous.  ``out`` (rows, N):
-    where the result goes (contiguous rows, any row stride); ``lib``: as for ``decode_linear``."""
+    where the result goes (contiguous rows, any row stride); ``lib``: as for ``decode_linear``.
+
+    Each factor is two fp16 terms, so a product is right to 2^-21 of itself and a result to about 2^-20 of the sum of its
+    products' sizes, besides the sums' own rounding, whatever the range of values in a row (the library's fp32 sums are off by
+    more at K = 1024).  Results that a row's smaller values could change by more than the terms hold of them, and those of
+    rows with an infinity or a NaN, are summed in fp32: correct, and slower than the library where most of them are."""
     _lib.require_cuda(x, "linear_f32")
     lib = _lib.load() if lib is None else lib
     K, N = x.shape[-1], weight.shape[0]
@@ -401,7 +406,8 @@ def linear_f32(x, weight, bias=None, out=None, lib=None):
 
 
 def linear(x, weight, bias=None):
-    """x @ weight.T + bias: fp32 rows in numbers through ``linear_f32``, the library's product otherwise."""
+    """x @ weight.T + bias: fp32 rows in numbers through ``linear_f32`` (see there for its error), the library's product
+    otherwise."""
     if linear_f32_supported(x, weight, bias):
         return linear_f32(x, weight, bias)
     return F.linear(x, weight, bias)

@@ -230,8 +230,11 @@ int atma_qkv_prep_decode(const void* q_gate, int64_t qg_row, int64_t qg_head, co
 int atma_add_rms_norm(const void* x, const void* y, const void* weight, void* x_out, void* h_out, int rows, int D,
                       float eps, int dtype, void* stream);
 
-/* fp32 linear layer on the tensor cores at fp32 accuracy: out[m][n] = sum_k x[m][k] * w[n][k] + bias[n] (bias may be
- * NULL); x rows and out rows with strides in elements, w [N][K] dense.  scratch: atma_linear_f32_scratch_bytes() bytes. */
+/* fp32 linear layer on the tensor cores: out[m][n] = sum_k x[m][k] * w[n][k] + bias[n] (bias may be NULL, else N values).
+ * Products are right to 2^-21 of themselves, whatever the range of values in a row; results are off by about 2^-20 of the sum
+ * of |x| |w| at most, besides the rounding of fp32 sums.  Results that the two fp16 terms of each factor do not settle (rows
+ * with an infinity or a NaN; large values that meet zeros and values 2^28 times smaller that do not) are summed in fp32.
+ * x rows and out rows with strides in elements, w [N][K] dense.  scratch: atma_linear_f32_scratch_bytes() bytes. */
 int atma_linear_f32(const float* x, int64_t x_row_stride, const float* w, const float* bias, float* out, int64_t out_row_stride,
                     int M, int N, int K, void* scratch, void* stream);
 int64_t atma_linear_f32_scratch_bytes(int M, int N, int K);

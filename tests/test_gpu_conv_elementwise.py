@@ -368,11 +368,18 @@ def test_decode_linear_rejects_what_it_does_not_serve():
     assert atma_b200.device_status() == 0
 
 
+def _product_bound(x, w):
+    """Two terms of each factor are right to 2^-23, the smallest product left out is 2^-22 of a product, the tensor core cuts off
+    at 2^-23 in each of a chunk's four large products: 2^-20.  The chunks' sums, or where fp32 arithmetic takes over 32 lanes' of
+    K / 32 products and then theirs, are rounded to 2^-24 each.  Subnormal results: half a unit for each."""
+    K = x.shape[1]
+    return x.double().abs() @ w.double().abs().t() * (2 ** -20 + (K / 32 + 6) * 2 ** -24) + (K + 1) * 2.0 ** -149
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 1, 1), (128, 64, 64), (129, 65, 63), (127, 4100, 257), (300, 1027, 130), (2000, 128, 2049)])
 @pytest.mark.parametrize("spread", [0.0, 4.0])
 def test_linear_f32(M, K, N, spread):
-    """Edges of tiles and planes, strided and unaligned rows, values of very different size in one row.  A product's terms
-    are right to 2^-22 and 2^-51 of their row's largest value, and fp32 sums add a few units of 2^-24."""
+    """Edges of tiles and planes, strided and unaligned rows, values of very different size in one row."""
     from atma_b200.inference_ops import linear_f32
     g = torch.Generator().manual_seed(M + K)
     wide = lambda *s: torch.randn(*s, generator=g) * torch.exp(torch.randn(*s, generator=g) * spread)      # noqa: E731
@@ -380,8 +387,7 @@ def test_linear_f32(M, K, N, spread):
     out = torch.full((M, N + 5), 7.0, device="cuda")
     y = linear_f32(x, w, b, out=out[:, 2:N + 2])
     xd, wd = x.double(), w.double()
-    bound = xd.abs() @ wd.abs().t() * 2 ** -20 + b.abs() * 2 ** -23
-    bound = bound + 2 ** -50 * (xd.abs().amax(1, True) * wd.abs().sum(1) + xd.abs().sum(1, True) * wd.abs().amax(1))
+    bound = _product_bound(x, w) + b.abs() * 2 ** -23
     assert ((y - (xd @ wd.t() + b)).abs() <= bound).all()
     assert (out[:, :2] == 7).all() and (out[:, N + 2:] == 7).all()
     assert torch.equal(linear_f32(x.contiguous(), w, b), y)
@@ -389,6 +395,33 @@ def test_linear_f32(M, K, N, spread):
     x[M // 2, 0], w[N // 2, K // 2] = float("inf"), float("nan")
     odd, want = linear_f32(x, w), (x.double() @ w.double().t())
     assert torch.equal(odd.isnan(), want.isnan()) and torch.equal(odd.isinf(), want.isinf())
+    assert atma_b200.device_status() == 0
+
+
+@pytest.mark.parametrize("small", [2.0 ** -20, 2.0 ** -27, 2.0 ** -29, 2.0 ** -37, 2.0 ** -51, 1e-30, 1e-44])
+@pytest.mark.parametrize("M,K,N", [(5, 3, 7), (130, 1024, 300), (257, 5000, 65)])
+def test_linear_f32_large_values_that_meet_zeros(M, K, N, small):
+    """A row's largest value times a zero, and small ones that make the result: to fp32 accuracy, whatever the distance between
+    them (subnormal results to half of their unit).  The same for a row of weights, and for rows where it is the other way round."""
+    from atma_b200.inference_ops import linear_f32
+    g = torch.Generator().manual_seed(K)
+    x, w = torch.randn(M, K, generator=g), torch.randn(N, K, generator=g)
+    x[::2, 1:] *= small
+    x[::2, 0] = 1.2345678
+    w[::3, 0] = 0                                                         # those rows' results come from the small values alone
+    w[1::3, 1:] *= small
+    x[1::4, 0] = 0
+    for scale in (1.0, 2.0 ** 60, 2.0 ** -60):
+        xs, ws = (x * scale).cuda(), w.cuda()
+        y, xd, wd = linear_f32(xs, ws), xs.double(), ws.double()
+        assert ((y - xd @ wd.t()).abs() <= _product_bound(xs, ws)).all()
+    for a, b in ((x, w), (w, x)):
+        a, b = a.clone(), b.clone()
+        a[0, K // 2], a[a.shape[0] // 2] = float("inf"), float("nan")
+        y, want = linear_f32(a.cuda(), b.cuda()).cpu(), a.double() @ b.double().t()
+        assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+        rest = want.isfinite()
+        assert ((y - want).abs() <= _product_bound(a, b))[rest].all()
     assert atma_b200.device_status() == 0
 
 
