@@ -132,11 +132,16 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a) {
       m[i] = mn;
       times<VM>(acc[i], al);
     }
-    // keys that some row of this warp sees: nothing beyond them enters its sums
-    const int j1 = min(min(kN, k_limit - k0), (int)fminf(fmaxf(ceilf(hi - koff) - (float)k0, 0.f), (float)kN));
-    const int j0 = a.window > 0 ? (int)fminf(fmaxf(lo - (float)a.window - koff - (float)k0, 0.f), (float)kN) & ~3 : 0;
+    // keys that some of the warp's rows see (j0 to j1 - 1) and those that all of them do (f0 to f1 - 1)
+    auto within = [&](float key) { return (int)fminf(fmaxf(key - koff - (float)k0, 0.f), (float)kN); };
+    const int j1 = min(min(kN, k_limit - k0), within(ceilf(hi))), f1 = min(j1, within(ceilf(lo)));
+    const int j0 = a.window > 0 ? within(lo - (float)a.window) & ~3 : 0, f0 = a.window > 0 ? (within(ceilf(hi) - (float)a.window) + 3) & ~3 : 0;
+    auto sees = [&](int i, int j) {
+      const float pos = (float)(k0 + j) + koff;
+      return pos < n[i] && (a.window <= 0 || pos >= n[i] - (float)a.window);
+    };
     copies_done();
-    weigh<VM>(sP, sKV, ty, tx, j0, j1, acc);
+    weigh<VM>(sP, sKV, ty, tx, j0, j1, f0, f1, sees, acc);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 

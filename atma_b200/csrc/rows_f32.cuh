@@ -75,12 +75,37 @@ __device__ __forceinline__ void dots(const float* q, const float* k, int ld, int
   }
 }
 
-// acc[i][.] += sum over keys j0 .. j1 - 1 (j0 a multiple of 4) of p[4 ty + i][j] v[j][.]
-template <int VM>
-__device__ __forceinline__ void weigh(const float* p, const float* v, int ty, int tx, int j0, int j1, uint64_t (&acc)[4][2 * VM]) {
+// acc[i][.] += sum over keys j0 .. j1 - 1 of p[4 ty + i][j] v[j][.].  Every row of the warp sees the keys from f0 to f1 - 1 (f0 a
+// multiple of 4 if there are four of them); for the others sees(i, j) tells, and a value that a row does not see stays out of
+// its sums, be it infinite or no number at all.  Edges are short, so their keys go one by one.
+template <int VM, typename Sees>
+__device__ __forceinline__ void weigh(const float* p, const float* v, int ty, int tx, int j0, int j1, int f0, int f1, Sees sees,
+                                      uint64_t (&acc)[4][2 * VM]) {
   const float* pr = p + 4 * ty * kLdP;
+  auto add = [&](int i, float f, const ulonglong2 (&x)[VM]) {
+    const uint64_t ff = pack2(f, f);
+#pragma unroll
+    for (int m = 0; m < VM; ++m) {
+      acc[i][2 * m] = fma2(x[m].x, ff, acc[i][2 * m]);
+      acc[i][2 * m + 1] = fma2(x[m].y, ff, acc[i][2 * m + 1]);
+    }
+  };
+  auto edge = [&](int from, int to) {
 #pragma unroll 1
-  for (int j = j0; j < j1; j += 4) {
+    for (int j = from; j < to; ++j) {
+      ulonglong2 x[VM];
+#pragma unroll
+      for (int m = 0; m < VM; ++m) x[m] = *reinterpret_cast<const ulonglong2*>(v + j * 64 * VM + 64 * m + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (sees(i, j)) add(i, pr[i * kLdP + j], x);
+    }
+  };
+  f0 = min(max(f0, j0), j1);
+  f1 = f0 + max(min(f1, j1) - f0, 0) / 4 * 4;
+  edge(j0, f0);
+#pragma unroll 1
+  for (int j = f0; j < f1; j += 4) {
     float4 w[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(pr + i * kLdP + j);
@@ -90,17 +115,10 @@ __device__ __forceinline__ void weigh(const float* p, const float* v, int ty, in
 #pragma unroll
       for (int m = 0; m < VM; ++m) x[m] = *reinterpret_cast<const ulonglong2*>(v + (j + e) * 64 * VM + 64 * m + 4 * tx);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float f = e == 0 ? w[i].x : (e == 1 ? w[i].y : (e == 2 ? w[i].z : w[i].w));
-        const uint64_t ff = pack2(f, f);
-#pragma unroll
-        for (int m = 0; m < VM; ++m) {
-          acc[i][2 * m] = fma2(x[m].x, ff, acc[i][2 * m]);
-          acc[i][2 * m + 1] = fma2(x[m].y, ff, acc[i][2 * m + 1]);
-        }
-      }
+      for (int i = 0; i < 4; ++i) add(i, e == 0 ? w[i].x : (e == 1 ? w[i].y : (e == 2 ? w[i].z : w[i].w)), x);
     }
   }
+  edge(f1, j1);
 }
 
 // over the 16 threads of a row

@@ -5,7 +5,7 @@
 // There a lane owns one key and a warp two rows: two loads from shared memory for two FMAs.  Here a thread owns 4 x 4 scores
 // and 4 rows x 4 VM channels (rows_f32.cuh), so that FMAs and shared memory are both busy; K and V take turns in one buffer,
 // V under the statistics, and two CTAs share an SM, one loading while the other computes.  Later rows have more keys, so
-// those of all heads come first.  Measured, 1500 rows, 8 heads, two maps of 64, 128 value channels: 1089 -> 549 us (679 with
+// those of all heads come first.  Measured, 1500 rows, 8 heads, two maps of 64, 128 value channels: 1089 -> 534 us (679 with
 // the heads one after another).
 #include "rows_f32.cuh"
 #include "softmax_attention.cuh"
@@ -83,9 +83,12 @@ softmax_rows_f32_kernel(const atma_softmax_args a) {
     __syncthreads();                           // the last tile's V is read
     fetch(K, kd, kd, ld);
     copies_done();
-    // columns that some row of the warp may see: nothing beyond them enters its sums
-    const int j1 = min(min(kN, n_keys - k0), first_pos + 8 - k0);
-    const int j0 = k0 >= a.keep_first ? max(0, first_pos - a.window + 1 - k0) & ~3 : 0;
+    // columns that some of the warp's rows see (j0 to j1 - 1) and those that all of them do (f0 to f1 - 1)
+    const int kept = a.keep_first - k0, opens = first_pos - a.window + 1 - k0;
+    int j1 = min(min(kN, n_keys - k0), first_pos + 8 - k0);
+    if (kept > 0 && opens >= kN) j1 = min(j1, kept);
+    const int j0 = kept > 0 ? 0 : max(opens, 0) & ~3, f1 = min(j1, first_pos + 1 - k0), f0 = kept >= f1 ? 0 : (opens + 7 + 3) & ~3;
+    auto sees = [&](int i, int j) { return key_visible(start + q0 + 4 * ty + i, k0 + j, a.window, a.keep_first); };
 #pragma unroll
     for (int t = 0; t < M; ++t) {
       float sc[4][4];
@@ -120,7 +123,7 @@ softmax_rows_f32_kernel(const atma_softmax_args a) {
     }
     copies_done();
 #pragma unroll
-    for (int t = 0; t < M; ++t) weigh<VM>(sP + t * kM * kLdP, sKV, ty, tx, j0, j1, acc[t]);
+    for (int t = 0; t < M; ++t) weigh<VM>(sP + t * kM * kLdP, sKV, ty, tx, j0, j1, f0, f1, sees, acc[t]);
   }
 
   const bool vec = a.out_rs % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;

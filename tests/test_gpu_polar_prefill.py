@@ -229,7 +229,7 @@ def test_tensor_core_path_is_taken_and_no_wait_ran_out():
 @pytest.mark.parametrize("window", [None, 37])
 def test_fp32_tiles_of_rows_against_short_calls(Tq, Tk, H, Hkv, dk, window):
     """The 64-row kernel against the 32-row kernel on the same rows in portions, whose key counts are not in order; both sum
-    at most 200 fp32 terms in their own order."""
+    at most 200 fp32 terms in their own order.  Infinite values reach the rows that see them and no others."""
     q, k, v = rand((2, H, Tq, dk), 1).cuda(), rand((2, Hkv, Tk, dk), 2).cuda(), rand((2, Hkv, Tk, dk), 3).cuda()
     n = (torch.arange(Tq) * 37 % Tk + 1).float().cuda()
     p = dict(v_null=rand((H, dk), 4).cuda(), null_base=rand((H,), 5).cuda(), null_slope_raw=rand((H,), 6).cuda(), len_gain_raw=rand((H,), 7).cuda(),
@@ -239,3 +239,12 @@ def test_fp32_tiles_of_rows_against_short_calls(Tq, Tk, H, Hkv, dk, window):
         s = slice(a, a + 32)
         wc, wm = atma_b200.polar_attention_fwd(q[:, :, s].contiguous(), k, v, n[s].contiguous(), window=window, is_causal=False, **p)
         assert max_rel(c[:, :, s], wc) < 1e-5 and max_rel(mag[:, :, s], wm) < 1e-5
+    for counts in (n, torch.arange(Tk - Tq + 1, Tk + 1).float().cuda()):
+        call = lambda: atma_b200.polar_attention_fwd(q, k, v, counts, window=window, is_causal=False, **p)[0]
+        c = call()
+        for at in {0, 3, Tk // 2, max(Tk - 66, 0), Tk - 4, Tk - 1}:
+            kept = v.clone()
+            v[:, :, at] = float("inf")
+            got, unseen = call(), (counts <= at) | (counts - (window or Tk) > at)
+            assert torch.equal(got[:, :, unseen], c[:, :, unseen]) and not got[:, :, ~unseen].isfinite().all(-1).any(), at
+            v.copy_(kept)

@@ -427,8 +427,9 @@ def test_saved_folder_command_line_and_replay(tmp_path, capsys, monkeypatch):
 @pytest.mark.parametrize("window,keep", [(EVERY, 0), (40, 3), (65, 70)])
 @pytest.mark.parametrize("rows,start", [(33, 0), (64, 1), (65, 63), (200, 130)])
 def test_fp32_tiles_of_rows_against_short_steps(H, G, maps, dim, vdim, window, keep, rows, start):
-    """The 64-row kernel on a prompt against the 16-row kernel on the same rows in portions of 32: edges of tiles, windows
-    and kept keys.  Both sum at most 330 fp32 terms in their own order.  An infinite value stays behind the rows in front."""
+    """The 64-row kernel on a prompt against 64 bits, and against the 16-row kernel on the same rows in portions of 32: edges of
+    tiles, windows and kept keys.  Both sum at most 330 fp32 terms in their own order.  Infinite values reach the rows that see
+    them and no others."""
     n = rows + start
     q, kc, vc = rand((rows, H, maps, dim), 1), rand((8, 64, G, maps * dim), 2), rand((8, 64, G, vdim), 3)
     q, kc, vc = q.cuda(), kc.cuda(), vc.cuda()
@@ -445,5 +446,20 @@ def test_fp32_tiles_of_rows_against_short_steps(H, G, maps, dim, vdim, window, k
         b = min(a + 32, rows)
         ops().softmax_prefill(q[a:b], kc, vc, group([b - a], [start + a], [0], table), want[a:b], **{**kw, "gate": kw["gate"][a:b]})
     assert max_rel(out, want) < 1e-5
-    vc[table[0][(n - 1) // 64], (n - 1) % 64] = float("inf")
-    assert torch.equal(whole()[:max(rows - 12, 0)], out[:max(rows - 12, 0)])
+    pos, key = torch.arange(start, n, device="cuda")[:, None], torch.arange(n, device="cuda")[None]
+    see = (key <= pos) & ((pos - key < window) | (key < keep))
+    k, v = (c[table[0]].flatten(0, 1)[:n].double().view(n, G, -1).repeat_interleave(H // G, 1) for c in (kc, vc))
+    o = 0
+    for m in range(maps):
+        s = torch.einsum("thd,nhd->htn", q[:, :, m].double(), k.view(n, H, maps, dim)[:, :, m]) * kw["scale"]
+        s = torch.cat([s.masked_fill(~see, float("-inf")), torch.full((H, rows, 1), kw["sink"], device="cuda", dtype=torch.float64)], -1)
+        o = o + (1.0 if m == 0 else -kw["lam"]) * torch.einsum("htn,nhd->thd", s.softmax(-1)[..., :n], v)
+    if maps == 2:
+        o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + kw["eps"]) * kw["out_scale"]
+    assert max_rel(out, o.flatten(1) * torch.sigmoid(kw["gate"].double())) < 1e-5
+    for at in {min(max(i, 0), n - 1) for i in (n - 1, n - 4, n - 70, start, keep, keep - 1, 0)}:
+        kept = vc.clone()
+        vc[table[0][at // 64], at % 64] = float("inf")
+        got, unseen = whole(), ~see[:, at]
+        assert torch.equal(got[unseen], out[unseen]) and not got[~unseen].isfinite().all(1).any(), at
+        vc.copy_(kept)
