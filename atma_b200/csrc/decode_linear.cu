@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "early.cuh"
+#include "gelu.cuh"
 #include "mma_sync.cuh"
 
 namespace atma {
@@ -158,8 +159,7 @@ decode_linear_kernel(const LinArgs a) {
     }
     float v = y[0];
     if constexpr (kGated == 2) {
-      const float z = y[0];
-      v = 0.5f * z * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z))) * y[1];
+      v = gelu_tanh_16(y[0]) * y[1];
     } else if constexpr (kGated == 1) {
       const float p = fmaxf(y[0], 0.f);
       float sq = p * p;

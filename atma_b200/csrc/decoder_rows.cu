@@ -1,8 +1,9 @@
 // Row operations of the decoder models: token + bigram and token + learned-position embeddings, the fp32 residual
 // stream with RMS norms of the stream or of what a sublayer adds to it, the feed-forward activations and the per-head
 // norm with a silu gate.  Everything is one pass over rows, 16 bytes per thread and access where the shapes allow it.
-#include "early.cuh"
 #include "common.cuh"
+#include "early.cuh"
+#include "gelu.cuh"
 #include "../../include/atma_decoder.h"
 
 namespace atma {
@@ -307,27 +308,6 @@ bias_squared_relu_kernel(const T* z, int64_t z_rs, const T* __restrict__ bias, T
 }
 
 // ---- gelu_tanh(gate) * up ---------------------------------------------------------------------------
-__device__ __forceinline__ float gelu_tanh(float z) {
-  const float c = 0.7978845608028654f;                    // sqrt(2 / pi)
-  return 0.5f * z * (1.0f + tanhf(c * fmaf(0.044715f * z * z, z, z)));
-}
-
-// For results that are rounded to 16 bits: the same as z / (1 + e^-2u) by the fast exponential and division (a few fp32 units in
-// the last place, and no cancellation below zero).  tanhf's instructions, not the 805 MB, set the time of 32768 x 4096: 160 us,
-// 118 now (6.8 TB/s).
-template <typename T>
-__device__ __forceinline__ float gelu_tanh_for(float z) {
-  if constexpr (sizeof(T) == 2) {
-    const float u = 0.7978845608028654f * fmaf(0.044715f * z * z, z, z);
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-2.0f * 1.4426950408889634f * u));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));        // infinity -> 0
-    return z * r;
-  } else {
-    return gelu_tanh(z);
-  }
-}
-
 template <typename T, int VEC>
 __global__ void gelu_gate_kernel(const T* __restrict__ gate, int64_t gate_rs, const T* __restrict__ up, int64_t up_rs,
                                  T* __restrict__ out, int64_t out_rs, int width) {
@@ -338,7 +318,10 @@ __global__ void gelu_gate_kernel(const T* __restrict__ gate, int64_t gate_rs, co
   const Pack<T, VEC> u = *reinterpret_cast<const Pack<T, VEC>*>(up + row * up_rs + c);
   Pack<T, VEC> o;
 #pragma unroll
-  for (int e = 0; e < VEC; ++e) o.e[e] = from_f32<T>(gelu_tanh_for<T>(to_f32(g.e[e])) * to_f32(u.e[e]));
+  for (int e = 0; e < VEC; ++e) {
+    const float z = to_f32(g.e[e]);
+    o.e[e] = from_f32<T>((sizeof(T) == 2 ? gelu_tanh_16(z) : gelu_tanh(z)) * to_f32(u.e[e]));
+  }
   *reinterpret_cast<Pack<T, VEC>*>(out + row * out_rs + c) = o;
 }
 

@@ -1,9 +1,12 @@
 """GPU: every mechanism of the Rizurax decoder against the plain oracle, then the whole model through the engine -
 prompts, portions, decoding, unequal batches, reused pages and slots, generation."""
 
+import math
+
 import pytest
 import torch
 
+import atma_b200
 from oracle import rizurax as R
 from tests.conftest import max_abs, max_rel
 from tests.gpu_util import rand
@@ -70,6 +73,36 @@ def test_gelu_gate(dtype, rows, width):
     ops().gelu_gate(g[:, :width], g[:, width:], out[:, 8:])
     want = R.gelu_tanh(gu[:, :width].double()) * gu[:, width:].double()
     assert max_rel(out[:, 8:], want) < (1e-6 if dtype == F32 else 6e-3) and out[:, :8].abs().max() == 0
+
+
+@pytest.mark.parametrize("dtype", [BF16, torch.float16])
+def test_gelu_over_all_16_bit_values(dtype):
+    """Every value there is, infinities and NaN among them, against 64 bits: half a unit in the last of 8 or 11 bits (2^-8,
+    2^-11), the stated error of the fast form (4 + 1.18 |2 u| units of 2^-23), and what may become zero: half the smallest fp16 value, |z| 2^-126 at
+    z = -11.3 from where the division gives zero.  A decoding step's gate is a prompt's, bit for bit."""
+    z = torch.arange(-2 ** 15, 2 ** 15, dtype=torch.int32).to(torch.int16).view(dtype).cuda()
+    zd = z.double()
+    u2 = 2 * math.sqrt(2 / math.pi) * (zd + 0.044715 * zd ** 3)
+    want = zd * torch.sigmoid(u2)                                        # 0.5 z (1 + tanh u) without its cancellation
+    w = torch.zeros(2 * z.numel(), 32, dtype=dtype, device="cuda")       # features [z | 1] from x = (1, 0, ...)
+    finite = z.isfinite()
+    w[:z.numel(), 0], w[z.numel():, 0] = torch.where(finite, z, torch.zeros_like(z)), 1
+    x = torch.zeros(3, 32, dtype=dtype, device="cuda")
+    x[:, 0] = 1
+    step = atma_b200.decode_linear(x, w, gated="gelu_tanh")
+    assert torch.equal(step[0], step[1]) and torch.equal(step[0], step[2])
+    results = [step[0][finite]]
+    if dtype == BF16:
+        gate = torch.empty(1, z.numel(), dtype=dtype, device="cuda")
+        ops().gelu_gate(z[None], torch.ones_like(z)[None], gate)
+        assert torch.equal(gate[0][finite], step[0][finite])
+        assert gate[0][z == float("inf")].item() == float("inf") and gate[0][z.isnan()].isnan().all()
+        results.append(gate[0][finite])
+    want, u2 = want[finite], u2[finite]
+    fast = (4 + 1.18 * u2.abs().clamp(max=100)) * 2.0 ** -23
+    bound = want.abs() * ((2.0 ** -8 if dtype == BF16 else 2.0 ** -11) + fast) + (11.3 * 2.0 ** -126 if dtype == BF16 else 2.0 ** -25)
+    for got in results:
+        assert ((got.double() - want).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("rows,n,k", [(1, 64, 96), (16, 128, 256), (9, 96, 64), (40, 128, 256), (3, 42, 45)])
