@@ -7,7 +7,10 @@
 //   rhs_i = beta_i (v_i - e_i S^T k_i)     A_ij = beta_i P_ij k_i.k_j (j < i)     T = (I + A)^-1
 //   o_i   = e_i S^T q_i + sum_{j<=i} R'_ij rhs_j        R' = (P_ij q_i.k_j, j <= i) T
 //   S     <- e_7 S + sum_j k'_j rhs_j^T                 k'_j = sum_{i>=j} P_7i T_ij k_i
-// Kernel 1 makes T's products R' and k' of every block, side by side; kernel 2 walks the blocks.  There a warp owns four
+// Kernel 1 makes T's products R' and k' of every block, side by side; kernel 2 walks the blocks.  Records take 1.6 KB per row and
+// head of 128, so inputs whose records would take over 1 GB (85000 rows of 8 heads) go in portions, and the one sequence that a
+// portion's end cuts hands its state on in the scratch.  Smaller portions would put sequences one behind the other that
+// can be walked side by side (128 MB: 4 x 8192 rows 3.3 ms instead of 1.6).  In kernel 2 a warp owns four
 // state columns, 16 lanes x DK / 16 rows for two of them; of the 16 products with k_i and q_i each lane ends up with one
 // (halving exchange), the right sides go round once, and the update needs nothing else.  Bound by issue slots: about 60
 // per row and warp, FMAs in pairs (f32x2).  Blocks of 16 rows would double the exchange and the factor work per row.
@@ -27,6 +30,7 @@ constexpr int kN = 8;                       // rows of a block
 constexpr int kExtra = 96;                  // floats behind a record's vectors: R' [8][8] | e [8] | beta [8] | pad
 constexpr int kAtE = kN * kN, kAtBeta = kAtE + kN;
 constexpr int kStages = 4;
+constexpr int64_t kMostBytes = 1 << 30;      // of the records that are there at a time
 
 __host__ __device__ constexpr int record_floats(int DK) { return 3 * kN * DK + kExtra; }
 // records in front of sequence s, whose first row is r0: enough for every sequence before it, without counting them
@@ -39,12 +43,19 @@ __device__ __forceinline__ Rows rows_of(const DeltaBlocks& a, int s) {
   return {r0, a.cu_rows[s + 1] - r0};
 }
 
+// A portion's first record, and the states [H][dk][dv] that come in and go out where a sequence is cut.
+struct Cut {
+  int64_t first;
+  const float* carry_in;
+  float* carry_out;
+};
+
 template <typename T, int DK>
 __global__ void __launch_bounds__(128)
-delta_blocks_factors_kernel(const DeltaBlocks a, float* __restrict__ recs, int64_t n_records) {
+delta_blocks_factors_kernel(const DeltaBlocks a, float* __restrict__ recs, int64_t n_records, int64_t first) {
   __shared__ __align__(16) float K[kN][DK + 4], Q[kN][DK + 4];
   __shared__ float g[kN], bt[kN], A[kN][kN], Rq[kN][kN], Tm[kN][kN];
-  const int64_t idx = blockIdx.x;
+  const int64_t idx = first + blockIdx.x;
   const int h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int lo = 0, hi = a.n_seqs - 1;            // the last sequence whose records begin at or before idx
   while (lo < hi) {
@@ -56,7 +67,7 @@ delta_blocks_factors_kernel(const DeltaBlocks a, float* __restrict__ recs, int64
   if (at < 0 || at >= seq.n) return;
   const int valid = min((int64_t)kN, seq.n - at);
   const int64_t row0 = seq.r0 + at;
-  float* rec = recs + ((int64_t)h * n_records + idx) * record_floats(DK);
+  float* rec = recs + ((int64_t)h * n_records + blockIdx.x) * record_floats(DK);
   const int hq = h / (a.H / a.Hq), hk = h / (a.H / a.G);
 
 #pragma unroll
@@ -153,28 +164,41 @@ delta_blocks_factors_kernel(const DeltaBlocks a, float* __restrict__ recs, int64
   }
 }
 
-template <typename T, int DK, int W>
+// CUT: one of several portions (5% slower, so not where there is one only).
+template <typename T, int DK, int W, bool CUT>
 __global__ void __launch_bounds__(W * 32)
-delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, int64_t n_records) {
+delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, int64_t n_records, const Cut p) {
   extern __shared__ __align__(16) float ring[];
   constexpr int R4 = DK / 64, kRec = record_floats(DK);        // quadruples of rows per lane
   const int tid = threadIdx.x, lane = tid & 31, l = lane & 15, half = lane >> 4;
   const int h = blockIdx.y, s = blockIdx.z;
   const int col = (blockIdx.x * W + (tid >> 5)) * 4 + half * 2;
   const bool c0 = col < a.dv, c1 = col + 1 < a.dv;
-  const Rows seq = rows_of(a, s);
+  Rows seq = rows_of(a, s);
+  int64_t record = first_record(seq.r0, s);            // that it begins with in this portion
+  int blocks = (seq.n + kN - 1) / kN;                  // it has there
+  bool begun = false, ends = true;                     // portions in front have rows of it; there are none behind
+  if constexpr (CUT) {
+    const int64_t ahead = record - p.first;
+    const int b0 = (int)max(-ahead, (int64_t)0), b1 = (int)min(n_records - ahead, (int64_t)blocks);
+    if (blocks == 0 ? ahead < 0 || ahead >= n_records : b0 >= b1) return;
+    begun = b0 > 0; ends = b1 == blocks;
+    blocks = b1 - b0;
+    record = ahead + b0;
+    seq.r0 += (int64_t)b0 * kN; seq.n -= b0 * kN;
+  }
   const int start = a.start_pos ? a.start_pos[s] : 1;
   const int64_t slot = a.slots ? a.slots[s] : s;
   T* o = static_cast<T*>(a.o) + (seq.r0 * a.H + h) * a.dv + col;
   const int64_t o_rs = (int64_t)a.H * a.dv;
   if (start < 0 || slot < 0) {
-    for (int r = l; r < seq.n; r += 16) {
+    for (int r = l; r < (CUT ? min(blocks * kN, seq.n) : seq.n); r += 16) {
       if (c0) o[r * o_rs] = from_f32<T>(0.f);
       if (c1) o[r * o_rs + 1] = from_f32<T>(0.f);
     }
     return;
   }
-  const int64_t plane = slot * a.state_ss + (int64_t)h * a.dk * a.dv + col;
+  const int64_t carry = (int64_t)h * a.dk * a.dv + col, plane = slot * a.state_ss + carry;
   uint64_t S[2][2 * R4];                    // [column][pair of rows]: rows 64 m + 4 l .. + 3
 #pragma unroll
   for (int m = 0; m < 2 * R4; ++m) {
@@ -182,17 +206,17 @@ delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, in
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int row = 64 * (m >> 1) + 4 * l + 2 * (m & 1) + e;
-      const float* p = a.state_in + plane + (int64_t)row * a.dv;
-      const bool ok = a.state_in != nullptr && start > 0 && row < a.dk;
-      x[0][e] = ok && c0 ? p[0] : 0.f;
-      x[1][e] = ok && c1 ? p[1] : 0.f;
+      const float* src = (begun ? p.carry_in + carry : a.state_in + plane) + (int64_t)row * a.dv;
+      const bool ok = (begun || (a.state_in != nullptr && start > 0)) && row < a.dk;
+      x[0][e] = ok && c0 ? src[0] : 0.f;
+      x[1][e] = ok && c1 ? src[1] : 0.f;
     }
     S[0][m] = pack2(x[0][0], x[0][1]);
     S[1][m] = pack2(x[1][0], x[1][1]);
   }
 
-  const float* rec = recs + ((int64_t)h * n_records + first_record(seq.r0, s)) * kRec;
-  const int NB = (seq.n + kN - 1) / kN;
+  const float* rec = recs + ((int64_t)h * n_records + record) * kRec;
+  const int NB = CUT ? blocks : (seq.n + kN - 1) / kN;
   auto stage = [&](int b) {
     if (b < NB) {
       const float* src = rec + (int64_t)b * kRec;
@@ -291,36 +315,50 @@ delta_blocks_walk_kernel(const DeltaBlocks a, const float* __restrict__ recs, in
     v_now = v_next; v_next = v_after;
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  if (a.state_out == nullptr) return;
+  if (ends && a.state_out == nullptr) return;
+  float* to = ends ? a.state_out + plane : p.carry_out + carry;
 #pragma unroll
   for (int m = 0; m < 2 * R4; ++m) {
     const float2 f0 = unpack2(S[0][m]), f1 = unpack2(S[1][m]);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int row = 64 * (m >> 1) + 4 * l + 2 * (m & 1) + e;
-      float* p = a.state_out + plane + (int64_t)row * a.dv;
-      if (row < a.dk && c0) p[0] = e ? f0.y : f0.x;
-      if (row < a.dk && c1) p[1] = e ? f1.y : f1.x;
+      float* dst = to + (int64_t)row * a.dv;
+      if (row < a.dk && c0) dst[0] = e ? f0.y : f0.x;
+      if (row < a.dk && c1) dst[1] = e ? f1.y : f1.x;
     }
   }
 }
 
 int padded(int dk) { return dk <= 64 ? 64 : (dk <= 128 ? 128 : 256); }
 int64_t records(int64_t total_rows, int n_seqs) { return total_rows / kN + n_seqs; }
+int64_t portion(int64_t n_records, int H, int dk) {
+  const int64_t fit = kMostBytes / ((int64_t)H * record_floats(padded(dk)) * 4);
+  return n_records <= fit ? n_records : (fit > 16 ? fit : 16);
+}
 
 template <typename T, int DK>
 int launch(const DeltaBlocks& a, float* recs, cudaStream_t st) {
-  const int64_t n = records(a.total_rows, a.n_seqs);
-  delta_blocks_factors_kernel<T, DK><<<dim3((unsigned)n, a.H), 128, 0, st>>>(a, recs, n);
+  const int64_t all = records(a.total_rows, a.n_seqs), n = portion(all, a.H, a.dk);
+  float* carry = recs + n * a.H * record_floats(DK);
+  const int64_t state = (int64_t)a.H * a.dk * a.dv;
   const int smem = kStages * record_floats(DK) * 4;
   // Every CTA reads its head's records again, so wide CTAs are better as long as they fill the chip.
-#define ATMA_WALK(W)                                                                                                       \
+#define ATMA_WALK(W, CUT)                                                                                                  \
   do {                                                                                                                     \
-    ATMA_CUDA_OK(cudaFuncSetAttribute(delta_blocks_walk_kernel<T, DK, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); \
-    delta_blocks_walk_kernel<T, DK, W><<<dim3((a.dv + 4 * W - 1) / (4 * W), a.H, a.n_seqs), W * 32, smem, st>>>(a, recs, n);    \
+    auto kern = delta_blocks_walk_kernel<T, DK, W, CUT>;                                                                   \
+    ATMA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));                           \
+    kern<<<dim3((a.dv + 4 * W - 1) / (4 * W), a.H, a.n_seqs), W * 32, smem, st>>>(a, recs, m, cut);                        \
   } while (0)
-  if ((int64_t)((a.dv + 31) / 32) * a.H * a.n_seqs >= sm_count_of_current_device()) ATMA_WALK(8);
-  else ATMA_WALK(2);
+  for (int64_t first = 0, i = 0; first < all; first += n, ++i) {
+    // two planes in turn: the state that comes in may be another sequence's than the one that goes out
+    const Cut cut{first, carry + (i & 1) * state, carry + (~i & 1) * state};
+    const int64_t m = first + n < all ? n : all - first;
+    delta_blocks_factors_kernel<T, DK><<<dim3((unsigned)m, a.H), 128, 0, st>>>(a, recs, m, first);
+    const bool wide = (int64_t)((a.dv + 31) / 32) * a.H * a.n_seqs >= sm_count_of_current_device();
+    if (n < all) { if (wide) ATMA_WALK(8, true); else ATMA_WALK(2, true); }
+    else { if (wide) ATMA_WALK(8, false); else ATMA_WALK(2, false); }
+  }
 #undef ATMA_WALK
   return launch_status("delta rule (fp32 arithmetic)");
 }
@@ -331,8 +369,10 @@ bool delta_blocks_supported(int64_t total_rows, int n_seqs, int H, int dk) {
   return dk > 0 && dk <= 256 && H > 0 && H <= 65535 && n_seqs > 0 && n_seqs <= 65535 && records(total_rows, n_seqs) < (int64_t(1) << 31);
 }
 
-int64_t delta_blocks_scratch_bytes(int64_t total_rows, int n_seqs, int H, int dk) {
-  return delta_blocks_supported(total_rows, n_seqs, H, dk) ? records(total_rows, n_seqs) * H * record_floats(padded(dk)) * 4 + 16 : 0;
+int64_t delta_blocks_scratch_bytes(int64_t total_rows, int n_seqs, int H, int dk, int dv) {
+  if (!delta_blocks_supported(total_rows, n_seqs, H, dk)) return 0;
+  const int64_t all = records(total_rows, n_seqs), n = portion(all, H, dk);
+  return n * H * record_floats(padded(dk)) * 4 + (n < all ? 2 * (int64_t)H * dk * dv * 4 : 0) + 16;
 }
 
 int delta_blocks_scan(const DeltaBlocks& a, void* scratch, cudaStream_t st) {

@@ -24,7 +24,7 @@ struct DeltaBlocks {
 };
 
 bool delta_blocks_supported(int64_t total_rows, int n_seqs, int H, int dk);
-int64_t delta_blocks_scratch_bytes(int64_t total_rows, int n_seqs, int H, int dk);
+int64_t delta_blocks_scratch_bytes(int64_t total_rows, int n_seqs, int H, int dk, int dv);
 int delta_blocks_scan(const DeltaBlocks& a, void* scratch, cudaStream_t st);
 
 }  // namespace atma

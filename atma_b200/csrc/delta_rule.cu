@@ -697,7 +697,7 @@ extern "C" int atma_delta_scan_path(const atma_delta_args* a) { return a != null
 extern "C" int64_t atma_delta_scan_scratch_bytes(const atma_delta_args* a) {
   if (a == nullptr) return 0;
   return delta_scan_sm100_supported(*a) ? delta_scan_sm100_scratch_bytes(*a)
-                                        : delta_blocks_scratch_bytes(a->total_rows, a->n_seqs, a->H, a->dim);
+                                        : delta_blocks_scratch_bytes(a->total_rows, a->n_seqs, a->H, a->dim, a->vdim);
 }
 
 extern "C" int atma_delta_scan(const atma_delta_args* a, const void* q, const void* k, const void* v, const float* q_inv,

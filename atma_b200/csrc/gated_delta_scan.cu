@@ -107,7 +107,7 @@ extern "C" int atma_gated_delta_scan_varlen_snapshots(const void* q, const void*
 }
 
 extern "C" int64_t atma_gated_delta_scan_scratch_bytes(int B, int T, int H, int dk, int dv) {
-  const int64_t fp32_path = delta_blocks_scratch_bytes((int64_t)B * T, B, H, dk);
+  const int64_t fp32_path = delta_blocks_scratch_bytes((int64_t)B * T, B, H, dk, dv);
   const int64_t mma_path = gated_delta_scan_mma_scratch_bytes(B, T, H);
   return fp32_path > mma_path ? fp32_path : mma_path;
 }

@@ -284,3 +284,22 @@ def test_fp32_blocks_of_rows(B, T, H, Hkv, dk, dv):
     v[:, T - 1] = float("inf")
     again, _ = _scan(q, k, v, glog, beta, S0)
     assert torch.equal(again[:, :T - 1], o[:, :T - 1])
+
+
+@pytest.mark.parametrize("dtype,B,T,H,Hkv,dk,dv", [(torch.bfloat16, 2, 15003, 64, 4, 65, 16), (torch.bfloat16, 3, 9000, 96, 1, 65, 3), (torch.float32, 1, 10561, 64, 1, 128, 4),
+                                                   (torch.float32, 1500, 9, 64, 64, 65, 4)])
+def test_fp32_blocks_in_portions(dtype, B, T, H, Hkv, dk, dv):
+    """Inputs whose records don't fit the scratch at a time, and whose portions end inside of sequences, at their ends and between
+    them: bit for bit what single sequences give in pieces of whole blocks, each with the state that the one in front left."""
+    q, k, v, glog, beta, S0 = (x.cuda() for x in _scan_inputs(B, T, H, dk, dv, dtype, seed=3, gamma_bias=1.0))
+    k, v = k[:, :, :Hkv].contiguous(), v[:, :, :Hkv].contiguous()
+    run = lambda *a, s: atma_b200.gated_delta.chunk_gated_delta_rule(*a, scale=dk ** -0.5, initial_state=s, output_final_state=True,      # noqa: E731
+                                                                     use_qk_l2norm_in_kernel=True)
+    o, S = run(q, k, v, glog, beta, s=S0)
+    for b in {0, B // 2, B - 1}:
+        state = S0[b:b + 1]
+        for a in range(0, T, 6400):
+            piece, state = run(*(x[b:b + 1, a:a + 6400].contiguous() for x in (q, k, v, glog, beta)), s=state)
+            assert torch.equal(o[b, a:a + 6400], piece[0])
+        assert torch.equal(S[b], state[0])
+    assert torch.equal(run(q, k, v, glog, beta, s=None)[0][:, 0], run(*(x[:, :1].contiguous() for x in (q, k, v, glog, beta)), s=None)[0][:, 0])

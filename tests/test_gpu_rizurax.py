@@ -379,6 +379,41 @@ def test_delta_long_sequences_cut_into_segments(shape, lens, first, shift):
     assert (state[0] == 33).all() and ops().device_status() == 0
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_delta_rule_in_portions_of_records(dtype):
+    """More blocks of rows than the scratch holds at a time, cut inside of sequences and between them, an empty and a padded one
+    among them: bit for bit what pieces of whole blocks give, and the row-by-row form (no scratch) to fp32 accuracy."""
+    H, G, K, V, lens, slots = 64, 2, 256, 8, [6000, 5, 0, 7000, 40, 5000, 3], [3, 0, 6, 5, -1, 1, 2]
+    starts = [0 if s >= 0 else -1 for s in slots]
+    w = ops().DeltaWeights(*(rand((n, 4), i, dtype, 0.6).cuda() for i, n in enumerate((G * K, G * K, H * V), 1)), rand((H,), 5).cuda() - 1,
+                           rand((H,), 6).cuda() - 2, (1 + rand((V,), 7, scale=0.3)).to(dtype).cuda(), heads=H, kv_heads=G, dim=K, vdim=V, unit_eps=1e-6,
+                           q_scale=K ** -0.5)
+    z = rand((sum(lens), w.channels + H * V + 2 * H), 8, dtype, 1.5).cuda()
+    tables = [_delta_tables(w, 7, dtype) for _ in range(3)]
+
+    def call(z, tab, *g, scratch=True):
+        parts = ops().DeltaParts(z, w, *tab, group(*g))
+        assert parts.scratch.numel() < 1.2 * 2 ** 30
+        parts.scratch = parts.scratch if scratch else None
+        parts.o.fill_(7)
+        parts.prepare()
+        parts.scan()
+        return parts.o
+
+    whole = call(z, tables[0], lens, starts, slots, [[0]] * len(lens))
+    rows = call(z, tables[1], lens, starts, slots, [[0]] * len(lens), scratch=False)
+    assert max_rel(whole, rows) < (1e-5 if dtype == F32 else 8e-3) and max_rel(tables[0][1], tables[1][1]) < 1e-5
+    at = 0
+    for n, first, slot in zip(lens, starts, slots):
+        for a in range(0, n, 4000):
+            m = min(4000, n - a)
+            piece = call(z[at:at + m], tables[2], [m], [a if slot >= 0 else -1], [slot], [[0]])
+            assert torch.equal(piece, whole[at:at + m]) and (slot >= 0 or not piece.any())
+            at += m
+    used = [s for s, n in zip(slots, lens) if s >= 0 and n > 0]
+    assert torch.equal(tables[0][1][used], tables[2][1][used]) and (tables[0][1][4] == 33).all() and not tables[0][1][6].any()
+
+
 # ---- the whole model through the engine ----------------------------------------------------------------------------------------
 _cache = {}
 
