@@ -19,8 +19,8 @@
 // Bound by L2 -> shared memory traffic (96 KB per 64 columns and CTA at BN = 256, 62 B per clock and SM if the tensor cores
 // were to wait for nothing).  Narrower BN where wide tiles would leave SMs without one; see pick_bn.
 // Measured with the split, out of HBM, beside the library's: 1500 x 8192 x 1024 118 us (499), 1500 x 1024 x 5120 95 us (346),
-// 4096 x 8192 x 1024 251 us (1094).  Below 128 rows, 64 columns or K = 64 the split costs more than it gives (32 x 512 x
-// 2048: 36 us against 26) and callers stay with the library.
+// 4096 x 8192 x 1024 251 us (1094).  Where one side is short or few tiles walk a long K the
+// library's is faster (32 x 512 x 2048: 26 us against 36) and callers stay with it.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status word for the host.
 #include "common.cuh"
 #include "linear_f32.cuh"

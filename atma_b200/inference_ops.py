@@ -334,10 +334,17 @@ def decode_linear_supported(x, weight, gated=False, k_unit=32, bias=None):
             x.data_ptr() % 16 == 0 and weight.data_ptr() % 16 == 0 and _bias_fits(bias, weight.shape[0]) and _one_device(x, weight, bias))
 
 
-# Fewer rows, or a narrower product: the library is faster.  Less work than 512 x 1024 x 1024: either takes less time on the
+# The library is faster where (library's time against linear_f32's, out of HBM)
+#   a side is short, so that splitting the others' rows is most of the work: 131072 x 64 x 64 47 us against 177, 65536 x 128 x 64
+#     45 against 105, 8192 x 1024 x 64 44 against 46; 4096 x 4096 x 128 103 against 77;
+#   the rows that are split make few sums: 16384 x 128 x 256 31 against 38; 8844 x 149 x 505 49 against 36;
+#   few tiles walk a long K, which the library cuts: 128 x 128 x 32768 143 against 365; 256 x 256 x 8192 109 against 103.
+# Random shapes inside of these lines, 128 to 11500 a side: 1.2 to 3.9 times faster, but for 1056 x 4224 x 128 (0.9).
+# Less work than 512 x 1024 x 1024: either takes less time on the
 # GPU than the host needs for a layer's calls, and the library's is the shorter one there (a block of a few hundred rows:
 # 1127 us with every product on linear_f32, 1090 without).
-LINEAR_F32_MIN_ROWS, LINEAR_F32_MIN_SIZE, LINEAR_F32_MIN_WORK = 128, 64, 1 << 29
+LINEAR_F32_MIN_SIZE, LINEAR_F32_MIN_WORK, LINEAR_F32_MIN_WORK_PER_ROW = 128, 1 << 29, 1 << 16
+LINEAR_F32_LONG_K, LINEAR_F32_LONG_K_MIN_RESULTS = 8192, 1 << 18
 LINEAR_F32_MAX_ROWS, LINEAR_F32_MAX_N, LINEAR_F32_MAX_K = 1 << 29, 1 << 21, 1 << 24      # what the entry takes
 
 
@@ -355,9 +362,14 @@ def linear_f32_supported(x, weight, bias=None):
     if x.ndim < 2 or weight.ndim != 2 or not weight.is_contiguous() or not _bias_fits(bias, weight.shape[0]) or not _one_device(*tensors):
         return False
     K, N = x.shape[-1], weight.shape[0]
-    if weight.shape[1] != K or min(K, N) < LINEAR_F32_MIN_SIZE or K > LINEAR_F32_MAX_K or N > LINEAR_F32_MAX_N:
+    if weight.shape[1] != K or K == 0:
         return False
-    if not LINEAR_F32_MIN_ROWS * K <= x.numel() <= LINEAR_F32_MAX_ROWS * K or x.numel() * N < LINEAR_F32_MIN_WORK:
+    M = x.numel() // K
+    if min(M, N, K) < LINEAR_F32_MIN_SIZE or M > LINEAR_F32_MAX_ROWS or N > LINEAR_F32_MAX_N or K > LINEAR_F32_MAX_K:
+        return False
+    if M * N * K < max(LINEAR_F32_MIN_WORK, LINEAR_F32_MIN_WORK_PER_ROW * (M + N)):
+        return False
+    if K > LINEAR_F32_LONG_K and M * N < LINEAR_F32_LONG_K_MIN_RESULTS:
         return False
     if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
         return False

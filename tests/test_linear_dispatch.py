@@ -47,7 +47,9 @@ def served(calls, x, w, b=None):
 
 
 @pytest.mark.parametrize("rows,k,n,yes", [(512, 1024, 1024, True), (511, 1024, 1024, False), (128, 4096, 1024, True), (127, 8192, 1024, False),
-                                          (1 << 17, 64, 64, True), (1 << 17, 63, 66, False), (1 << 17, 66, 63, False)])
+                                          (4096, 128, 4096, True), (8192, 127, 4096, False), (4096, 4096, 128, True), (8192, 4096, 127, False),
+                                          (1 << 17, 64, 64, False), (16384, 256, 128, False), (16384, 513, 131, True), (256, 8192, 256, True),
+                                          (256, 8224, 256, False), (512, 8224, 512, True), (128, 32768, 128, False)])
 def test_thresholds(calls, rows, k, n, yes):
     x, w, _ = product(rows, k, n)
     assert served(calls, x, w) is yes
