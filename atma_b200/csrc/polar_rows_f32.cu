@@ -27,20 +27,10 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
   const int h = blockIdx.x % a.H, b = blockIdx.y, kvh = h / (a.H / a.Hkv);
 
-  // ---- which query rows of which sequence ----
-  const bool packed = a.n_tiles > 0;
-  const int block = ((int)(gridDim.x - blockIdx.x) - 1) / a.H;
-  int q0 = block * kM, seq0 = 0, q_limit = a.Tq, k_limit = a.Tk;
-  if (packed) {
-    const int t = block / (128 / kM);
-    seq0 = a.tile_seq_start[t];
-    q0 = a.tile_q_start[t] + block % (128 / kM) * kM;
-    q_limit = k_limit = a.tile_seq_len[t];
-  }
-  if (q0 >= q_limit) return;
-  const float* Q = static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh + (int64_t)seq0 * a.q_st;
-  const float* K = static_cast<const float*>(a.k) + b * a.k_sb + kvh * a.k_sh + (int64_t)seq0 * a.k_st;
-  const float* V = static_cast<const float*>(a.v) + b * a.v_sb + kvh * a.v_sh + (int64_t)seq0 * a.v_st;
+  const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM, q_limit = a.Tq, k_limit = a.Tk;
+  const float* Q = static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh;
+  const float* K = static_cast<const float*>(a.k) + b * a.k_sb + kvh * a.k_sh;
+  const float* V = static_cast<const float*>(a.v) + b * a.v_sb + kvh * a.v_sh;
   for (int i = tid; i < kM * (DK / 4); i += kThreads) {
     const int r = i / (DK / 4), c = 4 * (i - r * (DK / 4));
     const bool there = q0 + r < q_limit;
@@ -54,7 +44,7 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a) {
   for (int i = 0; i < 4; ++i) {
     const int r = q0 + 4 * ty + i;
     const bool ok = r < q_limit;
-    n[i] = !ok ? 0.f : (packed ? (float)(r + 1) : (a.n_keys ? a.n_keys[r] : a.n_base + (float)(r + 1)));
+    n[i] = !ok ? 0.f : (a.n_keys ? a.n_keys[r] : a.n_base + (float)(r + 1));
     const float nc = fmaxf(a.window > 0 ? fminf(n[i], (float)a.window) : n[i], 1.0f);
     temp[i] = 1.0f + a.spg[h] * logf(nc);
     if (ok) { lo = fminf(lo, n[i]); hi = fmaxf(hi, n[i]); }
@@ -174,13 +164,13 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a) {
     }
     const float inv = 1.0f / fmaxf(sqrtf(row_sum(sq)), a.eps);
     if (ok) {
-      float* cp = static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)(seq0 + r) * a.c_st;
+      float* cp = static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)r * a.c_st;
 #pragma unroll
       for (int c = 0; c < 4 * VM; ++c) cp[64 * (c >> 2) + 4 * tx + (c & 3)] = sv[c] * inv;
       if (tx == 0) {
         const float n_eff = Lf * Lf / fmaxf(Q2f, 1e-30f);
         const float m_eff = n_eff * (Lf / fmaxf(Z, a.eps));
-        static_cast<float*>(a.mag)[b * a.mag_sb + h * a.mag_sh + (int64_t)(seq0 + r) * a.mag_st] = tanhf(a.beta[h] * log1pf(m_eff));
+        static_cast<float*>(a.mag)[b * a.mag_sb + h * a.mag_sh + (int64_t)r * a.mag_st] = tanhf(a.beta[h] * log1pf(m_eff));
       }
     }
   }
@@ -190,18 +180,18 @@ template <int DK>
 int launch(const atma_polar_prefill_args& a, cudaStream_t st) {
   const int smem = 4 * (kM * (DK + kPad) + kN * (DK + kPad) + kM * kLdP);
   ATMA_CUDA_OK(cudaFuncSetAttribute(polar_rows_f32_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  const int blocks = a.n_tiles > 0 ? a.n_tiles * (128 / kM) : (a.Tq + kM - 1) / kM;
-  polar_rows_f32_kernel<DK><<<dim3(blocks * a.H, a.B), kThreads, smem, st>>>(a);
+  polar_rows_f32_kernel<DK><<<dim3((a.Tq + kM - 1) / kM * a.H, a.B), kThreads, smem, st>>>(a);
   return launch_status("polar_prefill (fp32, 64 x 64)");
 }
 
 }  // namespace
 
-// Rows in quadruples of channels, and more rows than one CTA of the other kernel holds.
+// Rows in quadruples of channels, and more rows than one CTA of the other kernel holds.  Packed batches stay with that: they
+// are for 16-bit types.
 bool polar_rows_f32_supported(const atma_polar_prefill_args& a) {
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   auto rows = [](int64_t sb, int64_t sh, int64_t st) { return sb % 4 == 0 && sh % 4 == 0 && st % 4 == 0; };
-  return a.dtype == ATMA_F32 && (a.dk == 64 || a.dk == 128) && (a.n_tiles > 0 || a.Tq > 32) && al(a.q) && al(a.k) && al(a.v) &&
+  return a.dtype == ATMA_F32 && (a.dk == 64 || a.dk == 128) && a.n_tiles == 0 && a.Tq > 32 && al(a.q) && al(a.k) && al(a.v) &&
          rows(a.q_sb, a.q_sh, a.q_st) && rows(a.k_sb, a.k_sh, a.k_st) && rows(a.v_sb, a.v_sh, a.v_st);
 }
 

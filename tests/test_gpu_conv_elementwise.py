@@ -438,27 +438,32 @@ def test_decode_linear_with_a_short_last_range(B, N, K):
 
 
 def test_kernels_that_start_early_follow_a_join_in_a_graph():
-    """A chain of small launches, forked and joined as a decode step's, replayed: every kernel sees what those in front wrote."""
+    """A chain of small launches, forked and joined as a decode step's, replayed and run eagerly: every kernel sees what those
+    in front wrote, so both give what the same calls give when each has ended before the next is launched."""
     from atma_b200.inference_ops import add_rms_norm
     g = torch.Generator().manual_seed(1)
     x = torch.randn(4, 1024, generator=g).to(torch.bfloat16).cuda()
     w = (torch.randn(8, 1024, 1024, generator=g) / 32).to(torch.bfloat16).cuda()
     norm, side = torch.ones(1024, dtype=torch.bfloat16, device="cuda"), torch.cuda.Stream()
 
-    def chain():
+    def chain(ended=lambda: None):
         h = x
         for i in range(0, 8, 2):
             a = atma_b200.decode_linear(h, w[i])
+            ended()
             cur = torch.cuda.current_stream()
             side.wait_stream(cur)
             with torch.cuda.stream(side):
                 c = atma_b200.decode_linear(a, w[i + 1])
+            ended()
             b = atma_b200.decode_linear(a, w[i])
+            ended()
             cur.wait_stream(side)
             _, h = add_rms_norm(b, c, norm, 1e-6)
+            ended()
         return h
 
-    want = chain()
+    chain()
     torch.cuda.synchronize()
     side2 = torch.cuda.Stream()
     side2.wait_stream(torch.cuda.current_stream())
@@ -467,6 +472,6 @@ def test_kernels_that_start_early_follow_a_join_in_a_graph():
         got = chain()
     for s in range(30):
         x.copy_(torch.randn(4, 1024, generator=torch.Generator().manual_seed(s)))
+        want = chain(torch.cuda.synchronize)
         graph.replay()
-        assert torch.equal(got, chain())
-    assert want.shape == got.shape
+        assert torch.equal(got, want) and torch.equal(chain(), want)
