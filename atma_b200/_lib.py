@@ -188,6 +188,7 @@ _DECODER_SIGNATURES = {
     "atma_delta_prepare": (c_int, [POINTER(DeltaArgs)] + [c_void_p] * 8),
     "atma_delta_scan": (c_int, [POINTER(DeltaArgs)] + [c_void_p] * 10),
     "atma_delta_scan_path": (c_int, [POINTER(DeltaArgs)]),
+    "atma_delta_scan_longest": (c_int, [POINTER(DeltaArgs), c_int] + [c_void_p] * 10),
     "atma_delta_scan_scratch_bytes": (c_int64, [POINTER(DeltaArgs)]),
     "atma_delta_step": (c_int, [POINTER(DeltaArgs), c_void_p, c_void_p, c_int64, c_float, c_void_p]),
 }

@@ -111,6 +111,7 @@ __global__ void plan_kernel(const int32_t* __restrict__ cu_rows, const int32_t* 
     }
   }
   __syncwarp();
+  if (items == nullptr) return;
   int length = 1 << 30;                              // chunks of a segment
   if (n_seqs + 2 <= room) {
     int longest = 0;
@@ -516,8 +517,13 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int vblocks = p.vdim / kD;
   const int hv = blockIdx.x, h = hv / vblocks, g = h / (p.H / p.G);
-  if ((int)blockIdx.y >= (p.second ? p.plan->n_second : p.plan->n_first)) return;      // the whole CTA, before anything is allocated
-  const Item entry = p.items[(p.second ? p.max_items : 0) + blockIdx.y];
+  Item entry{(int)blockIdx.y, 0, 0, kWalk, -1, -1, -1, 0};
+  if (p.items == nullptr) {
+    entry.last = n_chunks_of(p.cu_chunks, blockIdx.y);
+  } else {
+    if ((int)blockIdx.y >= (p.second ? p.plan->n_second : p.plan->n_first)) return;    // the whole CTA, before anything is allocated
+    entry = p.items[(p.second ? p.max_items : 0) + blockIdx.y];
+  }
   const int b = entry.seq, n_chunks = entry.last - entry.first;
   if (n_chunks <= 0 || p.slots[b] < 0 || (kCuts && entry.kind == kTransfer && hv % vblocks != 0)) return;
   const int row_begin = p.cu_rows[b] + entry.first * kC, row_end = p.cu_rows[b + 1];
@@ -867,23 +873,30 @@ int64_t align_up(int64_t n) { return (n + 1023) & ~int64_t(1023); }
 // Where the scratch's parts lie, from launch-time sizes only.
 struct Layout {
   int room, max_items;                                // walks that fit the machine at a time; items of either launch
-  bool cuts;                                          // whether a sequence may be cut at all
+  bool cuts;                                          // whether a sequence may be cut
   int64_t cu, plan, items, chains, scal, recs, planes, bytes;
 };
-Layout layout_of(const atma_delta_args& a) {
+Layout layout_of(const atma_delta_args& a, int64_t longest_rows) {
   Layout l{};
   const int64_t n = max_chunks(a) * a.H;
   const int walks = a.H * (a.vdim / kD);
   l.room = sm_count_of_current_device() / walks;
-  l.cuts = a.n_seqs + 2 <= l.room && (a.total_rows + kC - 1) / kC > 6 + kComposeChunks;
-  l.max_items = l.cuts ? l.room : a.n_seqs;
+  // what plan_kernel decides, if every other sequence takes one walk: where it cannot cut, two launches and the plan are left
+  // out (4 x 500 rows 69 -> 60 us)
+  const bool space = a.n_seqs + 2 <= l.room && (a.total_rows + kC - 1) / kC > 6 + kComposeChunks;      // whatever the longest is
+  if (space) {
+    const int64_t longest = (longest_rows + kC - 1) / kC, parts = (l.room - a.n_seqs + 2) / 2, least = (longest + parts - 1) / parts;
+    const int64_t length = least > 4 ? least : 4;
+    l.cuts = length + (length + 1) / 2 + kComposeChunks < longest;
+  }
+  l.max_items = space ? l.room : a.n_seqs;
   l.plan = align_up(4 * ((int64_t)a.n_seqs + 1));
   l.items = l.plan + align_up(sizeof(Plan));
   l.chains = l.items + align_up(2 * (int64_t)l.max_items * sizeof(Item));
   l.scal = l.chains + align_up((int64_t)a.n_seqs * sizeof(Chain));
   l.recs = l.scal + n * kScal * 4;
   l.planes = l.recs + n * kRecBytes;
-  l.bytes = l.planes + (l.cuts ? (int64_t)(l.room / 2) * kPlanes * walks * kD * kD * 4 : 0);
+  l.bytes = l.planes + (space ? (int64_t)(l.room / 2) * kPlanes * walks * kD * kD * 4 : 0);
   return l;
 }
 
@@ -894,9 +907,9 @@ bool delta_scan_sm100_supported(const atma_delta_args& a) {
          max_chunks(a) * a.H * 256 < (int64_t(1) << 31);
 }
 
-int64_t delta_scan_sm100_scratch_bytes(const atma_delta_args& a) { return layout_of(a).bytes + 1024; }
+int64_t delta_scan_sm100_scratch_bytes(const atma_delta_args& a) { return layout_of(a, a.total_rows).bytes + 1024; }
 
-int delta_scan_sm100(const atma_delta_args& a, const void* q, const void* k, const void* v, const float* q_inv, const float* k_inv,
+int delta_scan_sm100(const atma_delta_args& a, int longest, const void* q, const void* k, const void* v, const float* q_inv, const float* k_inv,
                      const float* log_decay, const float* beta, void* o, void* scratch, cudaStream_t st) {
   ATMA_REQUIRE(scratch != nullptr, "delta_scan: scratch is required for this shape");
   auto al = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
@@ -904,12 +917,12 @@ int delta_scan_sm100(const atma_delta_args& a, const void* q, const void* k, con
   const int64_t NC = max_chunks(a);
   Params p{};
   uint8_t* base = reinterpret_cast<uint8_t*>(align_up((int64_t)reinterpret_cast<uintptr_t>(scratch)));
-  const Layout l = layout_of(a);
+  const Layout l = layout_of(a, longest < a.total_rows ? longest : a.total_rows);
   int32_t* cu_chunks = reinterpret_cast<int32_t*>(base);
   Plan* plan = reinterpret_cast<Plan*>(base + l.plan);
   Item* items = reinterpret_cast<Item*>(base + l.items);
   Chain* chains = reinterpret_cast<Chain*>(base + l.chains);
-  p.plan = plan; p.items = items; p.chains = chains; p.max_items = l.max_items;
+  p.plan = plan; p.items = l.cuts ? items : nullptr; p.chains = chains; p.max_items = l.max_items;
   p.planes = reinterpret_cast<float*>(base + l.planes);
   p.scal = reinterpret_cast<float*>(base + l.scal);
   p.recs = base + l.recs;
@@ -929,14 +942,14 @@ int delta_scan_sm100(const atma_delta_args& a, const void* q, const void* k, con
     rc = make_tmap_16bit_4d(&mm, p.recs, 1, dims, strides, box);
   }
   if (rc != ATMA_OK) return rc;
-  plan_kernel<<<1, 32, 0, st>>>(a.cu_rows, a.start_pos, a.n_seqs, l.cuts ? l.room : 0, cu_chunks, plan, items, l.max_items, chains);
+  plan_kernel<<<1, 32, 0, st>>>(a.cu_rows, a.start_pos, a.n_seqs, l.room, cu_chunks, plan, l.cuts ? items : nullptr, l.max_items, chains);
   const int64_t tiles = (NC + 1) / 2 * a.H;
   const int sms = sm_count_of_current_device();
   ATMA_CUDA_OK(cudaFuncSetAttribute(delta_factors_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFactorSmem));
   delta_factors_kernel<<<(unsigned)(tiles < 2 * sms ? tiles : 2 * sms), kThreads, kFactorSmem, st>>>(mq, mk, p);
   ATMA_CUDA_OK(cudaFuncSetAttribute(delta_recur_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecurSmem));
   const int walks = a.H * (a.vdim / kD);
-  const dim3 grid(walks, l.max_items);
+  const dim3 grid(walks, l.cuts ? l.max_items : a.n_seqs);
   if (l.cuts) {                                       // whether one is cut is decided on the device: the last two may find nothing to do
     ATMA_CUDA_OK(cudaFuncSetAttribute(delta_recur_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecurSmem));
     ATMA_CUDA_OK(cudaFuncSetAttribute(delta_compose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kComposeSmem));

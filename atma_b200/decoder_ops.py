@@ -234,7 +234,7 @@ class DeltaParts:
         _lib.require_cuda(z, "delta_prefill")
         w, n, dev = weights, z.shape[0], z.device
         self.lib, self.keep = _lib.load_decoder(), (z, weights, conv_table, state_table, group)
-        self.args = w.args(z, conv_table, state_table, group)
+        self.args, self.longest = w.args(z, conv_table, state_table, group), group.max_rows
         self.q = torch.empty((n, w.kv_heads, w.dim), device=dev, dtype=z.dtype)
         self.k = torch.empty_like(self.q)
         self.v = torch.empty((n, w.heads, w.vdim), device=dev, dtype=z.dtype)
@@ -251,7 +251,7 @@ class DeltaParts:
         _check(self.lib.atma_delta_prepare(ctypes.byref(self.args), _ptr(self.q), _ptr(self.k), _ptr(self.v), *self._factors(), _lib.stream_ptr()))
 
     def scan(self):
-        _check(self.lib.atma_delta_scan(ctypes.byref(self.args), _ptr(self.q), _ptr(self.k), _ptr(self.v), *self._factors(), _ptr(self.o),
+        _check(self.lib.atma_delta_scan_longest(ctypes.byref(self.args), self.longest, _ptr(self.q), _ptr(self.k), _ptr(self.v), *self._factors(), _ptr(self.o),
                                         _ptr(self.scratch), _lib.stream_ptr()))
 
 

@@ -135,6 +135,11 @@ int atma_delta_prepare(const atma_delta_args* args, void* q, void* k, void* v, f
  * serve the shape (atma_delta_scan_path() = 0): row by row, slower. */
 int atma_delta_scan(const atma_delta_args* args, const void* q, const void* k, const void* v, const float* q_inv, const float* k_inv,
                     const float* log_decay, const float* beta, void* o, void* scratch, void* stream);
+/* The same, told the most rows of a sequence (total_rows if that is not known): few long sequences are cut into segments, which
+ * takes launches of its own, and rows in ones and twos go row by row where that is faster.  A figure that is too small costs
+ * time only. */
+int atma_delta_scan_longest(const atma_delta_args* args, int longest, const void* q, const void* k, const void* v, const float* q_inv,
+                            const float* k_inv, const float* log_decay, const float* beta, void* o, void* scratch, void* stream);
 int atma_delta_scan_path(const atma_delta_args* args);
 int64_t atma_delta_scan_scratch_bytes(const atma_delta_args* args);
 /* One token per sequence, everything in one launch: convolutions, gates, recurrence, per-head norm with weight

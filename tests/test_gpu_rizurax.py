@@ -379,6 +379,24 @@ def test_delta_long_sequences_cut_into_segments(shape, lens, first, shift):
     assert (state[0] == 33).all() and ops().device_status() == 0
 
 
+@pytest.mark.parametrize("dtype,lens", [(BF16, [2113]), (BF16, [1300, 70, 1999]), (F32, [1, 2, 4, 3]), (F32, [5, 40])])
+def test_delta_scan_whatever_the_longest_is_said_to_be(dtype, lens):
+    """Cut or whole, in blocks or row by row: the figure chooses a kernel, the results stay."""
+    w = _delta_case((4, 2, 128, 128, 4), dtype, 1, 3)[1]
+    z = rand((sum(lens), w.channels + 4 * 128 + 8), 4, dtype, 1.5).cuda()
+    results = []
+    for longest in (max(lens), sum(lens), 1, 64):
+        conv, state = _delta_tables(w, len(lens), dtype)
+        parts = ops().DeltaParts(z, w, conv, state, group(lens, [0] * len(lens), list(range(len(lens))), [[0]] * len(lens)))
+        assert parts.longest == max(lens)
+        parts.longest = longest
+        parts.prepare()
+        parts.scan()
+        results.append((parts.o, state))
+    for o, state in results[1:]:
+        assert max_rel(o, results[0][0]) < (1e-5 if dtype == F32 else 8e-3) and max_rel(state, results[0][1]) < (1e-5 if dtype == F32 else 2e-4)
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 def test_delta_rule_in_portions_of_records(dtype):
     """More blocks of rows than the scratch holds at a time, cut inside of sequences and between them, an empty and a padded one
@@ -395,6 +413,7 @@ def test_delta_rule_in_portions_of_records(dtype):
         parts = ops().DeltaParts(z, w, *tab, group(*g))
         assert parts.scratch.numel() < 1.2 * 2 ** 30
         parts.scratch = parts.scratch if scratch else None
+        parts.longest = max(parts.longest, 8)             # in blocks also where a call has three rows
         parts.o.fill_(7)
         parts.prepare()
         parts.scan()
