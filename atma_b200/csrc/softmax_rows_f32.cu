@@ -173,8 +173,12 @@ int launch(const atma_softmax_args& a, cudaStream_t st) {
 
 }  // namespace
 
-// Rows in quadruples of channels, sizes that leave room for two CTAs, and more rows than two CTAs of the other kernel hold.
+// Rows in quadruples of channels, sizes that leave room for two CTAs, and more rows than two CTAs of the other kernel hold.  With
+// two maps and one page of keys at most, the other kernel's four times as many CTAs are faster while this one's leave most SMs
+// without any (8 heads, one prompt: 33 rows 23 us against 28, 128 rows 48 against 51; with 8000 keys in front 3470 against 2516).
 bool softmax_rows_f32_supported(const atma_softmax_args& a) {
+  const int64_t ctas = (int64_t)(a.max_rows + kM - 1) / kM * a.H * a.n_seqs;
+  if (a.maps == 2 && a.max_rows <= 128 && (int64_t)a.max_blocks * a.block_size <= 256 && 8 * ctas <= sm_count_of_current_device()) return false;
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return a.dtype == ATMA_F32 && a.max_rows > 32 && a.dim % 4 == 0 && a.vdim % 4 == 0 && a.maps * a.dim <= 128 && a.vdim <= 128 && al(a.q) &&
          al(a.k_cache) && al(a.v_cache);
