@@ -27,6 +27,7 @@ namespace atma {
 namespace {
 
 constexpr int kWarps = 16;                 // warps per CTA
+constexpr int kAhead = 8;                  // lines of a row that are asked for under the kernel in front: 16 KB per warp, 38 MB in all
 constexpr int kMaxRows = 16;               // batch rows (two n8 tiles)
 
 struct LinArgs {
@@ -56,9 +57,9 @@ decode_linear_kernel(const LinArgs a) {
   const int k0 = min(split * a.kper, a.K), kend = min(k0 + a.kper, a.K);
   const T* W = static_cast<const T*>(a.w);
   const T* X = static_cast<const T*>(a.x);
-  if (unit < a.units) {                                       // the warp's weights, a 128-byte line per lane
+  if (unit < a.units) {                                       // the warp's first weights, a 128-byte line per lane
     constexpr int kLine = 128 / (int)sizeof(T);
-    const int lines = (kend - k0 + kLine - 1) / kLine;
+    const int lines = min((kend - k0 + kLine - 1) / kLine, kAhead);
     for (int i = lane; i < 16 * kTiles * lines; i += 32) {
       const int r = i / lines, at = k0 + (i - r * lines) * kLine;
       prefetch_l2(W + ((int64_t)unit * 16 + (r & 15) + (r < 16 ? 0 : a.N / 2)) * a.K + at);
