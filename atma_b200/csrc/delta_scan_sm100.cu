@@ -882,7 +882,7 @@ Layout layout_of(const atma_delta_args& a, int64_t longest_rows) {
   const int walks = a.H * (a.vdim / kD);
   l.room = sm_count_of_current_device() / walks;
   // what plan_kernel decides, if every other sequence takes one walk: where it cannot cut, two launches and the plan are left
-  // out (4 x 500 rows 69 -> 60 us)
+  // out (4 x 500 rows 56 -> 51 us, one after another; 8 x 200 44 -> 38)
   const bool space = a.n_seqs + 2 <= l.room && (a.total_rows + kC - 1) / kC > 6 + kComposeChunks;      // whatever the longest is
   if (space) {
     const int64_t longest = (longest_rows + kC - 1) / kC, parts = (l.room - a.n_seqs + 2) / 2, least = (longest + parts - 1) / parts;
