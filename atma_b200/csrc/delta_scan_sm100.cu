@@ -282,6 +282,18 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             tma_load_4d(Ks + cb * 16384 + ci * 8192, &tmap_k, &bar.kq_full, cb * 64, m.g, t0, 0);
             tma_load_4d(Qs + cb * 16384 + ci * 8192, &tmap_q, &bar.kq_full, cb * 64, m.g, t0, 0);
           }
+        // the tiles' place is taken until the end of this one; meanwhile the next inputs come into L2
+        if (tile + gridDim.x < n_tiles) {
+          Meta mn;
+          tile_meta(p, tile + gridDim.x, mn);
+#pragma unroll
+          for (int ci = 0; ci < 2; ++ci)
+#pragma unroll
+            for (int cb = 0; cb < 2; ++cb) {
+              tma_prefetch_l2_4d(&tmap_k, cb * 64, mn.g, (int)mn.t0[ci], 0);
+              tma_prefetch_l2_4d(&tmap_q, cb * 64, mn.g, (int)mn.t0[ci], 0);
+            }
+        }
       }
     }
     __syncwarp();
@@ -317,16 +329,25 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const int ci = row >> 6, pr = row & 63;            // chunk of the tile, row inside the chunk
     const uint32_t lane_base = tbase + (uint32_t(32 * quad) << 16);
     uint32_t it = 0;
+    // a tile's coordinates and its row scalars are fetched a tile ahead
+    Meta m_next{};
+    float bt_next = 0.f, kinv_next = 0.f, qinv_next = 0.f, decay_next = 0.f;
+    auto fetch_tile = [&](int64_t tile) {
+      if (tile >= n_tiles) return;
+      tile_meta(p, tile, m_next);
+      const bool valid = pr < (ci ? m_next.rows[1] : m_next.rows[0]);
+      const int64_t t = (ci ? m_next.t0[1] : m_next.t0[0]) + pr;
+      bt_next = valid ? p.beta[t * p.H + m_next.h] : 0.f;
+      kinv_next = valid ? p.k_inv[t * p.G + m_next.g] : 0.f;
+      qinv_next = valid ? p.q_inv[t * p.G + m_next.g] : 0.f;
+      decay_next = valid ? p.log_decay[t * p.H + m_next.h] : 0.f;
+    };
+    fetch_tile(blockIdx.x);
     for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
-      Meta m;
-      tile_meta(p, tile, m);
-      const bool valid = pr < (ci ? m.rows[1] : m.rows[0]);
+      const Meta m = m_next;
       const int64_t rec = ci ? m.rec[1] : m.rec[0];
-      const int64_t t = (ci ? m.t0[1] : m.t0[0]) + pr;
-      const float bt_p = valid ? p.beta[t * p.H + m.h] : 0.f;
-      const float kinv_p = valid ? p.k_inv[t * p.G + m.g] : 0.f;
-      const float qinv_p = valid ? p.q_inv[t * p.G + m.g] : 0.f;
-      float run = valid ? p.log_decay[t * p.H + m.h] : 0.f;
+      const float bt_p = bt_next, kinv_p = kinv_next, qinv_p = qinv_next;
+      float run = decay_next;
       // decay prefix over the chunk's 64 rows (two warps)
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -370,8 +391,9 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int s = 32 * half + j + e;
-              const bool seen = which ? s <= pr : s < pr;
-              x[e] = seen ? f * (__expf(lg_p - s_lg[64 * ci + s]) * s_kinv[64 * ci + s]) * __uint_as_float(gm[j + e]) : 0.f;
+              // chosen after it is computed: as a condition around the exponential it is a branch for every element
+              const float value = f * (__expf(lg_p - s_lg[64 * ci + s]) * s_kinv[64 * ci + s]) * __uint_as_float(gm[j + e]);
+              x[e] = (which ? s <= pr : s < pr) ? value : 0.f;
             }
             *reinterpret_cast<float4*>(dst + j) = make_float4(x[0], x[1], x[2], x[3]);
           }
@@ -418,29 +440,30 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         worker_sync();
       }
-      // ---- M1 = T diag(beta): this thread's row, 32 columns, as two terms; zeros of M2 above the diagonal blocks ----
-      if (rec >= 0) {
-        uint8_t* r1 = p.recs + rec * (int64_t)kRecBytes + pr * 128 + half * 64;
+      fetch_tile(tile + gridDim.x);
+      // ---- M1 = T diag(beta) as two terms, and zeros of M2 above the diagonal blocks: eight threads per 128-byte row ----
 #pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
-          uint32_t hi[4], lo[4];
-          const bool above = ((32 * half + 8 * c4) >> 4) > (pr >> 4);
+      for (int i = 0; i < 4; ++i) {
+        const int idx = wtid + 256 * i, r = idx >> 3, ch = idx & 7, rp = r & 63, rc = r >> 6;
+        const int64_t to = rc ? m.rec[1] : m.rec[0];
+        const bool above = (ch >> 1) > (rp >> 4);
+        uint32_t hi[4] = {}, lo[4] = {};
+        if (!above) {
+          float x[8];
+          *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(Tf + r * kLd + 8 * ch);
+          *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(Tf + r * kLd + 8 * ch + 4);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int s = 32 * half + 8 * c4 + 2 * e;
-            float x = 0.f, y = 0.f;
-            if (!above) {
-              const float2 tt = *reinterpret_cast<const float2*>(Tf + row * kLd + s);
-              x = s <= pr ? tt.x * s_bt[64 * ci + s] : 0.f;
-              y = s + 1 <= pr ? tt.y * s_bt[64 * ci + s + 1] : 0.f;
-            }
-            split2(x, y, hi[e], lo[e]);
-          }
-          *reinterpret_cast<uint4*>(r1 + c4 * 16) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(r1 + 16384 + c4 * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          for (int e = 0; e < 8; ++e) x[e] = 8 * ch + e <= rp ? x[e] * s_bt[64 * rc + 8 * ch + e] : 0.f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) split2(x[2 * e], x[2 * e + 1], hi[e], lo[e]);
+        }
+        if (to >= 0) {
+          uint8_t* r1 = p.recs + to * (int64_t)kRecBytes + rp * 128 + ch * 16;
+          *reinterpret_cast<uint4*>(r1) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(r1 + 16384) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           if (above) {
-            *reinterpret_cast<uint4*>(r1 + 8192 + c4 * 16) = make_uint4(0u, 0u, 0u, 0u);
-            *reinterpret_cast<uint4*>(r1 + 24576 + c4 * 16) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(r1 + 8192) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(r1 + 24576) = make_uint4(0u, 0u, 0u, 0u);
           }
         }
       }
