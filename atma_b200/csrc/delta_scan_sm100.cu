@@ -267,7 +267,7 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
   if (warp == 0) {
     // ---- TMA producer ------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
         if (it > 0 && !mbar_wait(&bar.tile_free, (it - 1) & 1u, abort_flag)) break;
@@ -299,7 +299,7 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     __syncwarp();
   } else if (warp == 1) {
     // ---- MMA issuer --------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(128, 128, 1, 0, 0);
       const uint64_t hi_k = (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(16 >> 4) << 16);
       const uint64_t kd = hi_k | uint64_t((smem_u32(Ks) >> 4) & 0x3FFFu), qd = hi_k | uint64_t((smem_u32(Qs) >> 4) & 0x3FFFu);
@@ -573,7 +573,7 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
   if (warp == 0) {
     // ---- TMA producer ------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       for (int i = 0; i < n_chunks; ++i) {
         const int s = i % kStages;
         uint8_t* st = smem + s * kStageBytes;
@@ -596,7 +596,7 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     // ---- MMA issuer --------------------------------------------------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       // B rows as they lie: [K; Q] or [M1; M2]; without outputs only the first half
       const uint32_t idesc_k = !kCuts || item.kind == kWalk ? make_idesc(128, 128, 1, 0, 0) : make_idesc(128, 64, 1, 0, 0);
       constexpr uint32_t idesc_ds = make_idesc(128, 128, 1, 0, 1);     // B = K [s][k], MN-major

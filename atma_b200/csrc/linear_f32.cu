@@ -226,7 +226,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   volatile int* abort = &s_abort_v;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       int it = 0;
       for (; it < NK; ++it) {
         const int st = it % L::kStages;
@@ -240,7 +240,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       for (int i = max(0, it - L::kStages); i < it; ++i) mbar_wait(&full[i % L::kStages], (i / L::kStages) & 1, &alone);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(kBM, BN, 0, 0, 0);
       for (int it = 0; it < NK; ++it) {
         const int st = it % L::kStages, buf = it & 1;

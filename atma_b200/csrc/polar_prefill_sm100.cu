@@ -217,7 +217,7 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
   asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
   if (warp == 0) {
     // =============================== TMA producer ================================================
-    if (lane == 0) {
+    if (elect_one()) {
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         if (hi[t] > lo[t]) {
@@ -239,7 +239,7 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     __syncwarp();
   } else if (warp == 1) {
     // =============================== MMA issuer =================================================
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc(kBM, kBN, kBf16 ? 1 : 0, 0, 0);
       constexpr uint32_t idesc_pv = make_idesc(kBM, kDK, kBf16 ? 1 : 0, 0, 1);
       const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);

@@ -10,7 +10,7 @@
 //
 //   warp 0      TMA producer: the Q tiles once, K and V tiles (stream 0, stream 1, stream 0, ... or shared) through rings,
 //               with one map the output gate's tiles at the end
-//   warp 1      MMA issuer (one lane)
+//   warp 1      MMA issuer
 //   warps 2-3   idle (they complete the first warpgroup, whose registers are handed over)
 //   warps 4-7   softmax of stream 0, one thread per query row (= one TMEM lane), and its epilogue (two maps: half of the
 //               epilogue's channels)
@@ -134,7 +134,7 @@ softmax_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     if (warp == 0) {
       // ============================= TMA producer ==============================================
-      if (lane == 0 && n_kt > 0) {
+      if (n_kt > 0 && elect_one()) {
         const int32_t* bt = a.block_tables + seq * a.bt_stride;
         for (int m = 0; m < n_streams; ++m) {
           mbar_arrive_expect_tx(&bar.q_full[m], kMapTile);
@@ -180,7 +180,7 @@ softmax_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
       __syncwarp();
     } else if (warp == 1) {
       // ============================= MMA issuer ================================================
-      if (lane == 0 && n_kt > 0) {
+      if (n_kt > 0 && elect_one()) {
         constexpr uint32_t idesc_qk = make_idesc(kBM, kBN, 1, 0, 0);
         constexpr uint32_t idesc_pv = make_idesc(kBM, VD, 1, 0, 1);
         const uint32_t q_addr = smem_u32(sQ), k_addr = smem_u32(sK), v_addr = smem_u32(sV);
