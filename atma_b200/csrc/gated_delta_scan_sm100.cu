@@ -1,30 +1,40 @@
 // Gated-delta scan, the recurrence over chunks, on the 5th-generation tensor cores (sm_100a):
-// tcgen05.mma with TMEM accumulators, per-chunk factor records brought in by TMA.
+// tcgen05.mma with TMEM accumulators, per-chunk factor records and the rows of q, k, v brought in by TMA.
 //
 // One CTA owns one (recurrence, head) and the whole state S [dk][dv], held TRANSPOSED: every
 // thread of the eight state warps keeps 64 fp32 values of one row of S^T [v][k] in registers for
-// the whole sequence.  Per 64-token chunk, with the state-independent factors -W, Qg, Kt, U0^T, Rq
-// of gated_delta_scan.cuh (s, p = rows of the chunk; k, v = key / value channel):
+// the whole sequence.  Per 64-token chunk, with Tw, Tu, Rq and the row scalars of gated_delta_scan.cuh
+// (s, p = rows of the chunk; k, v = key / value channel):
 //
-//   MMA1a  U^T  = S^T (-W)^T            M=128 (v) N=64 (s)  K=128 (k)
-//   MMA1b  O^T  = S^T Qg^T              M=128 (v) N=64 (p)  K=128 (k)
-//   threads     U^T += U0^T -> 16-bit, back into TMEM
-//   MMA2a  dS^T = U^T Kt                M=128 (v) N=128 (k) K=64 (s);  threads: S^T = g_C S^T + dS^T
-//   MMA2b  O^T += U^T Rq^T              M=128 (v) N=64 (p)  K=64 (s)
+//   the chain
+//     MMA   U^T += S^T (-W)^T                 K=128 (k);   state warps: U^T -> 16 bits, times (g_C / g) k_inv, then as it is
+//     MMA   dS^T = (U (g_C / g) k_inv)^T K    N=128 (k);   state warps: S^T = g_C S^T + dS^T
+//   under the thread phase of U, for the next chunk
+//     MMA  -W^T = K^T Tw^T   M=128 (k) N=64 (p) K=64 (s);  W warps: -> 16 bits, shared memory (B operand)
+//   under the thread phase of S, issued by a warp of its own so that the chain's never waits for what these wait for
+//     MMA   U^T = V^T Tu^T of the next chunk; stays in TMEM
+//     MMA   O1^T = S^T Q^T,  O2^T = U^T Rq^T;  O warps: o = g q_inv O1 + O2
 //
-// The A operand of every product (the 16-bit copies of S^T and U^T) is read from TMEM, where the
-// state warps put it with tcgen05.st; only the B operands (the record tiles, exactly as TMA
-// delivers them) come from shared memory.  One SM's shared-memory bandwidth is what bounds this
-// kernel, so nothing the threads produce goes through shared memory, and no thread-written tile
-// needs a proxy fence.  All four accumulators have the value channel v on the 128 TMEM lanes, which
-// spreads both thread phases of the chunk-to-chunk critical path over all four warp schedulers.
+// Q, K, V and the record tiles are operands exactly as TMA delivers them; scalars per row are applied to fp32
+// accumulators.  fp16 has no room for U times an unbounded 1 / |k|, so there the helper warps scale the K rows in
+// shared memory instead.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
+// accumulators have a channel on the 128 TMEM lanes, which spreads the thread phases over all four schedulers.
 //
-//   warp 0      TMA producer: the pieces of each chunk record through a 3-stage ring
-//   warp 1      MMA issuer (one lane); owns the TMEM allocation
-//   warps 2-9   state warps; warp w works on TMEM lanes 32 (w % 4) .. +31 and on column half
-//               (w - 2) / 4 of whatever it reads (k for S^T, s for U^T, p for O^T)
-// TMEM (512 columns allocated): 16-bit S^T [0,64) | 16-bit U^T [64,96) | U^T fp32 [128,192) |
-// O^T_0 [192,256) | O^T_1 [256,320) | dS^T [320,448).
+// What bounds it is the latency of the chain, of which the two thread phases are half: 3000 clocks a chunk, 650 for S and 750
+// for U between a product's end and its successor's first operand, the products 330 and 600.  Measured with the chunk-local
+// stage, which no longer writes W, U0, Qg and Kt: 8 sequences of 16384 tokens, 8 heads, 327 + 414 us (617 + 385 with those
+// in 72 KB records), one of 65536 732 -> 606 us, 8 of 300 45 -> 39 us.
+//
+//   warp 0       TMA producer: V, Tw, Tu and K three chunks ahead, Q and Rq two
+//   warp 1       issues the chain's products and -W^T; owns the TMEM allocation
+//   warp 2       issues the other products (warp 3 fills the warpgroup)
+//   warps 4-11   state warps; warp w works on TMEM lanes 32 (w % 4) .. +31 and on column half
+//                (w - 4) / 4 of whatever it reads (k for S^T, p for U^T); with sixteen of them a phase
+//                takes longer, their waits and arrivals cost more than the shorter rows save
+//   warps 12-15  W warps, warps 16-19 O warps: TMEM lanes 32 (w % 4) .. +31
+// TMEM (512 columns allocated): 16-bit S^T [0,64) and, every other chunk, [64,128) | 16-bit U^T [128,160), scaled
+// [160,192) | U^T fp32 [192,256) | O1^T [256,320) | O2^T [320,384) | dS^T [384,512), where -W^T of the next chunk passes
+// through between the state's reading and the next dS^T.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status
 // word for the host.
 #include "common.cuh"
@@ -40,58 +50,54 @@ namespace {
 
 __device__ int g_scan_status = 0;
 
-constexpr int kThreads = 320;
-constexpr int kA1Bytes = 2 * kD * 128;            // [-W ; Qg]: [128 rows][128 k] 16-bit = two 64-column boxes of 16 KiB
-constexpr int kKtBytes = 2 * kC * 128;            // [64 s][128 k] = two boxes of 8 KiB
-constexpr int kU0Bytes = kD * 128;                // U0^T: [128 v][64 s], one box
-constexpr int kRqBytes = kC * 128;                // [64 p][64 s], one box
-constexpr int kStageBytes = kA1Bytes + kKtBytes + kU0Bytes + kRqBytes;   // 72 KiB
-constexpr int kStages = 3;
-constexpr int kSmemBytes = kStages * kStageBytes + 1024;
-constexpr int kRecRows = kRecBytes / 256;         // a record as rows of 128 16-bit values (288)
-constexpr int kRecRowsRq = kRecBytes / 128;       // ... and as rows of 64 values (576)
-constexpr uint32_t kColSb = 0, kColUb = 64, kColU = 128, kColO = 192, kColS = 320;
+constexpr int kStateWarps = 8, kHelpWarps = 4, kThreads = 32 * (4 + kStateWarps + 2 * kHelpWarps);
+// 640 threads are launched with 96 registers each, 61440; then 256 of them take 136 and 384 keep 64, together 59392
+constexpr int kStateRegs = 136, kOtherRegs = 64;
+constexpr int kRowBytes = kC * kD * 2;            // 64 rows of 128 channels: two boxes of 64 channels, 8 KiB each
+// rings: [V | Tw | Tu], [K], [Q | Rq], scalars; then -W^T [128 k][64 p]
+constexpr int kVts = 3, kVtBytes = kRowBytes + 2 * kTile64, kKs = 3, kQrs = 2, kQrBytes = kRowBytes + kTile64, kScs = 4, kScBytes = kScal * 4;
+constexpr int kOffK = kVts * kVtBytes, kOffQr = kOffK + kKs * kRowBytes, kOffW = kOffQr + kQrs * kQrBytes, kOffSc = kOffW + kD * 128,
+              kSmemBytes = kOffSc + kScs * kScBytes + 1024;
+constexpr uint32_t kColSb = 0, kColUb = 128, kColUs = 160, kColU = 192, kColO1 = 256, kColO2 = 320, kColS = 384, kColW = kColS;
 
 struct Barriers {
-  uint64_t a1_full[kStages], a1_empty[kStages], y_full[kStages], y_empty[kStages];
-  uint64_t o_free[2], o_done[2];
-  uint64_t sb_ready, ub_ready, u_full, s_done;
+  uint64_t vt_full[kVts], vt_empty[kVts], k_full[kKs], k_empty[kKs], qr_full[kQrs], qr_empty[kQrs], sc_full[kScs], sc_empty[kScs];
+  uint64_t w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
 };
 
 struct Params {
-  const float* gcs;
+  const float* scal;
   const float* initial_state;
   void* o;
   float* final_state;
-  int Tlen, H, NC, is_bf16;
+  int Tlen, H, Hkv, NC;
   RecMap map;
   VarLen var;
 };
 
-template <bool kBf16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (kBf16) {
-    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-  } else {
-    __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&h);
-  }
-}
-template <bool kBf16>
-__device__ __forceinline__ float2 unpack2(uint32_t v) {
-  if constexpr (kBf16) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-  else return __half22float2(*reinterpret_cast<__half2*>(&v));
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 
-// byte offset of the 16-byte chunk `chunk` (0..7) of row `row` inside a 128-byte-swizzled box
-__device__ __forceinline__ uint32_t box_off(int row, int chunk) {
-  return (uint32_t)(row * 128 + ((chunk ^ (row & 7)) << 4));
+// shared-memory descriptors of tiles with 128-byte rows: K-major, and MN-major in boxes of 8 KiB
+__device__ __forceinline__ uint64_t desc_k(uint32_t addr) {
+  return (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(16 >> 4) << 16) | uint64_t((addr >> 4) & 0x3FFFu);
+}
+__device__ __forceinline__ uint64_t desc_mn(uint32_t addr) {
+  return (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(8192 >> 4) << 16) | uint64_t((addr >> 4) & 0x3FFFu);
+}
+template <int kRegs, bool kMore>
+__device__ __forceinline__ void set_registers() {       // of every warp of a warpgroup
+  if constexpr (kMore) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
+  else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
 
-template <bool kBf16>
+// kWide: o is 4-byte aligned, two channels are stored at a time
+template <bool kBf16, bool kWide>
 __global__ void __launch_bounds__(kThreads, 1)
-scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_rec, const __grid_constant__ CUtensorMap tmap_rq, const Params p) {
+scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
+                        const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_rec, const Params p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ Barriers bar;
@@ -104,241 +110,392 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_rec, const __gr
   const int rb = packed ? 0 : p.map.rec[b];
   const bool zero_u0 = packed ? false : p.map.zero_u0[b] != 0;
   int c_begin, c_end;
-  int64_t tok_base, tok_end;
+  int64_t tok_in, tok_base, tok_end;                     // first token of the inputs; first and past-the-end token of o
   if (packed) {
     c_begin = p.var.cu_chunks[b]; c_end = p.var.cu_chunks[b + 1];
-    tok_base = p.var.cu_seqlens[b]; tok_end = p.var.cu_seqlens[b + 1];
+    tok_in = tok_base = p.var.cu_seqlens[b]; tok_end = p.var.cu_seqlens[b + 1];
   } else {
     c_begin = p.map.c_begin[b]; c_end = p.map.c_end[b] > 0 ? p.map.c_end[b] : p.NC;
     const int64_t orow0 = (int64_t)max(p.map.o_row[b], 0) * p.Tlen;  // the batch row of o this recurrence writes
+    tok_in = (int64_t)rb * p.Tlen + (int64_t)c_begin * kC;
     tok_base = orow0 + (int64_t)c_begin * kC;
     tok_end = orow0 + min((int64_t)p.Tlen, (int64_t)c_end * kC);
   }
   const int n_chunks = max(c_end - c_begin, 0);
   const int64_t rec0 = ((int64_t)rb * p.H + h) * p.NC + c_begin;     // first record of this recurrence
-  const float* gcs = p.gcs + rec0;
   const bool want_o = p.o != nullptr && (packed || p.map.o_row[b] >= 0);   // a negative row: this recurrence only carries state
 
   if (tid == 0) {
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&bar.a1_full[i], 1); mbar_init(&bar.a1_empty[i], 1);
-      mbar_init(&bar.y_full[i], 1); mbar_init(&bar.y_empty[i], 1);
-    }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bar.o_free[i], 8); mbar_init(&bar.o_done[i], 1); }
-    mbar_init(&bar.sb_ready, 8); mbar_init(&bar.ub_ready, 8);
-    mbar_init(&bar.u_full, 1); mbar_init(&bar.s_done, 1);
+    for (int i = 0; i < kVts; ++i) { mbar_init(&bar.vt_full[i], 1); mbar_init(&bar.vt_empty[i], 2); }
+    for (int i = 0; i < kKs; ++i) { mbar_init(&bar.k_full[i], 1); mbar_init(&bar.k_empty[i], 1); }
+    for (int i = 0; i < kQrs; ++i) { mbar_init(&bar.qr_full[i], 1); mbar_init(&bar.qr_empty[i], 1); }
+    for (int i = 0; i < kScs; ++i) { mbar_init(&bar.sc_full[i], 1); mbar_init(&bar.sc_empty[i], kStateWarps + (kBf16 ? 1 : 2) * kHelpWarps); }
+    mbar_init(&bar.sb_ready, kStateWarps); mbar_init(&bar.us_ready, kStateWarps); mbar_init(&bar.ub_ready, kStateWarps);
+    mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
+    mbar_init(&bar.w_done, 1); mbar_init(&bar.u_full, 1); mbar_init(&bar.s_done, 1); mbar_init(&bar.o_done, 1);
     s_abort = 0;
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc(&s_tmem_base, 512);
-  if (warp == 0 && lane == 0) { prefetch_tensormap(&tmap_rec); prefetch_tensormap(&tmap_rq); }
+  if (warp == 0 && lane == 0) { prefetch_tensormap(&tmap_q); prefetch_tensormap(&tmap_k); prefetch_tensormap(&tmap_v); prefetch_tensormap(&tmap_rec); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tbase = s_tmem_base;
   volatile int* abort_flag = &s_abort;
 
-  if (warp == 0) {
-    // =============================== TMA producer ================================================
-    if (lane == 0) {
-      for (int i = 0; i < n_chunks; ++i) {
-        const int s = i % kStages;
-        const uint32_t ph = (uint32_t)(i / kStages) & 1u;
-        uint8_t* st = smem + s * kStageBytes;
-        const int row = (int)((rec0 + i) * kRecRows), row64 = (int)((rec0 + i) * kRecRowsRq);
-        if (!mbar_wait(&bar.a1_empty[s], ph ^ 1u, abort_flag)) break;
-        mbar_arrive_expect_tx(&bar.a1_full[s], kA1Bytes);
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {                      // -W rows then Qg rows, two column boxes each
-          tma_load_4d(st + half * 16384, &tmap_rec, &bar.a1_full[s], half * 64, row, 0, 0);
-          tma_load_4d(st + half * 16384 + 8192, &tmap_rec, &bar.a1_full[s], half * 64, row + 64, 0, 0);
-        }
-        if (!mbar_wait(&bar.y_empty[s], ph ^ 1u, abort_flag)) break;
-        mbar_arrive_expect_tx(&bar.y_full[s], kKtBytes + kU0Bytes + kRqBytes);
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          tma_load_4d(st + kA1Bytes + half * 8192, &tmap_rec, &bar.y_full[s], half * 64, row + 128, 0, 0);
-          tma_load_4d(st + kA1Bytes + kKtBytes + half * 8192, &tmap_rq, &bar.y_full[s], 0, row64 + 384 + half * 64, 0, 0);
-        }
-        tma_load_4d(st + kA1Bytes + kKtBytes + kU0Bytes, &tmap_rq, &bar.y_full[s], 0, row64 + 512, 0, 0);
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // =============================== MMA issuer =================================================
-    if (lane == 0) {
-      constexpr int fmt = kBf16 ? 1 : 0;
-      constexpr uint32_t idesc_n64 = make_idesc(128, 64, fmt, 0, 0);     // B = W, Qg or Rq rows, K-major
-      constexpr uint32_t idesc_s = make_idesc(128, 128, fmt, 0, 1);      // dS^T = U^T Kt: B = Kt [s][k] MN-major
-      const uint64_t hi_k = (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(16 >> 4) << 16);
-      const uint64_t hi_mn64 = (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61) | (uint64_t(8192 >> 4) << 16);
-      bool ok = true;
-      for (int i = 0; i < n_chunks && ok; ++i) {
-        const int s = i % kStages, ob = i & 1;
-        const uint32_t ph = (uint32_t)(i / kStages) & 1u;
-        const uint32_t st = smem_u32(smem + s * kStageBytes);
-        const uint32_t tO = tbase + kColO + ob * 64;
-        const uint64_t a1 = hi_k | uint64_t((st >> 4) & 0x3FFFu);
-        ok = mbar_wait(&bar.sb_ready, (uint32_t)i & 1u, abort_flag);
-        if (ok) ok = mbar_wait(&bar.a1_full[s], ph, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t off = uint64_t(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4);
-          mma_ts(tbase + kColU, tbase + kColSb + kk * 8, a1 + off, idesc_n64, kk > 0);
-        }
-        tc_commit(&bar.u_full);
-        if (want_o) {
-          if (i >= 2) ok = mbar_wait(&bar.o_free[ob], (uint32_t)((i >> 1) - 1) & 1u, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint64_t off = uint64_t(((kk >> 2) * 16384 + (kk & 3) * 32) >> 4);
-            mma_ts(tO, tbase + kColSb + kk * 8, a1 + uint64_t(8192 >> 4) + off, idesc_n64, kk > 0);
+  if (warp < 4) {
+    set_registers<kOtherRegs, false>();
+    if (warp == 0) {
+      // =============================== TMA producer ================================================
+      if (elect_one()) {
+        const int hk = h / (p.H / p.Hkv);
+        for (int i = 0; i <= n_chunks; ++i) {
+          if (i < n_chunks) {
+            const int t0 = (int)(tok_in + (int64_t)i * kC), row = (int)((rec0 + i) * (3 * kC));
+            uint8_t* st = smem + i % kVts * kVtBytes;
+            uint64_t* full = &bar.vt_full[i % kVts];
+            if (!mbar_wait(&bar.vt_empty[i % kVts], ((uint32_t)(i / kVts) & 1u) ^ 1u, abort_flag)) break;
+            mbar_arrive_expect_tx(full, kVtBytes);
+            tma_load_4d(st + kRowBytes, &tmap_rec, full, 0, row, 0, 0);
+            tma_load_4d(st + kRowBytes + kTile64, &tmap_rec, full, 0, row + kC, 0, 0);
+            tma_load_4d(st, &tmap_v, full, 0, hk, t0, 0);
+            tma_load_4d(st + 8192, &tmap_v, full, 64, hk, t0, 0);
+            st = smem + kOffK + i % kKs * kRowBytes;
+            full = &bar.k_full[i % kKs];
+            if (!mbar_wait(&bar.k_empty[i % kKs], ((uint32_t)(i / kKs) & 1u) ^ 1u, abort_flag)) break;
+            mbar_arrive_expect_tx(full, kRowBytes);
+            tma_load_4d(st, &tmap_k, full, 0, hk, t0, 0);
+            tma_load_4d(st + 8192, &tmap_k, full, 64, hk, t0, 0);
+            full = &bar.sc_full[i % kScs];
+            if (!mbar_wait(&bar.sc_empty[i % kScs], ((uint32_t)(i / kScs) & 1u) ^ 1u, abort_flag)) break;
+            mbar_arrive_expect_tx(full, kScBytes);
+            bulk_load(smem + kOffSc + i % kScs * kScBytes, p.scal + (rec0 + i) * kScal, kScBytes, full);
+          }
+          const int c = i - 1;                           // what o needs comes a chunk behind
+          if (want_o && c >= 0) {
+            const int t0 = (int)(tok_in + (int64_t)c * kC), row = (int)((rec0 + c) * (3 * kC));
+            uint8_t* st = smem + kOffQr + c % kQrs * kQrBytes;
+            uint64_t* full = &bar.qr_full[c % kQrs];
+            if (!mbar_wait(&bar.qr_empty[c % kQrs], ((uint32_t)(c / kQrs) & 1u) ^ 1u, abort_flag)) break;
+            mbar_arrive_expect_tx(full, kQrBytes);
+            tma_load_4d(st, &tmap_q, full, 0, h, t0, 0);
+            tma_load_4d(st + 8192, &tmap_q, full, 64, h, t0, 0);
+            tma_load_4d(st + kRowBytes, &tmap_rec, full, 0, row + 2 * kC, 0, 0);
           }
         }
-        if (i + kStages < n_chunks) tc_commit(&bar.a1_empty[s]);    // nobody waits for the last ones
-        ok = mbar_wait(&bar.ub_ready, (uint32_t)i & 1u, abort_flag);
-        if (ok) ok = mbar_wait(&bar.y_full[s], ph, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        {
-          const uint64_t kt0 = hi_mn64 | uint64_t(((st + kA1Bytes) >> 4) & 0x3FFFu);
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // =============================== the chain's products =======================================
+      if (elect_one()) {
+        constexpr int fmt = kBf16 ? 1 : 0;
+        constexpr uint32_t idesc_w = make_idesc(128, 64, fmt, 0, 1);       // B = -W^T [k][p], MN-major
+        constexpr uint32_t idesc_s = make_idesc(128, 128, fmt, 0, 1);      // B = K [s][k], MN-major
+        constexpr uint32_t idesc_kt = make_idesc(128, 64, fmt, 1, 0);      // A = K rows [s][k], MN-major; B = Tw, K-major
+        const uint32_t base = smem_u32(smem);
+        const uint64_t wt = desc_mn(base + kOffW);
+        bool ok = true;
+        for (int i = -1; i < n_chunks && ok; ++i) {
+          const uint32_t pi = (uint32_t)i & 1u;
+          if (i >= 0) {
+            ok = mbar_wait(&bar.w_ready, pi, abort_flag) && mbar_wait(&bar.u0_done, pi, abort_flag) && mbar_wait(&bar.sb_ready, pi, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              mma_ts(tbase + kColU, tbase + kColSb + 64 * pi + kk * 8, wt + uint64_t((kk * 2048) >> 4), idesc_w, (kk > 0 || !zero_u0) ? 1u : 0u);
+            tc_commit(&bar.u_full);
+          }
+          const int n = i + 1;                           // -W^T of the next chunk, over dS^T, which has been read (sb_ready)
+          if (n < n_chunks) {
+            const uint32_t vt = base + n % kVts * kVtBytes, nkr = base + kOffK + n % kKs * kRowBytes;
+            ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && mbar_wait(&bar.k_full[n % kKs], (uint32_t)(n / kKs) & 1u, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              mma_ss(tbase + kColW, desc_mn(nkr) + uint64_t((kk * 2048) >> 4), desc_k(vt + kRowBytes) + uint64_t((kk * 32) >> 4), idesc_kt, kk > 0);
+            tc_commit(&bar.w_done);
+            tc_commit(&bar.vt_empty[n % kVts]);
+          }
+          if (i < 0) continue;
+          ok = mbar_wait(&bar.us_ready, pi, abort_flag) && (n == n_chunks || mbar_wait(&bar.w_read, pi ^ 1u, abort_flag));
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t kr = desc_mn(base + kOffK + i % kKs * kRowBytes);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_ts(tbase + kColS, tbase + kColUb + kk * 8, kt0 + uint64_t((kk * 2048) >> 4), idesc_s, kk > 0);
+            mma_ts(tbase + kColS, tbase + (kBf16 ? kColUs : kColUb) + kk * 8, kr + uint64_t((kk * 2048) >> 4), idesc_s, kk > 0);
+          tc_commit(&bar.s_done);
+          tc_commit(&bar.k_empty[i % kKs]);
         }
-        tc_commit(&bar.s_done);
-        if (want_o) {
-          const uint64_t rq0 = hi_k | uint64_t(((st + kA1Bytes + kKtBytes + kU0Bytes) >> 4) & 0x3FFFu);
+      }
+    } else if (warp == 2) {
+      // =============================== the other products =========================================
+      if (elect_one()) {
+        constexpr int fmt = kBf16 ? 1 : 0;
+        constexpr uint32_t idesc_vt = make_idesc(128, 64, fmt, 1, 0);      // A = V rows [s][v], MN-major; B = Tu, K-major
+        constexpr uint32_t idesc_n64 = make_idesc(128, 64, fmt, 0, 0);     // B = Q or Rq rows, K-major
+        const uint32_t base = smem_u32(smem);
+        bool ok = true;
+        for (int i = -1; i < n_chunks && ok; ++i) {
+          const int n = i + 1;                           // U0^T of the next chunk, once U^T of this one has been read
+          if (n < n_chunks) {
+            const uint32_t vt = base + n % kVts * kVtBytes;
+            ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && (i < 0 || mbar_wait(&bar.ub_ready, (uint32_t)i & 1u, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            if (!zero_u0) {
 #pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            mma_ts(tO, tbase + kColUb + kk * 8, rq0 + uint64_t((kk * 32) >> 4), idesc_n64, 1u);
-          tc_commit(&bar.o_done[ob]);
+              for (int kk = 0; kk < 4; ++kk)
+                mma_ss(tbase + kColU, desc_mn(vt) + uint64_t((kk * 2048) >> 4), desc_k(vt + kRowBytes + kTile64) + uint64_t((kk * 32) >> 4), idesc_vt, kk > 0);
+            }
+            tc_commit(&bar.u0_done);
+            tc_commit(&bar.vt_empty[n % kVts]);
+          }
+          if (i >= 0 && want_o) {
+            const uint32_t qr = base + kOffQr + i % kQrs * kQrBytes;
+            ok = mbar_wait(&bar.ub_ready, (uint32_t)i & 1u, abort_flag) && mbar_wait(&bar.qr_full[i % kQrs], (uint32_t)(i / kQrs) & 1u, abort_flag) &&
+                 (i == 0 || mbar_wait(&bar.o_free, (uint32_t)(i - 1) & 1u, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)
+              mma_ts(tbase + kColO1, tbase + kColSb + 64 * (i & 1) + kk * 8, desc_k(qr) + uint64_t(((kk >> 2) * 8192 + (kk & 3) * 32) >> 4), idesc_n64, kk > 0);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              mma_ts(tbase + kColO2, tbase + kColUb + kk * 8, desc_k(qr + kRowBytes) + uint64_t((kk * 32) >> 4), idesc_n64, kk > 0);
+            tc_commit(&bar.o_done);
+            tc_commit(&bar.qr_empty[i % kQrs]);
+          }
         }
-        if (i + kStages < n_chunks) tc_commit(&bar.y_empty[s]);
       }
     }
-    __syncwarp();
-  } else {
+  } else if (warp < 4 + kStateWarps) {
+    set_registers<kStateRegs, true>();
     // =============================== state warps ==================================================
-    const int quad = warp & 3, half = (warp - 2) >> 2;
+    const int quad = warp & 3, half = (warp - 4) >> 2;
     const int row = 32 * quad + lane;                    // TMEM lane = value channel v
     const uint32_t lane_base = tbase + (uint32_t(32 * quad) << 16);
 
     // where the state comes from and goes to: element (k, v) of the [dk][dv] plane, k = 64*half + j
-    const int srow = packed ? b : p.map.state_row[b];
-    const int64_t sbase = ((int64_t)srow * p.H + h) * kD * kD + (int64_t)(64 * half) * kD + row;
-    const float* s_in = p.initial_state ? p.initial_state + sbase : nullptr;
-    float* s_out = p.final_state ? p.final_state + sbase : nullptr;
-    if (packed && p.var.state_table != nullptr) {
-      float* trow = p.var.state_table + p.var.slots[b] * p.var.slot_stride + (int64_t)h * kD * kD + (int64_t)(64 * half) * kD + row;
-      s_in = (p.var.has_initial == nullptr || p.var.has_initial[b] != 0) ? trow : nullptr;
-      s_out = trow;
-    }
-    float* snap_base = nullptr;
-    if (packed && p.var.snapshots != nullptr)
-      snap_base = p.var.snapshots + ((int64_t)p.var.snap_offsets[b] * p.H + h) * kD * kD + (int64_t)(64 * half) * kD + row;
+    const int64_t plane = ((int64_t)h * kD + 64 * half) * kD + row;
+    auto table = [&] { return p.var.state_table + p.var.slots[b] * p.var.slot_stride + plane; };
+    const bool tabled = packed && p.var.state_table != nullptr;
+    const int64_t sbase = (int64_t)(packed ? b : p.map.state_row[b]) * p.H * kD * kD + plane;
 
-    float S[64];                                          // S^T[v = row][k = 64*half + j], fp32 master
+    float2 S[32];                                         // S^T[v = row][k = 64*half + j], fp32 master
+    {
+      const float* s_in = p.initial_state ? p.initial_state + sbase : nullptr;
+      if (tabled) s_in = (p.var.has_initial == nullptr || p.var.has_initial[b] != 0) ? table() : nullptr;
 #pragma unroll
-    for (int j = 0; j < 64; ++j) S[j] = s_in ? s_in[(int64_t)j * kD] : 0.f;
-    if (n_chunks == 0 && s_out != nullptr && s_out != s_in) {
-#pragma unroll
-      for (int j = 0; j < 64; ++j) s_out[(int64_t)j * kD] = S[j];
+      for (int j = 0; j < 32; ++j) S[j] = s_in ? make_float2(s_in[2 * j * kD], s_in[(2 * j + 1) * kD]) : make_float2(0.f, 0.f);
     }
+    auto put = [&](float* dst) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) { dst[2 * j * kD] = S[j].x; dst[(2 * j + 1) * kD] = S[j].y; }
+    };
     bool ok = true;
-    float g_next = n_chunks > 0 ? gcs[0] : 0.f;           // g_C of chunk i - 1, fetched one iteration ahead
-    for (int i = 0; i <= n_chunks && n_chunks > 0; ++i) {
-      const float gC = g_next;
-      if (i < n_chunks) g_next = gcs[i];
-      // ---- state phase: after this block S is the state before chunk i ---------------------------
+    float gC = 0.f;                                       // decay over the chunk before
+    for (int i = 0; i <= n_chunks; ++i) {
+      const uint32_t sb = lane_base + kColSb + 64 * (i & 1) + 32 * half;
+      // ---- state phase: after this block S is the state before chunk i, its 16-bit copy the A operand of U and O1 ------
       if (i > 0) {
-        ok = mbar_wait(&bar.s_done, (uint32_t)(i - 1) & 1u, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp(&bar.s_done, (uint32_t)(i - 1) & 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        uint32_t d[64];
-        tmem_ld32_nowait(lane_base + kColS + 64 * half, &d[0]);
-        tmem_ld32_nowait(lane_base + kColS + 64 * half + 32, &d[32]);
-        tmem_ld_wait();
+        uint32_t d[2][16];
+        tmem_ld16_nowait(lane_base + kColS + 64 * half, d[0]);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) { reg_fence(d[j]); S[j] = fmaf(gC, S[j], __uint_as_float(d[j])); }
-      }
-      if (i < n_chunks) {                               // 16-bit copy of S^T: the A operand of MMA1a/b
-        uint32_t w[32];
+        for (int part = 0; part < 4; ++part) {            // the next 16 columns are on their way while these are added
+          uint32_t(&x)[16] = d[part & 1];
+          tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) w[j] = pack2<kBf16>(S[2 * j], S[2 * j + 1]);
-        tmem_st32(lane_base + kColSb + 32 * half, w);
-        tmem_st_wait();
-        tc_fence_before();                                // also: the dS^T columns have been read, MMA2a may overwrite them
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.sb_ready);
-      }
-      // snapshot / final state: the state after i chunks
-      if (i > 0 && snap_base != nullptr && (i % p.var.snap_chunks) == 0 && tok_base + (int64_t)i * kC <= tok_end) {
-        float* dst = snap_base + (int64_t)(i / p.var.snap_chunks - 1) * p.H * kD * kD;
+          for (int j = 0; j < 16; ++j) reg_fence(x[j]);
+          if (part < 3) tmem_ld16_nowait(lane_base + kColS + 64 * half + 16 * (part + 1), d[(part + 1) & 1]);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) dst[(int64_t)j * kD] = S[j];
-      }
-      if (i == n_chunks && s_out != nullptr) {
+          for (int j = 0; j < 8; ++j)
+            S[8 * part + j] = __ffma2_rn(make_float2(gC, gC), S[8 * part + j], make_float2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1])));
+          uint32_t w[8];
 #pragma unroll
-        for (int j = 0; j < 64; ++j) s_out[(int64_t)j * kD] = S[j];
+          for (int j = 0; j < 8; ++j) w[j] = pack2<kBf16>(S[8 * part + j].x, S[8 * part + j].y);
+          tmem_st8(sb + 8 * part, w);
+        }
+      } else {
+#pragma unroll
+        for (int part = 0; part < 4; ++part) {
+          uint32_t w[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) w[j] = pack2<kBf16>(S[8 * part + j].x, S[8 * part + j].y);
+          tmem_st8(sb + 8 * part, w);
+        }
       }
+      tmem_st_wait();
+      tc_fence_before();                                  // also: the dS^T columns have been read, the next may overwrite them
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.sb_ready);          // nobody waits for the last one
+      // snapshot: the state after i chunks
+      if (packed && p.var.snapshots != nullptr && i > 0 && (i % p.var.snap_chunks) == 0 && tok_base + (int64_t)i * kC <= tok_end)
+        put(p.var.snapshots + ((int64_t)p.var.snap_offsets[b] + i / p.var.snap_chunks - 1) * p.H * kD * kD + plane);
+      if (i == n_chunks) break;
 
-      // ---- O^T of the previous chunk, one chunk behind: thread (v, half) holds rows p = 32*half .. +31 ----
-      if (want_o && i > 0) {
-        const int ci = i - 1, ob = ci & 1;
-        ok = mbar_wait(&bar.o_done[ob], (uint32_t)(ci >> 1) & 1u, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        uint32_t r[32];
-        tmem_ld32(lane_base + kColO + ob * 64 + 32 * half, r);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.o_free[ob]);
-        const int64_t t0 = tok_base + (int64_t)ci * kC + 32 * half;
-        uint16_t* ocol = reinterpret_cast<uint16_t*>(p.o) + (t0 * p.H + h) * kD + row;
-        const int n_ok = (int)min((int64_t)32, tok_end - t0);
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (j < n_ok) ocol[(int64_t)j * p.H * kD] = (uint16_t)(pack2<kBf16>(__uint_as_float(r[j]), 0.f) & 0xffffu);
-      }
-
-      // ---- U^T of this chunk: all 128 lanes, chunk rows 32*half .. +31 ------------------------------
-      if (i < n_chunks) {
-        const int s = i % kStages;
-        const uint32_t ph = (uint32_t)(i / kStages) & 1u;
-        ok = mbar_wait(&bar.u_full, (uint32_t)i & 1u, abort_flag);
-        if (ok && !zero_u0) ok = mbar_wait(&bar.y_full[s], ph, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
+      // ---- U^T of this chunk: chunk rows 32*half .. +31, as it is and scaled ------------------------------
+      const float* sc = reinterpret_cast<const float*>(smem + kOffSc + i % kScs * kScBytes);
+      ok = mbar_wait_warp(&bar.sc_full[i % kScs], (uint32_t)(i / kScs) & 1u, abort_flag);
+      if (!ok) break;
+      gC = sc[kScalG];
+      ok = mbar_wait_warp(&bar.u_full, (uint32_t)i & 1u, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      {
         uint32_t r[32];
         tmem_ld32(lane_base + kColU + 32 * half, r);
-        const uint8_t* u0_box = smem + s * kStageBytes + kA1Bytes + kKtBytes;
-        uint32_t ow[16];
+        if constexpr (kBf16) {
+          uint32_t w[16];
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          uint4 u0 = make_uint4(0u, 0u, 0u, 0u);
-          if (!zero_u0) u0 = *reinterpret_cast<const uint4*>(u0_box + box_off(row, 4 * half + ch));
-          const uint32_t uw[4] = {u0.x, u0.y, u0.z, u0.w};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 f = unpack2<kBf16>(uw[e]);
-            ow[4 * ch + e] = pack2<kBf16>(__uint_as_float(r[8 * ch + 2 * e]) + f.x, __uint_as_float(r[8 * ch + 2 * e + 1]) + f.y);
+          for (int j = 0; j < 16; j += 2) {
+            const float4 ks = *reinterpret_cast<const float4*>(sc + kScalK + 32 * half + 2 * j);
+            const float2 x = __fmul2_rn(make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), make_float2(ks.x, ks.y));
+            const float2 y = __fmul2_rn(make_float2(__uint_as_float(r[2 * j + 2]), __uint_as_float(r[2 * j + 3])), make_float2(ks.z, ks.w));
+            w[j] = pack2<kBf16>(x.x, x.y);
+            w[j + 1] = pack2<kBf16>(y.x, y.y);
           }
+          tmem_st16(lane_base + kColUs + 16 * half, w);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar.us_ready);
         }
-        tmem_st16(lane_base + kColUb + 16 * half, ow);
+        // the products of o one chunk back have read the plain copy, and the S^T that the next one will take the place of
+        if (want_o && i > 0 && !(ok = mbar_wait_warp(&bar.o_done, (uint32_t)(i - 1) & 1u, abort_flag))) break;
+        uint32_t w[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) w[j] = pack2<kBf16>(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+        tmem_st16(lane_base + kColUb + 16 * half, w);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.ub_ready);
+        if (lane == 0) {
+          if constexpr (!kBf16) mbar_arrive(&bar.us_ready);
+          mbar_arrive(&bar.ub_ready);
+          mbar_arrive(&bar.sc_empty[i % kScs]);
+        }
       }
-
+    }
+    if (ok) {
+      if (tabled) put(table());
+      else if (p.final_state != nullptr) put(p.final_state + sbase);
+    }
+  } else if (warp < 4 + kStateWarps + kHelpWarps) {
+    set_registers<kOtherRegs, false>();
+    // =============================== W warps ======================================================
+    const int row = 32 * (warp & 3) + lane;              // TMEM lane: key channel
+    const uint32_t lane_base = tbase + (uint32_t(32 * (warp & 3)) << 16);
+    for (int i = 0; i < n_chunks; ++i) {
+      const float* sc = reinterpret_cast<const float*>(smem + kOffSc + i % kScs * kScBytes);
+      if constexpr (!kBf16) {
+        if (!mbar_wait_warp(&bar.sc_full[i % kScs], (uint32_t)(i / kScs) & 1u, abort_flag)) break;
+      }
+      if (!mbar_wait_warp(&bar.w_done, (uint32_t)i & 1u, abort_flag)) break;       // the chain's product with the one before is done, too
+      tc_fence_after();
+      uint32_t w[32];
+#pragma unroll
+      for (int hh = 0; hh < 4; ++hh) {
+        uint32_t r[16];
+        tmem_ld16(lane_base + kColW + 16 * hh, r);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) w[8 * hh + e] = pack2<kBf16>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.w_read);
+      uint8_t* wt = smem + kOffW;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(wt + box_off(row, c)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+      if constexpr (!kBf16) {                            // K rows times (g_C / g) k_inv, in place: row row / 2, one box of it
+        const float f = sc[kScalK + (row >> 1)];
+        uint8_t* kr = smem + kOffK + i % kKs * kRowBytes + (row & 1) * 8192;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          uint4* at = reinterpret_cast<uint4*>(kr + box_off(row >> 1, c));
+          const uint4 u = *at;
+          const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+          uint32_t y[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 v = unpack2<kBf16>(x[e]);
+            y[e] = pack2<kBf16>(v.x * f, v.y * f);
+          }
+          *at = make_uint4(y[0], y[1], y[2], y[3]);
+        }
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&bar.w_ready);
+        if constexpr (!kBf16) mbar_arrive(&bar.sc_empty[i % kScs]);
+      }
+    }
+  } else {
+    set_registers<kOtherRegs, false>();
+    // =============================== O warps ======================================================
+    const int row = 32 * (warp & 3) + lane;              // TMEM lane: value channel
+    const uint32_t lane_base = tbase + (uint32_t(32 * (warp & 3)) << 16);
+    const int64_t orow = (int64_t)p.H * kD;
+    for (int i = 0; i < n_chunks; ++i) {
+      if (!mbar_wait_warp(&bar.sc_full[i % kScs], (uint32_t)(i / kScs) & 1u, abort_flag)) break;
+      if (!want_o) {                                     // not before the scalars are there: an arrival belongs to one use of their place
+        if (lane == 0) mbar_arrive(&bar.sc_empty[i % kScs]);
+        continue;
+      }
+      if (!mbar_wait_warp(&bar.o_done, (uint32_t)i & 1u, abort_flag)) break;
+      tc_fence_after();
+      const float* qs = reinterpret_cast<const float*>(smem + kOffSc + i % kScs * kScBytes) + kScalQ;
+      const int n_ok = (int)min((int64_t)kC, tok_end - (tok_base + (int64_t)i * kC));
+      uint16_t* first = static_cast<uint16_t*>(p.o) + ((tok_base + (int64_t)i * kC) * p.H + h) * kD + row;
+#pragma unroll 1
+      for (int hh = 0; hh < 4; ++hh) {
+        uint32_t x[16], y[16], w[8];                     // w: rows 2 j and 2 j + 1
+        tmem_ld16_nowait(lane_base + kColO1 + 16 * hh, x);
+        tmem_ld16_nowait(lane_base + kColO2 + 16 * hh, y);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          const float4 f = *reinterpret_cast<const float4*>(qs + 16 * hh + 2 * j);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { reg_fence(x[2 * j + e]); reg_fence(y[2 * j + e]); }
+          const float2 a = __ffma2_rn(make_float2(f.x, f.y), make_float2(__uint_as_float(x[2 * j]), __uint_as_float(x[2 * j + 1])),
+                                      make_float2(__uint_as_float(y[2 * j]), __uint_as_float(y[2 * j + 1])));
+          const float2 b2 = __ffma2_rn(make_float2(f.z, f.w), make_float2(__uint_as_float(x[2 * j + 2]), __uint_as_float(x[2 * j + 3])),
+                                       make_float2(__uint_as_float(y[2 * j + 2]), __uint_as_float(y[2 * j + 3])));
+          w[j] = pack2<kBf16>(a.x, a.y);
+          w[j + 1] = pack2<kBf16>(b2.x, b2.y);
+        }
+        if (hh == 3) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) { mbar_arrive(&bar.o_free); mbar_arrive(&bar.sc_empty[i % kScs]); }
+        }
+        if constexpr (kWide) {
+          // two lanes swap halves, so that an even one stores two channels of the even row, an odd one of the odd row
+          uint32_t* dst = reinterpret_cast<uint32_t*>(first - (lane & 1) + ((lane & 1) + 16 * hh) * orow);
+          const uint32_t pick = lane & 1 ? 0x3276u : 0x5410u;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const uint32_t other = __shfl_xor_sync(0xffffffffu, w[j], 1);
+            if (16 * hh + 2 * j + (lane & 1) < n_ok) *dst = __byte_perm(w[j], other, pick);
+            dst += orow;
+          }
+        } else {
+          uint16_t* dst = first + 16 * hh * orow;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (16 * hh + j < n_ok) *dst = (uint16_t)(w[j >> 1] >> (16 * (j & 1)));
+            dst += orow;
+          }
+        }
+      }
     }
   }
 
@@ -348,44 +505,35 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_rec, const __gr
   if (warp == 1) tmem_dealloc(tbase, 512);
 }
 
-int make_record_maps(CUtensorMap* rec, CUtensorMap* rq, const uint8_t* recs, int is_bf16, int64_t n_records) {
-  {
-    const uint64_t rows = (uint64_t)n_records * kRecRows;
-    const uint64_t dims[4] = {128, rows, 1, 1};
-    const int64_t strides[3] = {128, (int64_t)rows * 128, (int64_t)rows * 128};
-    const uint32_t box[4] = {64, 64, 1, 1};
-    int rc = make_tmap_16bit_4d(rec, recs, is_bf16, dims, strides, box);
-    if (rc != ATMA_OK) return rc;
-  }
-  const uint64_t rows = (uint64_t)n_records * kRecRowsRq;
-  const uint64_t dims[4] = {64, rows, 1, 1};
-  const int64_t strides[3] = {64, (int64_t)rows * 64, (int64_t)rows * 64};
-  const uint32_t box[4] = {64, 64, 1, 1};
-  return make_tmap_16bit_4d(rq, recs, is_bf16, dims, strides, box);
-}
-
 }  // namespace
 
-int gated_delta_recur_sm100(const uint8_t* recs, const float* gcs, int is_bf16, int64_t n_records, const float* initial_state,
-                            void* o, float* final_state, int Tlen, int H, int NC, int n_rec, const RecMap& map,
-                            const VarLen& var, cudaStream_t st) {
+int gated_delta_recur_sm100(const Rows& rows, const uint8_t* recs, const float* scal, int64_t n_records, const float* initial_state,
+                            void* o, float* final_state, int Tlen, int NC, int n_rec, const RecMap& map, const VarLen& var,
+                            cudaStream_t st) {
   if (n_rec <= 0 || n_records <= 0) return ATMA_OK;
-  if (n_records * kRecRowsRq >= (int64_t(1) << 31))
+  if (n_records * 3 * kC >= (int64_t(1) << 31))
     return fail(ATMA_ERR_INVALID, "gated_delta_scan: %lld chunk records exceed the tensor-map row range", (long long)n_records);
-  CUtensorMap mrec, mrq;
-  int rc = make_record_maps(&mrec, &mrq, recs, is_bf16, n_records);
+  if (rows.tokens >= (int64_t(1) << 31)) return fail(ATMA_ERR_INVALID, "gated_delta_scan: %lld tokens exceed the tensor-map range", (long long)rows.tokens);
+  CUtensorMap mq, mk, mv, mr;
+  int rc = make_rows_map(&mq, rows.q, rows.is_bf16, rows.H, rows.tokens);
+  if (rc == ATMA_OK) rc = make_rows_map(&mk, rows.k, rows.is_bf16, rows.Hkv, rows.tokens);
+  if (rc == ATMA_OK) rc = make_rows_map(&mv, rows.v, rows.is_bf16, rows.Hkv, rows.tokens);
+  if (rc == ATMA_OK) {
+    const uint64_t n = (uint64_t)n_records * 3 * kC;                 // a record as rows of 64 values
+    const uint64_t dims[4] = {64, n, 1, 1};
+    const int64_t strides[3] = {64, (int64_t)n * 64, (int64_t)n * 64};
+    const uint32_t box[4] = {64, 64, 1, 1};
+    rc = make_tmap_16bit_4d(&mr, recs, rows.is_bf16, dims, strides, box);
+  }
   if (rc != ATMA_OK) return rc;
   Params p{};
-  p.gcs = gcs; p.initial_state = initial_state; p.o = o; p.final_state = final_state;
-  p.Tlen = Tlen; p.H = H; p.NC = NC; p.is_bf16 = is_bf16; p.map = map; p.var = var;
-  const dim3 grid(H, n_rec);
-  if (is_bf16) {
-    ATMA_CUDA_OK(cudaFuncSetAttribute(scan_recur_sm100_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    scan_recur_sm100_kernel<true><<<grid, kThreads, kSmemBytes, st>>>(mrec, mrq, p);
-  } else {
-    ATMA_CUDA_OK(cudaFuncSetAttribute(scan_recur_sm100_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    scan_recur_sm100_kernel<false><<<grid, kThreads, kSmemBytes, st>>>(mrec, mrq, p);
-  }
+  p.scal = scal; p.initial_state = initial_state; p.o = o; p.final_state = final_state;
+  p.Tlen = Tlen; p.H = rows.H; p.Hkv = rows.Hkv; p.NC = NC; p.map = map; p.var = var;
+  const bool wide = (reinterpret_cast<uintptr_t>(o) & 3) == 0;
+  auto kernel = rows.is_bf16 ? (wide ? scan_recur_sm100_kernel<true, true> : scan_recur_sm100_kernel<true, false>)
+                             : (wide ? scan_recur_sm100_kernel<false, true> : scan_recur_sm100_kernel<false, false>);
+  ATMA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+  kernel<<<dim3(rows.H, n_rec), kThreads, kSmemBytes, st>>>(mq, mk, mv, mr, p);
   return launch_status("gated_delta_scan (recurrence, tcgen05)");
 }
 

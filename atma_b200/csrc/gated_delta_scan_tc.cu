@@ -2,13 +2,15 @@
 // tensor-core path.
 //
 // Same factorisation as the fp32 kernel (gated_delta_scan.cu):
-//   per chunk, independent of the state:  -W = -T diag(beta g) K,  U0 = T diag(beta) V,
-//       Qg = diag(g) Q,  Kt = diag(g_C/g) K,  Rq = tril((g_p/g_s) q_p.k_s),  T = (I + A)^-1
-//   per chunk, on the state S [dk][dv]:    U = U0 - W S;  O = Qg S + Rq U;  S <- g_C S + Kt^T U
+//   per chunk, independent of the state:  T = (I + A)^-1,  Rq = tril((g_p/g_s) q_p.k_s)
+//   per chunk, on the state S [dk][dv]:    U = T diag(beta) (V - diag(g) K S);  O = diag(g) Q S + Rq U;
+//       S <- g_C S + (diag(g_C/g) K)^T U
 // The chunk-local factors come from the tcgen05 kernel of gated_delta_local_sm100.cu (one record
 // per chunk and head in scratch memory), the recurrence over the chunks from the tcgen05 kernel of
 // gated_delta_scan_sm100.cu.  This file lays out the scratch, builds the packed-batch chunk
 // offsets and sequences the two launches.
+#include <tuple>
+
 #include "common.cuh"
 #include "gated_delta_scan.cuh"
 
@@ -27,6 +29,15 @@ __global__ void varlen_chunk_offsets_kernel(const int32_t* __restrict__ cu_seqle
       acc += (len + kC - 1) / kC;
       cu_chunks[i + 1] = acc;
     }
+  }
+}
+
+// The rows that a later call walks the factors of: dst (tokens, H, 128) from src (tokens, Hs, 128), heads repeated.
+__global__ void keep_rows_kernel(uint4* __restrict__ dst, const uint4* __restrict__ src, int64_t n, int H, int Hs) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t head = i >> 4, token = head / H;               // 16 pieces of 16 bytes per head
+    const int h = (int)(head - token * H) / (H / Hs);
+    dst[i] = src[((token * Hs + h) << 4) + (i & 15)];
   }
 }
 
@@ -120,12 +131,10 @@ bool gated_delta_scan_mma_supported(int dtype, int dk, int dv) {
   return (dtype == ATMA_BF16 || dtype == ATMA_F16) && dk == kD && dv == kD;
 }
 
-static int64_t record_bytes(int B, int T, int H) {
-  const int64_t NC = (T + kC - 1) / kC;
-  return ((int64_t)B * H * NC * kRecBytes + 255) / 256 * 256 + ((int64_t)B * H * NC * sizeof(float) + 255) / 256 * 256;
-}
+static int64_t round256(int64_t n) { return (n + 255) / 256 * 256; }
+static int64_t record_bytes(int B, int T, int H) { return round256((int64_t)B * H * ((T + kC - 1) / kC) * kScratchPerChunk); }
 
-// records | g_C | workspace of the segmented recurrence (sized for the largest segment count)
+// records | scalars of every chunk | rows kept for scan_recur | workspace of the segmented recurrence (sized for the largest segment count)
 int64_t gated_delta_scan_mma_scratch_bytes(int B, int T, int H) {
   const int NC = (T + kC - 1) / kC;
   int64_t ws = 0;
@@ -134,26 +143,31 @@ int64_t gated_delta_scan_mma_scratch_bytes(int B, int T, int H) {
   return record_bytes(B, T, H) + ws + 256;
 }
 
-static float* gc_array(void* scratch, int B, int H, int NC) {
-  uint8_t* recs = static_cast<uint8_t*>(scratch);
-  return reinterpret_cast<float*>(recs + (((int64_t)B * H * NC * kRecBytes + 255) / 256) * 256);
+static float* scal_array(void* scratch, int64_t n_records) { return reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + n_records * kRecBytes); }
+
+// where scan_factors keeps the rows: all heads, q | k | v
+static Rows kept_rows(void* scratch, int dtype, int B, int T, int H) {
+  const int64_t n = (int64_t)B * H * ((T + kC - 1) / kC), each = (int64_t)B * T * H * kD * 2;
+  uint8_t* at = static_cast<uint8_t*>(scratch) + n * (kRecBytes + kScal * 4);
+  return Rows{at, at + each, at + 2 * each, dtype == ATMA_BF16, H, H, (int64_t)B * T};
 }
 
-// Kernel A only: the chunk-local factors of B sequences into `scratch`.
+// Kernel A only: the chunk-local factors of B sequences into `scratch`, and the rows with them.
 int gated_delta_scan_mma_factors(const void* q, const void* k, const void* v, int dtype, const float* g,
                                  const float* beta, void* scratch, int B, int T, int H, int Hkv, int normalize_qk,
                                  float scale, cudaStream_t st) {
   const int NC = (T + kC - 1) / kC;
-  uint8_t* recs = static_cast<uint8_t*>(scratch);
-  float* gcs = gc_array(scratch, B, H, NC);
-  return gated_delta_local_sm100(q, k, v, dtype == ATMA_BF16, g, beta, recs, gcs, B, T, H, Hkv, NC, normalize_qk, scale, VarLen{},
-                                 (int64_t)B * T, st);
+  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T}, keep = kept_rows(scratch, dtype, B, T, H);
+  const int64_t n = (int64_t)B * T * H * 16;
+  const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
+  for (const auto& [to, from, heads] : {std::make_tuple(keep.q, q, H), std::make_tuple(keep.k, k, Hkv), std::make_tuple(keep.v, v, Hkv)})
+    keep_rows_kernel<<<grid, 256, 0, st>>>(static_cast<uint4*>(const_cast<void*>(to)), static_cast<const uint4*>(from), n, H, heads);
+  return gated_delta_local_sm100(rows, g, beta, static_cast<uint8_t*>(scratch), scal_array(scratch, (int64_t)B * H * NC), B, T, NC,
+                                 normalize_qk, scale, VarLen{}, st);
 }
 
-// Kernel B only: n_rec recurrences over the factors of a scratch built for B sequences.
-int gated_delta_scan_mma_recur(void* scratch, int dtype, int B, int T, int H, int n_rec, const int* rec_of,
-                               const int* zero_u0, const float* initial_state, void* o, float* final_state,
-                               cudaStream_t st) {
+static int recur_over(const Rows& rows, void* scratch, int B, int T, int n_rec, const int* rec_of, const int* zero_u0,
+                      const float* initial_state, void* o, float* final_state, cudaStream_t st) {
   const int NC = (T + kC - 1) / kC;
   if (n_rec < 1 || n_rec > kMaxRec) return fail(ATMA_ERR_INVALID, "gated_delta_scan_recur: n_rec=%d outside 1..%d", n_rec, kMaxRec);
   RecMap map{};
@@ -165,14 +179,20 @@ int gated_delta_scan_mma_recur(void* scratch, int dtype, int B, int T, int H, in
     if (map.rec[i] < 0 || map.rec[i] >= B)
       return fail(ATMA_ERR_INVALID, "gated_delta_scan_recur: rec_of[%d]=%d outside the %d factor sets", i, map.rec[i], B);
   }
-  const uint8_t* recs = static_cast<const uint8_t*>(scratch);
-  const float* gcs = gc_array(scratch, B, H, NC);
-  return gated_delta_recur_sm100(recs, gcs, dtype == ATMA_BF16, (int64_t)B * H * NC, initial_state, o, final_state, T, H, NC,
+  const int64_t n = (int64_t)B * rows.H * NC;
+  return gated_delta_recur_sm100(rows, static_cast<const uint8_t*>(scratch), scal_array(scratch, n), n, initial_state, o, final_state, T, NC,
                                  n_rec, map, VarLen{}, st);
 }
 
+// Kernel B only: n_rec recurrences over the factors of a scratch built for B sequences.
+int gated_delta_scan_mma_recur(void* scratch, int dtype, int B, int T, int H, int n_rec, const int* rec_of,
+                               const int* zero_u0, const float* initial_state, void* o, float* final_state,
+                               cudaStream_t st) {
+  return recur_over(kept_rows(scratch, dtype, B, T, H), scratch, B, T, n_rec, rec_of, zero_u0, initial_state, o, final_state, st);
+}
+
 // Packed batch: chunk offsets, factors of every chunk, one recurrence per sequence, all in one go.
-// Scratch layout: records of NCu = total/64 + n_seqs chunks per head | g_C | cu_chunks.
+// Scratch layout: records of NCu = total/64 + n_seqs chunks per head | scalars | cu_chunks.
 int64_t gated_delta_scan_mma_varlen_scratch_bytes(int64_t total_tokens, int n_seqs, int H) {
   const int64_t NCu = total_tokens / kC + n_seqs;
   return record_bytes(1, (int)(NCu * kC), H) + (((int64_t)n_seqs + 1) * 4 + 255) / 256 * 256 + 256;
@@ -186,15 +206,14 @@ int gated_delta_scan_mma_varlen(const void* q, const void* k, const void* v, int
                                 cudaStream_t st) {
   const int NCu = (int)(total_tokens / kC) + n_seqs;          // upper bound on the chunk count
   uint8_t* recs = static_cast<uint8_t*>(scratch);
-  float* gcs = gc_array(scratch, 1, H, NCu);
+  float* scal = scal_array(scratch, (int64_t)H * NCu);
   int32_t* cu_chunks = reinterpret_cast<int32_t*>(recs + record_bytes(1, NCu * kC, H));
   varlen_chunk_offsets_kernel<<<1, 32, 0, st>>>(cu_seqlens, cu_chunks, n_seqs);
   VarLen var{cu_seqlens, cu_chunks, n_seqs, slots, has_initial, state_table, slot_stride, snapshots, snap_offsets, snap_chunks};
-  const bool bf = dtype == ATMA_BF16;
-  int rc = gated_delta_local_sm100(q, k, v, bf, g, beta, recs, gcs, 1, 0, H, Hkv, NCu, normalize_qk, scale, var, total_tokens, st);
+  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, total_tokens};
+  int rc = gated_delta_local_sm100(rows, g, beta, recs, scal, 1, 0, NCu, normalize_qk, scale, var, st);
   if (rc != ATMA_OK) return rc;
-  return gated_delta_recur_sm100(recs, gcs, bf, (int64_t)H * NCu, initial_state, o, final_state, 0, H, NCu, n_seqs, RecMap{}, var,
-                                 st);
+  return gated_delta_recur_sm100(rows, recs, scal, (int64_t)H * NCu, initial_state, o, final_state, 0, NCu, n_seqs, RecMap{}, var, st);
 }
 
 // The whole scan.  `segments`: 1 = one recurrence per sequence; n > 1 = cut every sequence into n
@@ -207,13 +226,14 @@ int gated_delta_scan_mma_varlen(const void* q, const void* k, const void* v, int
 int gated_delta_scan_mma(const void* q, const void* k, const void* v, int dtype, const float* g, const float* beta,
                          const float* initial_state, void* o, float* final_state, void* scratch, int B, int T, int H,
                          int Hkv, int normalize_qk, float scale, int segments, cudaStream_t st) {
-  int rc = gated_delta_scan_mma_factors(q, k, v, dtype, g, beta, scratch, B, T, H, Hkv, normalize_qk, scale, st);
-  if (rc != ATMA_OK) return rc;
   const int NC = (T + kC - 1) / kC;
+  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T};
+  const uint8_t* recs = static_cast<const uint8_t*>(scratch);
+  float* scal = scal_array(scratch, (int64_t)B * H * NC);
+  int rc = gated_delta_local_sm100(rows, g, beta, static_cast<uint8_t*>(scratch), scal, B, T, NC, normalize_qk, scale, VarLen{}, st);
+  if (rc != ATMA_OK) return rc;
   const int NS = segments == 1 ? 1 : gated_delta_scan_segments(B, H, NC, segments);
   if (NS >= 2) {
-    const uint8_t* recs = static_cast<const uint8_t*>(scratch);
-    const float* gcs = gc_array(scratch, B, H, NC);
     float* ws = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + record_bytes(B, T, H));
     const int per_row = 2 * NS - 1, n1 = B * per_row, n2 = B * (NS - 1);
     const int64_t plane = (int64_t)H * kD * kD;
@@ -239,7 +259,6 @@ int gated_delta_scan_mma(const void* q, const void* k, const void* v, int dtype,
         m2.c_end[i] = (s + 1) * seg < NC ? (s + 1) * seg : NC;
       }
     }
-    const bool bf = dtype == ATMA_BF16;
     rc = launch_status("gated_delta_scan (segment setup)");
     if (rc != ATMA_OK) return rc;
     // pass 1 is one launch: the segment-0 recurrences write o, the (P, Q) recurrences carry state only
@@ -248,13 +267,13 @@ int gated_delta_scan_mma(const void* q, const void* k, const void* v, int dtype,
       m1.state_row[i] = i;
       if ((i % per_row) != 0) m1.o_row[i] = -1;
     }
-    rc = gated_delta_recur_sm100(recs, gcs, bf, (int64_t)B * H * NC, init1, o, fin1, T, H, NC, n1, m1, VarLen{}, st);
+    rc = gated_delta_recur_sm100(rows, recs, scal, (int64_t)B * H * NC, init1, o, fin1, T, NC, n1, m1, VarLen{}, st);
     if (rc != ATMA_OK) return rc;
     seg_compose_kernel<<<dim3(kD / 16, H, B), 256, 0, st>>>(fin1, init2, final_state, H, NS);
     rc = launch_status("gated_delta_scan (segment states)");
     if (rc != ATMA_OK) return rc;
     for (int i = 0; i < n2; ++i) m2.state_row[i] = i;
-    return gated_delta_recur_sm100(recs, gcs, bf, (int64_t)B * H * NC, init2, o, nullptr, T, H, NC, n2, m2, VarLen{}, st);
+    return gated_delta_recur_sm100(rows, recs, scal, (int64_t)B * H * NC, init2, o, nullptr, T, NC, n2, m2, VarLen{}, st);
   }
   int done = 0;
   while (done < B) {                                  // at most kMaxRec recurrences per launch
@@ -262,9 +281,8 @@ int gated_delta_scan_mma(const void* q, const void* k, const void* v, int dtype,
     int rec_of[kMaxRec];
     for (int i = 0; i < n; ++i) rec_of[i] = done + i;
     const int64_t so = (int64_t)done * H * kD * kD, oo = (int64_t)done * T * H * kD;
-    rc = gated_delta_scan_mma_recur(scratch, dtype, B, T, H, n, rec_of, nullptr,
-                                    initial_state ? initial_state + so : nullptr,
-                                    o ? (void*)((uint16_t*)o + oo) : nullptr, final_state ? final_state + so : nullptr, st);
+    rc = recur_over(rows, scratch, B, T, n, rec_of, nullptr, initial_state ? initial_state + so : nullptr,
+                    o ? (void*)((uint16_t*)o + oo) : nullptr, final_state ? final_state + so : nullptr, st);
     if (rc != ATMA_OK) return rc;
     done += n;
   }

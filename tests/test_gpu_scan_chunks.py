@@ -1,0 +1,70 @@
+"""The tensor-core scan where its chunks, halves and rings begin and end, and the forms of its two stages."""
+
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+import atma_b200
+import oracle
+from atma_b200 import _lib
+from atma_b200.gated_delta import scan_factors, scan_recur
+from conftest import max_rel
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(B, T, H, Hkv, dtype, seed, spread=0.0):
+    """``spread``: rows of k and q are scaled by powers of two up to 2^+-spread, which the normalisation takes out again."""
+    g = torch.Generator().manual_seed(seed)
+    q, k, v = (torch.randn(B, T, n, 128, generator=g) for n in (H, Hkv, Hkv))
+    if spread:
+        q, k = (x * 2.0 ** torch.empty(B, T, x.shape[2], 1).uniform_(-spread, spread, generator=g).round() for x in (q, k))
+    glog = F.logsigmoid(torch.randn(B, T, H, generator=g) + 2.0)
+    beta = torch.sigmoid(torch.randn(B, T, H, generator=g))
+    return [x.to(dtype) for x in (q, k, v)] + [glog, beta, torch.randn(B, H, 128, 128, generator=g) * 0.3]
+
+
+@pytest.mark.parametrize("spread", [0.0, 5.0])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H,Hkv", [(1, 1, 1, 1), (2, 63, 2, 1), (1, 64, 4, 2), (3, 65, 2, 2), (1, 127, 8, 2), (1, 193, 4, 1), (2, 449, 3, 3)])
+def test_chunk_edges(B, T, H, Hkv, dtype, spread):
+    q, k, v, glog, beta, S0 = inputs(B, T, H, Hkv, dtype, T + H, spread)
+    rep = lambda x: x.repeat_interleave(H // Hkv, 2)  # noqa: E731
+    o_ref, S_ref = oracle.chunk_gated_delta_rule_oracle(q, rep(k), rep(v), glog, beta, initial_state=S0)
+    o, S = atma_b200.chunk_gated_delta_rule(q=q.cuda(), k=k.cuda(), v=v.cuda(), g=glog.cuda(), beta=beta.cuda(), scale=1.0,
+                                            initial_state=S0.cuda(), output_final_state=True, use_qk_l2norm_in_kernel=True)
+    assert max_rel(o, o_ref) < 2e-2 and max_rel(S, S_ref) < 2e-2          # 16-bit operands, as for the other sizes of this scan
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H,Hkv", [(2, 320, 4, 2), (1, 1000, 2, 1)])
+def test_two_calls_equal_one(B, T, H, Hkv, dtype):
+    """scan_factors keeps the rows that scan_recur needs, so the inputs may change in between."""
+    q, k, v, glog, beta, S0 = (x.cuda() for x in inputs(B, T, H, Hkv, dtype, 5))
+    o, S = atma_b200.chunk_gated_delta_rule(q=q, k=k, v=v, g=glog, beta=beta, scale=1.0, initial_state=S0, output_final_state=True,
+                                            use_qk_l2norm_in_kernel=True, segments=1)
+    f = scan_factors(q, k, v, glog, beta)
+    for x in (q, k, v):
+        x.zero_()
+    o2, S2 = scan_recur(f, list(range(B)), initial_state=S0)
+    assert torch.equal(o, o2) and torch.equal(S, S2)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_outputs_two_bytes_off(dtype):
+    """o may start at any 16-bit value: from an odd one its values are stored one by one."""
+    B, T, H, Hkv = 2, 150, 3, 1
+    q, k, v, glog, beta, S0 = (x.cuda() for x in inputs(B, T, H, Hkv, dtype, 9))
+    lib = _lib.load()
+    scratch = torch.empty(lib.atma_gated_delta_scan_scratch_bytes(B, T, H, 128, 128), dtype=torch.uint8, device="cuda")
+    out = []
+    for off in (0, 1):
+        buf = torch.full((B * T * H * 128 + 2,), 7.0, dtype=dtype, device="cuda")
+        _lib.check(lib.atma_gated_delta_scan(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.dtype_code(q), _lib.ptr(glog), _lib.ptr(beta),
+                                             _lib.ptr(S0), ctypes.c_void_p(buf.data_ptr() + 2 * off), None, _lib.ptr(scratch), B, T, H, Hkv,
+                                             128, 128, 1, 1.0, _lib.stream_ptr()))
+        assert (buf[:off] == 7).all() and (buf[off + B * T * H * 128:] == 7).all()
+        out.append(buf[off:off + B * T * H * 128])
+    assert torch.equal(*out)
