@@ -607,11 +607,12 @@ int sm100_status_fetch_and_clear(int* out) {
 // the device; clears the flag).
 extern "C" int atma_device_status(int* status) {
   ATMA_REQUIRE(status != nullptr, "device_status: null out pointer");
-  int a = 0, b = 0, c = 0, d = 0;
+  int a = 0, b = 0, c = 0, d = 0, e = 0;
   int rc = atma::sm100_status_fetch_and_clear(&a);
   if (rc == ATMA_OK) rc = atma::scan_sm100_status_fetch_and_clear(&b);
   if (rc == ATMA_OK) rc = atma::scan_local_status_fetch_and_clear(&c);
   if (rc == ATMA_OK) rc = atma::linear_f32_status_fetch_and_clear(&d);
-  *status = a | b | c | d;
+  if (rc == ATMA_OK) rc = atma::polar_tf32_status_fetch_and_clear(&e);
+  *status = a | b | c | d | e;
   return rc;
 }

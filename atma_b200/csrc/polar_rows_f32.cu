@@ -1,10 +1,12 @@
-// Polar Attention prefill of fp32 tensors with a head size of 64 or 128, fp32 arithmetic, 64 rows x 64 keys per step: the
-// same results as polar_prefill_simt_kernel, which keeps the other types and sizes.
+// Polar Attention prefill of fp32 tensors with a head size of 64 or 128: on the tensor cores (attend_tf32.cuh) where there are
+// rows enough, else in fp32 arithmetic, 64 rows x 64 keys per step, with the same results as polar_prefill_simt_kernel, which
+// keeps the other types and sizes.
 //
 // There a lane owns one key and a warp four rows, with a shuffle for every weight; here a thread owns 4 x 4 scores and
 // 4 rows x DK / 16 channels (rows_f32.cuh).  K and V take turns in one buffer, V under the statistics, and two CTAs share an
 // SM; later rows have more keys, so those of all heads come first.  Measured, 2048 rows, 8 heads of 128: 1049 -> 423 us (527
 // with the heads one after another and the scores one channel at a time).
+#include "attend_tf32.cuh"
 #include "polar_prefill.cuh"
 #include "rows_f32.cuh"
 
@@ -17,7 +19,7 @@ constexpr float kNegBig = -1e38f;
 
 template <int DK>
 __global__ void __launch_bounds__(kThreads, 2)
-polar_rows_f32_kernel(const atma_polar_prefill_args a) {
+polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
   constexpr int VM = DK / 64, ld = DK + kPad;
   extern __shared__ __align__(16) float sm[];
   float* sQ = sm;                              // [64][ld]
@@ -28,6 +30,8 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a) {
   const int h = blockIdx.x % a.H, b = blockIdx.y, kvh = h / (a.H / a.Hkv);
 
   const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM, q_limit = a.Tq, k_limit = a.Tk;
+  // behind the tensor-core kernel: only the blocks that it has marked
+  if (marked && __float_as_uint(static_cast<const float*>(a.c)[b * a.c_sb + h * a.c_sh + (int64_t)q0 * a.c_st]) != attend_tf32::kRedo) return;
   const float* Q = static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh;
   const float* K = static_cast<const float*>(a.k) + b * a.k_sb + kvh * a.k_sh;
   const float* V = static_cast<const float*>(a.v) + b * a.v_sb + kvh * a.v_sh;
@@ -176,11 +180,145 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a) {
   }
 }
 
+// ---- the same on the tensor cores, 128 rows of a head per CTA ----------------------------------------------------------
+__device__ int g_polar_tf32_status = 0;
+
+struct PolarFront {
+  struct Row {
+    float n, f, temp, nc, koff;
+    int k_limit, window;
+    __device__ __forceinline__ float score(float s) const { return s * f; }
+    __device__ __forceinline__ bool sees(int key) const {
+      const float pos = (float)key + koff;
+      return (key < k_limit) & (pos < n) & ((window <= 0) | (pos >= n - (float)window));
+    }
+    __device__ __forceinline__ bool sees_all(int first, int last) const { return sees(first) & sees(last); }      // keys that are seen follow one another
+    __device__ __forceinline__ float start(int) const { return kNegBig; }
+    __device__ __forceinline__ float start_sum(int) const { return 0.f; }
+  };
+  const atma_polar_prefill_args& a;
+  int h, b, kvh, q0, j_begin, j_end;
+
+  __device__ __forceinline__ float count(int r) const {
+    return r >= a.Tq ? 0.f : (a.n_keys ? a.n_keys[r] : a.n_base + (float)(r + 1));
+  }
+  __device__ __forceinline__ PolarFront(const atma_polar_prefill_args& args, float (*s_n)[2]) : a(args) {
+    h = blockIdx.x % a.H; b = blockIdx.y; kvh = h / (a.H / a.Hkv);
+    q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * attend_tf32::kM;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 4) {
+      const int r = q0 + 32 * warp + lane;
+      float lo = r < a.Tq ? count(r) : 3.0e38f, hi = r < a.Tq ? lo : -1.0f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      }
+      if (lane == 0) { s_n[warp][0] = lo; s_n[warp][1] = hi; }
+    }
+    __syncthreads();
+    float lo = s_n[0][0], hi = s_n[0][1];
+#pragma unroll
+    for (int w = 1; w < 4; ++w) { lo = fminf(lo, s_n[w][0]); hi = fmaxf(hi, s_n[w][1]); }
+    const float koff = (float)a.key_offset;
+    j_end = max((int)fminf((float)a.Tk, ceilf(hi - koff)), 0);
+    j_begin = 0;
+    if (a.window > 0) {
+      const float first = lo - (float)a.window - koff;
+      if (first > 0.f) j_begin = (int)fminf(first, (float)a.Tk) / kN * kN;
+    }
+  }
+  __device__ __forceinline__ int tiles() const { return max(j_end - j_begin + kN - 1, 0) / kN; }
+  __device__ __forceinline__ int key0(int j) const { return j_begin + j * kN; }
+  __device__ __forceinline__ float q_scale() const { return 1.f; }
+  __device__ __forceinline__ const float* any() const { return static_cast<const float*>(a.q); }
+  __device__ __forceinline__ const float* q_row(int r) const {
+    return q0 + r < a.Tq ? static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh + (int64_t)(q0 + r) * a.q_st : nullptr;
+  }
+  __device__ __forceinline__ const float* k_row(int key) const {
+    return key < a.Tk ? static_cast<const float*>(a.k) + b * a.k_sb + kvh * a.k_sh + (int64_t)key * a.k_st : nullptr;
+  }
+  __device__ __forceinline__ const float* v_row(int key) const {
+    return key < a.Tk ? static_cast<const float*>(a.v) + b * a.v_sb + kvh * a.v_sh + (int64_t)key * a.v_st : nullptr;
+  }
+  __device__ __forceinline__ Row row(int r) const {
+    Row w;
+    w.n = count(q0 + r);
+    w.nc = fmaxf(a.window > 0 ? fminf(w.n, (float)a.window) : w.n, 1.0f);
+    w.temp = 1.0f + a.spg[h] * logf(w.nc);
+    w.f = w.temp * rsqrtf((float)attend_tf32::kD);
+    w.koff = (float)a.key_offset; w.k_limit = a.Tk; w.window = a.window;
+    return w;
+  }
+  __device__ __forceinline__ void finish(const Row& w, int r, int half, const float (&m)[1], const float (&l)[1], float q2, float (&O)[1][64],
+                                         attend_tf32::Shared& sh) const {
+    using namespace attend_tf32;
+    const bool ok = q0 + r < a.Tq;
+    sh.sum[half][0][r] = l[0]; sh.sum[half][1][r] = q2;
+    if (ok && !trusted(O[0], l[0])) sh.redo[r >> 6] = 1;
+    rows_sync();
+    const float a_n = w.temp * (a.null_base[h] + a.sps[h] * sqrtf(logf(w.nc + 1.0f)));
+    const float mn = fmaxf(m[0], a_n), al = expf(m[0] - mn), p_n = expf(a_n - mn);
+    const float Lf = (l[0] + sh.sum[half ^ 1][0][r]) * al, Q2f = (q2 + sh.sum[half ^ 1][1][r]) * al * al, Z = Lf + p_n;
+    const float* vn = a.v_null + h * kD + 64 * half;
+    float sq = 0.f;
+#pragma unroll
+    for (int c = 0; c < 64; ++c) {
+      O[0][c] = fmaf(O[0][c], al, p_n * vn[c]);
+      sq = fmaf(O[0][c], O[0][c], sq);
+    }
+    sh.sum[half][2][r] = sq;
+    rows_sync();
+    if (!ok) return;
+    float* cp = static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)(q0 + r) * a.c_st + 64 * half;
+    if (sh.redo[r >> 6]) {
+      if (half == 0 && (r & 63) == 0) cp[0] = __uint_as_float(kRedo);
+      return;
+    }
+    const float inv = 1.0f / fmaxf(sqrtf(sq + sh.sum[half ^ 1][2][r]), a.eps);
+    if ((reinterpret_cast<uintptr_t>(cp) & 15) == 0) {
+#pragma unroll
+      for (int c = 0; c < 64; c += 4)
+        *reinterpret_cast<float4*>(cp + c) = make_float4(O[0][c] * inv, O[0][c + 1] * inv, O[0][c + 2] * inv, O[0][c + 3] * inv);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 64; ++c) cp[c] = O[0][c] * inv;
+    }
+    if (half == 0) {
+      const float n_eff = Lf * Lf / fmaxf(Q2f, 1e-30f), m_eff = n_eff * (Lf / fmaxf(Z, a.eps));
+      static_cast<float*>(a.mag)[b * a.mag_sb + h * a.mag_sh + (int64_t)(q0 + r) * a.mag_st] = tanhf(a.beta[h] * log1pf(m_eff));
+    }
+  }
+};
+
+__global__ void __launch_bounds__(attend_tf32::kThreads, 1)
+polar_tf32_kernel(const __grid_constant__ atma_polar_prefill_args a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ attend_tf32::Shared sh;
+  __shared__ float s_n[4][2];
+  PolarFront front(a, s_n);
+  attend_tf32::attend<PolarFront, 1>(front, smem, sh, &g_polar_tf32_status);
+}
+
+// Head size 128, no statistics carried in or out (a marked block is done again from the inputs alone), and enough rows: 2048
+// rows, 8 heads 431 us on the 64 x 64 kernel, 130 here; 512 rows 100 and 60; 256 rows 57 and 49, where the calls' own launches are most of it.
+bool polar_tf32_supported(const atma_polar_prefill_args& a) {
+  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq >= 256;
+}
+
 template <int DK>
 int launch(const atma_polar_prefill_args& a, cudaStream_t st) {
+  const bool tf32 = polar_tf32_supported(a);
+  if (tf32) {
+    ATMA_CUDA_OK(cudaFuncSetAttribute(polar_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, attend_tf32::kSmemBytes));
+    polar_tf32_kernel<<<dim3((a.Tq + attend_tf32::kM - 1) / attend_tf32::kM * a.H, a.B), attend_tf32::kThreads, attend_tf32::kSmemBytes, st>>>(a);
+    const int rc = launch_status("polar_prefill (fp32, tensor cores)");
+    if (rc != ATMA_OK) return rc;
+  }
   const int smem = 4 * (kM * (DK + kPad) + kN * (DK + kPad) + kM * kLdP);
   ATMA_CUDA_OK(cudaFuncSetAttribute(polar_rows_f32_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  polar_rows_f32_kernel<DK><<<dim3((a.Tq + kM - 1) / kM * a.H, a.B), kThreads, smem, st>>>(a);
+  polar_rows_f32_kernel<DK><<<dim3((a.Tq + kM - 1) / kM * a.H, a.B), kThreads, smem, st>>>(a, tf32);
   return launch_status("polar_prefill (fp32, 64 x 64)");
 }
 
@@ -193,6 +331,14 @@ bool polar_rows_f32_supported(const atma_polar_prefill_args& a) {
   auto rows = [](int64_t sb, int64_t sh, int64_t st) { return sb % 4 == 0 && sh % 4 == 0 && st % 4 == 0; };
   return a.dtype == ATMA_F32 && (a.dk == 64 || a.dk == 128) && a.n_tiles == 0 && a.Tq > 32 && al(a.q) && al(a.k) && al(a.v) &&
          rows(a.q_sb, a.q_sh, a.q_st) && rows(a.k_sb, a.k_sh, a.k_st) && rows(a.v_sb, a.v_sh, a.v_st);
+}
+
+int polar_tf32_status_fetch_and_clear(int* out) {
+  int v = 0, zero = 0;
+  ATMA_CUDA_OK(cudaMemcpyFromSymbol(&v, g_polar_tf32_status, sizeof(int)));
+  if (v != 0) ATMA_CUDA_OK(cudaMemcpyToSymbol(g_polar_tf32_status, &zero, sizeof(int)));
+  *out = v;
+  return ATMA_OK;
 }
 
 int polar_rows_f32(const atma_polar_prefill_args& a, cudaStream_t st) { return a.dk == 64 ? launch<64>(a, st) : launch<128>(a, st); }

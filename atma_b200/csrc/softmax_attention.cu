@@ -226,10 +226,11 @@ extern "C" int64_t atma_softmax_decode_scratch_floats(int n_seqs, int H, int map
 
 extern "C" int atma_decoder_device_status(int* status) {
   ATMA_REQUIRE(status != nullptr, "decoder_device_status: null out pointer");
-  int a = 0, b = 0, c = 0;
+  int a = 0, b = 0, c = 0, d = 0;
   int rc = softmax_sm100_status_fetch_and_clear(&a);
   if (rc == ATMA_OK) rc = delta_sm100_status_fetch_and_clear(&b);
   if (rc == ATMA_OK) rc = linear_f32_status_fetch_and_clear(&c);
-  *status = a | b | c;
+  if (rc == ATMA_OK) rc = softmax_tf32_status_fetch_and_clear(&d);
+  *status = a | b | c | d;
   return rc;
 }

@@ -11,6 +11,7 @@ bool softmax_prefill_sm100_supported(const atma_softmax_args& a);
 int softmax_prefill_sm100(const atma_softmax_args& a, cudaStream_t st);
 bool softmax_rows_f32_supported(const atma_softmax_args& a);
 int softmax_rows_f32(const atma_softmax_args& a, cudaStream_t st);
+int softmax_tf32_status_fetch_and_clear(int* out);
 bool softmax_decode_mma_supported(const atma_softmax_args& a);
 int softmax_decode_mma(const atma_softmax_args& a, cudaStream_t st);
 int softmax_sm100_status_fetch_and_clear(int* out);

@@ -1,4 +1,5 @@
-// Causal softmax attention of fp32 prompts over a paged cache, fp32 arithmetic, 64 rows x 64 keys per step: one or two maps,
+// Causal softmax attention of fp32 prompts over a paged cache: on the tensor cores (attend_tf32.cuh) where there are rows enough,
+// else in fp32 arithmetic, 64 rows x 64 keys per step.  One or two maps,
 // windows, a sink, the differential combination and the output gate as in softmax_rows_kernel, which keeps the other types
 // and sizes and short steps.
 //
@@ -7,6 +8,7 @@
 // V under the statistics, and two CTAs share an SM, one loading while the other computes.  Later rows have more keys, so
 // those of all heads come first.  Measured, 1500 rows, 8 heads, two maps of 64, 128 value channels: 1089 -> 534 us (679 with
 // the heads one after another).
+#include "attend_tf32.cuh"
 #include "rows_f32.cuh"
 #include "softmax_attention.cuh"
 
@@ -18,7 +20,7 @@ using namespace rows_f32;
 
 template <int M, int VM>
 __global__ void __launch_bounds__(kThreads, 2)
-softmax_rows_f32_kernel(const atma_softmax_args a) {
+softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
   extern __shared__ __align__(16) float sm[];
   const int kd = M * a.dim, ld = kd + kPad;
   float* sQ = sm;                              // [64][ld]
@@ -32,6 +34,8 @@ softmax_rows_f32_kernel(const atma_softmax_args a) {
   const int start = a.start_pos[s];
   const int g = h / (a.H / a.G);
   float* out = static_cast<float*>(a.out);
+  // behind the tensor-core kernel: only the blocks that it has marked
+  if (marked && __float_as_uint(out[(int64_t)(r_begin + q0) * a.out_rs + (int64_t)h * a.vdim]) != attend_tf32::kRedo) return;
   if (start < 0) {                             // padded sequence
     for (int i = tid; i < min(kM, n_rows - q0) * a.vdim; i += kThreads)
       out[(int64_t)(r_begin + q0 + i / a.vdim) * a.out_rs + (int64_t)h * a.vdim + i % a.vdim] = 0.f;
@@ -158,6 +162,120 @@ softmax_rows_f32_kernel(const atma_softmax_args a) {
   }
 }
 
+// ---- the same on the tensor cores, 128 rows of a head per CTA: 128 channels of q and k in all, 128 of v ------------------
+__device__ int g_softmax_tf32_status = 0;
+
+template <int M>
+struct SoftmaxFront {
+  struct Row {
+    int pos, n_keys, window, keep;
+    float sink;
+    __device__ __forceinline__ float score(float s) const { return s; }
+    __device__ __forceinline__ bool sees(int key) const { return (key < n_keys) & (key <= pos) & ((pos - key < window) | (key < keep)); }
+    __device__ __forceinline__ bool sees_all(int first, int last) const { return (last < n_keys) & (last <= pos) & ((pos - first < window) | (last < keep)); }
+    __device__ __forceinline__ float start(int) const { return sink; }      // the sink is a key that was seen before the others
+    __device__ __forceinline__ float start_sum(int) const { return sink > -INFINITY ? 1.f : 0.f; }
+  };
+  const atma_softmax_args& a;
+  int s, h, g, q0, r_begin, n_rows, first, n_keys;
+  KeyTiles kt;
+
+  __device__ __forceinline__ SoftmaxFront(const atma_softmax_args& args, int seq, int head, int row0, int begin, int rows, int start)
+      : a(args), s(seq), h(head), g(head / (args.H / args.G)), q0(row0), r_begin(begin), n_rows(rows), first(start + row0),
+        n_keys(min(start + min(row0 + attend_tf32::kM, rows), args.max_blocks * args.block_size)),
+        kt(start + row0, start + min(row0 + attend_tf32::kM, rows) - 1, args.max_blocks * args.block_size, args.window, args.keep_first, kN) {}
+  __device__ __forceinline__ int tiles() const { return kt.n; }
+  __device__ __forceinline__ int key0(int j) const { return kt[j] * kN; }
+  __device__ __forceinline__ float q_scale() const { return a.scale; }
+  __device__ __forceinline__ const float* any() const { return static_cast<const float*>(a.q); }
+  __device__ __forceinline__ const float* q_row(int r) const {
+    return q0 + r < n_rows ? static_cast<const float*>(a.q) + ((int64_t)(r_begin + q0 + r) * a.H + h) * attend_tf32::kD : nullptr;
+  }
+  __device__ __forceinline__ const float* cached(const void* cache, int pos) const {
+    if (pos >= n_keys) return nullptr;
+    const int blk = pos / a.block_size, phys = min(max(a.block_tables[s * a.bt_stride + blk], 0), a.num_blocks - 1);
+    return static_cast<const float*>(cache) + (((int64_t)phys * a.block_size + (pos - blk * a.block_size)) * a.G + g) * attend_tf32::kD;
+  }
+  __device__ __forceinline__ const float* k_row(int key) const { return cached(a.k_cache, key); }
+  __device__ __forceinline__ const float* v_row(int key) const { return cached(a.v_cache, key); }
+  __device__ __forceinline__ Row row(int r) const { return Row{first + r, n_keys, a.window, a.keep_first, a.sink}; }
+  __device__ __forceinline__ void finish(const Row&, int r, int half, const float (&)[M], const float (&l)[M], float, float (&O)[M][64],
+                                         attend_tf32::Shared& sh) const {
+    using namespace attend_tf32;
+    const bool ok = q0 + r < n_rows;
+#pragma unroll
+    for (int t = 0; t < M; ++t) {
+      sh.sum[half][t][r] = l[t];
+      if (ok && !trusted(O[t], l[t])) sh.redo[r >> 6] = 1;
+    }
+    rows_sync();
+    float L[M], ss = 0.f;
+#pragma unroll
+    for (int t = 0; t < M; ++t) L[t] = l[t] + sh.sum[half ^ 1][t][r];
+#pragma unroll
+    for (int c = 0; c < 64; ++c) {
+      O[0][c] = L[0] > 0.f ? O[0][c] / L[0] : 0.f;
+      if constexpr (M == 2) O[0][c] -= L[M - 1] > 0.f ? a.lambda * (O[M - 1][c] / L[M - 1]) : 0.f;
+      ss = fmaf(O[0][c], O[0][c], ss);
+    }
+    sh.sum[half][2][r] = ss;
+    rows_sync();
+    if (!ok) return;
+    float* op = static_cast<float*>(a.out) + (int64_t)(r_begin + q0 + r) * a.out_rs + (int64_t)h * kD + 64 * half;
+    if (sh.redo[r >> 6]) {
+      if (half == 0 && (r & 63) == 0) op[0] = __uint_as_float(kRedo);
+      return;
+    }
+    float f = 1.f;
+    if constexpr (M == 2) f = a.out_scale / sqrtf((ss + sh.sum[half ^ 1][2][r]) / (float)kD + a.eps);
+    const float* gp = a.gate == nullptr ? nullptr : static_cast<const float*>(a.gate) + (int64_t)(r_begin + q0 + r) * a.gate_rs + (int64_t)h * kD + 64 * half;
+    const bool vec = (reinterpret_cast<uintptr_t>(op) & 15) == 0;
+#pragma unroll
+    for (int c = 0; c < 64; c += 4) {
+      float y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] = O[0][c + e] * f * (gp != nullptr ? sigmoid_gate(gp[c + e]) : 1.f);
+      if (vec) *reinterpret_cast<float4*>(op + c) = make_float4(y[0], y[1], y[2], y[3]);
+      else
+#pragma unroll
+        for (int e = 0; e < 4; ++e) op[c + e] = y[e];
+    }
+  }
+};
+
+template <int M>
+__global__ void __launch_bounds__(attend_tf32::kThreads, 1)
+softmax_tf32_kernel(const __grid_constant__ atma_softmax_args a) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ attend_tf32::Shared sh;
+  const int s = blockIdx.y, h = blockIdx.x % a.H;
+  const int r_begin = a.cu_rows[s], n_rows = a.cu_rows[s + 1] - r_begin, start = a.start_pos[s];
+  const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * attend_tf32::kM;
+  if (q0 >= n_rows) return;
+  if (start < 0) {                             // padded sequence
+    float* out = static_cast<float*>(a.out);
+    for (int i = threadIdx.x; i < min(attend_tf32::kM, n_rows - q0) * attend_tf32::kD; i += attend_tf32::kThreads)
+      out[(int64_t)(r_begin + q0 + i / attend_tf32::kD) * a.out_rs + (int64_t)h * attend_tf32::kD + i % attend_tf32::kD] = 0.f;
+    return;
+  }
+  SoftmaxFront<M> front(a, s, h, q0, r_begin, n_rows, start);
+  attend_tf32::attend<SoftmaxFront<M>, M>(front, smem, sh, &g_softmax_tf32_status);
+}
+
+// 128 channels in one map or two, 128 of v, and enough rows.  Two layers of two maps: 1500 rows, 8 heads 527 us on the 64 x 64
+// kernel, 145 here; 400 rows 143 and 57; 256 rows 91 and 49.
+bool softmax_tf32_supported(const atma_softmax_args& a) {
+  return a.maps * a.dim == attend_tf32::kD && a.vdim == attend_tf32::kD && a.max_rows >= 256;
+}
+
+template <int M>
+int launch_tf32(const atma_softmax_args& a, cudaStream_t st) {
+  ATMA_CUDA_OK(cudaFuncSetAttribute(softmax_tf32_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, attend_tf32::kSmemBytes));
+  softmax_tf32_kernel<M><<<dim3((a.max_rows + attend_tf32::kM - 1) / attend_tf32::kM * a.H, a.n_seqs), attend_tf32::kThreads, attend_tf32::kSmemBytes, st>>>(a);
+  return launch_status("softmax attention (fp32, tensor cores)");
+}
+
 int smem_bytes(const atma_softmax_args& a) {
   const int ld = a.maps * a.dim + kPad, vm = a.vdim <= 64 ? 64 : 128;
   return 4 * (kM * ld + kN * (ld > vm ? ld : vm) + a.maps * kM * kLdP);
@@ -166,8 +284,13 @@ int smem_bytes(const atma_softmax_args& a) {
 template <int M, int VM>
 int launch(const atma_softmax_args& a, cudaStream_t st) {
   const int smem = smem_bytes(a);
+  const bool tf32 = softmax_tf32_supported(a);
+  if (tf32) {
+    const int rc = launch_tf32<M>(a, st);
+    if (rc != ATMA_OK) return rc;
+  }
   ATMA_CUDA_OK(cudaFuncSetAttribute(softmax_rows_f32_kernel<M, VM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  softmax_rows_f32_kernel<M, VM><<<dim3((a.max_rows + kM - 1) / kM * a.H, a.n_seqs), kThreads, smem, st>>>(a);
+  softmax_rows_f32_kernel<M, VM><<<dim3((a.max_rows + kM - 1) / kM * a.H, a.n_seqs), kThreads, smem, st>>>(a, tf32);
   return launch_status("softmax attention (fp32, 64 x 64)");
 }
 
@@ -182,6 +305,14 @@ bool softmax_rows_f32_supported(const atma_softmax_args& a) {
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   return a.dtype == ATMA_F32 && a.max_rows > 32 && a.dim % 4 == 0 && a.vdim % 4 == 0 && a.maps * a.dim <= 128 && a.vdim <= 128 && al(a.q) &&
          al(a.k_cache) && al(a.v_cache);
+}
+
+int softmax_tf32_status_fetch_and_clear(int* out) {
+  int v = 0, zero = 0;
+  ATMA_CUDA_OK(cudaMemcpyFromSymbol(&v, g_softmax_tf32_status, sizeof(int)));
+  if (v != 0) ATMA_CUDA_OK(cudaMemcpyToSymbol(g_softmax_tf32_status, &zero, sizeof(int)));
+  *out = v;
+  return ATMA_OK;
 }
 
 int softmax_rows_f32(const atma_softmax_args& a, cudaStream_t st) {

@@ -1,0 +1,110 @@
+"""fp32 attention on the tensor cores (256 rows and more): against 64 bits, at the edges of its 128-row and 64-key tiles, and with
+values that its two-term products cannot hold."""
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+import atma_b200
+from atma_b200 import decoder_ops
+from tests.conftest import max_rel
+from tests.gpu_util import rand
+from tests.rizurax_util import group
+
+pytestmark = pytest.mark.gpu
+INF = float("inf")
+
+
+def params(H, d):
+    return dict(v_null=rand((H, d), 4).cuda(), null_base=rand((H,), 5).cuda(), null_slope_raw=rand((H,), 6).cuda(), len_gain_raw=rand((H,), 7).cuda(),
+                mag_beta_raw=rand((H,), 8).cuda())
+
+
+def polar64(q, k, v, n, p, window):
+    H, d = q.shape[1], q.shape[3]
+    q, k, v, n, p = q.double(), k.double().repeat_interleave(H // k.shape[1], 1), v.double().repeat_interleave(H // v.shape[1], 1), n.double(), {i: t.double() for i, t in p.items()}
+    key = torch.arange(k.shape[2], device="cuda")[None]
+    see = (key < n[:, None]) & (key >= n[:, None] - (window or 1 << 30))
+    nc = (n.clamp_max(window) if window else n).clamp_min(1)
+    temp = 1 + F.softplus(p["len_gain_raw"])[:, None] * torch.log(nc)
+    null = temp * (p["null_base"][:, None] + F.softplus(p["null_slope_raw"])[:, None] * torch.sqrt(torch.log(nc + 1)))
+    s = (q @ k.transpose(-1, -2) * (temp / d ** 0.5)[..., None]).masked_fill(~see, -INF)
+    w = torch.softmax(torch.cat([s, null[None, ..., None].expand(*s.shape[:-1], 1)], -1), -1)
+    w, w0 = w[..., :-1], w[..., -1:]
+    c = w @ v + w0 * p["v_null"][None, :, None]
+    real, sq = w.sum(-1), (w * w).sum(-1).clamp_min(1e-300)
+    return c / c.norm(dim=-1, keepdim=True), torch.tanh(F.softplus(p["mag_beta_raw"])[None, :, None] * torch.log1p(real * real / sq * real))
+
+
+@pytest.mark.parametrize("Tq,Tk", [(256, 256), (257, 300), (383, 383), (640, 700)])
+@pytest.mark.parametrize("B,H,Hkv", [(2, 4, 2), (1, 3, 1)])
+@pytest.mark.parametrize("window", [None, 100])
+def test_polar(Tq, Tk, B, H, Hkv, window):
+    """Errors of fp32 sums of at most 700 terms."""
+    q, k, v, p = rand((B, H, Tq, 128), 1).cuda(), rand((B, Hkv, Tk, 128), 2).cuda(), rand((B, Hkv, Tk, 128), 3).cuda(), params(H, 128)
+    for n in (torch.arange(Tk - Tq + 1, Tk + 1), torch.arange(Tq) * 37 % Tk + 1):
+        n = n.float().cuda()
+        c, mag = atma_b200.polar_attention_fwd(q, k, v, n, window=window, is_causal=False, **p)
+        wc, wm = polar64(q, k, v, n, p, window)
+        assert max_rel(c, wc) < 1e-5 and max_rel(mag, wm) < 1e-5
+
+
+@pytest.mark.parametrize("what,at,value", [("v", 5, INF), ("v", 200, float("nan")), ("k", 130, INF), ("k", 299, -INF), ("k", 64, float("nan")), ("q", 100, float("nan")), ("q", 255, INF),
+                                           ("q", 3, 3e38)])
+def test_polar_values_without_two_terms(what, at, value):
+    """One such value changes the rows that see it, as it does in portions of 64 rows on the other kernel, and no others."""
+    T, H = 300, 2
+    x = dict(q=rand((1, H, T, 128), 1).cuda(), k=rand((1, 1, T, 128), 2).cuda(), v=rand((1, 1, T, 128), 3).cuda())
+    p, n = params(H, 128), torch.arange(1, T + 1).float().cuda()
+    clean = atma_b200.polar_attention_fwd(x["q"], x["k"], x["v"], n, **p)
+    x[what][0, -1, at, 7] = value
+    got = atma_b200.polar_attention_fwd(x["q"], x["k"], x["v"], n, **p)
+    for a in range(0, T, 64):
+        s = slice(a, a + 64)
+        want = atma_b200.polar_attention_fwd(x["q"][:, :, s].contiguous(), x["k"], x["v"], n[s].contiguous(), is_causal=False, **p)
+        for g, w, was in zip(got, want, clean):
+            assert torch.equal(g[:, :, s].isfinite(), w.isfinite())
+            assert torch.allclose(g[:, :, s], w, atol=1e-5, rtol=1e-5, equal_nan=True)
+            if what != "q":
+                unseen = n[s] <= at
+                assert torch.allclose(g[:, :, s][:, :, unseen], was[:, :, s][:, :, unseen], atol=1e-5, rtol=1e-5)
+    if what != "q" and at >= 128:                                            # tiles in front of it keep their bits
+        far = at // 128 * 128
+        assert torch.equal(got[0][:, :, :far], clean[0][:, :, :far])
+
+
+@pytest.mark.parametrize("H,G,maps", [(2, 1, 1), (4, 2, 2), (3, 3, 2)])
+@pytest.mark.parametrize("window,keep", [(1 << 20, 0), (40, 3), (130, 70)])
+@pytest.mark.parametrize("rows,start", [(256, 0), (300, 77), (513, 1)])
+@pytest.mark.parametrize("bad", [None, INF, "small"])
+def test_softmax(H, G, maps, window, keep, rows, start, bad):
+    n, dim = rows + start, 128 // maps
+    pages = -(-n // 64)
+    q, kc, vc = rand((rows, H, maps, dim), 1).cuda(), rand((pages + 2, 64, G, 128), 2).cuda(), rand((pages + 2, 64, G, 128), 3).cuda()
+    table = [torch.randperm(pages + 2, generator=torch.Generator().manual_seed(1))[:pages].tolist()]
+    kw = dict(scale=dim ** -0.5, lam=0.3, out_scale=0.7, eps=1e-6, window=None if window > n else window, keep_first=keep, sink=0.5,
+              gate=rand((rows, H * 128), 4).cuda())
+    pos, key = torch.arange(start, n, device="cuda")[:, None], torch.arange(n, device="cuda")[None]
+    see = (key <= pos) & ((pos - key < window) | (key < keep))
+    k, v = (c[table[0]].flatten(0, 1)[:n].double().view(n, G, -1).repeat_interleave(H // G, 1) for c in (kc, vc))
+    o = 0
+    for m in range(maps):
+        s = torch.einsum("thd,nhd->htn", q[:, :, m].double(), k.view(n, H, maps, dim)[:, :, m]) * kw["scale"]
+        s = torch.cat([s.masked_fill(~see, -INF), torch.full((H, rows, 1), kw["sink"], device="cuda", dtype=torch.float64)], -1)
+        o = o + (1.0 if m == 0 else -kw["lam"]) * torch.einsum("htn,nhd->thd", s.softmax(-1)[..., :n], v)
+    if maps == 2:
+        o = o / torch.sqrt((o * o).mean(-1, keepdim=True) + kw["eps"]) * kw["out_scale"]
+    want = o.flatten(1) * torch.sigmoid(kw["gate"].double())
+    at = n - 70
+    if bad == "small":                                  # the second terms of such values would be lost
+        if maps == 2:
+            return                                       # ends in a norm that has no squares of them
+        vc *= 1e-34
+        want = want * 1e-34
+    elif bad is not None:
+        vc[table[0][at // 64], at % 64] = bad
+    out = torch.zeros(rows, H * 128, device="cuda")
+    decoder_ops.softmax_prefill(q, kc, vc, group([rows], [start], [0], table), out, **kw)
+    reached = see[:, at] if bad == INF else torch.zeros(rows, dtype=torch.bool, device="cuda")
+    assert max_rel(out[~reached], want[~reached]) < 1e-5
+    assert not out[reached].isfinite().all(1).any()
