@@ -13,14 +13,16 @@
 // activations among them, have next to none, and the test costs nothing that shows; where every result needs it, 1500 x 8192 x
 // 1024 takes 7.8 ms instead of 0.12, with one such row of x 0.31.
 //   split kernel: one CTA per row of x and of w, two fp16 planes each, the row's power of two and what it lost.
-//   product kernel: a CTA owns 128 rows x BN columns.  Warp 0 TMA (both planes of 64 columns of x and of w per stage),
-//   warp 1 MMA, warps 2-9 add the sums of one stage out of one half of the accumulator columns while the next stage's
-//   products go to the other half, scale them back and write whole 128-byte lines.
-// Bound by L2 -> shared memory traffic (96 KB per 64 columns and CTA at BN = 256, 62 B per clock and SM if the tensor cores
-// were to wait for nothing).  Narrower BN where wide tiles would leave SMs without one; see pick_bn.
-// Measured with the split, out of HBM, beside the library's: 1500 x 8192 x 1024 118 us (499), 1500 x 1024 x 5120 95 us (346),
-// 4096 x 8192 x 1024 251 us (1094).  Where one side is short or few tiles walk a long K the
-// library's is faster (32 x 512 x 2048: 26 us against 36) and callers stay with it.
+//   product kernel: a CTA per SM takes tiles of 128 rows x BN columns in turn.  Warp 0 TMA (both planes of 64 columns of x and of
+//   w per stage), warp 1 MMA, warps 2-9 add the sums of one stage out of one half of the accumulator columns while the next stage's
+//   products go to the other half, scale them back and write them, under the first two stages of the next tile.
+// Bound by the products (1536 clocks per 64 columns at BN = 256) and L2 -> shared memory traffic (96 KB for them, 1600 clocks) within
+// a tile, 1780 measured; between tiles by the results' way out: 18000 clocks a tile, as long as ten stages, with a loop over rows
+// and columns that loads, scales and stores one value, 6000 with four values at a time and the columns' figures fetched under the
+// products.  Narrower BN where wide tiles would leave SMs without one; see pick_bn.
+// Measured out of HBM, without the split (with it, beside the library's, 1500 x 8192 x 1024 103 us and 499): 1500 x 8192 x 1024
+// 93 -> 83 us, 4096 x 8192 x 1024 227 -> 179, 2048 x 1024 x 4096 59 -> 51, 512 x 1024 x 1024 16.4 -> 13.3.  Where one side is short or
+// few tiles walk a long K the library's is faster (32 x 512 x 2048: 26 us against 36) and callers stay with it.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status word for the host.
 #include "common.cuh"
 #include "linear_f32.cuh"
@@ -33,6 +35,7 @@ namespace {
 using namespace sm100;
 
 constexpr int kBM = 128, kBK = 64;
+constexpr int kOut = 16, kLd = kOut + 4;      // columns that leave at a time; floats between their rows: quarter warps meet no bank twice
 constexpr int kThreads = 320;
 constexpr int kLoBits = 11;                 // the second plane is 2^11 times what the first leaves
 constexpr float kWhole = 1.0f / (1 << 13);  // scaled values from here on are in the two terms to 2^-22 of themselves
@@ -146,7 +149,8 @@ struct Tile {
   static constexpr int kStages = BN == 256 ? 2 : (BN == 128 ? 3 : 4);
   static constexpr int kPlaneA = kBM * kBK * 2, kPlaneB = BN * kBK * 2;
   static constexpr int kStageBytes = 2 * (kPlaneA + kPlaneB);
-  static constexpr int kSmem = kStages * kStageBytes + 1024;
+  static constexpr int kStaging = 8 * 32 * kLd * 4;                       // results on their way out, a warp's 32 rows x 16 columns
+  static constexpr int kSmem = kStages * kStageBytes + kStaging + 1024;
   static constexpr int kCols = 2 * BN;      // TMEM columns
 };
 
@@ -159,33 +163,35 @@ struct Product {
   int M, N, K, Kp;
 };
 
-// A warp's rows from m0 on and its lanes' columns n: the results that the terms alone don't settle, in fp32 arithmetic.
-__device__ __noinline__ void sum_again(const Product& p, int m0, int rows, int n, const float* sums, int ld, const float* row_least, float least,
-                                       float bias) {
+// Results that the terms alone don't settle, in fp32 arithmetic: bit 4 i + j of a lane's `flags` is row m0 + lane / 4 + 8 i, column
+// n0 + 4 (lane % 4) + j.  Four at a time: their loads do not wait for one another.
+__device__ __noinline__ void sum_again(const Product& p, int m0, int n0, uint32_t flags) {
   const int lane = threadIdx.x & 31;
-  for (int r = 0; r < rows; ++r) {
-    uint32_t lanes = __ballot_sync(0xffffffffu, n < p.N && fabsf(sums[r * ld]) < row_least[r] + least);
-    const float* x = p.x + (m0 + r) * p.x_rs;
-    while (lanes != 0) {                    // four at a time: their loads do not wait for one another
+  for (int bit = 0; bit < 16; ++bit) {
+    uint32_t lanes = __ballot_sync(0xffffffffu, flags >> bit & 1);
+    while (lanes != 0) {
       int l[4];
       float acc[4] = {};
-      const float* w[4];
+      const float *x[4], *w[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         l[j] = j > 0 && lanes == 0 ? l[0] : __ffs(lanes) - 1;
         lanes &= lanes - 1;
-        w[j] = p.w + (int64_t)(n - lane + l[j]) * p.K;
+        x[j] = p.x + (int64_t)(m0 + (l[j] >> 2) + 8 * (bit >> 2)) * p.x_rs;
+        w[j] = p.w + (int64_t)(n0 + 4 * (l[j] & 3) + (bit & 3)) * p.K;
       }
 #pragma unroll 4
       for (int k = lane; k < p.K; k += 32) {
-        const float a = x[k];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] = fmaf(a, w[j][k], acc[j]);
+        for (int j = 0; j < 4; ++j) acc[j] = fmaf(x[j][k], w[j][k], acc[j]);
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float sum = warp_sum(acc[j]);
-        if (lane == l[j]) p.out[(m0 + r) * p.out_rs + n] = sum + bias;
+        if (lane == l[j]) {
+          const int n = n0 + 4 * (lane & 3) + (bit & 3);
+          p.out[(int64_t)(m0 + (lane >> 2) + 8 * (bit >> 2)) * p.out_rs + n] = sum + (p.bias ? p.bias[n] : 0.f);
+        }
       }
     }
   }
@@ -200,21 +206,17 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   __shared__ uint64_t full[L::kStages], empty[L::kStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort_v;
-  __shared__ int s_ex[kBM];
-  __shared__ float s_least[kBM];            // a result is trusted from here on
+  __shared__ int s_ex[8][32];               // of each warp's rows: the power of two
+  __shared__ __align__(16) int s_cex[2][BN];            // of the columns the same, and the bias; a warp may be a tile ahead of another
+  __shared__ __align__(16) float s_cleast[2][BN], s_cbias[2][BN];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
-
-  for (int i = tid; i < kBM; i += kThreads) {
-    s_ex[i] = m0 + i < p.M ? p.exps[m0 + i] : 0;
-    s_least[i] = m0 + i < p.M ? trusted_from(p.losses[m0 + i]) : 0.f;
-  }
+  const int m_tiles = (p.M + kBM - 1) / kBM, tiles = m_tiles * ((p.N + BN - 1) / BN);
 
   if (warp == 0) tmem_alloc(&s_tmem, L::kCols);
   if (tid == 32) {
     for (int i = 0; i < L::kStages; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 256); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); }
     s_abort_v = 0;
     fence_barrier_init();
   }
@@ -227,90 +229,152 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 
   if (warp == 0) {
     if (elect_one()) {
-      int it = 0;
-      for (; it < NK; ++it) {
-        const int st = it % L::kStages;
-        if (it >= L::kStages && !mbar_wait(&empty[st], (it / L::kStages - 1) & 1, abort)) break;
-        uint8_t* a = smem + st * L::kStageBytes;
-        mbar_arrive_expect_tx(&full[st], L::kStageBytes);
-        tma_load_4d(a, &tm_x, &full[st], it * kBK, m0, 0, 0);
-        tma_load_4d(a + 2 * L::kPlaneA, &tm_w, &full[st], it * kBK, n0, 0, 0);
+      uint32_t n = 0;                       // stages so far, over all tiles
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int m0 = tile % m_tiles * kBM, n0 = tile / m_tiles * BN;
+        for (int it = 0; it < NK; ++it, ++n) {
+          const uint32_t st = n % L::kStages;
+          if (n >= L::kStages && !(ok = mbar_wait(&empty[st], (n / L::kStages - 1) & 1, abort))) break;
+          uint8_t* a = smem + st * L::kStageBytes;
+          mbar_arrive_expect_tx(&full[st], L::kStageBytes);
+          tma_load_4d(a, &tm_x, &full[st], it * kBK, m0, 0, 0);
+          tma_load_4d(a + 2 * L::kPlaneA, &tm_w, &full[st], it * kBK, n0, 0, 0);
+        }
       }
       volatile int alone = 0;               // whatever the others do, the CTA does not end before its copies
-      for (int i = max(0, it - L::kStages); i < it; ++i) mbar_wait(&full[i % L::kStages], (i / L::kStages) & 1, &alone);
+      for (uint32_t i = n > L::kStages ? n - L::kStages : 0; i < n; ++i) mbar_wait(&full[i % L::kStages], (i / L::kStages) & 1, &alone);
     }
   } else if (warp == 1) {
     if (elect_one()) {
       constexpr uint32_t idesc = make_idesc(kBM, BN, 0, 0, 0);
-      for (int it = 0; it < NK; ++it) {
-        const int st = it % L::kStages, buf = it & 1;
-        if (it >= 2 && !mbar_wait(&acc_empty[buf], (it / 2 - 1) & 1, abort)) break;
-        if (!mbar_wait(&full[st], (it / L::kStages) & 1, abort)) break;
-        tc_fence_after();
-        const uint32_t a = smem_u32(smem + st * L::kStageBytes), b = a + 2 * L::kPlaneA, d = tmem + buf * BN;
+      uint32_t n = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        for (int it = 0; it < NK; ++it, ++n) {
+          const uint32_t st = n % L::kStages, buf = n & 1;
+          ok = (n < 2 || mbar_wait(&acc_empty[buf], (n / 2 - 1) & 1, abort)) && mbar_wait(&full[st], (n / L::kStages) & 1, abort);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t a = smem_u32(smem + st * L::kStageBytes), b = a + 2 * L::kPlaneA, d = tmem + buf * BN;
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {       // lo hi, hi lo, hi hi
-          const uint32_t at = a + (t == 0 ? L::kPlaneA : 0), bt = b + (t == 1 ? L::kPlaneB : 0);
+          for (int t = 0; t < 3; ++t) {     // lo hi, hi lo, hi hi
+            const uint32_t at = a + (t == 0 ? L::kPlaneA : 0), bt = b + (t == 1 ? L::kPlaneB : 0);
 #pragma unroll
-          for (int k = 0; k < kBK / 16; ++k) {
-            const uint64_t ad = make_sdesc_sw128(at + 32 * k, 16, 1024), bd = make_sdesc_sw128(bt + 32 * k, 16, 1024);
-            if (t == 2 && k == 0) mma_ss_onto_lo(d, ad, bd, idesc);
-            else mma_ss(d, ad, bd, idesc, t > 0 || k > 0);
+            for (int k = 0; k < kBK / 16; ++k) {
+              const uint64_t ad = make_sdesc_sw128(at + 32 * k, 16, 1024), bd = make_sdesc_sw128(bt + 32 * k, 16, 1024);
+              if (t == 2 && k == 0) mma_ss_onto_lo(d, ad, bd, idesc);
+              else mma_ss(d, ad, bd, idesc, t > 0 || k > 0);
+            }
           }
+          tc_commit(&empty[st]);
+          tc_commit(&acc_full[buf]);
         }
-        tc_commit(&empty[st]);
-        tc_commit(&acc_full[buf]);
       }
     }
   } else {
     constexpr int kMine = BN / 2;           // columns of a thread's row
-    const int quarter = warp & 3, side = (warp - 2) >> 2;
+    const int w = warp - 2, quarter = warp & 3, side = w >> 2;
     const uint32_t at = tmem + (uint32_t(32 * quarter) << 16) + side * kMine;
-    float acc[kMine];
-#pragma unroll
-    for (int i = 0; i < kMine; ++i) acc[i] = 0.f;
+    float* s = reinterpret_cast<float*>(smem + L::kStages * L::kStageBytes) + w * 32 * kLd;
+    const bool vec = p.out_rs % 4 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+    const int rr = lane >> 2, cc = 4 * (lane & 3);                   // what this lane stores: row rr + 8 i, four columns
+    uint32_t n_st = 0;
     bool ok = true;
-    for (int it = 0; it < NK; ++it) {
-      const int buf = it & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (it / 2) & 1, abort));
-      if (!ok) break;
-      tc_fence_after();
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+      const int mw = tile % m_tiles * kBM + 32 * quarter, nw = tile / m_tiles * BN + side * kMine, rows = min(32, p.M - mw);
+      const bool in_row = lane < rows;
+      const int ex = in_row ? p.exps[mw + lane] : 0;
+      const float row_least = in_row ? trusted_from(p.losses[mw + lane]) : 0.f, most_least = warp_max(row_least);
+      const int turn = tile / gridDim.x & 1;
+      int* cex = &s_cex[turn][side * kMine];
+      float *cleast = &s_cleast[turn][side * kMine], *cbias = &s_cbias[turn][side * kMine];
+      __syncwarp();                         // the last tile's rows have been read
+      s_ex[w][lane] = ex;
+      int most_e = -1000, least_e = 1000;
+      // under the first products; the four warps of these columns write the same
 #pragma unroll
-      for (int c = 0; c < kMine; c += 32) {
-        uint32_t r[32];
-        tmem_ld32(at + buf * BN + c, r);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[c + i] += __uint_as_float(r[i]);
+      for (int i = lane; i < kMine; i += 32) {
+        const bool in = nw + i < p.N;
+        cex[i] = in ? p.exps[p.M + nw + i] : 0;
+        cleast[i] = in ? trusted_from(p.losses[p.M + nw + i]) : -INFINITY;
+        cbias[i] = in && p.bias ? p.bias[nw + i] : 0.f;
+        most_e = max(most_e, cex[i]); least_e = min(least_e, cex[i]);
       }
-      tc_fence_before();
-      mbar_arrive(&acc_empty[buf]);
-    }
-    if (ok) {                               // every product is done: the stages' memory is free
-      constexpr int kLd = kMine + 1;
-      static_assert(8 * 32 * kLd * 4 <= L::kStages * L::kStageBytes, "the sums don't fit where the stages were");
-      float* s = reinterpret_cast<float*>(smem) + (warp - 2) * 32 * kLd;
+      // whether every result's power of two is a normal number; else it comes as two factors
+      const bool one_factor = __reduce_max_sync(0xffffffffu, most_e) + __reduce_max_sync(0xffffffffu, ex) <= 126 &&
+                              __reduce_min_sync(0xffffffffu, least_e) + __reduce_min_sync(0xffffffffu, ex) >= -127;
+      float acc[kMine];
 #pragma unroll
-      for (int i = 0; i < kMine; ++i) s[lane * kLd + i] = acc[i];
-      __syncwarp();
-      const int mw = m0 + 32 * quarter, rows = min(32, p.M - mw);
-      const int* ex = s_ex + 32 * quarter;
-      const float row_least = warp_max(s_least[32 * quarter + lane]);
-      for (int c = lane; c < kMine; c += 32) {
-        const int n = n0 + side * kMine + c;
-        const bool in = n < p.N;
-        const int ew = in ? p.exps[p.M + n] : 0;
-        const float least = in ? trusted_from(p.losses[p.M + n]) : 0.f;
-        const float bias = in && p.bias ? p.bias[n] : 0.f;
-        float low = INFINITY;
-#pragma unroll 8
-        for (int r = 0; r < rows; ++r) {
-          const float sum = s[r * kLd + c];
-          const int e = -(ex[r] + ew);
-          const float v = sum * pow2i(e / 2) * pow2i(e - e / 2);
-          low = fminf(low, fabsf(sum));
-          if (in) p.out[(int64_t)(mw + r) * p.out_rs + n] = v + bias;
+      for (int i = 0; i < kMine; ++i) acc[i] = 0.f;
+      for (int it = 0; it < NK; ++it, ++n_st) {
+        const uint32_t buf = n_st & 1;
+        ok = mbar_wait_warp(&acc_full[buf], (n_st / 2) & 1, abort);
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < kMine; c += 32) {
+          uint32_t r[32];
+          tmem_ld32(at + buf * BN + c, r);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) acc[c + i] += __uint_as_float(r[i]);
         }
-        if (__any_sync(0xffffffffu, in && low < row_least + least)) sum_again(p, mw, rows, n, s + c, kLd, s_least + 32 * quarter, least, bias);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+      }
+      if (!ok || rows <= 0) continue;
+      // 16 columns at a time through shared memory, so that rows leave in whole sectors.  The tensor cores have begun the next
+      // tile, but wait after two stages of it, so the common case is kept short: whole tiles, powers of two that are normal numbers.
+      const bool simple = one_factor && vec && rows == 32 && nw + kMine <= p.N;
+      float* to = p.out + (int64_t)(mw + rr) * p.out_rs + nw + cc;
+      const int64_t step = 8 * p.out_rs;
+      uint32_t flags[kMine / 32];           // 16 results of this lane in each half
+#pragma unroll
+      for (int c = 0; c < kMine; c += kOut) {
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < kOut; i += 4) *reinterpret_cast<float4*>(s + lane * kLd + i) = make_float4(acc[c + i], acc[c + i + 1], acc[c + i + 2], acc[c + i + 3]);
+        const int4 ew = *reinterpret_cast<const int4*>(cex + c + cc);
+        const float4 l4 = *reinterpret_cast<const float4*>(cleast + c + cc), bias = *reinterpret_cast<const float4*>(cbias + c + cc);
+        const float least = fmaxf(fmaxf(l4.x, l4.y), fmaxf(l4.z, l4.w)) + most_least;
+        __syncwarp();
+        uint32_t again = 0;                 // four results that may have to be summed again, per row
+        if (simple) {
+          const int fx = (127 - ew.x) << 23, fy = (127 - ew.y) << 23, fz = (127 - ew.z) << 23, fw = (127 - ew.w) << 23;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float4 q = *reinterpret_cast<const float4*>(s + (rr + 8 * i) * kLd + cc);
+            const int er = s_ex[w][rr + 8 * i] << 23;
+            again |= fminf(fminf(fabsf(q.x), fabsf(q.y)), fminf(fabsf(q.z), fabsf(q.w))) < least ? 15u << (4 * i) : 0u;
+            *reinterpret_cast<float4*>(to + i * step + c) =
+                make_float4(fmaf(q.x, __int_as_float(fx - er), bias.x), fmaf(q.y, __int_as_float(fy - er), bias.y),
+                            fmaf(q.z, __int_as_float(fz - er), bias.z), fmaf(q.w, __int_as_float(fw - er), bias.w));
+          }
+        } else {
+          const int e4[4] = {ew.x, ew.y, ew.z, ew.w}, left = p.N - (nw + c + cc);
+          const float b4[4] = {bias.x, bias.y, bias.z, bias.w};
+#pragma unroll 1
+          for (int i = 0; i < 4; ++i) {
+            const int r = rr + 8 * i;
+            if (r >= rows) break;
+            const float4 q = *reinterpret_cast<const float4*>(s + r * kLd + cc);
+            const float sum[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (j >= left) break;
+              const int e = -(s_ex[w][r] + e4[j]);
+              to[i * step + c + j] = fmaf(sum[j] * pow2i(e / 2), pow2i(e - e / 2), b4[j]);
+              if (fabsf(sum[j]) < least) again |= (left >= 4 ? 15u : (1u << left) - 1) << (4 * i);      // all four, as above
+            }
+          }
+        }
+        if ((c / kOut) & 1) flags[c / 32] |= again << 16; else flags[c / 32] = again;
+      }
+#pragma unroll
+      for (int c = 0; c < kMine; c += kOut) {
+        const uint32_t f = flags[c / 32] >> (16 * ((c / kOut) & 1)) & 0xffffu;
+        if (__any_sync(0xffffffffu, f != 0)) sum_again(p, mw, nw + c, f);
       }
     }
   }
@@ -335,7 +399,9 @@ int launch(const Product& p, const __half* xp, const __half* wp, cudaStream_t st
   if (rc == ATMA_OK) rc = make_map(&mw, wp, p.N, p.Kp, BN);
   if (rc != ATMA_OK) return rc;
   ATMA_CUDA_OK(cudaFuncSetAttribute(linear_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::kSmem));
-  linear_f32_kernel<BN><<<dim3((p.M + kBM - 1) / kBM, (p.N + BN - 1) / BN), kThreads, Tile<BN>::kSmem, st>>>(mx, mw, p);
+  const int64_t tiles = (int64_t)((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN);
+  const int sms = sm_count_of_current_device();
+  linear_f32_kernel<BN><<<(unsigned)(tiles < sms ? tiles : sms), kThreads, Tile<BN>::kSmem, st>>>(mx, mw, p);
   return launch_status("linear_f32 (tcgen05)");
 }
 
