@@ -117,6 +117,7 @@ _SIGNATURES = {
                                      c_float, c_int, c_void_p]),
     "atma_add_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p]),
     "atma_linear_f32": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "atma_linear_act": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "atma_linear_f32_scratch_bytes": (c_int64, [c_int, c_int, c_int]),
     "atma_decode_linear": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int,
                                    c_void_p]),
@@ -192,7 +193,7 @@ _DECODER_SIGNATURES = {
     "atma_delta_scan_scratch_bytes": (c_int64, [POINTER(DeltaArgs)]),
     "atma_delta_step": (c_int, [POINTER(DeltaArgs), c_void_p, c_void_p, c_int64, c_float, c_void_p]),
 }
-_SHARED_SYMBOLS = ("atma_last_error", "atma_decode_linear", "atma_linear_f32", "atma_linear_f32_scratch_bytes")
+_SHARED_SYMBOLS = ("atma_last_error", "atma_decode_linear", "atma_linear_act", "atma_linear_f32", "atma_linear_f32_scratch_bytes")
 
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
 DECODER_SYMBOLS = tuple(_DECODER_SIGNATURES)
@@ -245,7 +246,8 @@ def ptr(t):
 
 
 def stream_ptr():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream; every launch asks, and the number alone takes 0.4 us to get, the stream object 3.3."""
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def dtype_code(t):
