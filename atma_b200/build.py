@@ -22,7 +22,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIBS = {"b200": os.path.join(HERE, "libatma_b200.so"), "decoder": os.path.join(HERE, "libatma_decoder.so")}
 LIB = LIBS["b200"]
 
-SHARED = {"error.cu", "sm100_host.cu", "decode_linear.cu", "delta_blocks.cu", "linear_f32.cu"}
+SHARED = {"error.cu", "sm100_host.cu", "decode_linear.cu", "delta_blocks.cu", "linear_act.cu", "linear_f32.cu"}
 DECODER = {"decoder_rows.cu", "norm_store.cu", "rotary_store.cu", "softmax_attention.cu", "softmax_prefill_sm100.cu", "softmax_rows_f32.cu",
            "softmax_decode_mma.cu",
            "delta_rule.cu", "delta_scan_sm100.cu"}

@@ -23,6 +23,7 @@
 // the result is unchanged), which keeps the read-modify-write of O out of most iterations.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a
 // status word for the host.
+#include "linear_act.cuh"
 #include "linear_f32.cuh"
 #include "polar_prefill.cuh"
 #include "sm100.cuh"
@@ -607,12 +608,13 @@ int sm100_status_fetch_and_clear(int* out) {
 // the device; clears the flag).
 extern "C" int atma_device_status(int* status) {
   ATMA_REQUIRE(status != nullptr, "device_status: null out pointer");
-  int a = 0, b = 0, c = 0, d = 0, e = 0;
+  int a = 0, b = 0, c = 0, d = 0, e = 0, f = 0;
   int rc = atma::sm100_status_fetch_and_clear(&a);
   if (rc == ATMA_OK) rc = atma::scan_sm100_status_fetch_and_clear(&b);
   if (rc == ATMA_OK) rc = atma::scan_local_status_fetch_and_clear(&c);
   if (rc == ATMA_OK) rc = atma::linear_f32_status_fetch_and_clear(&d);
   if (rc == ATMA_OK) rc = atma::polar_tf32_status_fetch_and_clear(&e);
-  *status = a | b | c | d | e;
+  if (rc == ATMA_OK) rc = atma::linear_act_status_fetch_and_clear(&f);
+  *status = a | b | c | d | e | f;
   return rc;
 }

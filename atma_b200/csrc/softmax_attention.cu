@@ -4,6 +4,7 @@
 //
 // A CTA of eight warps holds 16 query rows of one head, two per warp.  Keys come in tiles of 32: a lane owns a key for
 // the scores, and vdim / 32 value channels for the weighted sum, so the softmax statistics of a row are warp reductions.
+#include "linear_act.cuh"
 #include "linear_f32.cuh"
 #include "softmax_attention.cuh"
 
@@ -226,11 +227,12 @@ extern "C" int64_t atma_softmax_decode_scratch_floats(int n_seqs, int H, int map
 
 extern "C" int atma_decoder_device_status(int* status) {
   ATMA_REQUIRE(status != nullptr, "decoder_device_status: null out pointer");
-  int a = 0, b = 0, c = 0, d = 0;
+  int a = 0, b = 0, c = 0, d = 0, e = 0;
   int rc = softmax_sm100_status_fetch_and_clear(&a);
   if (rc == ATMA_OK) rc = delta_sm100_status_fetch_and_clear(&b);
   if (rc == ATMA_OK) rc = linear_f32_status_fetch_and_clear(&c);
   if (rc == ATMA_OK) rc = softmax_tf32_status_fetch_and_clear(&d);
-  *status = a | b | c | d;
+  if (rc == ATMA_OK) rc = linear_act_status_fetch_and_clear(&e);
+  *status = a | b | c | d | e;
   return rc;
 }

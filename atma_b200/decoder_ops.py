@@ -294,18 +294,23 @@ def linear(x, weight, out=None):
 
 def squared_relu_linear(x, weight, bias=None):
     """relu(x @ weight.T + bias)^2."""
-    from .inference_ops import decode_linear, decode_linear_supported
+    from .inference_ops import decode_linear, decode_linear_supported, linear_act_if_faster
     if decode_linear_supported(x, weight):
         return decode_linear(x, weight, bias=bias, gated="plain_squared_relu", lib=_lib.load_decoder())
-    z = _product(x, weight)
-    return bias_squared_relu(z, bias, z)
+    y = linear_act_if_faster(x, weight, "plain_squared_relu", bias, lib=_lib.load_decoder())
+    if y is None:
+        z = _product(x, weight)
+        y = bias_squared_relu(z, bias, z)
+    return y
 
 
 def gelu_gated_linear(x, weight, out):
     """out = gelu_tanh(x @ gate.T) * (x @ up.T) with weight = [gate; up]."""
-    from .inference_ops import decode_linear, decode_linear_supported
+    from .inference_ops import decode_linear, decode_linear_supported, linear_act_if_faster
     if decode_linear_supported(x, weight, gated=True):
         return decode_linear(x, weight, gated="gelu_tanh", out=out, lib=_lib.load_decoder())
+    if linear_act_if_faster(x, weight, "gelu_tanh", out=out, lib=_lib.load_decoder()) is not None:
+        return out
     gu = _product(x, weight)
     half = weight.shape[0] // 2
     return gelu_gate(gu[:, :half], gu[:, half:], out)

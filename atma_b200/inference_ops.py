@@ -351,14 +351,27 @@ LINEAR_F32_MAX_ROWS, LINEAR_F32_MAX_N, LINEAR_F32_MAX_K = 1 << 29, 1 << 21, 1 <<
 _PLAIN = (torch.Tensor, torch.nn.Parameter)
 
 
+def _plain_call(tensors):
+    """Whether these are plain CUDA tensors in a call that nothing watches which a library product would obey: autograd, transforms,
+    tracing, autocast, modes that see every call."""
+    if any(type(t) not in _PLAIN or not t.is_cuda or t.is_neg() for t in tensors):
+        return False
+    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
+        return False
+    if torch.is_autocast_enabled() or torch.compiler.is_compiling() or torch.jit.is_tracing():
+        return False
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
+        return False
+    return not (torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack())
+
+
 def linear_f32_supported(x, weight, bias=None):
     """Whether ``linear_f32`` serves this product: plain fp32 tensors on the current CUDA device, a bias of N values or none,
     enough rows, and nothing around the call that a library product would obey (autograd, transforms, tracing, autocast,
     modes that see every call, a caller's choice of TF32)."""
     tensors = (x, weight) if bias is None else (x, weight, bias)
-    for t in tensors:
-        if type(t) not in _PLAIN or t.dtype != torch.float32 or not t.is_cuda or t.is_neg():
-            return False
+    if any(t.dtype != torch.float32 for t in tensors) or not _plain_call(tensors):
+        return False
     if x.ndim < 2 or weight.ndim != 2 or not weight.is_contiguous() or not _bias_fits(bias, weight.shape[0]) or not _one_device(*tensors):
         return False
     K, N = x.shape[-1], weight.shape[0]
@@ -370,14 +383,6 @@ def linear_f32_supported(x, weight, bias=None):
     if M * N * K < max(LINEAR_F32_MIN_WORK, LINEAR_F32_MIN_WORK_PER_ROW * (M + N)):
         return False
     if K > LINEAR_F32_LONG_K and M * N < LINEAR_F32_LONG_K_MIN_RESULTS:
-        return False
-    if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
-        return False
-    if torch.is_autocast_enabled() or torch.compiler.is_compiling() or torch.jit.is_tracing():
-        return False
-    if torch._C._functorch.peek_interpreter_stack() is not None or torch.autograd.forward_ad._current_level >= 0:
-        return False
-    if torch._C._len_torch_function_stack() or torch._C._len_torch_dispatch_stack():
         return False
     try:
         return not torch.backends.cuda.matmul.allow_tf32
@@ -461,4 +466,71 @@ def decode_linear(x, weight, bias=None, gated=False, out=None, lib=None, any_k=F
     entry = lib.atma_decode_linear_k8 if any_k else lib.atma_decode_linear
     _lib.check(entry(_lib.ptr(x), x.stride(0), _lib.ptr(weight), _lib.ptr(bias), _lib.ptr(out), out.stride(0),
                      B, N, K, gate, _lib.dtype_code(x), _lib.stream_ptr()), lib)
+    return out
+
+
+# ``linear_act`` against the library's product and the activation behind it, us out of HBM for its three forms (N, K = 8192, 1024):
+#   M = 12000 125, 132, 129 against 185, 181, 206; 3000 50, 52, 48 against 62, 60, 60; 1024 25, 25, 25 against 28, 28, 30.
+# Below that, 100 tiles of 256 x 256, its pairs of SMs are too few to hide that one tile takes 19 us from launch to end: 768 24, 25, 25
+# against 24, 24, 24; 300 20, 20, 19 against 17, 17, 19; 1500 x 4096 x 1024 25, 25, 24 against 24, 24, 23.  With a short K the activation
+# is most of the work and has eight warps an SM: 20000 x 2048 x 128 41, 47, 38 against 46, 42, 48; at 256 25, 28, 25 against 30, 32, 30
+# (16000 x 1024).  Rows that fill their tiles badly: 600 x 16384 x 2048 48, 49, 48 against 48, 46, 48.
+LINEAR_ACT_MIN_RESULTS, LINEAR_ACT_MIN_K, LINEAR_ACT_TILE = 100 * 65536, 256, 256
+
+
+def _linear_act_pays(M, N, K):
+    rows = -(-M // LINEAR_ACT_TILE) * LINEAR_ACT_TILE
+    return M * N >= LINEAR_ACT_MIN_RESULTS and K >= LINEAR_ACT_MIN_K and 5 * M >= 4 * rows
+
+
+def linear_act_supported(x, weight, gated, bias=None, out=None):
+    """Whether ``linear_act`` serves this product: plain 16-bit tensors on the current CUDA device as its entry takes them, and nothing
+    around the call that a library product would obey."""
+    if x.ndim != 2 or weight.ndim != 2:
+        return False
+    dtype, (M, K), N, halves = x.dtype, x.shape, weight.shape[0], _GATES[gated] in _HALVES
+    width = N // 2 if halves else N
+    if dtype not in _HALF_TYPES or M == 0 or M > 1 << 24 or N == 0 or N > 1 << 20 or N % (16 if halves else 8) or K == 0 or K > 1 << 20 or K % 8:
+        return False
+    tensors = [t for t in (x, weight, bias, out) if t is not None]
+    if not _plain_call(tensors) or not _one_device(*tensors):
+        return False
+    for t in tensors:
+        if t.dtype != dtype or t.data_ptr() % 16 and t is not bias:
+            return False
+    if not _rows_fit(x, M, K) or weight.shape[1] != K or not weight.is_contiguous() or (out is not None and not _rows_fit(out, M, width)):
+        return False
+    return bias is None or (bias.shape == (N,) and bias.is_contiguous())
+
+
+_HALF_TYPES = (torch.bfloat16, torch.float16)
+
+
+def _rows_fit(t, rows, cols):
+    step = t.stride(0)
+    return t.shape == (rows, cols) and t.stride(1) == 1 and step % 8 == 0 and cols <= step <= 1 << 24
+
+
+@torch.no_grad()
+def linear_act(x, weight, gated, bias=None, out=None, lib=None):
+    """The first product of an MLP with its activation, for many rows: ``gated``, ``out`` and ``lib`` as for ``decode_linear``."""
+    if not linear_act_supported(x, weight, gated, bias, out):
+        raise ValueError("linear_act does not serve this product")
+    return _linear_act(x, weight, gated, bias, out, lib)
+
+
+def linear_act_if_faster(x, weight, gated, bias=None, out=None, lib=None):
+    """``linear_act`` where it serves the product and takes less time than a library product with the activation behind it, else None."""
+    if not _linear_act_pays(x.shape[0], weight.shape[0], x.shape[-1]) or not linear_act_supported(x, weight, gated, bias, out):
+        return None
+    return _linear_act(x, weight, gated, bias, out, lib)
+
+
+def _linear_act(x, weight, gated, bias, out, lib):
+    lib, form = _lib.load() if lib is None else lib, _GATES[gated]
+    (M, K), N = x.shape, weight.shape[0]
+    if out is None:
+        out = torch.empty((M, N // 2 if form in _HALVES else N), device=x.device, dtype=x.dtype)
+    _lib.check(lib.atma_linear_act(x.data_ptr(), x.stride(0), weight.data_ptr(), None if bias is None else bias.data_ptr(), out.data_ptr(), out.stride(0),
+                                   M, N, K, form, _lib.dtype_code(x), _lib.stream_ptr()), lib)
     return out

@@ -36,7 +36,7 @@ from .gated_delta import gated_delta_decode_step, gated_delta_decode_step_fused,
 from .inference_ops import qkv_prep_prefill, sigmoid_gate_mul
 from .polar import polar_attention_fwd
 from .inference_ops import (add_rms_norm, decode_linear, decode_linear_supported, lfm2_conv_decode_step, lfm2_conv_packed, linear,
-                            qkv_prep_decode, rms_sigmoid_gate, softcap_logits, squared_relu_gate)
+                            linear_act_if_faster, qkv_prep_decode, rms_sigmoid_gate, softcap_logits, squared_relu_gate)
 from .layer import PackedMaps, global_attention_prefill_packed
 from .polar import DECODE_BESIDE_MAX_ROWS, polar_attention_decode
 
@@ -145,9 +145,11 @@ class AtmaModel:
         if self.small_batch_linear and decode_linear_supported(h, w, gated=True, bias=b):
             act = decode_linear(h, w, b, gated=True)            # fc GEMM and the squared-ReLU gate in one launch
         else:
-            fc = linear(h, w, b)
-            half = fc.shape[-1] // 2
-            act = squared_relu_gate(fc[:, :half], fc[:, half:])
+            act = linear_act_if_faster(h, w, True, b)
+            if act is None:
+                fc = linear(h, w, b)
+                half = fc.shape[-1] // 2
+                act = squared_relu_gate(fc[:, :half], fc[:, half:])
         return self._lin(act, f"blocks.{i}.mlp.proj")
 
     def logits(self, hidden):

@@ -239,6 +239,12 @@ int atma_linear_f32(const float* x, int64_t x_row_stride, const float* w, const 
                     int M, int N, int K, void* scratch, void* stream);
 int64_t atma_linear_f32_scratch_bytes(int M, int N, int K);
 
+/* The first product of an MLP with its activation, 16-bit types, on the tensor cores: forms as atma_decode_linear's `gated`, 1 to 3
+ * (1, 2: the weight holds two halves and out has N/2 columns).  x, weight [N][K] and out 16-byte aligned, row strides (elements)
+ * multiples of 8, K a multiple of 8, N of 16 (form 3: 8); bias may be NULL, else N values. */
+int atma_linear_act(const void* x, int64_t x_row_stride, const void* weight, const void* bias, void* out, int64_t out_row_stride,
+                    int M, int N, int K, int form, int dtype, void* stream);
+
 /* Weight-streaming linear layer for decode batches of up to 16 rows (16-bit types): out[b][n] =
  * sum_k x[b][k] * weight[n][k] + bias[n] (bias may be NULL), weight [N][K] dense in torch's Linear
  * layout, fp32 accumulation, one rounding to `dtype`.  gated = 1: the N outputs are the two halves
