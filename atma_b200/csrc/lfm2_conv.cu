@@ -142,11 +142,14 @@ __global__ void lfm2_conv_packed_kernel(const T* __restrict__ proj, int64_t proj
 }
 
 // Vector form of the packed prefill (D and the row strides multiples of 16 bytes, 16-byte aligned bases): thread =
-// 16 bytes of channels x a run of kLfmVecTok consecutive tokens.  The B and x' parts of all kLfmVecTok + K - 1 rows
-// are requested as 16-byte loads up front and multiplied into the gated input once per row; the C part is read where
-// the token is written.  Rows before a sequence start (saved state or zero) and the state write of a closing token
-// are rare and out of line.  Same rounding points and accumulation order as the scalar form.
-constexpr int kLfmVecTok = 4;
+// 16 bytes of channels x a run of kLfmVecTok consecutive tokens.  All rows of the run and the K - 1 in front are requested
+// as 16-byte loads up front, behind the weights and the sequence's numbers, which would cost a second latency after them.
+// Bound by bytes in flight: a run that meets the start or the end of a sequence (saved state or zero in front, a state to
+// write) is rare, goes out of line and reads its rows again, so that four CTAs fit an SM (for five the loads of a run find no
+// registers).  Three CTAs with the rare runs in line and the numbers asked for last: 12800 x 1024 36.9 us, 30.7 now; 32768 x 1024
+// 73.9, 57.4 now (4.7 TB/s).
+// Same rounding points and accumulation order as the scalar form.
+constexpr int kLfmVecTok = 4, kLfmVecCtas = 4;
 
 template <typename T> struct LfmVec16 {
   static constexpr int N = 16 / sizeof(T);
@@ -172,8 +175,52 @@ __device__ __noinline__ void lfm2_state_write(T* __restrict__ dst, const uint4* 
   }
 }
 
+// The tokens [t0, t0 + nt) of 16 bytes of channels, whatever sequences they belong to.
 template <typename T, int K>
-__global__ void __launch_bounds__(128, 3)
+__device__ __noinline__ void lfm2_run_general(const T* proj, int64_t proj_st, const T* w, T* out, int64_t out_st, T* state, const T* init_state,
+                                              int64_t state_ss, const int32_t* seq_start, const int32_t* seq_end, const int32_t* seq_slot,
+                                              int D, int t0, int nt, int d0) {
+  constexpr int N = LfmVec16<T>::N;
+#pragma unroll 1
+  for (int t = t0; t < t0 + nt; ++t) {
+    const int s0 = seq_start[t], e0 = seq_end[t], sl = seq_slot[t];
+    LfmVec16<T> prev[K];                              // prev[j] = gated input K-1-j rows before t as this sequence sees it
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const int src = t - (K - 1 - j);
+      if (src >= s0) {
+        const T* p = proj + (int64_t)src * proj_st + d0;
+        LfmVec16<T> b, x;
+        b.u = *reinterpret_cast<const uint4*>(p);
+        x.u = *reinterpret_cast<const uint4*>(p + 2 * D);
+#pragma unroll
+        for (int n = 0; n < N; ++n) prev[j].e[n] = from_f32<T>(to_f32(b.e[n]) * to_f32(x.e[n]));
+      } else {
+        prev[j].u = lfm2_row_before_start<T, K>(sl >= 0 ? init_state : nullptr,
+                                                (sl >= 0 ? sl * state_ss : 0) + (int64_t)d0 * (K - 1), s0 - src);
+      }
+    }
+    LfmVec16<T> cv, o;
+    cv.u = *reinterpret_cast<const uint4*>(proj + (int64_t)t * proj_st + D + d0);
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < K; ++j) acc = fmaf(to_f32(prev[j].e[n]), to_f32(w[(int64_t)(d0 + n) * K + j]), acc);
+      o.e[n] = from_f32<T>(to_f32(cv.e[n]) * round_through<T>(acc));
+    }
+    *reinterpret_cast<uint4*>(out + (int64_t)t * out_st + d0) = o.u;
+    if (t == e0 - 1 && sl >= 0 && state != nullptr) {
+      uint4 keep[K - 1];
+#pragma unroll
+      for (int j = 0; j < K - 1; ++j) keep[j] = prev[j + 1].u;
+      lfm2_state_write<T, K>(state + sl * state_ss + (int64_t)d0 * (K - 1), keep);
+    }
+  }
+}
+
+template <typename T, int K>
+__global__ void __launch_bounds__(128, kLfmVecCtas)
 lfm2_conv_packed_vec_kernel(const T* __restrict__ proj, int64_t proj_st, const T* __restrict__ w, T* __restrict__ out,
                             int64_t out_st, T* __restrict__ state, const T* __restrict__ init_state, int64_t state_ss,
                             const int32_t* __restrict__ seq_start, const int32_t* __restrict__ seq_end,
@@ -188,6 +235,16 @@ lfm2_conv_packed_vec_kernel(const T* __restrict__ proj, int64_t proj_st, const T
   const int d0 = cg * N;
   const int nt = min(kLfmVecTok, total - t0);
 
+  const int sa = seq_start[t0], sb = seq_start[t0 + nt - 1], ea = seq_end[t0 + nt - 1];
+  constexpr int kPieces = (N * K * (int)sizeof(T) + 15) / 16;       // the thread's N x K weights are neighbours in memory
+  LfmVec16<T> wv[kPieces];
+  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < kPieces; ++i) wv[i].u = *reinterpret_cast<const uint4*>(w + (int64_t)d0 * K + i * N);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N * K; ++i) wv[i / N].e[i % N] = w[(int64_t)d0 * K + i];
+  }
   LfmVec16<T> bx[kLfmVecTok + K - 1], xx[kLfmVecTok + K - 1], cc[kLfmVecTok];
 #pragma unroll
   for (int i = 0; i < kLfmVecTok + K - 1; ++i) {
@@ -204,89 +261,27 @@ lfm2_conv_packed_vec_kernel(const T* __restrict__ proj, int64_t proj_st, const T
 #pragma unroll
   for (int i = 0; i < kLfmVecTok; ++i)
     cc[i].u = i < nt ? *reinterpret_cast<const uint4*>(proj + (int64_t)(t0 + i) * proj_st + D + d0) : make_uint4(0u, 0u, 0u, 0u);
-  float wt[N][K];
-  if ((K * (int)sizeof(T) * N) % 16 == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
-    constexpr int kPieces = (N * K * (int)sizeof(T) + 15) / 16;     // the thread's N x K weights are neighbours in memory
-    LfmVec16<T> wv[kPieces];
-#pragma unroll
-    for (int i = 0; i < kPieces; ++i) wv[i].u = *reinterpret_cast<const uint4*>(w + (int64_t)d0 * K + i * N);
-#pragma unroll
-    for (int n = 0; n < N; ++n)
-#pragma unroll
-      for (int j = 0; j < K; ++j) wt[n][j] = to_f32(wv[(n * K + j) / N].e[(n * K + j) % N]);
-  } else {
-#pragma unroll
-    for (int n = 0; n < N; ++n)
-#pragma unroll
-      for (int j = 0; j < K; ++j) wt[n][j] = to_f32(w[(d0 + n) * K + j]);
+  // the run and its K-1 rows of left context lie inside one sequence that goes on behind it
+  if (nt < kLfmVecTok || sa != sb || ea <= t0 + nt || sa > t0 - (K - 1)) {
+    lfm2_run_general<T, K>(proj, proj_st, w, out, out_st, state, init_state, state_ss, seq_start, seq_end, seq_slot, D, t0, nt, d0);
+    return;
   }
   // gated input B * x' of every row of the run, rounded to T as eager materialises it (reuses bx)
 #pragma unroll
   for (int i = 0; i < kLfmVecTok + K - 1; ++i)
 #pragma unroll
     for (int n = 0; n < N; ++n) bx[i].e[n] = from_f32<T>(to_f32(bx[i].e[n]) * to_f32(xx[i].e[n]));
-
-  const int sa = seq_start[t0], ea = seq_end[t0 + nt - 1], sla = seq_slot[t0];
-  const bool uniform = sa == seq_start[t0 + nt - 1] && ea > t0 + nt;   // one sequence, not closed inside the run
-  if (uniform && sa <= t0 - (K - 1)) {
-    // common case: the run and its K-1 rows of left context lie inside one sequence
-    float win[K][N];
 #pragma unroll
-    for (int rl = 0; rl < kLfmVecTok + K - 1; ++rl) {
-#pragma unroll
-      for (int n = 0; n < N; ++n) win[rl % K][n] = to_f32(bx[rl].e[n]);
-      if (rl >= K - 1 && rl - (K - 1) < nt) {
-        LfmVec16<T> o;
-#pragma unroll
-        for (int n = 0; n < N; ++n) {
-          float acc = 0.f;
-#pragma unroll
-          for (int j = 0; j < K; ++j) acc = fmaf(win[(rl - (K - 1) + j) % K][n], wt[n][j], acc);
-          o.e[n] = from_f32<T>(to_f32(cc[rl - (K - 1)].e[n]) * round_through<T>(acc));
-        }
-        *reinterpret_cast<uint4*>(out + (int64_t)(t0 + rl - (K - 1)) * out_st + d0) = o.u;
-      }
-    }
-    return;
-  }
-#pragma unroll 1
-  for (int i = 0; i < nt; ++i) {
-    const int t = t0 + i;
-    const int s0 = uniform ? sa : seq_start[t], e0 = uniform ? ea : seq_end[t], sl = uniform ? sla : seq_slot[t];
-    LfmVec16<T> prev[K];                              // prev[j] = gated input K-1-j rows before t as this sequence sees it
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      const int src = t - (K - 1 - j);
-      if (src >= s0) {
-        const int idx = i + j;                        // bx[] index; selected without dynamic register indexing
-        uint4 u = bx[0].u;
-#pragma unroll
-        for (int q = 1; q < kLfmVecTok + K - 1; ++q) if (q == idx) u = bx[q].u;
-        prev[j].u = u;
-      } else {
-        prev[j].u = lfm2_row_before_start<T, K>(sl >= 0 ? init_state : nullptr,
-                                                (sl >= 0 ? sl * state_ss : 0) + (int64_t)d0 * (K - 1), s0 - src);
-      }
-    }
-    uint4 cu = cc[0].u;
-#pragma unroll
-    for (int q = 1; q < kLfmVecTok; ++q) if (q == i) cu = cc[q].u;
-    LfmVec16<T> cv, o;
-    cv.u = cu;
+  for (int i = 0; i < kLfmVecTok; ++i) {
+    LfmVec16<T> o;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       float acc = 0.f;
 #pragma unroll
-      for (int j = 0; j < K; ++j) acc = fmaf(to_f32(prev[j].e[n]), wt[n][j], acc);
-      o.e[n] = from_f32<T>(to_f32(cv.e[n]) * round_through<T>(acc));
+      for (int j = 0; j < K; ++j) acc = fmaf(to_f32(bx[i + j].e[n]), to_f32(wv[(n * K + j) / N].e[(n * K + j) % N]), acc);
+      o.e[n] = from_f32<T>(to_f32(cc[i].e[n]) * round_through<T>(acc));
     }
-    *reinterpret_cast<uint4*>(out + (int64_t)t * out_st + d0) = o.u;
-    if (t == e0 - 1 && sl >= 0 && state != nullptr) {
-      uint4 keep[K - 1];
-#pragma unroll
-      for (int j = 0; j < K - 1; ++j) keep[j] = prev[j + 1].u;
-      lfm2_state_write<T, K>(state + sl * state_ss + (int64_t)d0 * (K - 1), keep);
-    }
+    *reinterpret_cast<uint4*>(out + (int64_t)(t0 + i) * out_st + d0) = o.u;
   }
 }
 
