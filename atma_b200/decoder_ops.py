@@ -297,7 +297,7 @@ def squared_relu_linear(x, weight, bias=None):
     from .inference_ops import decode_linear, decode_linear_supported, linear_act_if_faster
     if decode_linear_supported(x, weight):
         return decode_linear(x, weight, bias=bias, gated="plain_squared_relu", lib=_lib.load_decoder())
-    y = linear_act_if_faster(x, weight, "plain_squared_relu", bias, lib=_lib.load_decoder())
+    y = linear_act_if_faster(x, weight, "plain_squared_relu", bias, lib=_lib.load_decoder()) if x.dtype == torch.bfloat16 else None
     if y is None:
         z = _product(x, weight)
         y = bias_squared_relu(z, bias, z)
@@ -309,7 +309,7 @@ def gelu_gated_linear(x, weight, out):
     from .inference_ops import decode_linear, decode_linear_supported, linear_act_if_faster
     if decode_linear_supported(x, weight, gated=True):
         return decode_linear(x, weight, gated="gelu_tanh", out=out, lib=_lib.load_decoder())
-    if linear_act_if_faster(x, weight, "gelu_tanh", out=out, lib=_lib.load_decoder()) is not None:
+    if x.dtype == torch.bfloat16 and linear_act_if_faster(x, weight, "gelu_tanh", out=out, lib=_lib.load_decoder()) is not None:
         return out
     gu = _product(x, weight)
     half = weight.shape[0] // 2

@@ -500,7 +500,15 @@ def linear_act_supported(x, weight, gated, bias=None, out=None):
             return False
     if not _rows_fit(x, M, K) or weight.shape[1] != K or not weight.is_contiguous() or (out is not None and not _rows_fit(out, M, width)):
         return False
+    if out is not None and any(_overlap(out, t) for t in tensors if t is not out):      # results leave while inputs are still read
+        return False
     return bias is None or (bias.shape == (N,) and bias.is_contiguous())
+
+
+def _overlap(a, b):
+    """Whether the stretches of memory between two tensors' first and last values meet."""
+    (a0, a1), (b0, b1) = ((t.data_ptr(), t.data_ptr() + t.element_size() * (1 + sum((n - 1) * s for n, s in zip(t.shape, t.stride())))) for t in (a, b))
+    return a0 < b1 and b0 < a1
 
 
 _HALF_TYPES = (torch.bfloat16, torch.float16)
