@@ -7,7 +7,8 @@ fourth one (i % 4 == 2) a global Polar + gated-delta layer, the others LFM2 gate
 each followed by the squared-ReLU gated MLP; final RMSNorm, LM head, logit soft-cap.  It takes
 the reference's ``state_dict`` as is (inference/utils/loader.py:5-39).
 
-Projections are cuBLAS (``linear_f32`` for fp32 prompts); everything between them is this library:
+Projections are cuBLAS (``linear_f32`` for fp32 prompts, ``linear_act`` for the MLP's first product and its gate over many rows);
+everything between them is this library:
 
     prefill (packed fresh prompts)          decode (one token per sequence, CUDA-graph safe)
     add_rms_norm                            add_rms_norm
@@ -16,7 +17,8 @@ Projections are cuBLAS (``linear_f32`` for fp32 prompts); everything between the
     polar_attention_packed_fwd              polar_attention_decode (c * sigmoid(gate) written by the merge)
     packed_gated_delta_prefill              gated_delta_decode_step_fused (gates from logits, RMSNorm * sigmoid(gate))
     sigmoid_gate_mul, rms_sigmoid_gate
-    squared_relu_gate, softcap_logits       squared_relu_gate, softcap_logits
+    linear_act or squared_relu_gate         squared_relu_gate
+    softcap_logits                          softcap_logits
 
 In decode a global layer is six launches: one GEMM for all of its input projections (q|gate, k,
 v, the two memory gates' logits, the memory's output gate - their weights concatenated once at
