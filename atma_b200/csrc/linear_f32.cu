@@ -206,9 +206,12 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   __shared__ uint64_t full[L::kStages], empty[L::kStages], acc_full[2], acc_empty[2];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort_v;
-  __shared__ int s_ex[8][32];               // of each warp's rows: the power of two
-  __shared__ __align__(16) int s_cex[2][BN];            // of the columns the same, and the bias; a warp may be a tile ahead of another
-  __shared__ __align__(16) float s_cleast[2][BN], s_cbias[2][BN];
+  // A warp's own figures of its rows (the power of two) and columns (the same, from where on a sum is trusted, the bias).  Four warps
+  // have the same columns, but no copy in common: a warp gives its accumulators away before it writes its results, so with K <= 128
+  // the next tile's products can be through, and another warp two tiles ahead, while it still reads.
+  __shared__ int s_ex[8][32];
+  __shared__ __align__(16) int s_cex[8][BN / 2];
+  __shared__ __align__(16) float s_cleast[8][BN / 2], s_cbias[8][BN / 2];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int m_tiles = (p.M + kBM - 1) / kBM, tiles = m_tiles * ((p.N + BN - 1) / BN);
@@ -286,13 +289,12 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       const bool in_row = lane < rows;
       const int ex = in_row ? p.exps[mw + lane] : 0;
       const float row_least = in_row ? trusted_from(p.losses[mw + lane]) : 0.f, most_least = warp_max(row_least);
-      const int turn = tile / gridDim.x & 1;
-      int* cex = &s_cex[turn][side * kMine];
-      float *cleast = &s_cleast[turn][side * kMine], *cbias = &s_cbias[turn][side * kMine];
-      __syncwarp();                         // the last tile's rows have been read
+      int* cex = s_cex[w];
+      float *cleast = s_cleast[w], *cbias = s_cbias[w];
+      __syncwarp();                         // the last tile's figures have been read
       s_ex[w][lane] = ex;
       int most_e = -1000, least_e = 1000;
-      // under the first products; the four warps of these columns write the same
+      // under the first products
 #pragma unroll
       for (int i = lane; i < kMine; i += 32) {
         const bool in = nw + i < p.N;
