@@ -13,7 +13,7 @@
 // activations among them, have next to none, and the test costs nothing that shows; where every result needs it, 1500 x 8192 x
 // 1024 takes 7.8 ms instead of 0.12, with one such row of x 0.31.
 //   split kernel: one CTA per row of x and of w, two fp16 planes each, the row's power of two and what it lost.
-//   product kernel: a CTA per SM takes tiles of 128 rows x BN columns in turn.  Warp 0 TMA (both planes of 64 columns of x and of
+//   product kernel: a CTA per SM takes tiles of 128 rows x BN columns in turn (a very long K: a CTA per tile).  Warp 0 TMA (both planes of 64 columns of x and of
 //   w per stage), warp 1 MMA, warps 2-9 add the sums of one stage out of one half of the accumulator columns while the next stage's
 //   products go to the other half, scale them back and write them, under the first two stages of the next tile.
 // Bound by the products (1536 clocks per 64 columns at BN = 256) and L2 -> shared memory traffic (96 KB for them, 1600 clocks) within
@@ -387,6 +387,11 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   if (tid == 0 && s_abort_v) atomicExch(&g_linear_status, 1);
 }
 
+// From here on a tile has a CTA to itself.  Tiles in turn have the next products wait while results are summed again, and a wait ends
+// after a second or two: a tile of 128 x 256 with nothing else took 2.6 ms at K = 1024 and takes in proportion to K.  What tiles in turn save,
+// some 12000 clocks each, is then less than 1.5 % of a tile's 512 stages.
+constexpr int kAloneK = 1 << 15;
+
 int make_map(CUtensorMap* out, const __half* planes, int rows, int Kp, int box_rows) {
   const uint64_t dims[4] = {(uint64_t)Kp, (uint64_t)rows, 2, 1};
   const int64_t strides[3] = {Kp, (int64_t)rows * Kp, 2 * (int64_t)rows * Kp};
@@ -403,7 +408,8 @@ int launch(const Product& p, const __half* xp, const __half* wp, cudaStream_t st
   ATMA_CUDA_OK(cudaFuncSetAttribute(linear_f32_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<BN>::kSmem));
   const int64_t tiles = (int64_t)((p.M + kBM - 1) / kBM) * ((p.N + BN - 1) / BN);
   const int sms = sm_count_of_current_device();
-  linear_f32_kernel<BN><<<(unsigned)(tiles < sms ? tiles : sms), kThreads, Tile<BN>::kSmem, st>>>(mx, mw, p);
+  const bool in_turn = tiles > sms && p.Kp < kAloneK;
+  linear_f32_kernel<BN><<<(unsigned)(in_turn ? sms : tiles), kThreads, Tile<BN>::kSmem, st>>>(mx, mw, p);
   return launch_status("linear_f32 (tcgen05)");
 }
 

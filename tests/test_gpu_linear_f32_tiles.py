@@ -37,3 +37,18 @@ def test_tiles_in_turn(M, K, N, again):
             off = (y[part] - (x[part].double() @ w.double().t() + b)).abs()
             assert (off <= _product_bound(x[part], w) + b.abs() * 2 ** -23).all()
     assert atma_b200.device_status() == 0
+
+
+@pytest.mark.parametrize("K", [2 ** 15 - 64, 2 ** 15 - 63, 2 ** 15])       # tiles in turn, and from 2^15 on (padded to 64) a CTA per tile
+def test_long_sums_that_are_all_taken_again(K):
+    """176 tiles; every other tile of rows is summed again from one end to the other, while other warps wait for it."""
+    M, N = 2000, 2600
+    g = torch.Generator(device="cuda").manual_seed(K)
+    x, w = torch.randn(M, K, generator=g, device="cuda"), torch.randn(N, K, generator=g, device="cuda")
+    x[(torch.arange(M, device="cuda") // 128) % 2 == 0, 1:] *= 2.0 ** -29
+    w[:, 0] = 0
+    y = linear_f32(x, w)
+    for r in range(0, M, 500):
+        part = slice(r, r + 500)
+        assert ((y[part] - x[part].double() @ w.double().t()).abs() <= _product_bound(x[part], w)).all()
+    assert atma_b200.device_status() == 0
