@@ -388,7 +388,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 }
 
 // From here on a tile has a CTA to itself.  Tiles in turn have the next products wait while results are summed again, and a wait ends
-// after a second or two: a tile of 128 x 256 with nothing else took 2.6 ms at K = 1024 and takes in proportion to K.  What tiles in turn save,
+// after 1.1 s: a tile of 128 x 256 with nothing else took 2.6 ms at K = 1024, 24 at 8192, 150 at 32704.  What tiles in turn save,
 // some 12000 clocks each, is then less than 1.5 % of a tile's 512 stages.
 constexpr int kAloneK = 1 << 15;
 

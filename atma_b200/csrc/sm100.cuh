@@ -46,8 +46,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // another thread of the CTA has given up) the wait returns false; the caller then leaves its
 // loop, the CTA frees its TMEM and returns, and the host finds a non-zero device status word.
 // Short code on purpose: it stands in every loop of kernels whose warps do different things, and
-// those have to share the instruction cache.
-constexpr uint32_t kWaitLimitClocks = 3900000000u;   // 2 s
+// those have to share the instruction cache.  The clock has 32 bits, so the limit is half of its range: a poll falls into the
+// other half unless the waiting thread itself stands still for as long.  1.1 s at 1.9 GHz, longer at lower clocks.
+constexpr uint32_t kWaitLimitClocks = 1u << 31;
 
 __device__ __forceinline__ uint32_t clock32() {
   uint32_t t;
