@@ -13,6 +13,7 @@
 //          T = (I + A)^-1: 16 x 16 diagonal blocks by substitution (fp32), then the blocks below
 //          the diagonal level by level with mma.sync tf32 (G_il = -T_ii A_il; T_ij = sum_l G_il T_lj)
 //          Tw[p][s] = -T[p][s] beta_s g_s k_inv_s,  Tu[p][s] = T[p][s] beta_s    -> record
+//          (fp16: k_inv without a power of two, see gated_delta_scan.cuh)
 //
 // The row scalings of the right-hand sides are in the columns of T, so that the recurrence multiplies
 // Tw and Tu with the K and V rows as they are.
@@ -62,6 +63,13 @@ struct Params {
   int n_pairs; int64_t n_tiles;
   VarLen var;
 };
+
+// x = pow2 * the result, which is in [1/2, 1); x > 0 and normal
+__device__ __forceinline__ float without_pow2(float x, float& pow2) {
+  const uint32_t b = __float_as_uint(x);
+  pow2 = __uint_as_float((b & 0x7f800000u) + 0x00800000u);
+  return __uint_as_float((b & 0x007fffffu) | 0x3f000000u);
+}
 
 __device__ __forceinline__ void worker_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
@@ -272,17 +280,20 @@ scan_local_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         if (half) s_qinv[row] = inv * p.scale; else s_kinv[row] = inv;
       }
       worker_sync();
+      float k_left = s_kinv[row], k_pow2 = 1.f;          // what Tw and the scalars have of k_inv, and what the K rows get
+      if (!kBf16 && p.normalize) k_left = without_pow2(k_left, k_pow2);
       if (half == 0) {
         if (quad & 1) run += s_wsum[quad - 1];           // second warp of the chunk
         s_lg[row] = run;
-        s_wsc[row] = -s_bt[row] * __expf(run) * s_kinv[row];       // column scale of Tw
+        s_wsc[row] = -s_bt[row] * __expf(run) * k_left;  // column scale of Tw
       }
       worker_sync();
       const float lg_p = s_lg[row], bt_p = s_bt[row], lg_C = s_lg[64 * ci + 63], kinv_p = s_kinv[row], qinv_p = s_qinv[row];
       if (half == 0 && rec >= 0) {
         float* sc = p.scal + rec * kScal;
         sc[kScalQ + pr] = valid ? __expf(lg_p) * qinv_p : 0.f;
-        sc[kScalK + pr] = valid ? __expf(lg_C - lg_p) * kinv_p : 0.f;
+        sc[kScalK + pr] = valid ? __expf(lg_C - lg_p) * k_left : 0.f;
+        if constexpr (!kBf16) sc[kScalP + pr] = k_pow2;
         if (pr == kC - 1) sc[kScalG] = __expf(run);
       }
 

@@ -16,8 +16,9 @@
 //     MMA   O1^T = S^T Q^T,  O2^T = U^T Rq^T;  O warps: o = g q_inv O1 + O2
 //
 // Q, K, V and the record tiles are operands exactly as TMA delivers them; scalars per row are applied to fp32
-// accumulators.  fp16 has no room for U times an unbounded 1 / |k|, so there the helper warps scale the K rows in
-// shared memory instead.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
+// accumulators.  fp16 has no room for an unbounded 1 / |k|, neither in Tw nor in U, so there the W warps bring the K rows
+// in shared memory to a length between 1 and 2 by a power of two, which loses nothing, a chunk ahead of the first product
+// that reads them, and k_inv stands for what is left, a factor between 1/2 and 1.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
 // accumulators have a channel on the 128 TMEM lanes, which spreads the thread phases over all four schedulers.
 //
 // What bounds it is the latency of the chain, of which the two thread phases are half: 3000 clocks a chunk, 650 for S and 750
@@ -62,7 +63,7 @@ constexpr uint32_t kColSb = 0, kColUb = 128, kColUs = 160, kColU = 192, kColO1 =
 
 struct Barriers {
   uint64_t vt_full[kVts], vt_empty[kVts], k_full[kKs], k_empty[kKs], qr_full[kQrs], qr_empty[kQrs], sc_full[kScs], sc_empty[kScs];
-  uint64_t w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
+  uint64_t rows_ready, w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
 };
 
 struct Params {
@@ -131,7 +132,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     for (int i = 0; i < kQrs; ++i) { mbar_init(&bar.qr_full[i], 1); mbar_init(&bar.qr_empty[i], 1); }
     for (int i = 0; i < kScs; ++i) { mbar_init(&bar.sc_full[i], 1); mbar_init(&bar.sc_empty[i], kStateWarps + (kBf16 ? 1 : 2) * kHelpWarps); }
     mbar_init(&bar.sb_ready, kStateWarps); mbar_init(&bar.us_ready, kStateWarps); mbar_init(&bar.ub_ready, kStateWarps);
-    mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
+    mbar_init(&bar.rows_ready, kHelpWarps); mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
     mbar_init(&bar.w_done, 1); mbar_init(&bar.u_full, 1); mbar_init(&bar.s_done, 1); mbar_init(&bar.o_done, 1);
     s_abort = 0;
     fence_barrier_init();
@@ -210,7 +211,8 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           const int n = i + 1;                           // -W^T of the next chunk, over dS^T, which has been read (sb_ready)
           if (n < n_chunks) {
             const uint32_t vt = base + n % kVts * kVtBytes, nkr = base + kOffK + n % kKs * kRowBytes;
-            ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && mbar_wait(&bar.k_full[n % kKs], (uint32_t)(n / kKs) & 1u, abort_flag);
+            ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && mbar_wait(&bar.k_full[n % kKs], (uint32_t)(n / kKs) & 1u, abort_flag) &&
+                 (kBf16 || mbar_wait(&bar.rows_ready, (uint32_t)n & 1u, abort_flag));
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
@@ -226,7 +228,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           const uint64_t kr = desc_mn(base + kOffK + i % kKs * kRowBytes);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            mma_ts(tbase + kColS, tbase + (kBf16 ? kColUs : kColUb) + kk * 8, kr + uint64_t((kk * 2048) >> 4), idesc_s, kk > 0);
+            mma_ts(tbase + kColS, tbase + kColUs + kk * 8, kr + uint64_t((kk * 2048) >> 4), idesc_s, kk > 0);
           tc_commit(&bar.s_done);
           tc_commit(&bar.k_empty[i % kKs]);
         }
@@ -351,7 +353,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       {
         uint32_t r[32];
         tmem_ld32(lane_base + kColU + 32 * half, r);
-        if constexpr (kBf16) {
+        {
           uint32_t w[16];
 #pragma unroll
           for (int j = 0; j < 16; j += 2) {
@@ -377,7 +379,6 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if constexpr (!kBf16) mbar_arrive(&bar.us_ready);
           mbar_arrive(&bar.ub_ready);
           mbar_arrive(&bar.sc_empty[i % kScs]);
         }
@@ -392,11 +393,33 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     // =============================== W warps ======================================================
     const int row = 32 * (warp & 3) + lane;              // TMEM lane: key channel
     const uint32_t lane_base = tbase + (uint32_t(32 * (warp & 3)) << 16);
-    for (int i = 0; i < n_chunks; ++i) {
-      const float* sc = reinterpret_cast<const float*>(smem + kOffSc + i % kScs * kScBytes);
-      if constexpr (!kBf16) {
-        if (!mbar_wait_warp(&bar.sc_full[i % kScs], (uint32_t)(i / kScs) & 1u, abort_flag)) break;
+    // K rows of a chunk times their powers of two, in place: this thread's is row / 2, one box of it
+    auto prepare = [&](int c) {
+      const float* sc = reinterpret_cast<const float*>(smem + kOffSc + c % kScs * kScBytes);
+      if (!mbar_wait_warp(&bar.sc_full[c % kScs], (uint32_t)(c / kScs) & 1u, abort_flag) ||
+          !mbar_wait_warp(&bar.k_full[c % kKs], (uint32_t)(c / kKs) & 1u, abort_flag)) return false;
+      const float f = sc[kScalP + (row >> 1)];
+      uint8_t* kr = smem + kOffK + c % kKs * kRowBytes + (row & 1) * 8192;
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        uint4* at = reinterpret_cast<uint4*>(kr + box_off(row >> 1, ch));
+        const uint4 u = *at;
+        const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+        uint32_t y[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = unpack2<kBf16>(x[e]);
+          y[e] = pack2<kBf16>(v.x * f, v.y * f);
+        }
+        *at = make_uint4(y[0], y[1], y[2], y[3]);
       }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(&bar.rows_ready); mbar_arrive(&bar.sc_empty[c % kScs]); }
+      return true;
+    };
+    bool ok = kBf16 || n_chunks == 0 || prepare(0);
+    for (int i = 0; i < n_chunks && ok; ++i) {
       if (!mbar_wait_warp(&bar.w_done, (uint32_t)i & 1u, abort_flag)) break;       // the chain's product with the one before is done, too
       tc_fence_after();
       uint32_t w[32];
@@ -413,29 +436,10 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       uint8_t* wt = smem + kOffW;
 #pragma unroll
       for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(wt + box_off(row, c)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-      if constexpr (!kBf16) {                            // K rows times (g_C / g) k_inv, in place: row row / 2, one box of it
-        const float f = sc[kScalK + (row >> 1)];
-        uint8_t* kr = smem + kOffK + i % kKs * kRowBytes + (row & 1) * 8192;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          uint4* at = reinterpret_cast<uint4*>(kr + box_off(row >> 1, c));
-          const uint4 u = *at;
-          const uint32_t x[4] = {u.x, u.y, u.z, u.w};
-          uint32_t y[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 v = unpack2<kBf16>(x[e]);
-            y[e] = pack2<kBf16>(v.x * f, v.y * f);
-          }
-          *at = make_uint4(y[0], y[1], y[2], y[3]);
-        }
-      }
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&bar.w_ready);
-        if constexpr (!kBf16) mbar_arrive(&bar.sc_empty[i % kScs]);
-      }
+      if (lane == 0) mbar_arrive(&bar.w_ready);
+      if (!kBf16 && i + 1 < n_chunks) ok = prepare(i + 1);
     }
   } else {
     set_registers<kOtherRegs, false>();

@@ -39,6 +39,22 @@ def test_chunk_edges(B, T, H, Hkv, dtype, spread):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T", [40, 64, 200])
+def test_key_rows_without_a_length(T, dtype):
+    """1 / |k| of rows of zeros and of rows of the type's smallest numbers is beyond fp16; the normalisation makes nothing of the
+    ones and unit vectors of the others."""
+    q, k, v, glog, beta, S0 = inputs(2, T, 2, 1, dtype, T)
+    k[:, 3::7] = 0
+    k[:, 5::11] = torch.randn(k[:, 5::11].shape, generator=torch.Generator().manual_seed(1)).sign().to(dtype) * 2.0 ** -24
+    k[:, 8::13] *= 1000
+    v[:, 1::9] *= 2000                                                    # U of the size of what fp16 holds
+    o_ref, S_ref = oracle.chunk_gated_delta_rule_oracle(q, k, v, glog, beta, initial_state=S0)
+    o, S = atma_b200.chunk_gated_delta_rule(q=q.cuda(), k=k.cuda(), v=v.cuda(), g=glog.cuda(), beta=beta.cuda(), scale=1.0,
+                                            initial_state=S0.cuda(), output_final_state=True, use_qk_l2norm_in_kernel=True)
+    assert max_rel(o, o_ref) < 2e-2 and max_rel(S, S_ref) < 2e-2          # as above
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,T,H,Hkv", [(2, 320, 4, 2), (1, 1000, 2, 1)])
 def test_two_calls_equal_one(B, T, H, Hkv, dtype):
     """scan_factors keeps the rows that scan_recur needs, so the inputs may change in between."""
