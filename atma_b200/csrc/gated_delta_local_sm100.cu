@@ -277,11 +277,12 @@ scan_local_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             }
           }
         const float inv = p.normalize ? 1.0f / fmaxf(sqrtf(sum[0] + sum[1]), 1e-12f) : 1.0f;
-        if (half) s_qinv[row] = inv * p.scale; else s_kinv[row] = inv;
+        // rows behind the sequence's end are another's, or nothing: whatever they hold, their factors are zero
+        if (half) s_qinv[row] = valid ? inv * p.scale : 0.f; else s_kinv[row] = valid ? inv : 0.f;
       }
       worker_sync();
       float k_left = s_kinv[row], k_pow2 = 1.f;          // what Tw and the scalars have of k_inv, and what the K rows get
-      if (!kBf16 && p.normalize) k_left = without_pow2(k_left, k_pow2);
+      if (!kBf16 && p.normalize && valid) k_left = without_pow2(k_left, k_pow2);
       if (half == 0) {
         if (quad & 1) run += s_wsum[quad - 1];           // second warp of the chunk
         s_lg[row] = run;
@@ -303,6 +304,7 @@ scan_local_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       tc_fence_after();
       {
         uint32_t rq[16];
+        const int own = valid, sees = valid ? pr : 0;    // columns s < sees, and s = pr if the row is the sequence's
         // rows 0-31 of a chunk see no column of its second half: that warp only writes zeros
         if (half == 1 && (quad & 1) == 0) {
 #pragma unroll
@@ -322,8 +324,8 @@ scan_local_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
               reg_fence(gk[j + e]); reg_fence(gq[j + e]);
               const int s = 32 * half + j + e;
               const float dec = __expf(lg_p - s_lg[64 * ci + s]) * s_kinv[64 * ci + s];
-              a2[e] = (s < pr) ? bt_p * dec * kinv_p * __uint_as_float(gk[j + e]) : 0.f;
-              r2[e] = (s <= pr) ? dec * qinv_p * __uint_as_float(gq[j + e]) : 0.f;
+              a2[e] = (s < sees) ? bt_p * dec * kinv_p * __uint_as_float(gk[j + e]) : 0.f;
+              r2[e] = (s < sees + own) ? dec * qinv_p * __uint_as_float(gq[j + e]) : 0.f;
             }
             *reinterpret_cast<float2*>(Af + row * kLd + 32 * half + j) = make_float2(a2[0], a2[1]);
             rq[j >> 1] = pack2<kBf16>(r2[0], r2[1]);

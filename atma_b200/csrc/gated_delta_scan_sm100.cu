@@ -18,7 +18,8 @@
 // Q, K, V and the record tiles are operands exactly as TMA delivers them; scalars per row are applied to fp32
 // accumulators.  fp16 has no room for an unbounded 1 / |k|, neither in Tw nor in U, so there the W warps bring the K rows
 // in shared memory to a length between 1 and 2 by a power of two, which loses nothing, a chunk ahead of the first product
-// that reads them, and k_inv stands for what is left, a factor between 1/2 and 1.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
+// that reads them, and k_inv stands for what is left, a factor between 1/2 and 1.  Behind the last rows of a sequence a
+// chunk holds another's, whose factors are zero; they may be infinite or no numbers, so the W warps clear them.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
 // accumulators have a channel on the 128 TMEM lanes, which spreads the thread phases over all four schedulers.
 //
 // What bounds it is the latency of the chain, of which the two thread phases are half: 3000 clocks a chunk, 650 for S and 750
@@ -63,7 +64,7 @@ constexpr uint32_t kColSb = 0, kColUb = 128, kColUs = 160, kColU = 192, kColO1 =
 
 struct Barriers {
   uint64_t vt_full[kVts], vt_empty[kVts], k_full[kKs], k_empty[kKs], qr_full[kQrs], qr_empty[kQrs], sc_full[kScs], sc_empty[kScs];
-  uint64_t rows_ready, w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
+  uint64_t k_ready, v_ready, w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
 };
 
 struct Params {
@@ -123,6 +124,9 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     tok_end = orow0 + min((int64_t)p.Tlen, (int64_t)c_end * kC);
   }
   const int n_chunks = max(c_end - c_begin, 0);
+  const int last_rows = (int)(tok_end - tok_base - (int64_t)(n_chunks - 1) * kC);    // of the last chunk
+  auto partial = [&](int c) { return c == n_chunks - 1 && last_rows < kC; };
+  auto prepared = [&](int c) { return !kBf16 || partial(c); };       // chunks whose K rows the W warps work on first
   const int64_t rec0 = ((int64_t)rb * p.H + h) * p.NC + c_begin;     // first record of this recurrence
   const bool want_o = p.o != nullptr && (packed || p.map.o_row[b] >= 0);   // a negative row: this recurrence only carries state
 
@@ -132,7 +136,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     for (int i = 0; i < kQrs; ++i) { mbar_init(&bar.qr_full[i], 1); mbar_init(&bar.qr_empty[i], 1); }
     for (int i = 0; i < kScs; ++i) { mbar_init(&bar.sc_full[i], 1); mbar_init(&bar.sc_empty[i], kStateWarps + (kBf16 ? 1 : 2) * kHelpWarps); }
     mbar_init(&bar.sb_ready, kStateWarps); mbar_init(&bar.us_ready, kStateWarps); mbar_init(&bar.ub_ready, kStateWarps);
-    mbar_init(&bar.rows_ready, kHelpWarps); mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
+    mbar_init(&bar.k_ready, kHelpWarps); mbar_init(&bar.v_ready, kHelpWarps); mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
     mbar_init(&bar.w_done, 1); mbar_init(&bar.u_full, 1); mbar_init(&bar.s_done, 1); mbar_init(&bar.o_done, 1);
     s_abort = 0;
     fence_barrier_init();
@@ -212,7 +216,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           if (n < n_chunks) {
             const uint32_t vt = base + n % kVts * kVtBytes, nkr = base + kOffK + n % kKs * kRowBytes;
             ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && mbar_wait(&bar.k_full[n % kKs], (uint32_t)(n / kKs) & 1u, abort_flag) &&
-                 (kBf16 || mbar_wait(&bar.rows_ready, (uint32_t)n & 1u, abort_flag));
+                 (!prepared(n) || mbar_wait(&bar.k_ready, kBf16 ? 0u : (uint32_t)n & 1u, abort_flag));
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
@@ -245,7 +249,8 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           const int n = i + 1;                           // U0^T of the next chunk, once U^T of this one has been read
           if (n < n_chunks) {
             const uint32_t vt = base + n % kVts * kVtBytes;
-            ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && (i < 0 || mbar_wait(&bar.ub_ready, (uint32_t)i & 1u, abort_flag));
+            ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && (i < 0 || mbar_wait(&bar.ub_ready, (uint32_t)i & 1u, abort_flag)) &&
+                 (!partial(n) || mbar_wait(&bar.v_ready, 0, abort_flag));
             if (!ok) break;
             tc_fence_after();
             if (!zero_u0) {
@@ -393,32 +398,52 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     // =============================== W warps ======================================================
     const int row = 32 * (warp & 3) + lane;              // TMEM lane: key channel
     const uint32_t lane_base = tbase + (uint32_t(32 * (warp & 3)) << 16);
-    // K rows of a chunk times their powers of two, in place: this thread's is row / 2, one box of it
+    // in place, this thread's row is row / 2, one box of it: K rows times their powers of two (fp16); zeros for what is not the sequence's
     auto prepare = [&](int c) {
-      const float* sc = reinterpret_cast<const float*>(smem + kOffSc + c % kScs * kScBytes);
-      if (!mbar_wait_warp(&bar.sc_full[c % kScs], (uint32_t)(c / kScs) & 1u, abort_flag) ||
-          !mbar_wait_warp(&bar.k_full[c % kKs], (uint32_t)(c / kKs) & 1u, abort_flag)) return false;
-      const float f = sc[kScalP + (row >> 1)];
-      uint8_t* kr = smem + kOffK + c % kKs * kRowBytes + (row & 1) * 8192;
+      const bool other = partial(c) && (row >> 1) >= last_rows;
+      const uint32_t box = (row & 1) * 8192;
+      uint8_t* kr = smem + kOffK + c % kKs * kRowBytes + box;
+      if (!mbar_wait_warp(&bar.k_full[c % kKs], (uint32_t)(c / kKs) & 1u, abort_flag)) return false;
+      float f = 1.f;
+      if constexpr (!kBf16) {
+        if (!mbar_wait_warp(&bar.sc_full[c % kScs], (uint32_t)(c / kScs) & 1u, abort_flag)) return false;
+        f = reinterpret_cast<const float*>(smem + kOffSc + c % kScs * kScBytes)[kScalP + (row >> 1)];
+      }
+      if (!kBf16 || other) {
 #pragma unroll
-      for (int ch = 0; ch < 8; ++ch) {
-        uint4* at = reinterpret_cast<uint4*>(kr + box_off(row >> 1, ch));
-        const uint4 u = *at;
-        const uint32_t x[4] = {u.x, u.y, u.z, u.w};
-        uint32_t y[4];
+        for (int ch = 0; ch < 8; ++ch) {
+          uint4* at = reinterpret_cast<uint4*>(kr + box_off(row >> 1, ch));
+          const uint4 u = other ? make_uint4(0u, 0u, 0u, 0u) : *at;
+          const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+          uint32_t y[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 v = unpack2<kBf16>(x[e]);
-          y[e] = pack2<kBf16>(v.x * f, v.y * f);
+          for (int e = 0; e < 4; ++e) {
+            const float2 v = unpack2<kBf16>(x[e]);
+            y[e] = pack2<kBf16>(v.x * f, v.y * f);
+          }
+          *at = make_uint4(y[0], y[1], y[2], y[3]);
         }
-        *at = make_uint4(y[0], y[1], y[2], y[3]);
       }
       fence_proxy_async();
       __syncwarp();
-      if (lane == 0) { mbar_arrive(&bar.rows_ready); mbar_arrive(&bar.sc_empty[c % kScs]); }
+      if (lane == 0) {
+        mbar_arrive(&bar.k_ready);
+        if constexpr (!kBf16) mbar_arrive(&bar.sc_empty[c % kScs]);
+      }
+      if (partial(c)) {
+        if (!mbar_wait_warp(&bar.vt_full[c % kVts], (uint32_t)(c / kVts) & 1u, abort_flag)) return false;
+        if (other) {
+#pragma unroll
+          for (int ch = 0; ch < 8; ++ch)
+            *reinterpret_cast<uint4*>(smem + c % kVts * kVtBytes + box + box_off(row >> 1, ch)) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.v_ready);
+      }
       return true;
     };
-    bool ok = kBf16 || n_chunks == 0 || prepare(0);
+    bool ok = n_chunks == 0 || !prepared(0) || prepare(0);
     for (int i = 0; i < n_chunks && ok; ++i) {
       if (!mbar_wait_warp(&bar.w_done, (uint32_t)i & 1u, abort_flag)) break;       // the chain's product with the one before is done, too
       tc_fence_after();
@@ -439,7 +464,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.w_ready);
-      if (!kBf16 && i + 1 < n_chunks) ok = prepare(i + 1);
+      if (i + 1 < n_chunks && prepared(i + 1)) ok = prepare(i + 1);
     }
   } else {
     set_registers<kOtherRegs, false>();

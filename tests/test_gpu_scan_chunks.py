@@ -55,6 +55,42 @@ def test_key_rows_without_a_length(T, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("lengths", [(65, 70), (1, 1, 200), (127, 5), (64, 64), (17, 300, 30), (193, 2, 61)])
+def test_a_sequence_keeps_its_bits_whatever_its_neighbours_hold(lengths, bad, dtype):
+    """A chunk holds rows of the next sequence behind a sequence's last ones.  Every other sequence's rows go bad, the others' outputs
+    and states stay as they were; packed, and as rows of a batch."""
+    n, total, H, Hkv = len(lengths), sum(lengths), 3, 1
+    at = [sum(lengths[:i]) for i in range(n + 1)]
+
+    def packed(x, S0):
+        table = S0.clone()
+        o = atma_b200.packed_gated_delta_prefill(*(t[0].cuda() for t in x), torch.tensor(at), table, torch.arange(n).cuda())
+        return [(o[at[i]:at[i + 1]], table[i]) for i in range(n)]
+
+    def dense(x, S0):
+        o, S = atma_b200.chunk_gated_delta_rule(**dict(zip(("q", "k", "v", "g", "beta"), (t.cuda() for t in x))), scale=1.0, initial_state=S0,
+                                                output_final_state=True, use_qk_l2norm_in_kernel=True)
+        return list(zip(o, S))
+
+    x = inputs(1, total, H, Hkv, dtype, total)[:5]
+    S0 = torch.randn(n, H, 128, 128, generator=torch.Generator().manual_seed(3)).cuda() * 0.3
+    cases = [(packed, x, lambda t, i: t[:, at[i]:at[i + 1]], S0)]
+    cases += [(dense, inputs(3, T, H, Hkv, dtype, T)[:5], lambda t, i: t[i:i + 1], S0[:1].expand(3, -1, -1, -1)) for T in set(lengths)]
+    for call, x, part, S in cases:
+        want = call(x, S)
+        for first in (0, 1):
+            y = [t.clone() for t in x]
+            for i in range(first, len(want), 2):
+                for t in y[:3]:
+                    part(t, i)[:, ::2] = bad
+            for i, (g, w) in enumerate(zip(call(y, S), want)):
+                if i % 2 != first:
+                    assert torch.equal(g[0], w[0]) and torch.equal(g[1], w[1])
+    assert atma_b200.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("B,T,H,Hkv", [(2, 320, 4, 2), (1, 1000, 2, 1)])
 def test_two_calls_equal_one(B, T, H, Hkv, dtype):
     """scan_factors keeps the rows that scan_recur needs, so the inputs may change in between."""
