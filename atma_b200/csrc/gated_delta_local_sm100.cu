@@ -64,10 +64,12 @@ struct Params {
   VarLen var;
 };
 
-// x = pow2 * the result, which is in [1/2, 1); x > 0 and normal
-__device__ __forceinline__ float without_pow2(float x, float& pow2) {
+// 1 / |k| of fp16 rows (2^-20 to 2^24, or there is no row) as a factor from 1/2 to 1 and the product of two powers of two
+__device__ __forceinline__ float without_pow2(float x, __half2& pow2) {
   const uint32_t b = __float_as_uint(x);
-  pow2 = __uint_as_float((b & 0x7f800000u) + 0x00800000u);
+  const int e = (int)(b >> 23) - 126;
+  if (e < -24 || e > 26) { pow2 = __float2half2_rn(0.f); return 0.f; }
+  pow2 = __floats2half2_rn(__int_as_float((127 + (e >> 1)) << 23), __int_as_float((127 + e - (e >> 1)) << 23));
   return __uint_as_float((b & 0x007fffffu) | 0x3f000000u);
 }
 
@@ -281,8 +283,14 @@ scan_local_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         if (half) s_qinv[row] = valid ? inv * p.scale : 0.f; else s_kinv[row] = valid ? inv : 0.f;
       }
       worker_sync();
-      float k_left = s_kinv[row], k_pow2 = 1.f;          // what Tw and the scalars have of k_inv, and what the K rows get
-      if (!kBf16 && p.normalize && valid) k_left = without_pow2(k_left, k_pow2);
+      float k_left = s_kinv[row];                        // what Tw and the scalars have of k_inv, and what the K rows get
+      __half2 k_pow2 = __float2half2_rn(1.f);
+      bool far = false;
+      if constexpr (!kBf16) {
+        auto beyond = [](float x) { return x > 1.0078125f || (x > 0.f && x < 0.015625f); };
+        far = __any_sync(0xffffffffu, p.normalize && (beyond(k_left) || beyond(s_kinv[row ^ 32])));       // of the chunk
+        if (far) k_left = without_pow2(k_left, k_pow2);
+      }
       if (half == 0) {
         if (quad & 1) run += s_wsum[quad - 1];           // second warp of the chunk
         s_lg[row] = run;
@@ -294,8 +302,8 @@ scan_local_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         float* sc = p.scal + rec * kScal;
         sc[kScalQ + pr] = valid ? __expf(lg_p) * qinv_p : 0.f;
         sc[kScalK + pr] = valid ? __expf(lg_C - lg_p) * k_left : 0.f;
-        if constexpr (!kBf16) sc[kScalP + pr] = k_pow2;
-        if (pr == kC - 1) sc[kScalG] = __expf(run);
+        if (far) reinterpret_cast<__half2*>(sc)[kScalP + pr] = k_pow2;
+        if (pr == kC - 1) { sc[kScalG] = __expf(run); sc[kScalFar] = far; }
       }
 
       // ---- A (fp32, shared memory) and Rq (record) from the Gram matrices -------------------------------

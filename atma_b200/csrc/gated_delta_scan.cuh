@@ -14,12 +14,14 @@ namespace scan {
 constexpr int kC = 64, kD = 128;
 // One record per (sequence, head, chunk): three 16-bit row-major [64 p][64 s] tiles
 //   Tw = -T diag(beta g k_inv) | Tu = T diag(beta) | Rq = tril((g_p / g_s) q^_p.k^_s)          T = (I + A)^-1
-// and, in a second array, one float per row for each of g q_inv scale and (g_C / g) k_inv, then g_C.  In fp16 k_inv is split: a
-// power of two per row (kScalP), which the recurrence multiplies the K rows with, and a factor from 1/2 to 1, which takes its place here.  The rows of q, k and v
+// and, in a second array, one float per row for each of g q_inv scale and (g_C / g) k_inv, then g_C.  Behind it, in
+// fp16, whether the chunk has a row of a length outside of [1, 64] (kScalFar): k_inv is then split in all of its rows, a power of two per row,
+// which the recurrence multiplies the K rows with, and a factor from 1/2 to 1, which takes its place here.  The power is there as
+// two fp16 ones (kScalP), whose product can be beyond what fp16 holds.  The rows of q, k and v
 // themselves are read again by the recurrence, which makes -W = Tw K and U0 = Tu V beside its chain: a record with
 // W, U0, Qg and Kt in it is 72 KB of writes and reads for what takes 24, and rounds each of them to 16 bits.
 constexpr int kTile64 = kC * kC * 2, kRecTw = 0, kRecTu = kTile64, kRecRq = 2 * kTile64, kRecBytes = 3 * kTile64;
-constexpr int kScalQ = 0, kScalK = kC, kScalG = 2 * kC, kScalP = 3 * kC, kScal = 256;                    // floats
+constexpr int kScalQ = 0, kScalK = kC, kScalG = 2 * kC, kScalFar = 2 * kC + 1, kScalP = 3 * kC, kScal = 256;                    // floats
 // Scratch per chunk and head: record, scalars, and the rows of q, k, v that scan_factors keeps for scan_recur (whose
 // callers hand it nothing but the scratch).  Packed batches count the same.
 constexpr int kScratchPerChunk = kRecBytes + kScal * 4 + 3 * kC * kD * 2;

@@ -16,10 +16,11 @@
 //     MMA   O1^T = S^T Q^T,  O2^T = U^T Rq^T;  O warps: o = g q_inv O1 + O2
 //
 // Q, K, V and the record tiles are operands exactly as TMA delivers them; scalars per row are applied to fp32
-// accumulators.  fp16 has no room for an unbounded 1 / |k|, neither in Tw nor in U, so there the W warps bring the K rows
-// in shared memory to a length between 1 and 2 by a power of two, which loses nothing, a chunk ahead of the first product
-// that reads them, and k_inv stands for what is left, a factor between 1/2 and 1.  Behind the last rows of a sequence a
-// chunk holds another's, whose factors are zero; they may be infinite or no numbers, so the W warps clear them.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
+// accumulators.  fp16 has no room for an unbounded 1 / |k|, neither in Tw nor in U, so in chunks with very short or long
+// rows a warp brings the K rows in shared memory to a length between 1 and 2 by a power of two, which loses nothing, ahead of
+// the first product that reads them, and k_inv stands for what is left, a factor between 1/2 and 1.  The rows arrive shortly before
+// that product, so this costs such a chunk 2000 clocks.  Behind the last rows of a sequence a
+// chunk holds another's, whose factors are zero; they may be infinite or no numbers, so the same warp clears them.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
 // accumulators have a channel on the 128 TMEM lanes, which spreads the thread phases over all four schedulers.
 //
 // What bounds it is the latency of the chain, of which the two thread phases are half: 3000 clocks a chunk, 650 for S and 750
@@ -29,7 +30,8 @@
 //
 //   warp 0       TMA producer: V, Tw, Tu and K three chunks ahead, Q and Rq two
 //   warp 1       issues the chain's products and -W^T; owns the TMEM allocation
-//   warp 2       issues the other products (warp 3 fills the warpgroup)
+//   warp 2       issues the other products
+//   warp 3       K and V rows in place, where they need it
 //   warps 4-11   state warps; warp w works on TMEM lanes 32 (w % 4) .. +31 and on column half
 //                (w - 4) / 4 of whatever it reads (k for S^T, p for U^T); with sixteen of them a phase
 //                takes longer, their waits and arrivals cost more than the shorter rows save
@@ -60,11 +62,11 @@ constexpr int kRowBytes = kC * kD * 2;            // 64 rows of 128 channels: tw
 constexpr int kVts = 3, kVtBytes = kRowBytes + 2 * kTile64, kKs = 3, kQrs = 2, kQrBytes = kRowBytes + kTile64, kScs = 4, kScBytes = kScal * 4;
 constexpr int kOffK = kVts * kVtBytes, kOffQr = kOffK + kKs * kRowBytes, kOffW = kOffQr + kQrs * kQrBytes, kOffSc = kOffW + kD * 128,
               kSmemBytes = kOffSc + kScs * kScBytes + 1024;
-constexpr uint32_t kColSb = 0, kColUb = 128, kColUs = 160, kColU = 192, kColO1 = 256, kColO2 = 320, kColS = 384, kColW = kColS;
+constexpr uint32_t kColSb = 0, kColUb = 128, kColUs = 160, kColU = 192, kColO1 = 256, kColO2 = 320, kColS = 384;
 
 struct Barriers {
   uint64_t vt_full[kVts], vt_empty[kVts], k_full[kKs], k_empty[kKs], qr_full[kQrs], qr_empty[kQrs], sc_full[kScs], sc_empty[kScs];
-  uint64_t k_ready, v_ready, w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
+  uint64_t last_sent, k_ready[kKs], v_ready, w_done, w_read, w_ready, u0_done, sb_ready, u_full, us_ready, ub_ready, s_done, o_done, o_free;
 };
 
 struct Params {
@@ -125,18 +127,19 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   }
   const int n_chunks = max(c_end - c_begin, 0);
   const int last_rows = (int)(tok_end - tok_base - (int64_t)(n_chunks - 1) * kC);    // of the last chunk
-  auto partial = [&](int c) { return c == n_chunks - 1 && last_rows < kC; };
-  auto prepared = [&](int c) { return !kBf16 || partial(c); };       // chunks whose K rows the W warps work on first
-  const int64_t rec0 = ((int64_t)rb * p.H + h) * p.NC + c_begin;     // first record of this recurrence
   const bool want_o = p.o != nullptr && (packed || p.map.o_row[b] >= 0);   // a negative row: this recurrence only carries state
+  const uint32_t col_w = want_o ? kColS : kColO1;                    // see TMEM above
+  auto partial = [&](int c) { return c == n_chunks - 1 && last_rows < kC; };
+  auto prepared = [&](int c) { return !kBf16 || partial(c); };       // chunks whose K rows warp 3 works on first
+  const int64_t rec0 = ((int64_t)rb * p.H + h) * p.NC + c_begin;     // first record of this recurrence
 
   if (tid == 0) {
     for (int i = 0; i < kVts; ++i) { mbar_init(&bar.vt_full[i], 1); mbar_init(&bar.vt_empty[i], 2); }
-    for (int i = 0; i < kKs; ++i) { mbar_init(&bar.k_full[i], 1); mbar_init(&bar.k_empty[i], 1); }
+    for (int i = 0; i < kKs; ++i) { mbar_init(&bar.k_full[i], 1); mbar_init(&bar.k_empty[i], 1); mbar_init(&bar.k_ready[i], 1); }
     for (int i = 0; i < kQrs; ++i) { mbar_init(&bar.qr_full[i], 1); mbar_init(&bar.qr_empty[i], 1); }
-    for (int i = 0; i < kScs; ++i) { mbar_init(&bar.sc_full[i], 1); mbar_init(&bar.sc_empty[i], kStateWarps + (kBf16 ? 1 : 2) * kHelpWarps); }
+    for (int i = 0; i < kScs; ++i) { mbar_init(&bar.sc_full[i], 1); mbar_init(&bar.sc_empty[i], kStateWarps + kHelpWarps + (kBf16 ? 0 : 1)); }
     mbar_init(&bar.sb_ready, kStateWarps); mbar_init(&bar.us_ready, kStateWarps); mbar_init(&bar.ub_ready, kStateWarps);
-    mbar_init(&bar.k_ready, kHelpWarps); mbar_init(&bar.v_ready, kHelpWarps); mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
+    mbar_init(&bar.last_sent, 1); mbar_init(&bar.v_ready, 1); mbar_init(&bar.w_read, kHelpWarps); mbar_init(&bar.w_ready, kHelpWarps); mbar_init(&bar.u0_done, 1); mbar_init(&bar.o_free, kHelpWarps);
     mbar_init(&bar.w_done, 1); mbar_init(&bar.u_full, 1); mbar_init(&bar.s_done, 1); mbar_init(&bar.o_done, 1);
     s_abort = 0;
     fence_barrier_init();
@@ -176,6 +179,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             if (!mbar_wait(&bar.sc_empty[i % kScs], ((uint32_t)(i / kScs) & 1u) ^ 1u, abort_flag)) break;
             mbar_arrive_expect_tx(full, kScBytes);
             bulk_load(smem + kOffSc + i % kScs * kScBytes, p.scal + (rec0 + i) * kScal, kScBytes, full);
+            if (kBf16 && i == n_chunks - 1) mbar_arrive(&bar.last_sent);
           }
           const int c = i - 1;                           // what o needs comes a chunk behind
           if (want_o && c >= 0) {
@@ -216,17 +220,17 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
           if (n < n_chunks) {
             const uint32_t vt = base + n % kVts * kVtBytes, nkr = base + kOffK + n % kKs * kRowBytes;
             ok = mbar_wait(&bar.vt_full[n % kVts], (uint32_t)(n / kVts) & 1u, abort_flag) && mbar_wait(&bar.k_full[n % kKs], (uint32_t)(n / kKs) & 1u, abort_flag) &&
-                 (!prepared(n) || mbar_wait(&bar.k_ready, kBf16 ? 0u : (uint32_t)n & 1u, abort_flag));
+                 (!prepared(n) || mbar_wait(&bar.k_ready[n % kKs], kBf16 ? 0u : (uint32_t)(n / kKs) & 1u, abort_flag));
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-              mma_ss(tbase + kColW, desc_mn(nkr) + uint64_t((kk * 2048) >> 4), desc_k(vt + kRowBytes) + uint64_t((kk * 32) >> 4), idesc_kt, kk > 0);
+              mma_ss(tbase + col_w, desc_mn(nkr) + uint64_t((kk * 2048) >> 4), desc_k(vt + kRowBytes) + uint64_t((kk * 32) >> 4), idesc_kt, kk > 0);
             tc_commit(&bar.w_done);
             tc_commit(&bar.vt_empty[n % kVts]);
           }
           if (i < 0) continue;
-          ok = mbar_wait(&bar.us_ready, pi, abort_flag) && (n == n_chunks || mbar_wait(&bar.w_read, pi ^ 1u, abort_flag));
+          ok = mbar_wait(&bar.us_ready, pi, abort_flag) && (!want_o || n == n_chunks || mbar_wait(&bar.w_read, pi ^ 1u, abort_flag));
           if (!ok) break;
           tc_fence_after();
           const uint64_t kr = desc_mn(base + kOffK + i % kKs * kRowBytes);
@@ -276,6 +280,54 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             tc_commit(&bar.o_done);
             tc_commit(&bar.qr_empty[i % kQrs]);
           }
+        }
+      }
+    } else {
+      // =============================== rows in place ==============================================
+      // zeros for what is not the sequence's; in fp16 K rows times their powers of two, if a chunk has any: eight lanes a row
+      for (int c = kBf16 ? max(n_chunks - 1, 0) : 0; c < n_chunks; ++c) {
+        if (!prepared(c)) break;
+        // K and V have been asked for before either of these, so their barriers are in this chunk's phase
+        if (!(kBf16 ? mbar_wait_warp(&bar.last_sent, 0, abort_flag) : mbar_wait_warp(&bar.sc_full[c % kScs], (uint32_t)(c / kScs) & 1u, abort_flag))) break;
+        const float* sc = reinterpret_cast<const float*>(smem + kOffSc + c % kScs * kScBytes);
+        const bool scaled = !kBf16 && sc[kScalFar] != 0.f;
+        const int rows = partial(c) ? last_rows : kC;
+        if (scaled || rows < kC) {
+          if (!mbar_wait_warp(&bar.k_full[c % kKs], (uint32_t)(c / kKs) & 1u, abort_flag)) break;
+          uint8_t* kr = smem + kOffK + c % kKs * kRowBytes;
+#pragma unroll 8
+          for (int i = 0; i < 32; ++i) {                 // both boxes of a row one after the other
+            const int r = 4 * (i >> 1) + (lane >> 3);
+            uint4* at = reinterpret_cast<uint4*>(kr + (i & 1) * 8192 + box_off(r, lane & 7));
+            if (r >= rows) {
+              *at = make_uint4(0u, 0u, 0u, 0u);
+            } else if (scaled) {
+              uint4 u = *at;
+              const __half2 f = reinterpret_cast<const __half2*>(sc)[kScalP + r], f1 = __low2half2(f), f2 = __high2half2(f);
+              __half2* v = reinterpret_cast<__half2*>(&u);
+#pragma unroll
+              for (int e = 0; e < 4; ++e) v[e] = __hmul2(__hmul2(v[e], f1), f2);
+              *at = u;
+            }
+          }
+          fence_proxy_async();
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&bar.k_ready[c % kKs]);
+          if constexpr (!kBf16) mbar_arrive(&bar.sc_empty[c % kScs]);
+        }
+        if (rows < kC) {
+          if (!mbar_wait_warp(&bar.vt_full[c % kVts], (uint32_t)(c / kVts) & 1u, abort_flag)) break;
+          uint8_t* vr = smem + c % kVts * kVtBytes;
+#pragma unroll 4
+          for (int i = 0; i < 32; ++i) {
+            const int r = 4 * (i >> 1) + (lane >> 3);
+            if (r >= rows) *reinterpret_cast<uint4*>(vr + (i & 1) * 8192 + box_off(r, lane & 7)) = make_uint4(0u, 0u, 0u, 0u);
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar.v_ready);
         }
       }
     }
@@ -398,60 +450,14 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     // =============================== W warps ======================================================
     const int row = 32 * (warp & 3) + lane;              // TMEM lane: key channel
     const uint32_t lane_base = tbase + (uint32_t(32 * (warp & 3)) << 16);
-    // in place, this thread's row is row / 2, one box of it: K rows times their powers of two (fp16); zeros for what is not the sequence's
-    auto prepare = [&](int c) {
-      const bool other = partial(c) && (row >> 1) >= last_rows;
-      const uint32_t box = (row & 1) * 8192;
-      uint8_t* kr = smem + kOffK + c % kKs * kRowBytes + box;
-      if (!mbar_wait_warp(&bar.k_full[c % kKs], (uint32_t)(c / kKs) & 1u, abort_flag)) return false;
-      float f = 1.f;
-      if constexpr (!kBf16) {
-        if (!mbar_wait_warp(&bar.sc_full[c % kScs], (uint32_t)(c / kScs) & 1u, abort_flag)) return false;
-        f = reinterpret_cast<const float*>(smem + kOffSc + c % kScs * kScBytes)[kScalP + (row >> 1)];
-      }
-      if (!kBf16 || other) {
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {
-          uint4* at = reinterpret_cast<uint4*>(kr + box_off(row >> 1, ch));
-          const uint4 u = other ? make_uint4(0u, 0u, 0u, 0u) : *at;
-          const uint32_t x[4] = {u.x, u.y, u.z, u.w};
-          uint32_t y[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 v = unpack2<kBf16>(x[e]);
-            y[e] = pack2<kBf16>(v.x * f, v.y * f);
-          }
-          *at = make_uint4(y[0], y[1], y[2], y[3]);
-        }
-      }
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&bar.k_ready);
-        if constexpr (!kBf16) mbar_arrive(&bar.sc_empty[c % kScs]);
-      }
-      if (partial(c)) {
-        if (!mbar_wait_warp(&bar.vt_full[c % kVts], (uint32_t)(c / kVts) & 1u, abort_flag)) return false;
-        if (other) {
-#pragma unroll
-          for (int ch = 0; ch < 8; ++ch)
-            *reinterpret_cast<uint4*>(smem + c % kVts * kVtBytes + box + box_off(row >> 1, ch)) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.v_ready);
-      }
-      return true;
-    };
-    bool ok = n_chunks == 0 || !prepared(0) || prepare(0);
-    for (int i = 0; i < n_chunks && ok; ++i) {
+    for (int i = 0; i < n_chunks; ++i) {
       if (!mbar_wait_warp(&bar.w_done, (uint32_t)i & 1u, abort_flag)) break;       // the chain's product with the one before is done, too
       tc_fence_after();
       uint32_t w[32];
 #pragma unroll
       for (int hh = 0; hh < 4; ++hh) {
         uint32_t r[16];
-        tmem_ld16(lane_base + kColW + 16 * hh, r);
+        tmem_ld16(lane_base + col_w + 16 * hh, r);
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[8 * hh + e] = pack2<kBf16>(__uint_as_float(r[2 * e]), __uint_as_float(r[2 * e + 1]));
       }
@@ -464,7 +470,6 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       fence_proxy_async();
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar.w_ready);
-      if (i + 1 < n_chunks && prepared(i + 1)) ok = prepare(i + 1);
     }
   } else {
     set_registers<kOtherRegs, false>();
