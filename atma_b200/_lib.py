@@ -130,6 +130,10 @@ _SIGNATURES = {
                                               c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),
     "atma_gated_delta_scan_recur": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                             POINTER(c_int), POINTER(c_int), c_void_p, c_void_p, c_void_p, c_void_p]),
+    "atma_gated_delta_scan_factors_alone": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),
+    "atma_gated_delta_scan_recur_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
+                                            POINTER(c_int), POINTER(c_int), c_void_p, c_void_p, c_void_p, c_void_p]),
     "atma_gated_delta_scan_varlen": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int,
                                              c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),

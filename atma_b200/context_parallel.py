@@ -77,7 +77,7 @@ class CudaBackend:
 
     def scan_factors(self, q, k, v, g, beta):
         from .gated_delta import scan_factors
-        return scan_factors(q, k, v, g, beta, scale=1.0, use_qk_l2norm_in_kernel=True)
+        return scan_factors(q, k, v, g, beta, scale=1.0, use_qk_l2norm_in_kernel=True, keep_rows=False)      # nobody else has the joined parts
 
     def scan_recur(self, factors, rec_of, initial_state, zero_value, want_output):
         from .gated_delta import scan_recur

@@ -15,9 +15,9 @@ int gated_delta_scan_mma(const void* q, const void* k, const void* v, int dtype,
 
 int gated_delta_scan_mma_factors(const void* q, const void* k, const void* v, int dtype, const float* g,
                                  const float* beta, void* scratch, int B, int T, int H, int Hkv, int normalize_qk,
-                                 float scale, cudaStream_t st);
-int gated_delta_scan_mma_recur(void* scratch, int dtype, int B, int T, int H, int n_rec, const int* rec_of,
-                               const int* zero_u0, const float* initial_state, void* o, float* final_state,
+                                 float scale, bool keep_rows, cudaStream_t st);
+int gated_delta_scan_mma_recur(const void* q, const void* k, const void* v, int Hkv, void* scratch, int dtype, int B, int T, int H,
+                               int n_rec, const int* rec_of, const int* zero_u0, const float* initial_state, void* o, float* final_state,
                                cudaStream_t st);
 int64_t gated_delta_scan_mma_varlen_scratch_bytes(int64_t total_tokens, int n_seqs, int H);
 int gated_delta_scan_mma_varlen(const void* q, const void* k, const void* v, int dtype, const float* g, const float* beta,
@@ -31,15 +31,26 @@ int gated_delta_scan_mma_varlen(const void* q, const void* k, const void* v, int
 
 using namespace atma;
 
-extern "C" int atma_gated_delta_scan_factors(const void* q, const void* k, const void* v, int dtype, const float* g,
-                                             const float* beta, void* scratch, int B, int T, int H, int Hkv, int dk,
-                                             int dv, int normalize_qk, float scale, void* stream) {
+static int scan_factors_impl(const void* q, const void* k, const void* v, int dtype, const float* g, const float* beta, void* scratch, int B,
+                             int T, int H, int Hkv, int dk, int dv, int normalize_qk, float scale, bool keep_rows, void* stream) {
   ATMA_REQUIRE(gated_delta_scan_mma_supported(dtype, dk, dv),
                "gated_delta_scan_factors: needs 16-bit inputs with dk = dv = 128 (got dtype %d, dk %d, dv %d)", dtype, dk, dv);
   ATMA_REQUIRE(B > 0 && T > 0 && H > 0 && Hkv > 0 && H % Hkv == 0, "gated_delta_scan_factors: bad shape");
   ATMA_REQUIRE(scratch != nullptr && (uintptr_t)scratch % 256 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 &&
                    (uintptr_t)v % 16 == 0, "gated_delta_scan_factors: scratch must be 256-byte and inputs 16-byte aligned");
-  return gated_delta_scan_mma_factors(q, k, v, dtype, g, beta, scratch, B, T, H, Hkv, normalize_qk, scale, (cudaStream_t)stream);
+  return gated_delta_scan_mma_factors(q, k, v, dtype, g, beta, scratch, B, T, H, Hkv, normalize_qk, scale, keep_rows, (cudaStream_t)stream);
+}
+
+extern "C" int atma_gated_delta_scan_factors(const void* q, const void* k, const void* v, int dtype, const float* g,
+                                             const float* beta, void* scratch, int B, int T, int H, int Hkv, int dk,
+                                             int dv, int normalize_qk, float scale, void* stream) {
+  return scan_factors_impl(q, k, v, dtype, g, beta, scratch, B, T, H, Hkv, dk, dv, normalize_qk, scale, true, stream);
+}
+
+extern "C" int atma_gated_delta_scan_factors_alone(const void* q, const void* k, const void* v, int dtype, const float* g,
+                                                   const float* beta, void* scratch, int B, int T, int H, int Hkv, int dk,
+                                                   int dv, int normalize_qk, float scale, void* stream) {
+  return scan_factors_impl(q, k, v, dtype, g, beta, scratch, B, T, H, Hkv, dk, dv, normalize_qk, scale, false, stream);
 }
 
 extern "C" int atma_gated_delta_scan_recur(void* scratch, int dtype, int B, int T, int H, int dk, int dv, int n_rec,
@@ -47,7 +58,18 @@ extern "C" int atma_gated_delta_scan_recur(void* scratch, int dtype, int B, int 
                                            float* final_state, void* stream) {
   ATMA_REQUIRE(gated_delta_scan_mma_supported(dtype, dk, dv), "gated_delta_scan_recur: needs 16-bit, dk = dv = 128");
   ATMA_REQUIRE(scratch != nullptr && B > 0 && T > 0 && H > 0, "gated_delta_scan_recur: bad arguments");
-  return gated_delta_scan_mma_recur(scratch, dtype, B, T, H, n_rec, rec_of, zero_u0, initial_state, o, final_state,
+  return gated_delta_scan_mma_recur(nullptr, nullptr, nullptr, H, scratch, dtype, B, T, H, n_rec, rec_of, zero_u0, initial_state, o, final_state,
+                                    (cudaStream_t)stream);
+}
+
+extern "C" int atma_gated_delta_scan_recur_rows(const void* q, const void* k, const void* v, int Hkv, void* scratch, int dtype, int B, int T,
+                                                int H, int dk, int dv, int n_rec, const int* rec_of, const int* zero_u0,
+                                                const float* initial_state, void* o, float* final_state, void* stream) {
+  ATMA_REQUIRE(gated_delta_scan_mma_supported(dtype, dk, dv), "gated_delta_scan_recur_rows: needs 16-bit, dk = dv = 128");
+  ATMA_REQUIRE(scratch != nullptr && B > 0 && T > 0 && H > 0 && Hkv > 0 && H % Hkv == 0, "gated_delta_scan_recur_rows: bad arguments");
+  ATMA_REQUIRE(q != nullptr && k != nullptr && v != nullptr && (uintptr_t)q % 16 == 0 && (uintptr_t)k % 16 == 0 && (uintptr_t)v % 16 == 0,
+               "gated_delta_scan_recur_rows: q, k and v must be 16-byte aligned");
+  return gated_delta_scan_mma_recur(q, k, v, Hkv, scratch, dtype, B, T, H, n_rec, rec_of, zero_u0, initial_state, o, final_state,
                                     (cudaStream_t)stream);
 }
 

@@ -316,15 +316,17 @@ def chunk_gated_delta_rule(q=None, k=None, v=None, g=None, beta=None, scale=None
 class ScanFactors:
     """Handle on the per-chunk factors of B sequences (see ``scan_factors``)."""
 
-    def __init__(self, scratch, B, T, H, dk, dv, dtype, device):
+    def __init__(self, scratch, B, T, H, dk, dv, dtype, device, rows=None):
         self.scratch, self.B, self.T, self.H, self.dk, self.dv, self.dtype, self.device = scratch, B, T, H, dk, dv, dtype, device
+        self.rows = rows                                   # q, k, v where the scratch has no copy of them
 
 
 @torch.no_grad()
-def scan_factors(q, k, v, g, beta, scale=1.0, use_qk_l2norm_in_kernel=True):
+def scan_factors(q, k, v, g, beta, scale=1.0, use_qk_l2norm_in_kernel=True, keep_rows=True):
     """First half of ``chunk_gated_delta_rule`` for a sequence that is split across GPUs: the
     state-independent per-chunk factors (16-bit inputs, dk = dv = 128).  The returned handle owns
-    its scratch memory; pass it to ``scan_recur`` any number of times."""
+    its scratch memory; pass it to ``scan_recur`` any number of times.  It has a copy of q, k and v, which the recurrences
+    read again; ``keep_rows=False`` leaves that out and the tensors themselves are read, so nobody may write to them meanwhile."""
     _lib.require_cuda(q, "scan_factors")
     lib = _lib.load()
     B, T, H, dk = q.shape
@@ -332,10 +334,10 @@ def scan_factors(q, k, v, g, beta, scale=1.0, use_qk_l2norm_in_kernel=True):
     q, k, v = q.contiguous(), k.to(q.dtype).contiguous(), v.to(q.dtype).contiguous()
     g, beta = g.float().contiguous(), beta.float().contiguous()
     scratch = torch.empty(int(lib.atma_gated_delta_scan_scratch_bytes(B, T, H, dk, dv)), device=q.device, dtype=torch.uint8)
-    _lib.check(lib.atma_gated_delta_scan_factors(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.dtype_code(q), _lib.ptr(g),
-                                                 _lib.ptr(beta), _lib.ptr(scratch), B, T, H, Hkv, dk, dv,
-                                                 1 if use_qk_l2norm_in_kernel else 0, float(scale), _lib.stream_ptr()))
-    return ScanFactors(scratch, B, T, H, dk, dv, q.dtype, q.device)
+    entry = lib.atma_gated_delta_scan_factors if keep_rows else lib.atma_gated_delta_scan_factors_alone
+    _lib.check(entry(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.dtype_code(q), _lib.ptr(g), _lib.ptr(beta), _lib.ptr(scratch), B, T, H, Hkv,
+                     dk, dv, 1 if use_qk_l2norm_in_kernel else 0, float(scale), _lib.stream_ptr()))
+    return ScanFactors(scratch, B, T, H, dk, dv, q.dtype, q.device, None if keep_rows else (q, k, v))
 
 
 @torch.no_grad()
@@ -354,7 +356,11 @@ def scan_recur(factors, rec_of, initial_state=None, zero_value=None, want_output
         initial_state = initial_state.float().contiguous()
     o = torch.empty((n, f.T, f.H, f.dv), device=f.device, dtype=f.dtype) if want_output else None
     final = torch.empty((n, f.H, f.dk, f.dv), device=f.device, dtype=torch.float32)
-    _lib.check(lib.atma_gated_delta_scan_recur(_lib.ptr(f.scratch), _lib.DTYPE_CODE[f.dtype], f.B, f.T, f.H, f.dk, f.dv, n,
-                                               rec_arr, zero_arr, _lib.ptr(initial_state), _lib.ptr(o), _lib.ptr(final),
-                                               _lib.stream_ptr()))
+    args = (_lib.ptr(f.scratch), _lib.DTYPE_CODE[f.dtype], f.B, f.T, f.H, f.dk, f.dv, n, rec_arr, zero_arr, _lib.ptr(initial_state),
+            _lib.ptr(o), _lib.ptr(final), _lib.stream_ptr())
+    if f.rows is None:
+        _lib.check(lib.atma_gated_delta_scan_recur(*args))
+    else:
+        q, k, v = f.rows
+        _lib.check(lib.atma_gated_delta_scan_recur_rows(_lib.ptr(q), _lib.ptr(k), _lib.ptr(v), k.shape[2], *args))
     return o, final

@@ -316,6 +316,16 @@ int atma_gated_delta_scan_recur(void* scratch, int dtype, int B, int T, int H, i
                                 int n_rec, const int* rec_of, const int* zero_u0,
                                 const float* initial_state, void* o, float* final_state,
                                 void* stream);
+/* The same for callers that still have q, k and v as they were when the recurrences run: _factors keeps a copy of them in
+ * the scratch, these two do not. */
+int atma_gated_delta_scan_factors_alone(const void* q, const void* k, const void* v, int dtype,
+                                        const float* g, const float* beta, void* scratch,
+                                        int B, int T, int H, int Hkv, int dk, int dv,
+                                        int normalize_qk, float scale, void* stream);
+int atma_gated_delta_scan_recur_rows(const void* q, const void* k, const void* v, int Hkv, void* scratch, int dtype,
+                                     int B, int T, int H, int dk, int dv, int n_rec, const int* rec_of,
+                                     const int* zero_u0, const float* initial_state, void* o, float* final_state,
+                                     void* stream);
 
 /* ----------------------------------------------------------------------------------
  * Packed ("varlen") gated-delta prefill: n_seqs sequences of different lengths back to back

@@ -105,6 +105,18 @@ def test_two_calls_equal_one(B, T, H, Hkv, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,T,H,Hkv", [(2, 320, 4, 2), (1, 1000, 2, 1)])
+def test_two_calls_over_the_rows_themselves(B, T, H, Hkv, dtype):
+    """Without a copy the recurrences give what they give with one: outputs, states, and states with v = 0."""
+    q, k, v, glog, beta, S0 = (x.cuda() for x in inputs(B, T, H, Hkv, dtype, 6))
+    fs = [scan_factors(q, k, v, glog, beta, keep_rows=keep) for keep in (True, False)]
+    for want_output in (True, False):
+        for zero in (None, [True] * B):
+            (o, S), (o2, S2) = (scan_recur(f, list(range(B)), S0, zero, want_output) for f in fs)
+            assert torch.equal(S, S2) and (not want_output or torch.equal(o, o2))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_outputs_two_bytes_off(dtype):
     """o may start at any 16-bit value: from an odd one its values are stored one by one."""
     B, T, H, Hkv = 2, 150, 3, 1
