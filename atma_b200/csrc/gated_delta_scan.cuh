@@ -23,7 +23,7 @@ constexpr int kC = 64, kD = 128;
 constexpr int kTile64 = kC * kC * 2, kRecTw = 0, kRecTu = kTile64, kRecRq = 2 * kTile64, kRecBytes = 3 * kTile64;
 constexpr int kScalQ = 0, kScalK = kC, kScalG = 2 * kC, kScalFar = 2 * kC + 1, kScalP = 3 * kC, kScal = 256;                    // floats
 // Scratch per chunk and head: record, scalars, and the rows of q, k, v that scan_factors keeps for scan_recur (whose
-// callers hand it nothing but the scratch).  Packed batches count the same.
+// callers hand it nothing but the scratch), and the whole scans where results take the inputs' place.
 constexpr int kScratchPerChunk = kRecBytes + kScal * 4 + 3 * kC * kD * 2;
 
 template <bool kBf16>

@@ -145,26 +145,39 @@ int64_t gated_delta_scan_mma_scratch_bytes(int B, int T, int H) {
 
 static float* scal_array(void* scratch, int64_t n_records) { return reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + n_records * kRecBytes); }
 
-// where scan_factors keeps the rows: all heads, q | k | v
-static Rows kept_rows(void* scratch, int dtype, int B, int T, int H) {
-  const int64_t n = (int64_t)B * H * ((T + kC - 1) / kC), each = (int64_t)B * T * H * kD * 2;
-  uint8_t* at = static_cast<uint8_t*>(scratch) + n * (kRecBytes + kScal * 4);
-  return Rows{at, at + each, at + 2 * each, dtype == ATMA_BF16, H, H, (int64_t)B * T};
+// where a copy of the rows is kept: behind the records, all heads, q | k | v
+static Rows kept_rows(void* scratch, bool is_bf16, int64_t n_records, int64_t tokens, int H) {
+  const int64_t each = tokens * H * kD * 2;
+  uint8_t* at = static_cast<uint8_t*>(scratch) + n_records * (kRecBytes + kScal * 4);
+  return Rows{at, at + each, at + 2 * each, is_bf16, H, H, tokens};
 }
 
-// Kernel A only: the chunk-local factors of B sequences into `scratch`, and the rows with them (8 heads and 2 of k and v, 2 x 16384
-// rows: 46 of 165 us).
+// makes it (8 heads and 2 of k and v, 2 x 16384 rows: 46 us)
+static Rows keep_rows(const Rows& r, void* scratch, int64_t n_records, cudaStream_t st) {
+  const Rows keep = kept_rows(scratch, r.is_bf16, n_records, r.tokens, r.H);
+  const int64_t n = r.tokens * r.H * 16;
+  const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
+  for (const auto& [to, from, heads] : {std::make_tuple(keep.q, r.q, r.H), std::make_tuple(keep.k, r.k, r.Hkv), std::make_tuple(keep.v, r.v, r.Hkv)})
+    keep_rows_kernel<<<grid, 256, 0, st>>>(static_cast<uint4*>(const_cast<void*>(to)), static_cast<const uint4*>(from), n, r.H, heads);
+  return keep;
+}
+
+// Results that take the place of inputs: a recurrence reads rows of q, k and v while others' results are written.
+static bool meets(const void* o, const Rows& r) {
+  const auto in = [&](const void* x, int heads) {
+    const auto a = reinterpret_cast<uintptr_t>(o), b = reinterpret_cast<uintptr_t>(x), row = (uintptr_t)r.tokens * kD * 2;
+    return a < b + row * heads && b < a + row * r.H;
+  };
+  return o != nullptr && (in(r.q, r.H) || in(r.k, r.Hkv) || in(r.v, r.Hkv));
+}
+
+// Kernel A only: the chunk-local factors of B sequences into `scratch`, and the rows with them.
 int gated_delta_scan_mma_factors(const void* q, const void* k, const void* v, int dtype, const float* g,
                                  const float* beta, void* scratch, int B, int T, int H, int Hkv, int normalize_qk,
-                                 float scale, bool keep_rows, cudaStream_t st) {
+                                 float scale, bool keep, cudaStream_t st) {
   const int NC = (T + kC - 1) / kC;
-  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T}, keep = kept_rows(scratch, dtype, B, T, H);
-  if (!keep_rows) return gated_delta_local_sm100(rows, g, beta, static_cast<uint8_t*>(scratch), scal_array(scratch, (int64_t)B * H * NC), B, T, NC,
-                                                 normalize_qk, scale, VarLen{}, st);
-  const int64_t n = (int64_t)B * T * H * 16;
-  const int grid = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
-  for (const auto& [to, from, heads] : {std::make_tuple(keep.q, q, H), std::make_tuple(keep.k, k, Hkv), std::make_tuple(keep.v, v, Hkv)})
-    keep_rows_kernel<<<grid, 256, 0, st>>>(static_cast<uint4*>(const_cast<void*>(to)), static_cast<const uint4*>(from), n, H, heads);
+  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T};
+  if (keep) keep_rows(rows, scratch, (int64_t)B * H * NC, st);
   return gated_delta_local_sm100(rows, g, beta, static_cast<uint8_t*>(scratch), scal_array(scratch, (int64_t)B * H * NC), B, T, NC,
                                  normalize_qk, scale, VarLen{}, st);
 }
@@ -191,7 +204,8 @@ static int recur_over(const Rows& rows, void* scratch, int B, int T, int n_rec, 
 int gated_delta_scan_mma_recur(const void* q, const void* k, const void* v, int Hkv, void* scratch, int dtype, int B, int T, int H,
                                int n_rec, const int* rec_of, const int* zero_u0, const float* initial_state, void* o, float* final_state,
                                cudaStream_t st) {
-  const Rows rows = q == nullptr ? kept_rows(scratch, dtype, B, T, H) : Rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T};
+  const int64_t n = (int64_t)B * H * ((T + kC - 1) / kC), tokens = (int64_t)B * T;
+  const Rows rows = q == nullptr ? kept_rows(scratch, dtype == ATMA_BF16, n, tokens, H) : Rows{q, k, v, dtype == ATMA_BF16, H, Hkv, tokens};
   return recur_over(rows, scratch, B, T, n_rec, rec_of, zero_u0, initial_state, o, final_state, st);
 }
 
@@ -214,7 +228,8 @@ int gated_delta_scan_mma_varlen(const void* q, const void* k, const void* v, int
   int32_t* cu_chunks = reinterpret_cast<int32_t*>(recs + record_bytes(1, NCu * kC, H));
   varlen_chunk_offsets_kernel<<<1, 32, 0, st>>>(cu_seqlens, cu_chunks, n_seqs);
   VarLen var{cu_seqlens, cu_chunks, n_seqs, slots, has_initial, state_table, slot_stride, snapshots, snap_offsets, snap_chunks};
-  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, total_tokens};
+  Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, total_tokens};
+  if (meets(o, rows)) rows = keep_rows(rows, scratch, (int64_t)H * NCu, st);
   int rc = gated_delta_local_sm100(rows, g, beta, recs, scal, 1, 0, NCu, normalize_qk, scale, var, st);
   if (rc != ATMA_OK) return rc;
   return gated_delta_recur_sm100(rows, recs, scal, (int64_t)H * NCu, initial_state, o, final_state, 0, NCu, n_seqs, RecMap{}, var, st);
@@ -231,7 +246,8 @@ int gated_delta_scan_mma(const void* q, const void* k, const void* v, int dtype,
                          const float* initial_state, void* o, float* final_state, void* scratch, int B, int T, int H,
                          int Hkv, int normalize_qk, float scale, int segments, cudaStream_t st) {
   const int NC = (T + kC - 1) / kC;
-  const Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T};
+  Rows rows{q, k, v, dtype == ATMA_BF16, H, Hkv, (int64_t)B * T};
+  if (meets(o, rows)) rows = keep_rows(rows, scratch, (int64_t)B * H * NC, st);
   const uint8_t* recs = static_cast<const uint8_t*>(scratch);
   float* scal = scal_array(scratch, (int64_t)B * H * NC);
   int rc = gated_delta_local_sm100(rows, g, beta, static_cast<uint8_t*>(scratch), scal, B, T, NC, normalize_qk, scale, VarLen{}, st);

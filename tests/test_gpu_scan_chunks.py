@@ -132,3 +132,35 @@ def test_outputs_two_bytes_off(dtype):
         assert (buf[:off] == 7).all() and (buf[off + B * T * H * 128:] == 7).all()
         out.append(buf[off:off + B * T * H * 128])
     assert torch.equal(*out)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("place", ["q", "k", "v", "behind k"])
+@pytest.mark.parametrize("T,segments", [(150, 1), (4096, 4)])
+def test_outputs_in_the_place_of_inputs(T, segments, place, dtype):
+    """o over q, k or v, or over the end of one and what follows: the rows are read before o is written, in both passes over segments
+    and in packed batches."""
+    B, H = 2, 2
+    x = [t.cuda() for t in inputs(B, T, H, H, dtype, 11)]
+    lib, n = _lib.load(), B * T * H * 128
+    scratch = torch.empty(max(lib.atma_gated_delta_scan_scratch_bytes(B, T, H, 128, 128),
+                              lib.atma_gated_delta_scan_varlen_scratch_bytes(B * T, 2, H, 128, 128)), dtype=torch.uint8, device="cuda")
+    cu = torch.tensor([0, T - 3, B * T], dtype=torch.int32, device="cuda")
+    for packed in (False, True):
+        out = []
+        for over in (False, True):
+            buf = torch.zeros(4 * n, dtype=dtype, device="cuda")
+            for i in range(3):
+                buf[i * n:(i + 1) * n] = x[i].flatten()
+            q, k, v = (buf.data_ptr() + 2 * i * n for i in range(3))
+            at = (3 * n if not over else n + n // 2 + 128 if place == "behind k" else "qkv".index(place) * n)
+            o = ctypes.c_void_p(buf.data_ptr() + 2 * at)
+            if packed:
+                _lib.check(lib.atma_gated_delta_scan_varlen(q, k, v, _lib.dtype_code(x[0]), _lib.ptr(x[3]), _lib.ptr(x[4]), _lib.ptr(cu), 2, B * T,
+                                                            _lib.ptr(x[5]), None, None, 0, None, None, o, _lib.ptr(scratch), H, H, 128, 128, 1, 1.0,
+                                                            _lib.stream_ptr()))
+            else:
+                _lib.check(lib.atma_gated_delta_scan_segmented(q, k, v, _lib.dtype_code(x[0]), _lib.ptr(x[3]), _lib.ptr(x[4]), _lib.ptr(x[5]), o, None,
+                                                               _lib.ptr(scratch), B, T, H, H, 128, 128, 1, 1.0, segments, _lib.stream_ptr()))
+            out.append(buf[at:at + n].clone())
+        assert torch.equal(*out)
