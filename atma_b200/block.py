@@ -92,6 +92,7 @@ def global_block_forward(x, sd, *, head_dim, num_kv_heads, window=None, mem_chun
     Hkv = num_kv_heads
     if B * T > 0 and _side_by_side(sd, D, H, Hkv, dk):
         rows = x.reshape(B * T, D)
+        eps = torch.finfo(torch.float32).eps if eps is None else eps          # as F.rms_norm's None, 16-bit inputs included
         _, h = add_rms_norm(rows, None, sd["norm1.weight"], eps)
         out, S = _mixed(x, h, sd, H, Hkv, dk, window, mem_gamma_bias, mem_beta_bias, initial_state)
         rows, h = add_rms_norm(rows, out, sd["norm2.weight"], eps)

@@ -50,3 +50,24 @@ def test_forms_that_go_one_by_one():
     del w["attn.mem.proj.weight"]
     x = rand((1, 20, 64), 9).cuda()
     assert not block._side_by_side(w, 64, 4, 1, 32) and block.global_block_forward(x, w, head_dim=32, num_kv_heads=1).shape == x.shape
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.bfloat16, 3e-2)])      # as above
+@pytest.mark.parametrize("what", ["eps"])
+def test_arguments_of_every_kind(monkeypatch, what, dtype, tol):
+    """No epsilon, biases of the memory's gates as tensors, convolutions of different lengths: as one operation at a time takes them."""
+    B, T, D, H, G, dk = 2, 70, 256, 4, 2, 64
+    w, x = weights(D, H, G, dk, True, dtype), rand((B, T, D), 9, dtype).cuda() * (1e-3 if what == "eps" else 1)
+    kw = dict(head_dim=dk, num_kv_heads=G, return_state=True)
+    if what == "eps":
+        kw["eps"] = None
+    elif what == "taps":
+        w["attn.canon_k.weight"] = w["attn.canon_k.weight"][..., 1:].contiguous()
+    else:
+        shape = {"head biases": (H,), "row biases": (B, T, H), "biases of one value": (1,)}[what]
+        kw.update(mem_gamma_bias=rand(shape, 3).cuda() + 3, mem_beta_bias=rand(shape, 4).cuda())
+    assert block._side_by_side(w, D, H, G, dk) == (what != "taps")
+    got, S = block.global_block_forward(x, w, **kw)
+    monkeypatch.setattr(block, "_side_by_side", lambda *a: False)
+    want, Sw = block.global_block_forward(x, w, **kw)
+    assert max_rel(got, want) < tol and max_rel(S, Sw) < tol
