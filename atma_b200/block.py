@@ -70,8 +70,9 @@ def _mixed(x, h, sd, H, Hkv, dk, window, mem_gamma_bias, mem_beta_bias, initial_
                                  null_base=sd["attn.null_base"], null_slope_raw=sd["attn.null_slope_raw"],
                                  len_gain_raw=sd["attn.len_gain_raw"], mag_beta_raw=sd["attn.mag_beta_raw"], window=window)
     c = c[0].transpose(0, 1) if B == 1 else c.transpose(1, 2).reshape(n, H, dk)
-    g, beta = (t.float() + bias if bias else t.float() for t, bias in ((g, mem_gamma_bias), (beta, mem_beta_bias)))
-    r, S = chunk_gated_delta_rule(q=q, k=k, v=v, g=F.logsigmoid(g).view(B, T, H), beta=torch.sigmoid(beta).view(B, T, H), scale=1.0,
+    logits = [t.float().view(B, T, H) for t in (g, beta)]
+    g, beta = (t if isinstance(bias, (int, float)) and bias == 0 else t + bias for t, bias in zip(logits, (mem_gamma_bias, mem_beta_bias)))
+    r, S = chunk_gated_delta_rule(q=q, k=k, v=v, g=F.logsigmoid(g), beta=torch.sigmoid(beta), scale=1.0,
                                   initial_state=initial_state, output_final_state=True, use_qk_l2norm_in_kernel=True)
     act = torch.cat([sigmoid_gate_mul(c, q_gate[..., dk:]).view(n, Hd), rms_sigmoid_gate(r.view(n, H, dk), mem_gate),
                      mag.transpose(1, 2).reshape(n, H)], 1)
