@@ -50,7 +50,8 @@ def _side_by_side(sd, D, H, Hkv, dk):
     """Whether the projections can go as one product and their parts be read in place."""
     if any(n + ".weight" not in sd for n in IN + OUT) or len({n + ".bias" in sd for n in IN}) != 1:
         return False
-    return dk % 8 == 0 and dk <= 128 and D <= 4096 and (2 * H) % 8 == 0 and 2 <= sd["attn.canon_q.weight"].shape[-1] <= 4
+    taps = {sd[f"attn.canon_{i}.weight"].shape[-1] for i in "qkv"}
+    return dk % 8 == 0 and dk <= 128 and D <= 4096 and (2 * H) % 8 == 0 and len(taps) == 1 and 2 <= min(taps) <= 4
 
 
 def _mixed(x, h, sd, H, Hkv, dk, window, mem_gamma_bias, mem_beta_bias, initial_state):

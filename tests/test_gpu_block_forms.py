@@ -53,7 +53,7 @@ def test_forms_that_go_one_by_one():
 
 
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.bfloat16, 3e-2)])      # as above
-@pytest.mark.parametrize("what", ["eps", "head biases", "row biases", "biases of one value"])
+@pytest.mark.parametrize("what", ["eps", "head biases", "row biases", "biases of one value", "taps"])
 def test_arguments_of_every_kind(monkeypatch, what, dtype, tol):
     """No epsilon, biases of the memory's gates as tensors, convolutions of different lengths: as one operation at a time takes them."""
     B, T, D, H, G, dk = 2, 70, 256, 4, 2, 64
