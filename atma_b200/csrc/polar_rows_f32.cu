@@ -303,8 +303,9 @@ polar_tf32_kernel(const __grid_constant__ atma_polar_prefill_args a) {
 
 // Head size 128, no statistics carried in or out (a marked block is done again from the inputs alone), and enough rows: 2048
 // rows, 8 heads 431 us on the 64 x 64 kernel, 130 here; 512 rows 100 and 60; 256 rows 57 and 49, where the calls' own launches are most of it.
+// Results that take the place of q: the mark would be in the rows that are read again.
 bool polar_tf32_supported(const atma_polar_prefill_args& a) {
-  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq >= 256;
+  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq >= 256 && a.c != a.q;
 }
 
 template <int DK>

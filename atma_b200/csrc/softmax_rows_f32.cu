@@ -264,9 +264,10 @@ softmax_tf32_kernel(const __grid_constant__ atma_softmax_args a) {
 }
 
 // 128 channels in one map or two, 128 of v, and enough rows.  Two layers of two maps: 1500 rows, 8 heads 527 us on the 64 x 64
-// kernel, 145 here; 400 rows 143 and 57; 256 rows 91 and 49.
+// kernel, 145 here; 400 rows 143 and 57; 256 rows 91 and 49.  Results that take the place of q or the gate: the mark would be in
+// the rows that are read again.
 bool softmax_tf32_supported(const atma_softmax_args& a) {
-  return a.maps * a.dim == attend_tf32::kD && a.vdim == attend_tf32::kD && a.max_rows >= 256;
+  return a.maps * a.dim == attend_tf32::kD && a.vdim == attend_tf32::kD && a.max_rows >= 256 && a.out != a.q && a.out != a.gate;
 }
 
 template <int M>

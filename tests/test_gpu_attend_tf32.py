@@ -1,12 +1,14 @@
 """fp32 attention on the tensor cores (256 rows and more): against 64 bits, at the edges of its 128-row and 64-key tiles, and with
 values that its two-term products cannot hold."""
 
+import ctypes
+
 import pytest
 import torch
 import torch.nn.functional as F
 
 import atma_b200
-from atma_b200 import decoder_ops
+from atma_b200 import _lib, decoder_ops
 from tests.conftest import max_rel
 from tests.gpu_util import rand
 from tests.rizurax_util import group
@@ -108,3 +110,41 @@ def test_softmax(H, G, maps, window, keep, rows, start, bad):
     reached = see[:, at] if bad == INF else torch.zeros(rows, dtype=torch.bool, device="cuda")
     assert max_rel(out[~reached], want[~reached]) < 1e-5
     assert not out[reached].isfinite().all(1).any()
+
+
+@pytest.mark.parametrize("maps", [1, 2])
+@pytest.mark.parametrize("over", ["q", "gate"])
+def test_softmax_in_the_place_of_an_input(over, maps):
+    """out over q or over the gate, with rows whose blocks are done again (an infinite value in the middle): as with an out of its own."""
+    rows, H, G = 400, 2, 1
+    q, kc, vc = rand((rows, H, maps, 128 // maps), 1).cuda(), rand((7, 64, G, 128), 2).cuda(), rand((7, 64, G, 128), 3).cuda()
+    vc[3, 10] = INF
+    kw = dict(scale=0.1, lam=0.3, out_scale=0.7, eps=1e-6, window=None, keep_first=0, sink=0.5)
+    gate = rand((rows, H * 128), 4).cuda()
+    g = group([rows], [0], [0], [list(range(7))])
+    want = decoder_ops.softmax_prefill(q, kc, vc, g, torch.zeros(rows, H * 128, device="cuda"), gate=gate, **kw)
+    out = q.view(rows, H * 128) if over == "q" else gate
+    got = decoder_ops.softmax_prefill(q, kc, vc, g, out, gate=gate, **kw)
+    assert torch.equal(got.isfinite(), want.isfinite()) and torch.allclose(got, want, atol=1e-5, rtol=1e-5, equal_nan=True)
+
+
+def test_polar_in_the_place_of_q():
+    T, H = 300, 2
+    q, k, v = (rand((1, n, T, 128), i).cuda() for i, n in enumerate((H, 1, 1)))
+    v[0, 0, 150, 3] = INF
+    p, n = params(H, 128), torch.arange(1, T + 1).float().cuda()
+    want = atma_b200.polar_attention_fwd(q, k, v, n, **p)
+    spg, sps, beta = (F.softplus(p[i]) for i in ("len_gain_raw", "null_slope_raw", "mag_beta_raw"))
+    x, mag = q.clone(), torch.zeros(1, H, T, device="cuda")
+    a = _lib.PolarPrefillArgs()
+    for name, t in (("q", x), ("k", k), ("v", v), ("c", x)):
+        setattr(a, name, t.data_ptr())
+        for i, d in enumerate(("sb", "sh", "st")):
+            setattr(a, f"{name}_{d}", t.stride(i))
+    a.mag, a.mag_sb, a.mag_sh, a.mag_st = mag.data_ptr(), mag.stride(0), mag.stride(1), mag.stride(2)
+    a.n_keys, a.spg, a.sps, a.beta = n.data_ptr(), spg.data_ptr(), sps.data_ptr(), beta.data_ptr()
+    a.null_base, a.v_null = p["null_base"].data_ptr(), p["v_null"].data_ptr()
+    a.B, a.H, a.Hkv, a.Tq, a.Tk, a.dk, a.dtype, a.eps, a.finalize = 1, H, 1, T, T, 128, _lib.dtype_code(q), 1e-6, 1
+    _lib.check(_lib.load().atma_polar_prefill(ctypes.byref(a), _lib.stream_ptr()))
+    for g, w in zip((x, mag), want):
+        assert torch.equal(g.isfinite(), w.isfinite()) and torch.allclose(g, w, atol=1e-5, rtol=1e-5, equal_nan=True)
