@@ -3,9 +3,18 @@
 //
 // Every operand is the sum of two tf32 terms, x = hi + lo with hi rounded to nearest, which leaves 2^-22 of it; three products
 // of terms - lo hi, hi lo, hi hi, small ones first - leave out 2^-22 of a product, with random signs.  The tensor core rounds its
-// fp32 sums towards zero, so a sum stays there for 64 channels of a score and for 64 keys of a result only: scores of 128
-// channels are two sums, added in registers, and so are the keys' results, in registers for the whole row.  What is
+// fp32 sums towards zero, which makes weights smaller together, so that next to a null key's weight they are off by more than
+// fp32 arithmetic's.  So a sum stays there for 16 channels of a score (32 with two maps, where a score has 64) and for 64 keys of a
+// result only; the others are made in registers.  What is
 // elementwise (scores, maxima, exponentials, sums of weights) is fp32 arithmetic as in the other fp32 kernels.
+// Errors of rows by the keys they see, 2-norm against 64 bits, products|64 x 64 kernels (2048 rows, 8 heads; 1e-7), and products with
+// one sum for 64 channels:
+//                         keys:  1       2-4     5-16    17-64   65-128  129-256 257-1024 -2048     1   2-4 -16 -64 -128 -256 -1024 -2048
+//   Polar, null key             1.0|1.0 1.4|1.3 1.8|1.7 2.4|2.3 2.8|2.6 3.0|2.9 3.4|3.6  3.7|4.2    1.2 1.7 2.5 3.7 4.2  4.6  5.4  6.0
+//   softmax, one map            0.4|0   1.2|1.0 1.6|1.6 2.4|2.2 2.8|2.7 2.9|3.4 3.1|5.2  3.2|7.4    0.4 1.4 2.1 3.2 3.7  3.9  4.2  4.3
+//   softmax, two maps           0.8|0.7 1.3|1.3 1.6|1.8 1.9|2.5 2.1|3.3 2.2|4.1 2.4|5.9  2.6|8.5    0.8 1.6 1.8 2.2 2.5  2.6  2.9  3.0
+// With one map, 64-row blocks with a row that sees fewer than 128 keys (few_keys) are for fp32 arithmetic: both blocks of a CTA, as a
+// prompt's first two, are done so at once, half of the threads each, beside the other CTAs' longer walks; one alone is marked.
 // A value that is infinite or no number, or results so small that their lo terms vanish, make a CTA mark 64-row blocks of its
 // output (kRedo); the 64 x 64 kernels of rows_f32.cuh run behind it on marked blocks only, and decide what such values give.
 //
@@ -14,11 +23,12 @@
 //   warps 8-11   keys: raw rows by cp.async a step ahead, then both terms of K [key][channel] and of V^T [channel][key] into
 //                shared memory, K-major with 128-byte swizzle
 //   warp 12      issues the products; owns the TMEM allocation (warps 13-15 fill the warpgroup)
-// TMEM (512 columns): Q hi [0,128) lo [128,256) | scores [256,320) and, of the other 64 channels, [320,384), then the weights
-// hi and lo in their place | the step's result [384,512).
-// A step of 64 keys takes 7700 clocks: three products at half the 16-bit rate, 1536 for the scores and 1536 for the result, with
+// TMEM (512 columns): Q hi [0,128) lo [128,256) | two sums of scores [256,384), then the weights hi and lo in their place |
+// the step's result [384,512), with one map the other two sums before.  With one map pairs of sums take the places in turn, the next
+// pair's products under the reading of the one in front, for next to nothing; sum by sum it was 1500 clocks a step.
+// A step of 64 keys takes 8000 clocks: three products at half the 16-bit rate, 1536 for the scores and 1536 for the result, with
 // their waits 4000; 1400 for the weights; what is left are scores, sums and hand-overs.  TMEM is full, so the next scores wait
-// for this step's result.  Errors against 64 bits: a model of 1500 rows 1.2e-6 -> 9.9e-7, a block of 2048 3.6e-7 as before.
+// for this step's result.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status word for the host.
 #pragma once
 
@@ -31,6 +41,7 @@ namespace attend_tf32 {
 using namespace sm100;
 
 constexpr int kM = 128, kN = 64, kD = 128, kThreads = 512;
+constexpr int few_keys(int maps) { return maps == 1 ? kM : 0; }
 constexpr uint32_t kRedo = 0x7fc0a11cu;              // a NaN that no arithmetic gives, in a block's first value
 constexpr int kTerm = kN * kD * 4;                   // one term of K or V
 constexpr int kOffK = 0, kOffV = 2 * kTerm, kOffRawK = 4 * kTerm, kOffRawV = 5 * kTerm, kSmemBytes = 6 * kTerm + 1024;
@@ -39,7 +50,7 @@ constexpr int kRowRegs = 208, kKeyRegs = 56, kMmaRegs = 40;          // 256 x 20
 static_assert(256 * kRowRegs + 128 * kKeyRegs + 128 * kMmaRegs <= kThreads * 128, "more registers than the block is launched with");
 
 struct Shared {
-  uint64_t q_ready, k_full, k_empty, v_full, v_empty, s_full, p_full, o_full, o_free;
+  uint64_t q_ready, k_full, k_empty, v_full, v_empty, s_full[2], s_free[2], p_full, o_full, o_free;
   uint32_t tmem;
   int abort, redo[2];
   float max[2][kM], sum[2][3][kM];                   // what the two halves of a row tell each other
@@ -65,6 +76,8 @@ __device__ __forceinline__ uint64_t desc(uint32_t addr) { return make_sdesc_sw12
 
 // Front: what a kernel attends to.  Front(args, shared): the CTA's rows and keys, told by all threads together, ends with a barrier;
 //   tiles(), key0(j)      steps and their first keys
+//   has(r), few(r)        whether row r is there, and sees keys, but fewer than few_keys; plain(smem, scratch) the rows in fp32 arithmetic
+//   mark(block)           a block of 64 rows (0, 1), if it has any, to be done again
 //   q_row(r), q_scale()   pointer to 128 channels of row r (0 .. 127) or null
 //   k_row(key), v_row(key), or null
 //   Row: row(r) with score(s), sees(key) and sees_all(first, last), without branches; start(t) and start_sum(t)
@@ -72,10 +85,19 @@ __device__ __forceinline__ uint64_t desc(uint32_t addr) { return make_sdesc_sw12
 template <typename Front, int M>
 __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int* status) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool few = tid < kM && f.few(tid);
+  const int few0 = __syncthreads_or(few && tid < kM / 2), few1 = __syncthreads_or(few && tid >= kM / 2);
+  if constexpr (few_keys(M) > 0) {
+    if (few0 && (few1 || !f.has(kM / 2))) {
+      f.plain(smem, reinterpret_cast<float (*)[2]>(sh.max));
+      return;
+    }
+  }
   if (tid == 0) {
     mbar_init(&sh.q_ready, 8); mbar_init(&sh.k_full, 4); mbar_init(&sh.k_empty, 1); mbar_init(&sh.v_full, 4); mbar_init(&sh.v_empty, 1);
-    mbar_init(&sh.s_full, 1); mbar_init(&sh.p_full, 8); mbar_init(&sh.o_full, 1); mbar_init(&sh.o_free, 8);
-    sh.abort = 0; sh.redo[0] = sh.redo[1] = 0;
+    for (int i = 0; i < 2; ++i) { mbar_init(&sh.s_full[i], 1); mbar_init(&sh.s_free[i], 8); }
+    mbar_init(&sh.p_full, 8); mbar_init(&sh.o_full, 1); mbar_init(&sh.o_free, 8);
+    sh.abort = 0; sh.redo[0] = few0; sh.redo[1] = few1;
     fence_barrier_init();
   }
   if (warp == 12) tmem_alloc(&sh.tmem, 512);
@@ -85,6 +107,7 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
   const uint32_t tbase = sh.tmem;
   volatile int* abort_flag = &sh.abort;
   const int n_tiles = f.tiles();
+  constexpr int kSum = M == 1 ? 16 : 32, kPairs = kD / M / (2 * kSum);           // channels that are summed in the tensor core; pairs of such sums
 
   if (warp < 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
@@ -129,25 +152,43 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
       const int key0 = f.key0(j) + 32 * half;
 #pragma unroll
       for (int t = 0; t < M; ++t, ++it) {
-        mbar_wait_warp(&sh.s_full, it & 1u, abort_flag);
-        tc_fence_after();
-        uint32_t s[32];
-        tmem_ld32(lane_base + kColS + 32 * half, s);
-        if constexpr (M == 1) {
-          uint32_t s2[32];
-          tmem_ld32(lane_base + kColS + 64 + 32 * half, s2);
+        float s[32] = {};
+#pragma unroll 1
+        for (int g = 0; g < kPairs; ++g) {
+          mbar_wait_warp(&sh.s_full[g & 1], (kPairs > 2 ? g >> 1 : it) & 1u, abort_flag);
+          tc_fence_after();
+          const uint32_t at = lane_base + kColS + 128 * (g & 1) + 32 * half;
+          if constexpr (M == 1) {
+            uint32_t x[64];
+            tmem_ld32_nowait(at, x);
+            tmem_ld32_nowait(at + 64, x + 32);
+            tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) s[i] = __float_as_uint(__uint_as_float(s[i]) + __uint_as_float(s2[i]));
+            for (int i = 0; i < 64; ++i) { reg_fence(x[i]); s[i & 31] += __uint_as_float(x[i]); }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 128; c += 64) {        // there are no registers for both
+              uint32_t x[32];
+              tmem_ld32(at + c, x);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) s[i] += __uint_as_float(x[i]);
+            }
+          }
+          if (g + 2 < kPairs) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.s_free[g & 1]);
+          }
         }
         float top = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) s[i] = __float_as_uint(row.score(__uint_as_float(s[i])));
+        for (int i = 0; i < 32; ++i) s[i] = row.score(s[i]);
         if (!__all_sync(0xffffffffu, row.sees_all(key0, key0 + 31))) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) s[i] = row.sees(key0 + i) ? s[i] : 0xff800000u;
+          for (int i = 0; i < 32; ++i) s[i] = row.sees(key0 + i) ? s[i] : -INFINITY;
         }
 #pragma unroll
-        for (int i = 0; i < 32; ++i) top = fmaxf(top, __uint_as_float(s[i]));
+        for (int i = 0; i < 32; ++i) top = fmaxf(top, s[i]);
         sh.max[half][r] = top;
         rows_sync();
         const float mn = fmaxf(m[t], fmaxf(top, sh.max[half ^ 1][r]));
@@ -159,7 +200,7 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
           uint32_t hi[16], lo[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float p = expf(__uint_as_float(s[c + i]) - from);
+            const float p = expf(s[c + i] - from);
             sum += p;
             sq = fmaf(p, p, sq);
             hi[i] = __float_as_uint(hi_term(p));
@@ -258,23 +299,29 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
         ok = mbar_wait(&sh.k_full, (uint32_t)j & 1u, abort_flag);
         for (int t = 0; t < M && ok; ++t, ++it) {
           tc_fence_after();
-          // scores of 64 channels at a time: of this map, or both halves of the one there is
-#pragma unroll
-          for (int g = 0; g < (M == 1 ? 2 : 1); ++g) {
-            const int ch = 64 * (M == 1 ? g : t);
+          for (int g = 0; g < kPairs && ok; ++g) {    // rolled, terms as well: their descriptors at once would not fit this warp's registers
+            // the second place is the result's: the one in front has been read
+            if (g == 1 && it > 0) ok = mbar_wait(&sh.o_free, (it - 1) & 1u, abort_flag);
+            if (g > 1) ok = mbar_wait(&sh.s_free[g & 1], it & 1u, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
 #pragma unroll 1
-            for (int term = 0; term < 3; ++term) {   // rolled: descriptors of all terms at once would not fit this warp's registers
-              const uint32_t qa = tbase + kColQ + (term == 0 ? 128 : 0) + ch;
-              const uint64_t kd = desc(ka + (term == 1 ? kTerm : 0) + ch / 32 * (kN * 128));
+            for (int c = 0; c < 2; ++c) {
+              const int step = ((t * kPairs + g) * 2 + c) * (kSum / 8);
+#pragma unroll 1
+              for (int term = 0; term < 3; ++term) {
 #pragma unroll
-              for (int k = 0; k < 8; ++k)
-                mma_ts_tf32(tbase + kColS + 64 * g, qa + 8 * k, kd + uint64_t(((k >> 2) * (kN * 128) + (k & 3) * 32) >> 4), idesc_tf32(kN), (term > 0 || k > 0) ? 1u : 0u);
+                for (int k = step; k < step + kSum / 8; ++k)
+                  mma_ts_tf32(tbase + kColS + 128 * (g & 1) + 64 * c, tbase + kColQ + (term == 0 ? 128 : 0) + 8 * k,
+                              desc(ka + (term == 1 ? kTerm : 0) + (k >> 2) * (kN * 128) + (k & 3) * 32), idesc_tf32(kN), (term > 0 || k > step) ? 1u : 0u);
+              }
             }
+            tc_commit(&sh.s_full[g & 1]);
           }
-          tc_commit(&sh.s_full);
+          if (!ok) break;
           if (t == M - 1) tc_commit(&sh.k_empty);
           ok = mbar_wait(&sh.p_full, it & 1u, abort_flag) && mbar_wait(&sh.v_full, (uint32_t)j & 1u, abort_flag) &&
-               (it == 0 || mbar_wait(&sh.o_free, (it - 1) & 1u, abort_flag));
+               (kPairs > 1 || it == 0 || mbar_wait(&sh.o_free, (it - 1) & 1u, abort_flag));
           if (!ok) break;
           tc_fence_after();
 #pragma unroll 1

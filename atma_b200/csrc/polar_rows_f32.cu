@@ -17,21 +17,17 @@ namespace {
 using namespace rows_f32;
 constexpr float kNegBig = -1e38f;
 
-template <int DK>
-__global__ void __launch_bounds__(kThreads, 2)
-polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
+template <int DK> constexpr int kBlockBytes = 4 * (kM * (DK + kPad) + kN * (DK + kPad) + kM * kLdP);
+
+// rows q0 .. q0 + 63 of a head
+template <int DK, int kOf>
+__device__ __forceinline__ void polar_block(const atma_polar_prefill_args& a, int h, int b, int q0, float* sm, float (*s_n)[2]) {
   constexpr int VM = DK / 64, ld = DK + kPad;
-  extern __shared__ __align__(16) float sm[];
   float* sQ = sm;                              // [64][ld]
   float* sKV = sQ + kM * ld;                   // K [64][ld], then V [64][DK]
   float* sP = sKV + kN * ld;                   // [64][kLdP]
-  __shared__ float s_lo[kThreads / 32], s_hi[kThreads / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
-  const int h = blockIdx.x % a.H, b = blockIdx.y, kvh = h / (a.H / a.Hkv);
-
-  const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM, q_limit = a.Tq, k_limit = a.Tk;
-  // behind the tensor-core kernel: only the blocks that it has marked
-  if (marked && __float_as_uint(static_cast<const float*>(a.c)[b * a.c_sb + h * a.c_sh + (int64_t)q0 * a.c_st]) != attend_tf32::kRedo) return;
+  const int tid = threadIdx.x & (kThreads - 1), lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
+  const int kvh = h / (a.H / a.Hkv), q_limit = a.Tq, k_limit = a.Tk;
   const float* Q = static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh;
   const float* K = static_cast<const float*>(a.k) + b * a.k_sb + kvh * a.k_sh;
   const float* V = static_cast<const float*>(a.v) + b * a.v_sb + kvh * a.v_sh;
@@ -69,11 +65,11 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
   const float inv_sqrt_dk = rsqrtf((float)DK);
   lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, 16));
   hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, 16));
-  if (lane == 0) { s_lo[warp] = lo; s_hi[warp] = hi; }
-  __syncthreads();
+  if (lane == 0) { s_n[warp][0] = lo; s_n[warp][1] = hi; }
+  block_sync<kOf>();
   float all_lo = lo, all_hi = hi;
 #pragma unroll
-  for (int w = 0; w < kThreads / 32; ++w) { all_lo = fminf(all_lo, s_lo[w]); all_hi = fmaxf(all_hi, s_hi[w]); }
+  for (int w = 0; w < kThreads / 32; ++w) { all_lo = fminf(all_lo, s_n[w][0]); all_hi = fmaxf(all_hi, s_n[w][1]); }
 
   // ---- key tiles that some row sees ----
   const float koff = (float)a.key_offset;
@@ -91,12 +87,12 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
         copy16(sKV + j * dst_ld + c, there ? src + (int64_t)(k0 + j) * stride + c : src, there);
       }
     };
-    __syncthreads();                           // the last tile's V is read
+    block_sync<kOf>();                           // the last tile's V is read
     fetch(K, a.k_st, ld);
-    copies_done();
+    copies_done<kOf>();
     float sc[4][4];
     dots<true>(sQ, sKV, ld, DK / 4, ty, tx, sc);
-    __syncthreads();
+    block_sync<kOf>();
     fetch(V, a.v_st, DK);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -134,7 +130,7 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
       const float pos = (float)(k0 + j) + koff;
       return pos < n[i] && (a.window <= 0 || pos >= n[i] - (float)a.window);
     };
-    copies_done();
+    copies_done<kOf>();
     weigh<VM>(sP, sKV, ty, tx, j0, j1, f0, f1, sees, acc);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -178,6 +174,17 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
       }
     }
   }
+}
+
+template <int DK>
+__global__ void __launch_bounds__(kThreads, 2)
+polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
+  extern __shared__ __align__(16) float sm[];
+  __shared__ float s_n[kThreads / 32][2];
+  const int h = blockIdx.x % a.H, b = blockIdx.y, q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM;
+  // behind the tensor-core kernel: only the blocks that it has marked
+  if (marked && __float_as_uint(static_cast<const float*>(a.c)[b * a.c_sb + h * a.c_sh + (int64_t)q0 * a.c_st]) != attend_tf32::kRedo) return;
+  polar_block<DK, 1>(a, h, b, q0, sm, s_n);
 }
 
 // ---- the same on the tensor cores, 128 rows of a head per CTA ----------------------------------------------------------
@@ -231,6 +238,21 @@ struct PolarFront {
   __device__ __forceinline__ int tiles() const { return max(j_end - j_begin + kN - 1, 0) / kN; }
   __device__ __forceinline__ int key0(int j) const { return j_begin + j * kN; }
   __device__ __forceinline__ float q_scale() const { return 1.f; }
+  __device__ __forceinline__ bool has(int r) const { return q0 + r < a.Tq; }
+  __device__ __forceinline__ bool few(int r) const {
+    const float n = count(q0 + r), first = fmaxf(a.window > 0 ? n - (float)a.window : 0.f, (float)a.key_offset);
+    const float seen = fminf(n, (float)a.key_offset + (float)a.Tk) - first;
+    return has(r) && seen > 0.f && seen < (float)attend_tf32::few_keys(1);
+  }
+  __device__ __forceinline__ float* result(int r) const { return static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)(q0 + r) * a.c_st; }
+  __device__ __forceinline__ void mark(int block) const { if (has(64 * block)) *result(64 * block) = __uint_as_float(attend_tf32::kRedo); }
+  // blocks of few keys in fp32 arithmetic, half of the CTA's threads each
+  __device__ __forceinline__ void plain(uint8_t* smem, float (*s_n)[2]) const {
+    static_assert(2 * kBlockBytes<attend_tf32::kD> <= attend_tf32::kSmemBytes - 1024, "two blocks fit");
+    const int block = threadIdx.x >> 8;
+    if (has(64 * block))
+      polar_block<attend_tf32::kD, 2>(a, h, b, q0 + 64 * block, reinterpret_cast<float*>(smem + block * kBlockBytes<attend_tf32::kD>), s_n + 8 * block);
+  }
   __device__ __forceinline__ const float* any() const { return static_cast<const float*>(a.q); }
   __device__ __forceinline__ const float* q_row(int r) const {
     return q0 + r < a.Tq ? static_cast<const float*>(a.q) + b * a.q_sb + h * a.q_sh + (int64_t)(q0 + r) * a.q_st : nullptr;
@@ -270,9 +292,9 @@ struct PolarFront {
     sh.sum[half][2][r] = sq;
     rows_sync();
     if (!ok) return;
-    float* cp = static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)(q0 + r) * a.c_st + 64 * half;
+    float* cp = result(r) + 64 * half;
     if (sh.redo[r >> 6]) {
-      if (half == 0 && (r & 63) == 0) cp[0] = __uint_as_float(kRedo);
+      if (half == 0 && (r & 63) == 0) mark(r >> 6);
       return;
     }
     const float inv = 1.0f / fmaxf(sqrtf(sq + sh.sum[half ^ 1][2][r]), a.eps);
@@ -302,10 +324,11 @@ polar_tf32_kernel(const __grid_constant__ atma_polar_prefill_args a) {
 }
 
 // Head size 128, no statistics carried in or out (a marked block is done again from the inputs alone), and enough rows: 2048
-// rows, 8 heads 431 us on the 64 x 64 kernel, 130 here; 512 rows 100 and 60; 256 rows 57 and 49, where the calls' own launches are most of it.
-// Results that take the place of q: the mark would be in the rows that are read again.
+// rows, 8 heads, the call's own launches counted, 453 us on the 64 x 64 kernel, 155 here; 512 rows 111 and 58; 256 rows 69 and 52.
+// Results that take the place of q: the mark would be in the rows that are read again.  Windows of fewer than few_keys keys: every block
+// would be left to the 64 x 64 kernel.
 bool polar_tf32_supported(const atma_polar_prefill_args& a) {
-  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq >= 256 && a.c != a.q;
+  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq >= 256 && a.c != a.q && (a.window <= 0 || a.window >= attend_tf32::few_keys(1));
 }
 
 template <int DK>
@@ -317,7 +340,7 @@ int launch(const atma_polar_prefill_args& a, cudaStream_t st) {
     const int rc = launch_status("polar_prefill (fp32, tensor cores)");
     if (rc != ATMA_OK) return rc;
   }
-  const int smem = 4 * (kM * (DK + kPad) + kN * (DK + kPad) + kM * kLdP);
+  constexpr int smem = kBlockBytes<DK>;
   ATMA_CUDA_OK(cudaFuncSetAttribute(polar_rows_f32_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   polar_rows_f32_kernel<DK><<<dim3((a.Tq + kM - 1) / kM * a.H, a.B), kThreads, smem, st>>>(a, tf32);
   return launch_status("polar_prefill (fp32, 64 x 64)");

@@ -19,9 +19,16 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool there)
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
                ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
+// The 256 threads of a block of 64 rows: of a CTA, or (kOf 2) half of a CTA that has two blocks.
+template <int kOf>
+__device__ __forceinline__ void block_sync() {
+  if constexpr (kOf == 1) __syncthreads();
+  else asm volatile("bar.sync %0, 256;" ::"r"(1 + (int)(threadIdx.x >> 8)) : "memory");
+}
+template <int kOf>
 __device__ __forceinline__ void copies_done() {
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
+  block_sync<kOf>();
 }
 
 // s[i][j] = row 4 ty + i times key tx + 16 j over n4 quadruples of channels.  PAIRS: even and odd channels in sums of their own,

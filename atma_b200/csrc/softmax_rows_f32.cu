@@ -18,24 +18,16 @@ namespace {
 
 using namespace rows_f32;
 
-template <int M, int VM>
-__global__ void __launch_bounds__(kThreads, 2)
-softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
-  extern __shared__ __align__(16) float sm[];
+// rows q0 .. q0 + 63 of a sequence's head
+template <int M, int VM, int kOf>
+__device__ __forceinline__ void softmax_block(const atma_softmax_args& a, int s, int h, int q0, float* sm) {
   const int kd = M * a.dim, ld = kd + kPad;
   float* sQ = sm;                              // [64][ld]
   float* sKV = sQ + kM * ld;                   // K [64][ld], then V [64][64 VM]
   float* sP = sKV + kN * max(ld, 64 * VM);     // [M][64][kLdP]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
-  const int s = blockIdx.y, h = blockIdx.x % a.H;
-  const int r_begin = a.cu_rows[s], n_rows = a.cu_rows[s + 1] - r_begin;
-  const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM;
-  if (q0 >= n_rows) return;
-  const int start = a.start_pos[s];
-  const int g = h / (a.H / a.G);
+  const int tid = threadIdx.x & (kThreads - 1), lane = tid & 31, warp = tid >> 5, tx = lane & 15, ty = 2 * warp + (lane >> 4);
+  const int r_begin = a.cu_rows[s], n_rows = a.cu_rows[s + 1] - r_begin, start = a.start_pos[s], g = h / (a.H / a.G);
   float* out = static_cast<float*>(a.out);
-  // behind the tensor-core kernel: only the blocks that it has marked
-  if (marked && __float_as_uint(out[(int64_t)(r_begin + q0) * a.out_rs + (int64_t)h * a.vdim]) != attend_tf32::kRedo) return;
   if (start < 0) {                             // padded sequence
     for (int i = tid; i < min(kM, n_rows - q0) * a.vdim; i += kThreads)
       out[(int64_t)(r_begin + q0 + i / a.vdim) * a.out_rs + (int64_t)h * a.vdim + i % a.vdim] = 0.f;
@@ -84,9 +76,9 @@ softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
         copy16(sKV + j * dst_ld + c, src, there);
       }
     };
-    __syncthreads();                           // the last tile's V is read
+    block_sync<kOf>();                           // the last tile's V is read
     fetch(K, kd, kd, ld);
-    copies_done();
+    copies_done<kOf>();
     // columns that some of the warp's rows see (j0 to j1 - 1) and those that all of them do (f0 to f1 - 1)
     const int kept = a.keep_first - k0, opens = first_pos - a.window + 1 - k0;
     int j1 = min(min(kN, n_keys - k0), first_pos + 8 - k0);
@@ -98,7 +90,7 @@ softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
       float sc[4][4];
       dots<M == 1>(sQ + t * a.dim, sKV + t * a.dim, ld, a.dim / 4, ty, tx, sc);
       if (t == M - 1) {
-        __syncthreads();                       // K is read
+        block_sync<kOf>();                       // K is read
         fetch(V, a.vdim, 64 * VM, 64 * VM);
       }
 #pragma unroll
@@ -125,7 +117,7 @@ softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
         times<VM>(acc[t][i], al);
       }
     }
-    copies_done();
+    copies_done<kOf>();
 #pragma unroll
     for (int t = 0; t < M; ++t) weigh<VM>(sP + t * kM * kLdP, sKV, ty, tx, j0, j1, f0, f1, sees, acc[t]);
   }
@@ -162,6 +154,17 @@ softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
   }
 }
 
+template <int M, int VM>
+__global__ void __launch_bounds__(kThreads, 2)
+softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
+  extern __shared__ __align__(16) float sm[];
+  const int s = blockIdx.y, h = blockIdx.x % a.H, q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * kM;
+  if (q0 >= a.cu_rows[s + 1] - a.cu_rows[s]) return;
+  // behind the tensor-core kernel: only the blocks that it has marked
+  if (marked && __float_as_uint(static_cast<const float*>(a.out)[(int64_t)(a.cu_rows[s] + q0) * a.out_rs + (int64_t)h * a.vdim]) != attend_tf32::kRedo) return;
+  softmax_block<M, VM, 1>(a, s, h, q0, sm);
+}
+
 // ---- the same on the tensor cores, 128 rows of a head per CTA: 128 channels of q and k in all, 128 of v ------------------
 __device__ int g_softmax_tf32_status = 0;
 
@@ -187,6 +190,23 @@ struct SoftmaxFront {
   __device__ __forceinline__ int tiles() const { return kt.n; }
   __device__ __forceinline__ int key0(int j) const { return kt[j] * kN; }
   __device__ __forceinline__ float q_scale() const { return a.scale; }
+  __device__ __forceinline__ bool has(int r) const { return q0 + r < n_rows; }
+  __device__ __forceinline__ bool few(int r) const {
+    const int last = min(first + r + 1, n_keys), opens = first + r + 1 - a.window;      // keys [opens, last) and those that are kept
+    const int seen = opens > 0 ? max(last - opens, 0) + min(max(a.keep_first, 0), opens) : last;
+    return has(r) && seen > 0 && seen < attend_tf32::few_keys(M);
+  }
+  __device__ __forceinline__ float* result(int r) const {
+    return static_cast<float*>(a.out) + (int64_t)(r_begin + q0 + r) * a.out_rs + (int64_t)h * attend_tf32::kD;
+  }
+  __device__ __forceinline__ void mark(int block) const { if (has(64 * block)) *result(64 * block) = __uint_as_float(attend_tf32::kRedo); }
+  // blocks of few keys in fp32 arithmetic, half of the CTA's threads each
+  __device__ __forceinline__ void plain(uint8_t* smem, float (*)[2]) const {
+    constexpr int kBytes = 4 * (kM * (attend_tf32::kD + kPad) + kN * (attend_tf32::kD + kPad) + M * kM * kLdP);
+    static_assert(M == 2 || 2 * kBytes <= attend_tf32::kSmemBytes - 1024, "two blocks fit");
+    const int block = threadIdx.x >> 8;
+    if (has(64 * block)) softmax_block<M, 2, 2>(a, s, h, q0 + 64 * block, reinterpret_cast<float*>(smem + block * kBytes));
+  }
   __device__ __forceinline__ const float* any() const { return static_cast<const float*>(a.q); }
   __device__ __forceinline__ const float* q_row(int r) const {
     return q0 + r < n_rows ? static_cast<const float*>(a.q) + ((int64_t)(r_begin + q0 + r) * a.H + h) * attend_tf32::kD : nullptr;
@@ -221,9 +241,9 @@ struct SoftmaxFront {
     sh.sum[half][2][r] = ss;
     rows_sync();
     if (!ok) return;
-    float* op = static_cast<float*>(a.out) + (int64_t)(r_begin + q0 + r) * a.out_rs + (int64_t)h * kD + 64 * half;
+    float* op = result(r) + 64 * half;
     if (sh.redo[r >> 6]) {
-      if (half == 0 && (r & 63) == 0) op[0] = __uint_as_float(kRedo);
+      if (half == 0 && (r & 63) == 0) mark(r >> 6);
       return;
     }
     float f = 1.f;
@@ -263,10 +283,13 @@ softmax_tf32_kernel(const __grid_constant__ atma_softmax_args a) {
   attend_tf32::attend<SoftmaxFront<M>, M>(front, smem, sh, &g_softmax_tf32_status);
 }
 
-// 128 channels in one map or two, 128 of v, and enough rows.  Two layers of two maps: 1500 rows, 8 heads 527 us on the 64 x 64
-// kernel, 145 here; 400 rows 143 and 57; 256 rows 91 and 49.  Results that take the place of q or the gate: the mark would be in
-// the rows that are read again.
+// 128 channels in one map or two, 128 of v, and enough rows.  Two maps, 8 heads, the call's own launches counted: 1500 rows 545 us on
+// the 64 x 64 kernel, 173 here; 400 rows 158 and 83; 256 rows 104 and 73.  One map: 363 and 136, 107 and 75, 72 and 75.  Results that take the place of q or the gate: the mark would be in
+// the rows that are read again.  Short windows: with one map every block would be left to the 64 x 64 kernel (few_keys); with two that is
+// faster while its CTAs have an SM each (a window of 8, 400 rows 59 us against 69, 1500 rows 76 against 73; of 64, 66 and 69, 86 and 71).
 bool softmax_tf32_supported(const atma_softmax_args& a) {
+  const int64_t ctas = (int64_t)(a.max_rows + kM - 1) / kM * a.H * a.n_seqs, seen = (int64_t)a.window + (a.keep_first > 0 ? a.keep_first : 0);
+  if (seen < attend_tf32::few_keys(1) && (a.maps == 1 || ctas <= sm_count_of_current_device())) return false;
   return a.maps * a.dim == attend_tf32::kD && a.vdim == attend_tf32::kD && a.max_rows >= 256 && a.out != a.q && a.out != a.gate;
 }
 
