@@ -145,9 +145,10 @@ __global__ void lfm2_conv_packed_kernel(const T* __restrict__ proj, int64_t proj
 // 16 bytes of channels x a run of kLfmVecTok consecutive tokens.  All rows of the run and the K - 1 in front are requested
 // as 16-byte loads up front, behind the weights and the sequence's numbers, which would cost a second latency after them.
 // Bound by bytes in flight: a run that meets the start or the end of a sequence (saved state or zero in front, a state to
-// write) is rare, goes out of line and reads its rows again, so that four CTAs fit an SM (for five the loads of a run find no
-// registers).  Three CTAs with the rare runs in line and the numbers asked for last: 12800 x 1024 36.9 us, 30.7 now; 32768 x 1024
-// 73.9, 57.4 now (4.7 TB/s).
+// write) goes out of line and reads its rows again, so that four CTAs fit an SM (for five the loads of a run find no
+// registers).  12800 x 1024, 16 bits, in sequences of 3000 tokens: three CTAs with such runs in line and the numbers asked for last 35.5
+// us, 26.7 now; of 30 tokens 39 and 29, of 5 58 and 39; in 32 bits 43 and 37, 47 and 41, 58 and 56.  The call out of line stands at the
+// end: in front of the common case it costs that its registers (bf16: 250 bytes of spills, 49 us).
 // Same rounding points and accumulation order as the scalar form.
 constexpr int kLfmVecTok = 4, kLfmVecCtas = 4;
 
@@ -161,60 +162,105 @@ __device__ __noinline__ uint4 lfm2_row_before_start(const T* __restrict__ init_s
   LfmVec16<T> r;
 #pragma unroll
   for (int n = 0; n < LfmVec16<T>::N; ++n)
-    r.e[n] = init_state != nullptr ? init_state[base + (int64_t)n * (K - 1) + (K - 1 - rows_before)] : from_f32<T>(0.f);
+    r.e[n] = init_state[base + (int64_t)n * (K - 1) + (K - 1 - rows_before)];
   return r.u;
 }
 template <typename T, int K>
 __device__ __noinline__ void lfm2_state_write(T* __restrict__ dst, const uint4* keep) {
+  constexpr int N = LfmVec16<T>::N;
+  LfmVec16<T> r[K - 1], o[K - 1];                     // dst[n][j], N (K-1) values in one piece
 #pragma unroll
-  for (int j = 0; j < K - 1; ++j) {
-    LfmVec16<T> r;
-    r.u = keep[j];
+  for (int j = 0; j < K - 1; ++j) r[j].u = keep[j];
 #pragma unroll
-    for (int n = 0; n < LfmVec16<T>::N; ++n) dst[(int64_t)n * (K - 1) + j] = r.e[n];
+  for (int i = 0; i < N * (K - 1); ++i) o[i / N].e[i % N] = r[i % (K - 1)].e[i / (K - 1)];
+  if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+#pragma unroll
+    for (int j = 0; j < K - 1; ++j) reinterpret_cast<uint4*>(dst)[j] = o[j].u;
+  } else {
+#pragma unroll
+    for (int i = 0; i < N * (K - 1); ++i) dst[i] = o[i / N].e[i % N];
   }
 }
 
-// The tokens [t0, t0 + nt) of 16 bytes of channels, whatever sequences they belong to.
+// a thread's N x K weights, neighbours in memory
+template <typename T, int K>
+struct LfmTaps {
+  static constexpr int N = LfmVec16<T>::N;
+  LfmVec16<T> v[K];
+  __device__ __forceinline__ explicit LfmTaps(const T* w) {
+    if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+#pragma unroll
+      for (int i = 0; i < K; ++i) v[i].u = reinterpret_cast<const uint4*>(w)[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < N * K; ++i) v[i / N].e[i % N] = w[i];
+    }
+  }
+  __device__ __forceinline__ float operator()(int n, int j) const { return to_f32(v[(n * K + j) / N].e[(n * K + j) % N]); }
+};
+
+// The tokens [t0, t0 + nt) of 16 bytes of channels, whatever sequences they belong to.  Everything is asked for at once here, too:
+// a packed batch of short sequences has no other runs (token after token, rows read again for each, 12800 x 1024 in sequences of 5
+// took 64 us in 16 bits and 80 in 32).
 template <typename T, int K>
 __device__ __noinline__ void lfm2_run_general(const T* proj, int64_t proj_st, const T* w, T* out, int64_t out_st, T* state, const T* init_state,
                                               int64_t state_ss, const int32_t* seq_start, const int32_t* seq_end, const int32_t* seq_slot,
                                               int D, int t0, int nt, int d0) {
-  constexpr int N = LfmVec16<T>::N;
-#pragma unroll 1
-  for (int t = t0; t < t0 + nt; ++t) {
-    const int s0 = seq_start[t], e0 = seq_end[t], sl = seq_slot[t];
+  constexpr int N = LfmVec16<T>::N, kRows = kLfmVecTok + K - 1;
+  int s0[kLfmVecTok], e0[kLfmVecTok], sl[kLfmVecTok];
+#pragma unroll
+  for (int i = 0; i < kLfmVecTok; ++i) {
+    const int t = t0 + min(i, nt - 1);
+    s0[i] = seq_start[t]; e0[i] = seq_end[t]; sl[i] = seq_slot[t];
+  }
+  const LfmTaps<T, K> wt(w + (int64_t)d0 * K);
+  LfmVec16<T> g[kRows], x[kRows], cc[kLfmVecTok];
+#pragma unroll
+  for (int i = 0; i < kRows; ++i) {
+    const int t = t0 - (K - 1) + i;
+    g[i].u = x[i].u = make_uint4(0u, 0u, 0u, 0u);
+    if (t >= 0 && t < t0 + nt) {
+      const T* p = proj + (int64_t)t * proj_st + d0;
+      g[i].u = *reinterpret_cast<const uint4*>(p);
+      x[i].u = *reinterpret_cast<const uint4*>(p + 2 * D);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kLfmVecTok; ++i)
+    if (i < nt) cc[i].u = *reinterpret_cast<const uint4*>(proj + (int64_t)(t0 + i) * proj_st + D + d0);
+#pragma unroll
+  for (int i = 0; i < kRows; ++i)
+#pragma unroll
+    for (int n = 0; n < N; ++n) g[i].e[n] = from_f32<T>(to_f32(g[i].e[n]) * to_f32(x[i].e[n]));
+#pragma unroll
+  for (int i = 0; i < kLfmVecTok; ++i) {
+    if (i >= nt) break;
+    const int t = t0 + i;
     LfmVec16<T> prev[K];                              // prev[j] = gated input K-1-j rows before t as this sequence sees it
 #pragma unroll
     for (int j = 0; j < K; ++j) {
       const int src = t - (K - 1 - j);
-      if (src >= s0) {
-        const T* p = proj + (int64_t)src * proj_st + d0;
-        LfmVec16<T> b, x;
-        b.u = *reinterpret_cast<const uint4*>(p);
-        x.u = *reinterpret_cast<const uint4*>(p + 2 * D);
-#pragma unroll
-        for (int n = 0; n < N; ++n) prev[j].e[n] = from_f32<T>(to_f32(b.e[n]) * to_f32(x.e[n]));
-      } else {
-        prev[j].u = lfm2_row_before_start<T, K>(sl >= 0 ? init_state : nullptr,
-                                                (sl >= 0 ? sl * state_ss : 0) + (int64_t)d0 * (K - 1), s0 - src);
+      prev[j].u = g[i + j].u;
+      if (src < s0[i]) {
+        prev[j].u = make_uint4(0u, 0u, 0u, 0u);
+        if (sl[i] >= 0 && init_state != nullptr)
+          prev[j].u = lfm2_row_before_start<T, K>(init_state, sl[i] * state_ss + (int64_t)d0 * (K - 1), s0[i] - src);
       }
     }
-    LfmVec16<T> cv, o;
-    cv.u = *reinterpret_cast<const uint4*>(proj + (int64_t)t * proj_st + D + d0);
+    LfmVec16<T> o;
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       float acc = 0.f;
 #pragma unroll
-      for (int j = 0; j < K; ++j) acc = fmaf(to_f32(prev[j].e[n]), to_f32(w[(int64_t)(d0 + n) * K + j]), acc);
-      o.e[n] = from_f32<T>(to_f32(cv.e[n]) * round_through<T>(acc));
+      for (int j = 0; j < K; ++j) acc = fmaf(to_f32(prev[j].e[n]), wt(n, j), acc);
+      o.e[n] = from_f32<T>(to_f32(cc[i].e[n]) * round_through<T>(acc));
     }
     *reinterpret_cast<uint4*>(out + (int64_t)t * out_st + d0) = o.u;
-    if (t == e0 - 1 && sl >= 0 && state != nullptr) {
+    if (t == e0[i] - 1 && sl[i] >= 0 && state != nullptr) {
       uint4 keep[K - 1];
 #pragma unroll
       for (int j = 0; j < K - 1; ++j) keep[j] = prev[j + 1].u;
-      lfm2_state_write<T, K>(state + sl * state_ss + (int64_t)d0 * (K - 1), keep);
+      lfm2_state_write<T, K>(state + sl[i] * state_ss + (int64_t)d0 * (K - 1), keep);
     }
   }
 }
@@ -236,15 +282,7 @@ lfm2_conv_packed_vec_kernel(const T* __restrict__ proj, int64_t proj_st, const T
   const int nt = min(kLfmVecTok, total - t0);
 
   const int sa = seq_start[t0], sb = seq_start[t0 + nt - 1], ea = seq_end[t0 + nt - 1];
-  constexpr int kPieces = (N * K * (int)sizeof(T) + 15) / 16;       // the thread's N x K weights are neighbours in memory
-  LfmVec16<T> wv[kPieces];
-  if ((reinterpret_cast<uintptr_t>(w) & 15) == 0) {
-#pragma unroll
-    for (int i = 0; i < kPieces; ++i) wv[i].u = *reinterpret_cast<const uint4*>(w + (int64_t)d0 * K + i * N);
-  } else {
-#pragma unroll
-    for (int i = 0; i < N * K; ++i) wv[i / N].e[i % N] = w[(int64_t)d0 * K + i];
-  }
+  const LfmTaps<T, K> wt(w + (int64_t)d0 * K);
   LfmVec16<T> bx[kLfmVecTok + K - 1], xx[kLfmVecTok + K - 1], cc[kLfmVecTok];
 #pragma unroll
   for (int i = 0; i < kLfmVecTok + K - 1; ++i) {
@@ -262,27 +300,27 @@ lfm2_conv_packed_vec_kernel(const T* __restrict__ proj, int64_t proj_st, const T
   for (int i = 0; i < kLfmVecTok; ++i)
     cc[i].u = i < nt ? *reinterpret_cast<const uint4*>(proj + (int64_t)(t0 + i) * proj_st + D + d0) : make_uint4(0u, 0u, 0u, 0u);
   // the run and its K-1 rows of left context lie inside one sequence that goes on behind it
-  if (nt < kLfmVecTok || sa != sb || ea <= t0 + nt || sa > t0 - (K - 1)) {
-    lfm2_run_general<T, K>(proj, proj_st, w, out, out_st, state, init_state, state_ss, seq_start, seq_end, seq_slot, D, t0, nt, d0);
+  if (nt == kLfmVecTok && sa == sb && ea > t0 + nt && sa <= t0 - (K - 1)) {
+    // gated input B * x' of every row of the run, rounded to T as eager materialises it (reuses bx)
+#pragma unroll
+    for (int i = 0; i < kLfmVecTok + K - 1; ++i)
+#pragma unroll
+      for (int n = 0; n < N; ++n) bx[i].e[n] = from_f32<T>(to_f32(bx[i].e[n]) * to_f32(xx[i].e[n]));
+#pragma unroll
+    for (int i = 0; i < kLfmVecTok; ++i) {
+      LfmVec16<T> o;
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        float acc = 0.f;
+#pragma unroll
+        for (int j = 0; j < K; ++j) acc = fmaf(to_f32(bx[i + j].e[n]), wt(n, j), acc);
+        o.e[n] = from_f32<T>(to_f32(cc[i].e[n]) * round_through<T>(acc));
+      }
+      *reinterpret_cast<uint4*>(out + (int64_t)(t0 + i) * out_st + d0) = o.u;
+    }
     return;
   }
-  // gated input B * x' of every row of the run, rounded to T as eager materialises it (reuses bx)
-#pragma unroll
-  for (int i = 0; i < kLfmVecTok + K - 1; ++i)
-#pragma unroll
-    for (int n = 0; n < N; ++n) bx[i].e[n] = from_f32<T>(to_f32(bx[i].e[n]) * to_f32(xx[i].e[n]));
-#pragma unroll
-  for (int i = 0; i < kLfmVecTok; ++i) {
-    LfmVec16<T> o;
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-      float acc = 0.f;
-#pragma unroll
-      for (int j = 0; j < K; ++j) acc = fmaf(to_f32(bx[i + j].e[n]), to_f32(wv[(n * K + j) / N].e[(n * K + j) % N]), acc);
-      o.e[n] = from_f32<T>(to_f32(cc[i].e[n]) * round_through<T>(acc));
-    }
-    *reinterpret_cast<uint4*>(out + (int64_t)(t0 + i) * out_st + d0) = o.u;
-  }
+  lfm2_run_general<T, K>(proj, proj_st, w, out, out_st, state, init_state, state_ss, seq_start, seq_end, seq_slot, D, t0, nt, d0);
 }
 
 template <typename T>
