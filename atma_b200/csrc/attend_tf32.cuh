@@ -74,9 +74,17 @@ __device__ __forceinline__ void mma_ts_tf32(uint32_t d_tmem, uint32_t a_tmem, ui
 __host__ __device__ constexpr uint32_t idesc_tf32(int N) { return (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(kM >> 4) << 24); }
 __device__ __forceinline__ uint64_t desc(uint32_t addr) { return make_sdesc_sw128(addr, 16, 1024); }
 
+// The CTA's first row.  Later rows have more keys, so they come first, but for the very first, which go row by row of keys (few_keys) and
+// take as long as four to six steps.
+template <int M>
+__device__ __forceinline__ int first_row(int heads) {
+  const int tiles = gridDim.x / heads, at = blockIdx.x / heads;
+  return (few_keys(M) > 0 ? (at == 0 ? 0 : tiles - at) : tiles - 1 - at) * kM;
+}
+
 // Front: what a kernel attends to.  Front(args, shared): the CTA's rows and keys, told by all threads together, ends with a barrier;
 //   tiles(), key0(j)      steps and their first keys
-//   has(r), few(r)        whether row r is there, and sees keys, but fewer than few_keys; plain(smem, scratch) the rows in fp32 arithmetic
+//   has(r), few(r)        whether row r is there, and sees keys, but fewer than few_keys; plain() the CTA's rows in fp32 arithmetic
 //   mark(block)           a block of 64 rows (0, 1), if it has any, to be done again
 //   q_row(r), q_scale()   pointer to 128 channels of row r (0 .. 127) or null
 //   k_row(key), v_row(key), or null
@@ -89,7 +97,7 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
   const int few0 = __syncthreads_or(few && tid < kM / 2), few1 = __syncthreads_or(few && tid >= kM / 2);
   if constexpr (few_keys(M) > 0) {
     if (few0 && (few1 || !f.has(kM / 2))) {
-      f.plain(smem, reinterpret_cast<float (*)[2]>(sh.max));
+      f.plain();
       return;
     }
   }
@@ -218,16 +226,28 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
         m[t] = mn;
         mbar_wait_warp(&sh.o_full, it & 1u, abort_flag);
         tc_fence_after();
+        if constexpr (M == 1) {                       // the next step's second pair of sums waits for this place
+          uint32_t o[64];
+          tmem_ld32_nowait(lane_base + kColO + 64 * half, o);
+          tmem_ld32_nowait(lane_base + kColO + 64 * half + 32, o + 32);
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.o_free);
 #pragma unroll
-        for (int c = 0; c < 64; c += 16) {
-          uint32_t o[16];
-          tmem_ld16(lane_base + kColO + 64 * half + c, o);
+          for (int i = 0; i < 64; ++i) { reg_fence(o[i]); O[t][i] = fmaf(O[t][i], al, __uint_as_float(o[i])); }
+        } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) O[t][c + i] = fmaf(O[t][c + i], al, __uint_as_float(o[i]));
+          for (int c = 0; c < 64; c += 16) {
+            uint32_t o[16];
+            tmem_ld16(lane_base + kColO + 64 * half + c, o);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) O[t][c + i] = fmaf(O[t][c + i], al, __uint_as_float(o[i]));
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sh.o_free);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh.o_free);
       }
     }
     f.finish(row, r, half, m, l, q2, O, sh);

@@ -188,6 +188,14 @@ polar_rows_f32_kernel(const atma_polar_prefill_args a, int marked) {
 }
 
 // ---- the same on the tensor cores, 128 rows of a head per CTA ----------------------------------------------------------
+// a block of the tensor-core kernel's CTA, `at` bytes into its shared memory (a pointer would not be known to be shared); a function of
+// its own, so that it takes none of that kernel's registers
+__device__ __noinline__ void polar_half_block(const atma_polar_prefill_args& a, int h, int b, int q0, int at) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ float s_n[2][8][2];
+  polar_block<attend_tf32::kD, 2>(a, h, b, q0, reinterpret_cast<float*>(smem_raw + at), s_n[threadIdx.x >> 8]);
+}
+
 __device__ int g_polar_tf32_status = 0;
 
 struct PolarFront {
@@ -211,7 +219,7 @@ struct PolarFront {
   }
   __device__ __forceinline__ PolarFront(const atma_polar_prefill_args& args, float (*s_n)[2]) : a(args) {
     h = blockIdx.x % a.H; b = blockIdx.y; kvh = h / (a.H / a.Hkv);
-    q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * attend_tf32::kM;
+    q0 = attend_tf32::first_row<1>(a.H);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp < 4) {
       const int r = q0 + 32 * warp + lane;
@@ -247,11 +255,10 @@ struct PolarFront {
   __device__ __forceinline__ float* result(int r) const { return static_cast<float*>(a.c) + b * a.c_sb + h * a.c_sh + (int64_t)(q0 + r) * a.c_st; }
   __device__ __forceinline__ void mark(int block) const { if (has(64 * block)) *result(64 * block) = __uint_as_float(attend_tf32::kRedo); }
   // blocks of few keys in fp32 arithmetic, half of the CTA's threads each
-  __device__ __forceinline__ void plain(uint8_t* smem, float (*s_n)[2]) const {
-    static_assert(2 * kBlockBytes<attend_tf32::kD> <= attend_tf32::kSmemBytes - 1024, "two blocks fit");
+  __device__ __forceinline__ void plain() const {
+    static_assert(2 * kBlockBytes<attend_tf32::kD> <= attend_tf32::kSmemBytes, "two blocks fit");
     const int block = threadIdx.x >> 8;
-    if (has(64 * block))
-      polar_block<attend_tf32::kD, 2>(a, h, b, q0 + 64 * block, reinterpret_cast<float*>(smem + block * kBlockBytes<attend_tf32::kD>), s_n + 8 * block);
+    if (has(64 * block)) polar_half_block(a, h, b, q0 + 64 * block, block * kBlockBytes<attend_tf32::kD>);
   }
   __device__ __forceinline__ const float* any() const { return static_cast<const float*>(a.q); }
   __device__ __forceinline__ const float* q_row(int r) const {
@@ -324,11 +331,12 @@ polar_tf32_kernel(const __grid_constant__ atma_polar_prefill_args a) {
 }
 
 // Head size 128, no statistics carried in or out (a marked block is done again from the inputs alone), and enough rows: 2048
-// rows, 8 heads, the call's own launches counted, 453 us on the 64 x 64 kernel, 155 here; 512 rows 111 and 58; 256 rows 69 and 52.
+// rows, 8 heads, the call's own launches counted, 432 us on the 64 x 64 kernel, 146 here; 512 rows 100 and 58; 300 rows 66 and 58; 256 rows 55 and
+// 58 (with two CTAs a head one is for fp32 arithmetic).
 // Results that take the place of q: the mark would be in the rows that are read again.  Windows of fewer than few_keys keys: every block
 // would be left to the 64 x 64 kernel.
 bool polar_tf32_supported(const atma_polar_prefill_args& a) {
-  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq >= 256 && a.c != a.q && (a.window <= 0 || a.window >= attend_tf32::few_keys(1));
+  return a.dk == 128 && a.finalize && a.stats_in_m == nullptr && a.Tq > 256 && a.c != a.q && (a.window <= 0 || a.window >= attend_tf32::few_keys(1));
 }
 
 template <int DK>

@@ -168,6 +168,14 @@ softmax_rows_f32_kernel(const atma_softmax_args a, int marked) {
 // ---- the same on the tensor cores, 128 rows of a head per CTA: 128 channels of q and k in all, 128 of v ------------------
 __device__ int g_softmax_tf32_status = 0;
 
+// a block of the tensor-core kernel's CTA, `at` bytes into its shared memory (a pointer would not be known to be shared); a function of
+// its own, so that it takes none of that kernel's registers
+template <int M>
+__device__ __noinline__ void softmax_half_block(const atma_softmax_args& a, int s, int h, int q0, int at) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  softmax_block<M, 2, 2>(a, s, h, q0, reinterpret_cast<float*>(smem_raw + at));
+}
+
 template <int M>
 struct SoftmaxFront {
   struct Row {
@@ -201,11 +209,11 @@ struct SoftmaxFront {
   }
   __device__ __forceinline__ void mark(int block) const { if (has(64 * block)) *result(64 * block) = __uint_as_float(attend_tf32::kRedo); }
   // blocks of few keys in fp32 arithmetic, half of the CTA's threads each
-  __device__ __forceinline__ void plain(uint8_t* smem, float (*)[2]) const {
+  __device__ __forceinline__ void plain() const {
     constexpr int kBytes = 4 * (kM * (attend_tf32::kD + kPad) + kN * (attend_tf32::kD + kPad) + M * kM * kLdP);
-    static_assert(M == 2 || 2 * kBytes <= attend_tf32::kSmemBytes - 1024, "two blocks fit");
+    static_assert(M == 2 || 2 * kBytes <= attend_tf32::kSmemBytes, "two blocks fit");
     const int block = threadIdx.x >> 8;
-    if (has(64 * block)) softmax_block<M, 2, 2>(a, s, h, q0 + 64 * block, reinterpret_cast<float*>(smem + block * kBytes));
+    if (has(64 * block)) softmax_half_block<M>(a, s, h, q0 + 64 * block, block * kBytes);
   }
   __device__ __forceinline__ const float* any() const { return static_cast<const float*>(a.q); }
   __device__ __forceinline__ const float* q_row(int r) const {
@@ -271,7 +279,7 @@ softmax_tf32_kernel(const __grid_constant__ atma_softmax_args a) {
   __shared__ attend_tf32::Shared sh;
   const int s = blockIdx.y, h = blockIdx.x % a.H;
   const int r_begin = a.cu_rows[s], n_rows = a.cu_rows[s + 1] - r_begin, start = a.start_pos[s];
-  const int q0 = ((int)(gridDim.x - blockIdx.x) - 1) / a.H * attend_tf32::kM;
+  const int q0 = attend_tf32::first_row<M>(a.H);
   if (q0 >= n_rows) return;
   if (start < 0) {                             // padded sequence
     float* out = static_cast<float*>(a.out);
@@ -283,14 +291,14 @@ softmax_tf32_kernel(const __grid_constant__ atma_softmax_args a) {
   attend_tf32::attend<SoftmaxFront<M>, M>(front, smem, sh, &g_softmax_tf32_status);
 }
 
-// 128 channels in one map or two, 128 of v, and enough rows.  Two maps, 8 heads, the call's own launches counted: 1500 rows 545 us on
-// the 64 x 64 kernel, 173 here; 400 rows 158 and 83; 256 rows 104 and 73.  One map: 363 and 136, 107 and 75, 72 and 75.  Results that take the place of q or the gate: the mark would be in
+// 128 channels in one map or two, 128 of v, and enough rows.  Two maps, 8 heads, the call's own launches counted: 1500 rows 547 us on
+// the 64 x 64 kernel, 175 here; 400 rows 156 and 83; 256 rows 104 and 75.  One map: 363 and 132, 106 and 79, 72 and 77.  Results that take the place of q or the gate: the mark would be in
 // the rows that are read again.  Short windows: with one map every block would be left to the 64 x 64 kernel (few_keys); with two that is
 // faster while its CTAs have an SM each (a window of 8, 400 rows 59 us against 69, 1500 rows 76 against 73; of 64, 66 and 69, 86 and 71).
 bool softmax_tf32_supported(const atma_softmax_args& a) {
   const int64_t ctas = (int64_t)(a.max_rows + kM - 1) / kM * a.H * a.n_seqs, seen = (int64_t)a.window + (a.keep_first > 0 ? a.keep_first : 0);
   if (seen < attend_tf32::few_keys(1) && (a.maps == 1 || ctas <= sm_count_of_current_device())) return false;
-  return a.maps * a.dim == attend_tf32::kD && a.vdim == attend_tf32::kD && a.max_rows >= 256 && a.out != a.q && a.out != a.gate;
+  return a.maps * a.dim == attend_tf32::kD && a.vdim == attend_tf32::kD && a.max_rows >= (a.maps == 1 ? 257 : 256) && a.out != a.q && a.out != a.gate;
 }
 
 template <int M>

@@ -1,4 +1,4 @@
-"""fp32 attention on the tensor cores (256 rows and more): against 64 bits, at the edges of its 128-row and 64-key tiles, and with
+"""fp32 attention on the tensor cores (257 rows and more, 256 with two maps): against 64 bits, at the edges of its 128-row and 64-key tiles, and with
 values that its two-term products cannot hold."""
 
 import ctypes
