@@ -437,7 +437,6 @@ def profile_case(which):
     elif which == "linear":
         # the MLP of one layer at decode batch 8 (hidden 1024, 4x): fc + gate (16.8 MB of weights), proj (8.4 MB); the
         # weights cycle through 12 copies (302 MB) so that every launch reads them from HBM, not from L2
-        import torch.nn.functional as F
         D, Fh, copies = 1024, 4096, 12
         w_fc = [(torch.randn(2 * Fh, D, generator=g) / 32).bfloat16().to(dev) for _ in range(copies)]
         w_pr = [(torch.randn(D, Fh, generator=g) / 64).bfloat16().to(dev) for _ in range(copies)]
