@@ -152,7 +152,7 @@ static Rows kept_rows(void* scratch, bool is_bf16, int64_t n_records, int64_t to
   return Rows{at, at + each, at + 2 * each, is_bf16, H, H, tokens};
 }
 
-// makes it (8 heads and 2 of k and v, 2 x 16384 rows: 46 us)
+// makes it (8 heads and 2 of k and v, 2 x 16384 rows: 72 of 165 us with the factors)
 static Rows keep_rows(const Rows& r, void* scratch, int64_t n_records, cudaStream_t st) {
   const Rows keep = kept_rows(scratch, r.is_bf16, n_records, r.tokens, r.H);
   const int64_t n = r.tokens * r.H * 16;

@@ -11,7 +11,7 @@
 // itself - large values that meet zeros and small ones that do not - is summed again in fp32 from the inputs, a warp for
 // four, and so are the results of a row with an infinity or a NaN, which has no fp16 terms.  Rows of random values, squared
 // activations among them, have next to none, and the test costs nothing that shows; where every result needs it, 1500 x 8192 x
-// 1024 takes 7.8 ms instead of 0.12, with one such row of x 0.31.
+// 1024 takes 12 ms instead of 0.11 (7.8 while every tile had its CTA), with one such row of x 0.31.
 //   split kernel: one CTA per row of x and of w, two fp16 planes each, the row's power of two and what it lost.
 //   product kernel: a CTA per SM takes tiles of 128 rows x BN columns in turn (a very long K: a CTA per tile).  Warp 0 TMA (both planes of 64 columns of x and of
 //   w per stage), warp 1 MMA, warps 2-9 add the sums of one stage out of one half of the accumulator columns while the next stage's
