@@ -332,11 +332,13 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     // a tile's coordinates and its row scalars are fetched a tile ahead
     Meta m_next{};
     float bt_next = 0.f, kinv_next = 0.f, qinv_next = 0.f, decay_next = 0.f;
+    int sees_next = 0;                                 // columns s < sees of A, s <= sees of Rq; a row behind the sequence's end: none
     auto fetch_tile = [&](int64_t tile) {
       if (tile >= n_tiles) return;
       tile_meta(p, tile, m_next);
       const bool valid = pr < (ci ? m_next.rows[1] : m_next.rows[0]);
       const int64_t t = (ci ? m_next.t0[1] : m_next.t0[0]) + pr;
+      sees_next = valid ? pr : -1;
       bt_next = valid ? p.beta[t * p.H + m_next.h] : 0.f;
       kinv_next = valid ? p.k_inv[t * p.G + m_next.g] : 0.f;
       qinv_next = valid ? p.q_inv[t * p.G + m_next.g] : 0.f;
@@ -347,6 +349,7 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       const Meta m = m_next;
       const int64_t rec = ci ? m.rec[1] : m.rec[0];
       const float bt_p = bt_next, kinv_p = kinv_next, qinv_p = qinv_next;
+      const int sees = sees_next;
       float run = decay_next;
       // decay prefix over the chunk's 64 rows (two warps)
 #pragma unroll
@@ -393,7 +396,7 @@ delta_factors_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
               const int s = 32 * half + j + e;
               // chosen after it is computed: as a condition around the exponential it is a branch for every element
               const float value = f * (__expf(lg_p - s_lg[64 * ci + s]) * s_kinv[64 * ci + s]) * __uint_as_float(gm[j + e]);
-              x[e] = (which ? s <= pr : s < pr) ? value : 0.f;
+              x[e] = (which ? s <= sees : s < sees) ? value : 0.f;
             }
             *reinterpret_cast<float4*>(dst + j) = make_float4(x[0], x[1], x[2], x[3]);
           }
@@ -738,6 +741,20 @@ delta_recur_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
         for (int j = 0; j < 16; j += 2)
           split2(fmaf(-ek[j], __uint_as_float(pr[j]), vv[j]), fmaf(-ek[j + 1], __uint_as_float(pr[j + 1]), vv[j + 1]), hi[j >> 1], lo[j >> 1]);
+        if (i == n_chunks - 1 && row_end - (row_begin + i * kC) < kC) {
+          // Rows behind the sequence's end are another's.  Their factors are zero, but they may be infinite or no numbers: no R, and
+          // zeros for K, whose product with S has been read, in front of the product with U
+          const int left = row_end - (row_begin + i * kC);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const uint32_t keep = 16 * qt + j < left ? 0xffffffffu : j & 1 ? 0x0000ffffu : 0xffff0000u;
+            hi[j >> 1] &= keep; lo[j >> 1] &= keep;
+          }
+          uint8_t* kr = smem + s * kStageBytes + kOffKQ;
+          for (int at = tid - 64 + left * 16; at < kC * 16; at += 32 * kStateWarps)      // 16 pieces of 16 bytes a row, eight in each box
+            *reinterpret_cast<uint4*>(kr + ((at & 8) << 11) + (at >> 4) * 128 + ((at & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+          fence_proxy_async();
+        }
         tmem_st8(lane_base + kColR + 8 * qt, hi);
         tmem_st8(lane_base + kColR + 32 + 8 * qt, lo);
         tmem_st_wait();
