@@ -11,7 +11,7 @@
 // itself - large values that meet zeros and small ones that do not - is summed again in fp32 from the inputs, a warp for
 // four, and so are the results of a row with an infinity or a NaN, which has no fp16 terms.  Rows of random values, squared
 // activations among them, have next to none, and the test costs nothing that shows; where every result needs it, 1500 x 8192 x
-// 1024 takes 12 ms instead of 0.11 (7.8 while every tile had its CTA), with one such row of x 0.31.
+// 1024 takes 9.9 ms instead of 0.11 (7.7 while every tile had its CTA), with one such row of x 0.31.
 //   split kernel: one CTA per row of x and of w, two fp16 planes each, the row's power of two and what it lost.
 //   product kernel: a CTA per SM takes tiles of 128 rows x BN columns in turn (a very long K: a CTA per tile).  Warp 0 TMA (both planes of 64 columns of x and of
 //   w per stage), warp 1 MMA, warps 2-9 add the sums of one stage out of one half of the accumulator columns while the next stage's
@@ -164,33 +164,41 @@ struct Product {
 };
 
 // Results that the terms alone don't settle, in fp32 arithmetic: bit 4 i + j of a lane's `flags` is row m0 + lane / 4 + 8 i, column
-// n0 + 4 (lane % 4) + j.  Four at a time: their loads do not wait for one another.
+// n0 + 4 (lane % 4) + j.  Four of a row at a time: their loads do not wait for one another, and x is read once for them (for each of
+// them, 1500 x 8192 x 1024 with nothing but such results took 11.4 ms).
 __device__ __noinline__ void sum_again(const Product& p, int m0, int n0, uint32_t flags) {
   const int lane = threadIdx.x & 31;
-  for (int bit = 0; bit < 16; ++bit) {
-    uint32_t lanes = __ballot_sync(0xffffffffu, flags >> bit & 1);
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {
+    uint32_t mine = (flags >> (4 * i) & 15u) << (4 * (lane & 3));            // the row's 16 columns, from its four lanes
+    mine |= __shfl_xor_sync(0xffffffffu, mine, 1);
+    mine |= __shfl_xor_sync(0xffffffffu, mine, 2);
+    uint32_t lanes = __ballot_sync(0xffffffffu, mine != 0) & 0x11111111u;
     while (lanes != 0) {
-      int l[4];
-      float acc[4] = {};
-      const float *x[4], *w[4];
+      const int from = __ffs(lanes) - 1, row = m0 + (from >> 2) + 8 * i;
+      lanes &= lanes - 1;
+      uint32_t cols = __shfl_sync(0xffffffffu, mine, from);
+      const float* x = p.x + (int64_t)row * p.x_rs;
+      while (cols != 0) {
+        int c[4];
+        float acc[4] = {};
+        const float* w[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        l[j] = j > 0 && lanes == 0 ? l[0] : __ffs(lanes) - 1;
-        lanes &= lanes - 1;
-        x[j] = p.x + (int64_t)(m0 + (l[j] >> 2) + 8 * (bit >> 2)) * p.x_rs;
-        w[j] = p.w + (int64_t)(n0 + 4 * (l[j] & 3) + (bit & 3)) * p.K;
-      }
+        for (int j = 0; j < 4; ++j) {
+          c[j] = j > 0 && cols == 0 ? c[0] : __ffs(cols) - 1;
+          cols &= cols - 1;
+          w[j] = p.w + (int64_t)(n0 + c[j]) * p.K;
+        }
 #pragma unroll 4
-      for (int k = lane; k < p.K; k += 32) {
+        for (int k = lane; k < p.K; k += 32) {
+          const float a = x[k];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[j] = fmaf(x[j][k], w[j][k], acc[j]);
-      }
+          for (int j = 0; j < 4; ++j) acc[j] = fmaf(a, w[j][k], acc[j]);
+        }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float sum = warp_sum(acc[j]);
-        if (lane == l[j]) {
-          const int n = n0 + 4 * (lane & 3) + (bit & 3);
-          p.out[(int64_t)(m0 + (lane >> 2) + 8 * (bit >> 2)) * p.out_rs + n] = sum + (p.bias ? p.bias[n] : 0.f);
+        for (int j = 0; j < 4; ++j) {
+          const float sum = warp_sum(acc[j]);
+          if (lane == j) p.out[(int64_t)row * p.out_rs + n0 + c[j]] = sum + (p.bias ? p.bias[n0 + c[j]] : 0.f);
         }
       }
     }
@@ -388,7 +396,7 @@ linear_f32_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
 }
 
 // From here on a tile has a CTA to itself.  Tiles in turn have the next products wait while results are summed again, and a wait ends
-// after 1.1 s: a tile of 128 x 256 with nothing else took 2.6 ms at K = 1024, 24 at 8192, 150 at 32704.  What tiles in turn save,
+// after 1.1 s: a tile of 128 x 256 with nothing else took 3.3 ms at K = 1024, 20 at 8192, 160 at 32704.  What tiles in turn save,
 // some 12000 clocks each, is then less than 1.5 % of a tile's 512 stages.
 constexpr int kAloneK = 1 << 15;
 
