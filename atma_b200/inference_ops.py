@@ -475,12 +475,22 @@ def decode_linear(x, weight, bias=None, gated=False, out=None, lib=None, any_k=F
 # against 24, 24, 24; 300 20, 20, 19 against 17, 17, 19; 1500 x 4096 x 1024 25, 25, 24 against 24, 24, 23.  With a short K the activation
 # is most of the work and has eight warps an SM: 20000 x 2048 x 128 41, 47, 38 against 46, 42, 48; at 256 25, 28, 25 against 30, 32, 30
 # (16000 x 1024).  Rows that fill their tiles badly: 600 x 16384 x 2048 48, 49, 48 against 48, 46, 48.
+# The 74 pairs of SMs take tiles in turn, and what the last turn leaves idle has to be made up for by what the activation would take behind
+# the product, 346 / K of its time (six bytes a result for two at the HBM's rate, against 2 K operations).  40 random shapes inside of the
+# lines above, by (share of the turns that is filled) x (1 + 346 / K): 0.81 to 0.83 0.83 to 0.98 of the speed (8399 x 1792 x 5568 179, 181, 178
+# against 161, 155, 157), 0.85 and 0.86 0.99 to 1.08, 0.92 0.95 (14080 x 2432 x 7808 361 against 341), from 0.98 on 1.01 to 1.4, but for two of less
+# than 30 us.
 LINEAR_ACT_MIN_RESULTS, LINEAR_ACT_MIN_K, LINEAR_ACT_TILE = 100 * 65536, 256, 256
+LINEAR_ACT_PAIRS, LINEAR_ACT_SAVES, LINEAR_ACT_FILLED = 74, 346, 0.95
 
 
 def _linear_act_pays(M, N, K):
-    rows = -(-M // LINEAR_ACT_TILE) * LINEAR_ACT_TILE
-    return M * N >= LINEAR_ACT_MIN_RESULTS and K >= LINEAR_ACT_MIN_K and 5 * M >= 4 * rows
+    tiles_m, tiles_n = -(-M // LINEAR_ACT_TILE), -(-N // LINEAR_ACT_TILE)      # of 256 features, whether they are two halves' or not
+    if M * N < LINEAR_ACT_MIN_RESULTS or K < LINEAR_ACT_MIN_K or 5 * M < 4 * tiles_m * LINEAR_ACT_TILE:
+        return False
+    turns = -(-tiles_m * tiles_n // LINEAR_ACT_PAIRS)
+    filled = M * N / (turns * LINEAR_ACT_PAIRS * LINEAR_ACT_TILE ** 2)
+    return filled * (1 + LINEAR_ACT_SAVES / K) >= LINEAR_ACT_FILLED
 
 
 def linear_act_supported(x, weight, gated, bias=None, out=None):

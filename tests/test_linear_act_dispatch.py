@@ -104,3 +104,11 @@ def test_half_precision_of_the_decoders(calls):
     decoder_ops.squared_relu_linear(x, w, b)
     decoder_ops.gelu_gated_linear(x, w, torch.zeros(M, N // 2, dtype=torch.float16))
     assert calls == ["relu", "gate"]
+
+
+@pytest.mark.parametrize("rows,k,n,yes", [(8399, 5568, 1792, False), (14080, 7808, 2432, False), (1635, 7744, 9472, False), (1281, 3200, 5568, False),
+                                          (24320, 5376, 4160, True), (5628, 5120, 3264, True), (6955, 3392, 4480, True), (2816, 256, 3776, True),
+                                          (12000, 1024, 8192, True), (3000, 1024, 8192, True), (4096, 2048, 16384, True)])
+def test_sizes_whose_last_turn_is_nearly_empty(rows, k, n, yes):
+    """Measured on both sides of the line."""
+    assert io._linear_act_pays(rows, n, k) is yes
