@@ -187,7 +187,8 @@ add_rms_norm_kernel(const T* __restrict__ x, const T* __restrict__ y, const T* _
 // The same for rows whose length is a multiple of eight values (16-byte aligned): one CTA per row, eight values
 // per thread, so that a row is one round of loads, a block reduction and one round of stores -
 // the latency of a decode step's 2 x layers launches of this kernel, not its bandwidth, is what counts.  In fp32, 2048 rows of
-// 1024 take 16 us with a warp per row, 6.7 so (25 MB with the add: 3.8 at the HBM's rate).
+// 1024 take 16 us with a warp per row, 6.7 so (25 MB with the add: 3.8 at the HBM's rate).  Many short rows of fp32 are bound by the number
+// of CTAs (65536 rows of 64, 128, 256, 512: 74, 74, 74, 86 us; 18, 29, 49, 109 with a warp per row) and stay with warps.
 template <typename T>
 __global__ void __launch_bounds__(512)
 add_rms_norm_row_kernel(const T* x, const T* y, const T* w, T* x_out, T* h_out, int D, float eps) {
@@ -299,7 +300,8 @@ extern "C" int atma_add_rms_norm(const void* x, const void* y, const void* weigh
   if (rows <= 0) return ATMA_OK;
   cudaStream_t st = (cudaStream_t)stream;
   auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  if (D % 8 == 0 && al16(x) && al16(y) && al16(weight) && al16(x_out) && al16(h_out)) {
+  const bool wide = dtype != ATMA_F32 || D >= 512 || rows <= 2048;
+  if (wide && D % 8 == 0 && al16(x) && al16(y) && al16(weight) && al16(x_out) && al16(h_out)) {
     const int threads = ((D / 8 + 31) / 32) * 32;                // <= 512 for D <= 4096
     ATMA_DISPATCH_DTYPE(dtype, T, {
       launch_early(rows, add_rms_norm_row_kernel<T>, rows, threads, 0, st, (const T*)x, (const T*)y, (const T*)weight, (T*)x_out, (T*)h_out, D, eps);

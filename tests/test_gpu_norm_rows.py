@@ -20,3 +20,9 @@ def test_fp32_rows(rows, D):
     assert (h.double() - want).abs().max() <= 2.0 ** -24 * 16 * want.abs().max()
     lead = torch.randn(rows * D + 1, device="cuda")[1:].view(rows, D)                # rows that are not 16-byte aligned
     assert torch.allclose(add_rms_norm(lead, None, w, 1e-6)[1], add_rms_norm(lead.clone(), None, w, 1e-6)[1], rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("rows,D", [(2048, 504), (2049, 504), (2049, 512), (3000, 8)])
+def test_many_fp32_rows(rows, D):
+    """From 2049 rows on a row of fewer than 512 values has a warp."""
+    test_fp32_rows(rows, D)
