@@ -75,7 +75,7 @@ __host__ __device__ constexpr uint32_t idesc_tf32(int N) { return (1u << 4) | (2
 __device__ __forceinline__ uint64_t desc(uint32_t addr) { return make_sdesc_sw128(addr, 16, 1024); }
 
 // The CTA's first row.  Later rows have more keys, so they come first, but for the very first, which go row by row of keys (few_keys) and
-// take as long as four to six steps.
+// take as long as a dozen steps.
 template <int M>
 __device__ __forceinline__ int first_row(int heads) {
   const int tiles = gridDim.x / heads, at = blockIdx.x / heads;
