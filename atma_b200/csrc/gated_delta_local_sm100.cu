@@ -19,7 +19,7 @@
 // Tw and Tu with the K and V rows as they are.
 // What bounds it is the serial chain of a tile's thread phases (Gram rows, substitution, four levels of
 // blocks), so two CTAs share an SM: T takes the place of the K and Q tiles, which are dead once the Gram
-// matrices are there (98 KB).  8 sequences of 16384 tokens, 8 heads: 327 us (0.75 GB
+// matrices are there (98 KB).  8 sequences of 16384 tokens, 8 heads: 330 us (0.75 GB
 // moved); one CTA per SM that also made W and U0 and wrote 72 KB a chunk took 617 us.
 //
 //   warp 0      TMA producer        warp 1      MMA issuer; owns the TMEM allocation

@@ -19,14 +19,16 @@
 // accumulators.  fp16 has no room for an unbounded 1 / |k|, neither in Tw nor in U, so in chunks with very short or long
 // rows a warp brings the K rows in shared memory to a length between 1 and 2 by a power of two, which loses nothing, ahead of
 // the first product that reads them, and k_inv stands for what is left, a factor between 1/2 and 1.  The rows arrive shortly before
-// that product, so this costs such a chunk 2000 clocks.  Behind the last rows of a sequence a
-// chunk holds another's, whose factors are zero; they may be infinite or no numbers, so the same warp clears them.  The A operands of the chain (16-bit copies of S^T and U^T) are read from TMEM.  All
-// accumulators have a channel on the 128 TMEM lanes, which spreads the thread phases over all four schedulers.
+// that product, so this costs such a chunk 2000 clocks.  Behind the last rows of a sequence a chunk holds another's, whose
+// factors are zero; they may be infinite or no numbers, so the same warp clears them.  The A operands of the chain (16-bit
+// copies of S^T and U^T) are read from TMEM.  All accumulators have a channel on the 128 TMEM lanes, which spreads the thread
+// phases over all four schedulers.
 //
-// What bounds it is the latency of the chain, of which the two thread phases are half: 3000 clocks a chunk, 650 for S and 750
-// for U between a product's end and its successor's first operand, the products 330 and 600.  Measured with the chunk-local
-// stage, which no longer writes W, U0, Qg and Kt: 8 sequences of 16384 tokens, 8 heads, 327 + 414 us (617 + 385 with those
-// in 72 KB records), one of 65536 732 -> 606 us, 8 of 300 45 -> 39 us.
+// What bounds it is the latency of the chain: 3000 to 3300 clocks a chunk, 1000 for the state's phase and its hand-over, 420 for U's
+// products, 850 for U's phase, up to 600 of waiting for the next -W to leave dS^T's columns, 450 to 640 for dS's products; 2750
+// without outputs, where -W has columns of its own.  Measured with the chunk-local stage, which no longer writes W, U0, Qg and
+// Kt: 8 sequences of 16384 tokens, 8 heads, 330 + 412 us (617 + 385 with those in 72 KB records; fp16 995 -> 753 in all), 8 of 300
+// 44 -> 36 us.  Context-parallel walks, 2 x 16384: state only 333 -> 349 us, with outputs 382 -> 412, factors 164 -> 93.
 //
 //   warp 0       TMA producer: V, Tw, Tu and K three chunks ahead, Q and Rq two
 //   warp 1       issues the chain's products and -W^T; owns the TMEM allocation
@@ -38,7 +40,7 @@
 //   warps 12-15  W warps, warps 16-19 O warps: TMEM lanes 32 (w % 4) .. +31
 // TMEM (512 columns allocated): 16-bit S^T [0,64) and, every other chunk, [64,128) | 16-bit U^T [128,160), scaled
 // [160,192) | U^T fp32 [192,256) | O1^T [256,320) | O2^T [320,384) | dS^T [384,512), where -W^T of the next chunk passes
-// through between the state's reading and the next dS^T.
+// through between the state's reading and the next dS^T; without outputs in O1^T's place.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status
 // word for the host.
 #include "common.cuh"
@@ -128,7 +130,7 @@ scan_recur_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   const int n_chunks = max(c_end - c_begin, 0);
   const int last_rows = (int)(tok_end - tok_base - (int64_t)(n_chunks - 1) * kC);    // of the last chunk
   const bool want_o = p.o != nullptr && (packed || p.map.o_row[b] >= 0);   // a negative row: this recurrence only carries state
-  const uint32_t col_w = want_o ? kColS : kColO1;                    // see TMEM above
+  const uint32_t col_w = want_o ? kColS : kColO1;                    // without outputs the chain need not wait for its reading
   auto partial = [&](int c) { return c == n_chunks - 1 && last_rows < kC; };
   auto prepared = [&](int c) { return !kBf16 || partial(c); };       // chunks whose K rows warp 3 works on first
   const int64_t rec0 = ((int64_t)rb * p.H + h) * p.NC + c_begin;     // first record of this recurrence
