@@ -9,7 +9,8 @@
 //
 //   warp 0      TMA producer: Q tiles once, then K and V tiles through 2-stage rings
 //   warp 1      MMA issuer (one lane): S_t = Q_t K_j^T (SS), O_t += P_t V_j (P read from TMEM)
-//   warps 2-3   idle (they complete the first warpgroup, whose registers are handed over)
+//   warp 2      packed: zeros behind the sequence's end in its last V tile
+//   warp 3      idle (it completes the first warpgroup, whose registers are handed over)
 //   warps 4-7   softmax + epilogue of tile 0, one thread per query row (= one TMEM lane)
 //   warps 8-11  softmax + epilogue of tile 1
 // The first warpgroup shrinks to 88 registers per thread (setmaxnreg) so that each softmax
@@ -64,7 +65,7 @@ __device__ int g_sm100_status = 0;
 struct Barriers {
   uint64_t q_full[2];
   uint64_t k_full[kStages], k_empty[kStages], v_full[kStages], v_empty[kStages];
-  uint64_t s_full[2], p_full[2], o_final[2];
+  uint64_t s_full[2], p_full[2], o_final[2], v_sent, v_clean;
 };
 
 __device__ __forceinline__ void tma_tile(void* dst, const CUtensorMap* m, uint64_t* bar, const int (&pos)[3],
@@ -154,6 +155,7 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       mbar_init(&bar.k_full[i], 1); mbar_init(&bar.k_empty[i], 1);
       mbar_init(&bar.v_full[i], 1); mbar_init(&bar.v_empty[i], 1);
     }
+    mbar_init(&bar.v_sent, 1); mbar_init(&bar.v_clean, 1);
     s_abort = 0;
     fence_barrier_init();
   }
@@ -208,6 +210,8 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
     jmin = a0 ? (a1 ? min(lo[0], lo[1]) : lo[0]) : (a1 ? lo[1] : 0);
     jmax = a0 ? (a1 ? max(hi[0], hi[1]) : hi[0]) : (a1 ? hi[1] : 0);
   }
+  // packed: keys of the last tile, if the sequence ends inside of it (elsewhere the tensor does, and the tile has zeros there)
+  const int last_keys = packed && jmax > jmin ? k_limit - (jmax - 1) * kBN : kBN;
   // all per-tile scalars are selected with ternaries so that they stay in registers
   auto active = [&](int t, int j) { return t ? (j >= lo[1] && j < hi[1]) : (j >= lo[0] && j < hi[0]); };
   volatile int* abort_flag = &s_abort;
@@ -235,6 +239,7 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
         if (!mbar_wait(&bar.v_empty[s], ph ^ 1u, abort_flag)) break;
         mbar_arrive_expect_tx(&bar.v_full[s], kTileBytes);
         tma_tile(sV + s * kTileBytes, &tmap_v, &bar.v_full[s], p.vpos, seq_row0 + j * kBN, kvh, b);
+        if (j == jmax - 1) mbar_arrive(&bar.v_sent);
       }
     }
     __syncwarp();
@@ -289,7 +294,10 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
           for (int t = 0; t < 2; ++t) {
             if (ok && active(t, j)) {
               ok = mbar_wait(&bar.p_full[t], (uint32_t)(j - lo[t]) & 1u, abort_flag);
-              if (ok && !v_ready) { ok = mbar_wait(&bar.v_full[s], ph, abort_flag); v_ready = true; }
+              if (ok && !v_ready) {
+                ok = mbar_wait(&bar.v_full[s], ph, abort_flag) && (j + 1 < jmax || last_keys >= kBN || mbar_wait(&bar.v_clean, 0, abort_flag));
+                v_ready = true;
+              }
               if (ok) {
                 tc_fence_after();
                 issue_pv(t, s, carry_in || j > lo[t]);
@@ -315,6 +323,18 @@ polar_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const __g
       }
     }
     __syncwarp();
+  } else if (warp == 2 && last_keys < kBN && mbar_wait_warp(&bar.v_sent, 0, abort_flag)) {
+    // V rows behind a packed sequence's end in its last key tile are the next one's: zeros (a weight of zero times a NaN is one)
+    const int it = jmax - 1 - jmin, s = it % kStages;
+    if (mbar_wait_warp(&bar.v_full[s], (uint32_t)(it / kStages) & 1u, abort_flag)) {
+      for (int at = 8 * last_keys + lane; at < 8 * kBN; at += 32) {                       // 16-byte pieces of rows of 128 bytes, two boxes
+        *reinterpret_cast<uint4*>(sV + s * kTileBytes + 16 * at) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(sV + s * kTileBytes + kTileBytes / 2 + 16 * at) = make_uint4(0u, 0u, 0u, 0u);
+      }
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar.v_clean);
+    }
   }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");

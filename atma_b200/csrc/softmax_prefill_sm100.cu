@@ -11,7 +11,8 @@
 //   warp 0      TMA producer: the Q tiles once, K and V tiles (stream 0, stream 1, stream 0, ... or shared) through rings,
 //               with one map the output gate's tiles at the end
 //   warp 1      MMA issuer
-//   warps 2-3   idle (they complete the first warpgroup, whose registers are handed over)
+//   warp 2      V rows behind the sequence's end in its last key tile: zeros, whatever the page holds there (a weight of zero times a NaN is one)
+//   warp 3      idle (it completes the first warpgroup, whose registers are handed over)
 //   warps 4-7   softmax of stream 0, one thread per query row (= one TMEM lane), and its epilogue (two maps: half of the
 //               epilogue's channels)
 //   warps 8-11  softmax of stream 1; its epilogue or the other half
@@ -55,7 +56,7 @@ template <int KS>
 struct Barriers {
   uint64_t q_full[2];
   uint64_t k_full[KS], k_empty[KS], v_full[kVStages], v_empty[kVStages];
-  uint64_t s_full[2], p_full[2], o_final[2], g_full[2];
+  uint64_t s_full[2], p_full[2], o_final[2], g_full[2], v_sent, v_clean[2];
 };
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -106,12 +107,15 @@ softmax_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
   const int r_begin = a.cu_rows[seq], n_rows = a.cu_rows[seq + 1] - r_begin, start = a.start_pos[seq];
   const KeyTiles tiles(start + row0, start + min(row0 + kBM, n_rows) - 1, a.max_blocks * a.block_size, a.window, a.keep_first, kBN);
   const int n_kt = start < 0 || row0 >= n_rows ? 0 : tiles.n;
+  // keys of the last tile, if the sequence ends inside of it
+  const int last_keys = n_kt == 0 ? kBN : min(start + n_rows, a.max_blocks * a.block_size) - (WIN ? tiles[n_kt - 1] : n_kt - 1) * kBN;
 
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bar.q_full[i], 1); mbar_init(&bar.s_full[i], 1);
-      mbar_init(&bar.p_full[i], 4); mbar_init(&bar.o_final[i], 1); mbar_init(&bar.g_full[i], 1);
+      mbar_init(&bar.p_full[i], 4); mbar_init(&bar.o_final[i], 1); mbar_init(&bar.g_full[i], 1); mbar_init(&bar.v_clean[i], 1);
     }
+    mbar_init(&bar.v_sent, 1);
     for (int i = 0; i < KS; ++i) { mbar_init(&bar.k_full[i], 1); mbar_init(&bar.k_empty[i], 1); }
     for (int i = 0; i < kVStages; ++i) { mbar_init(&bar.v_full[i], 1); mbar_init(&bar.v_empty[i], 1); }
     s_abort = 0;
@@ -166,6 +170,7 @@ softmax_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
               tma_load_4d(sV + s * kVTile + cb * kBox, &tmap_v, &bar.v_full[s], (m == 0 ? g0 : g1) * VD + cb * 64, row, 0, 0);
           }
         }
+        if (ok) mbar_arrive(&bar.v_sent);
         if (MAPS == 1 && a.gate != nullptr) {
           const int i = nk * n_kt - 1;                            // once the last K tile is given back nobody reads Q any more
           ok = ok && (!C::kGateOverQ || mbar_wait(&bar.k_empty[i % KS], (uint32_t)(i / KS) & 1u, abort_flag));
@@ -223,7 +228,8 @@ softmax_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
           for (int m = 0; m < 2; ++m) {
             if (!ok || m >= n_streams) break;
             const int i = nv == 2 ? 2 * j + m : j, vs = i % kVStages;
-            ok = mbar_wait(&bar.p_full[m], (uint32_t)j & 1u, abort_flag) && mbar_wait(&bar.v_full[vs], (uint32_t)(i / kVStages) & 1u, abort_flag);
+            ok = mbar_wait(&bar.p_full[m], (uint32_t)j & 1u, abort_flag) && mbar_wait(&bar.v_full[vs], (uint32_t)(i / kVStages) & 1u, abort_flag) &&
+                 (more || last_keys >= kBN || mbar_wait(&bar.v_clean[nv == 2 ? m : 0], 0, abort_flag));
             if (!ok) break;
             tc_fence_after();
             issue_pv(m, vs, j > 0);
@@ -234,6 +240,18 @@ softmax_prefill_sm100_kernel(const __grid_constant__ CUtensorMap tmap_q, const _
         }
       }
       __syncwarp();
+    } else if (warp == 2 && last_keys < kBN && mbar_wait_warp(&bar.v_sent, 0, abort_flag)) {      // from here on v_full means the last tiles
+      for (int m = 0; m < nv; ++m) {
+        const int i = nv * (n_kt - 1) + m, s = i % kVStages;
+        if (!mbar_wait_warp(&bar.v_full[s], (uint32_t)(i / kVStages) & 1u, abort_flag)) break;
+#pragma unroll
+        for (int cb = 0; cb < VD / 64; ++cb)
+          for (int at = 8 * last_keys + lane; at < 8 * kBN; at += 32)                     // 16-byte pieces of rows of 128 bytes
+            *reinterpret_cast<uint4*>(sV + s * kVTile + cb * kBox + 16 * at) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.v_clean[m]);
+      }
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 208;");
