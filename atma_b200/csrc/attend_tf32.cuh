@@ -26,7 +26,7 @@
 // TMEM (512 columns): Q hi [0,128) lo [128,256) | two sums of scores [256,384), then the weights hi and lo in their place |
 // the step's result [384,512), with one map the other two sums before.  With one map pairs of sums take the places in turn, the next
 // pair's products under the reading of the one in front, for next to nothing; sum by sum it was 1500 clocks a step.
-// A step of 64 keys takes 8000 clocks: three products at half the 16-bit rate, 1536 for the scores and 1536 for the result, with
+// A step of 64 keys takes 7800 clocks: three products at half the 16-bit rate, 1536 for the scores and 1536 for the result, with
 // their waits 4000; 1400 for the weights; what is left are scores, sums and hand-overs.  TMEM is full, so the next scores wait
 // for this step's result.
 // Every mbarrier wait is bounded; on expiry the CTA frees its TMEM, returns and leaves a status word for the host.
@@ -312,14 +312,14 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kMmaRegs));
     if (warp == 12 && elect_one()) {
-      const uint32_t ka = smem_u32(smem + kOffK), va = smem_u32(smem + kOffV);
+      const uint64_t k_desc = desc(smem_u32(smem + kOffK)), v_desc = desc(smem_u32(smem + kOffV));
       bool ok = n_tiles == 0 || mbar_wait(&sh.q_ready, 0, abort_flag);
       uint32_t it = 0;
       for (int j = 0; j < n_tiles && ok; ++j) {
         ok = mbar_wait(&sh.k_full, (uint32_t)j & 1u, abort_flag);
         for (int t = 0; t < M && ok; ++t, ++it) {
           tc_fence_after();
-          for (int g = 0; g < kPairs && ok; ++g) {    // rolled, terms as well: their descriptors at once would not fit this warp's registers
+          for (int g = 0; g < kPairs && ok; ++g) {    // rolled: all descriptors at once would not fit this warp's registers
             // the second place is the result's: the one in front has been read
             if (g == 1 && it > 0) ok = mbar_wait(&sh.o_free, (it - 1) & 1u, abort_flag);
             if (g > 1) ok = mbar_wait(&sh.s_free[g & 1], it & 1u, abort_flag);
@@ -327,14 +327,15 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
             tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < 2; ++c) {
+              // few instructions between products: 32 clocks each, and with descriptors made for every one the issue took twice that
               const int step = ((t * kPairs + g) * 2 + c) * (kSum / 8);
-#pragma unroll 1
-              for (int term = 0; term < 3; ++term) {
+              const uint32_t d = tbase + kColS + 128 * (g & 1) + 64 * c, qa = tbase + kColQ + 8 * step;
+              const uint64_t kd = k_desc + uint64_t(((step >> 2) * (kN * 128) + (step & 3) * 32) >> 4);
 #pragma unroll
-                for (int k = step; k < step + kSum / 8; ++k)
-                  mma_ts_tf32(tbase + kColS + 128 * (g & 1) + 64 * c, tbase + kColQ + (term == 0 ? 128 : 0) + 8 * k,
-                              desc(ka + (term == 1 ? kTerm : 0) + (k >> 2) * (kN * 128) + (k & 3) * 32), idesc_tf32(kN), (term > 0 || k > step) ? 1u : 0u);
-              }
+              for (int term = 0; term < 3; ++term)
+#pragma unroll
+                for (int k = 0; k < kSum / 8; ++k)
+                  mma_ts_tf32(d, qa + (term == 0 ? 128 : 0) + 8 * k, kd + uint64_t(((term == 1 ? kTerm : 0) + 32 * k) >> 4), idesc_tf32(kN), (term > 0 || k > 0) ? 1u : 0u);
             }
             tc_commit(&sh.s_full[g & 1]);
           }
@@ -347,7 +348,7 @@ __device__ __forceinline__ void attend(Front& f, uint8_t* smem, Shared& sh, int*
 #pragma unroll 1
           for (int term = 0; term < 3; ++term) {
             const uint32_t pa = tbase + kColP + (term == 0 ? 64 : 0);
-            const uint64_t vd = desc(va + (term == 1 ? kTerm : 0));
+            const uint64_t vd = v_desc + uint64_t((term == 1 ? kTerm : 0) >> 4);
 #pragma unroll
             for (int k = 0; k < 8; ++k)
               mma_ts_tf32(tbase + kColO, pa + 8 * k, vd + uint64_t(((k >> 2) * (kD * 128) + (k & 3) * 32) >> 4), idesc_tf32(kD), (term > 0 || k > 0) ? 1u : 0u);

@@ -331,7 +331,7 @@ polar_tf32_kernel(const __grid_constant__ atma_polar_prefill_args a) {
 }
 
 // Head size 128, no statistics carried in or out (a marked block is done again from the inputs alone), and enough rows: 2048
-// rows, 8 heads, the call's own launches counted, 432 us on the 64 x 64 kernel, 146 here; 512 rows 100 and 58; 300 rows 66 and 58; 256 rows 55 and
+// rows, 8 heads, the call's own launches counted, 432 us on the 64 x 64 kernel, 136 here; 512 rows 100 and 60; 300 rows 66 and 60; 256 rows 55 and
 // 58 (with two CTAs a head one is for fp32 arithmetic).
 // Results that take the place of q: the mark would be in the rows that are read again.  Windows of fewer than few_keys keys: every block
 // would be left to the 64 x 64 kernel.

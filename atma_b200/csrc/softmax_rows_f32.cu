@@ -292,7 +292,7 @@ softmax_tf32_kernel(const __grid_constant__ atma_softmax_args a) {
 }
 
 // 128 channels in one map or two, 128 of v, and enough rows.  Two maps, 8 heads, the call's own launches counted: 1500 rows 547 us on
-// the 64 x 64 kernel, 175 here; 400 rows 156 and 83; 256 rows 104 and 75.  One map: 363 and 132, 106 and 79, 72 and 77.  Results that take the place of q or the gate: the mark would be in
+// the 64 x 64 kernel, 173 here; 400 rows 156 and 83; 256 rows 104 and 73.  One map: 363 and 130, 106 and 80, 72 and 77.  Results that take the place of q or the gate: the mark would be in
 // the rows that are read again.  Short windows: with one map every block would be left to the 64 x 64 kernel (few_keys); with two that is
 // faster while its CTAs have an SM each (a window of 8, 400 rows 59 us against 69, 1500 rows 76 against 73; of 64, 66 and 69, 86 and 71).
 bool softmax_tf32_supported(const atma_softmax_args& a) {
